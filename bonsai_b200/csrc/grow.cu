@@ -33,16 +33,15 @@ namespace
 
 constexpr uint32_t k_threads    = 256;
 constexpr uint32_t k_part_rows  = 4096; // rows per partition chunk
-constexpr uint32_t k_build_rows = 4096; // rows per histogram-build chunk (exact)
+constexpr uint32_t k_build_rows = 2048; // rows per histogram-build chunk (exact)
 constexpr uint32_t k_qbuild_rows = 2048;  // rows per histogram-build chunk (quantised)
 constexpr uint32_t k_qctas = 148;        // persistent quantised-histogram CTAs per tile (one per SM)
 constexpr uint32_t k_qthreads    = 512;   // threads per quantised-histogram CTA
 constexpr uint32_t k_tthreads    = 1024;  // threads per conflict-free (u8) histogram CTA
-constexpr uint32_t k_warps_feat = 8;    // features per count/scatter CTA
 constexpr uint32_t k_find_thr   = 128;  // threads per (node, feature) find CTA
-constexpr uint32_t k_chain_stg  = 32;   // elements per lane per cp.async stage
-constexpr uint32_t k_chain_nst  = 4;    // cp.async stages per lane
 constexpr uint32_t k_max_bins   = 4096; // per feature, this engine's ceiling
+constexpr uint32_t k_exact_bins = 3679; // and the exact form's
+constexpr uint32_t k_no_sel_tile = 0xFFFFFFFFu; // an unused slot of a selection's tile table
 constexpr uint32_t k_plan_thr   = 512;  // plan kernels: one thread per node
 
 // The walked tree's decision heap (depthwise trees, depth <= 8): slot h's
@@ -312,200 +311,340 @@ __global__ void root_totals_kernel(Node *nodes, float2 const *hist, uint32_t con
 }
 
 // ------------------------------------------------------- histogram build ----
-// The plain form's cells must equal the CPU fill's serial float chains, so
-// each built node's rows are stably counting-sorted by bin per feature
-// (count -> offsets -> scatter), after which every cell's (g, h) values sit
-// contiguous in the node's row order and one lane folds each cell.
+// The plain form's cells must equal the CPU fill's serial float chains: each
+// cell's (g, h) values added one by one in the node's row order. Two kernels:
+//
+// sort_kernel: a CTA takes one 2,048-row chunk of a built node and one mirror
+// tile, brings each row's 32-byte tile and gradient pair into shared memory
+// once, and counting-sorts the rows by bin, stably, feature after feature
+// (four features at a time, a group of four warps each). A node of one chunk
+// is finished here, a thread per bin adding its run; the others' sorted pairs
+// go to memory, coalesced, with the chunk's bin offsets.
+//
+// chain_kernel: a warp takes 32 bins of a (node, feature), a lane per bin, and
+// streams that range of the node's chunks in order through a shared-memory
+// ring, each lane adding its runs.
+//
+// A bin's run is an even number of pairs, an odd one ending with a pair of
+// +0.0: two pairs are then one aligned 16-byte read. Adding +0.0 changes
+// nothing -- a sum that starts at +0.0 is never -0.0 under round-to-nearest.
+//
+// A chunk is sorted on its own: no counting pass over the node comes first,
+// rows and tiles are read once for all of a tile's features, and the payload
+// is written and read in whole lines. The former form -- a counting pass, a
+// per-node offset pass, a scatter of single pairs to 256 open places per
+// feature and a chain reading one line per lane -- took 32.7 ms per tree of
+// the 10M x 28 depth-8 logloss fit; these two take 11.5 (sort 6.6, bound by
+// the integer pipe's ballots; chain 4.9, by the largest nodes' serial chains).
 
-template <typename BinT>
-__global__ void __launch_bounds__(k_threads)
-    count_kernel(Ctl const *ctl, Chunk const *bchunks, uint32_t const *rows,
-                 void const *bins, uint64_t n_pad, uint32_t const *sel,
-                 uint32_t const *sel_nb, uint32_t nfb, uint32_t *ccount, uint32_t cs)
+constexpr uint32_t k_xgthr   = 128; // a group: one feature at a time
+constexpr uint32_t k_xgwarps = k_xgthr / 32;
+constexpr uint32_t k_xsteps  = k_build_rows / k_xgthr; // rows per lane and feature
+constexpr uint32_t k_xgroups = 4;  // groups per CTA, where their tables fit
+static_assert(2 * k_build_rows <= 0x1000, "a place in a padded chunk takes 12 bits");
+
+// A group's barrier (barrier 0 is the CTA's).
+__device__ __forceinline__ void group_sync(uint32_t group)
 {
-    pdl_enter();
-    extern __shared__ uint32_t cnt_s[]; // [k_warps_feat][cs]
-    uint32_t const             c = blockIdx.x;
-    if (c >= ctl->n_bchunks)
-    {
-        return;
-    }
-    Chunk const    ch   = bchunks[c];
-    uint32_t const lane = threadIdx.x & 31;
-    uint32_t const w    = threadIdx.x >> 5;
-    uint32_t const j    = (blockIdx.y * k_warps_feat) + w;
-    if (j >= nfb)
-    {
-        return;
-    }
-    uint32_t const f   = sel[j];
-    uint32_t const nb  = sel_nb[j];
-    uint32_t      *cnt = cnt_s + (w * cs);
-    for (uint32_t b = lane; b < nb; b += 32)
-    {
-        cnt[b] = 0;
-    }
-    __syncwarp();
-    for (uint32_t k = lane; k < ch.count; k += 32)
-    {
-        uint32_t const r = rows[ch.begin + k];
-        atomicAdd(&cnt[bin_at<BinT>(bins, n_pad, f, r)], 1U);
-    }
-    __syncwarp();
-    uint32_t *out = ccount + ((static_cast<uint64_t>(c) * nfb + j) * cs);
-    for (uint32_t b = lane; b < nb; b += 32)
-    {
-        out[b] = cnt[b];
-    }
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(k_xgthr) : "memory");
 }
 
-// Per (built node, feature): bin totals over the node's chunks, their
-// exclusive scan (the bin segments of the node's sorted payload), and each
-// chunk's per-bin write base, in place of its counts.
-__global__ void __launch_bounds__(k_threads)
-    offsets_kernel(Ctl const *ctl, uint32_t const *brange, uint32_t *ccount,
-                   uint32_t *seg, uint32_t const *sel_nb, uint32_t nfb, uint32_t cs,
-                   Chunk const *bchunks)
+// Adds a pair to a pair: two IEEE float adds in one instruction.
+__device__ __forceinline__ void add_pair(float2 &a, float2 const b)
 {
-    pdl_enter();
-    __shared__ uint32_t tot_s[k_max_bins];
-    __shared__ uint32_t carry_s;
-    uint32_t const      i = blockIdx.x;
-    if (i >= ctl->n_build)
-    {
-        return;
-    }
-    uint32_t const j  = blockIdx.y;
-    uint32_t const nb = sel_nb[j];
-    uint32_t const c0 = brange[i];
-    uint32_t const c1 = brange[i + 1];
-    for (uint32_t b = threadIdx.x; b < nb; b += k_threads)
-    {
-        uint32_t s = 0;
-        for (uint32_t c = c0; c < c1; ++c)
-        {
-            s += ccount[((static_cast<uint64_t>(c) * nfb + j) * cs) + b];
-        }
-        tot_s[b] = s;
-    }
-    if (threadIdx.x == 0)
-    {
-        carry_s = 0;
-    }
-    __syncthreads();
-    // exclusive scan over bins, 256 at a time
-    for (uint32_t b0 = 0; b0 < nb; b0 += k_threads)
-    {
-        uint32_t const b     = b0 + threadIdx.x;
-        uint32_t const v     = b < nb ? tot_s[b] : 0;
-        uint32_t       total = 0;
-        uint32_t const ex    = block_excl_scan<k_threads>(v, &total);
-        uint32_t const carry = carry_s;
-        if (b < nb)
-        {
-            tot_s[b] = carry + ex;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            carry_s = carry + total;
-        }
-        __syncthreads();
-    }
-    uint32_t *sg = seg + ((static_cast<uint64_t>(i) * nfb + j) * cs);
-    for (uint32_t b = threadIdx.x; b < nb; b += k_threads)
-    {
-        uint32_t run = tot_s[b];
-        sg[b]        = run;
-        for (uint32_t c = c0; c < c1; ++c)
-        {
-            uint32_t *p = ccount + ((static_cast<uint64_t>(c) * nfb + j) * cs) + b;
-            uint32_t  v = *p;
-            *p          = run;
-            run += v;
-        }
-    }
-    if (threadIdx.x == 0)
-    {
-        sg[nb] = carry_s;
-    }
-    (void)bchunks;
+    auto      &x = reinterpret_cast<unsigned long long &>(a);
+    auto const y = reinterpret_cast<unsigned long long const &>(b);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(y));
 }
 
-template <typename BinT>
-__global__ void __launch_bounds__(k_threads)
-    scatter_kernel(Ctl const *ctl, Chunk const *bchunks, uint32_t const *rows,
-                   void const *bins, uint64_t n_pad, float2 const *gh,
-                   uint32_t const *sel, uint32_t const *sel_nb, uint32_t nfb,
-                   uint32_t const *ccount, uint32_t cs, float2 *payload,
-                   uint64_t p_stride)
+// 16-bit words of a chunk's offset row: its bins in whole warps of 32, the
+// end after the last one, and room to keep rows 16-byte aligned.
+__host__ __device__ inline uint32_t offset_stride(uint32_t max_nb)
 {
-    pdl_enter();
-    extern __shared__ unsigned char smem_raw[];
-    uint32_t const c = blockIdx.x;
-    if (c >= ctl->n_bchunks)
+    return (((max_nb + 31) / 32) * 32) + 8;
+}
+
+// Pairs that padding may add to a chunk (even).
+__host__ __device__ inline uint32_t chunk_pads(uint32_t max_nb)
+{
+    return (min(max_nb, k_build_rows) + 1) & ~1u;
+}
+
+// Where chunk c (the x-th of its node, whose rows begin at base among the
+// built rows) has its sorted pairs: its rows' place, rounded down to a whole
+// 16 bytes, after every earlier chunk's padding.
+__device__ __forceinline__ uint64_t chunk_at(uint32_t base, uint32_t x, uint32_t c,
+                                             uint32_t max_nb)
+{
+    return ((uint64_t{base} + (uint64_t{x} * k_build_rows)) & ~uint64_t{1}) +
+           (uint64_t{c} * (chunk_pads(max_nb) + 2));
+}
+
+// Bytes of sort_kernel's dynamic shared memory.
+inline size_t sort_smem(uint32_t max_nb, uint32_t groups)
+{
+    size_t const row = ((max_nb + 1) / 2) * 4; // one warp's counters, 16 bits a bin
+    return (size_t{k_build_rows} * (k_mirror_bytes + sizeof(float2))) + 16 +
+           (groups * ((size_t{k_build_rows + chunk_pads(max_nb)} * 2) + (k_xgwarps * row)));
+}
+
+// Ranks a warp's rows within their bins, in row order: key[st] is the code of
+// the lane's row of step st (0xFFFF: none) and leaves with its rank -- the
+// rows before it in its bin, in this warp's run -- in its high half; cnt16
+// leaves holding each bin's rows. The lanes of one bin are found from a
+// ballot per bit of the code: the match instruction takes about 59 cycles of
+// an SM a warp here (root sort of 10M rows 2,509 us with it, 1,384 with the
+// ballots, which the integer pipe bounds).
+template <uint32_t BITS>
+__device__ __forceinline__ void rank_rows(uint32_t (&key)[k_xsteps], uint16_t *cnt16)
+{
+#pragma unroll
+    for (uint32_t st = 0; st < k_xsteps; ++st)
     {
-        return;
-    }
-    Chunk const ch     = bchunks[c];
-    auto       *rows_s = reinterpret_cast<uint32_t *>(smem_raw);
-    auto       *gh_s   = reinterpret_cast<float2 *>(rows_s + k_build_rows);
-    auto       *base_s = reinterpret_cast<uint32_t *>(gh_s + k_build_rows);
-    auto       *bins_s = reinterpret_cast<BinT *>(base_s + (k_warps_feat * cs));
-    for (uint32_t k = threadIdx.x; k < ch.count; k += k_threads)
-    {
-        uint32_t const r = rows[ch.begin + k];
-        rows_s[k]        = r;
-        gh_s[k]          = gh[r];
-    }
-    __syncthreads();
-    uint32_t const lane = threadIdx.x & 31;
-    uint32_t const w    = threadIdx.x >> 5;
-    uint32_t const j    = (blockIdx.y * k_warps_feat) + w;
-    if (j >= nfb)
-    {
-        return;
-    }
-    uint32_t const  f    = sel[j];
-    uint32_t const  nb   = sel_nb[j];
-    uint32_t       *base = base_s + (w * cs);
-    BinT           *bw   = bins_s + (w * k_build_rows);
-    uint32_t const *off  = ccount + ((static_cast<uint64_t>(c) * nfb + j) * cs);
-    for (uint32_t b = lane; b < nb; b += 32)
-    {
-        base[b] = off[b];
-    }
-    for (uint32_t k = lane; k < ch.count; k += 32)
-    {
-        bw[k] = static_cast<BinT>(bin_at<BinT>(bins, n_pad, f, rows_s[k]));
-    }
-    __syncwarp();
-    float2 *out = payload + (static_cast<uint64_t>(j) * p_stride) + ch.aux;
-    for (uint32_t k0 = 0; k0 < ch.count; k0 += 32)
-    {
-        uint32_t const k     = k0 + lane;
-        bool const     valid = k < ch.count;
-        uint32_t const b     = valid ? static_cast<uint32_t>(bw[k]) : 0xFFFFFFFFu;
-        uint32_t const peers = __match_any_sync(0xFFFFFFFFu, b);
-        uint32_t       pos   = 0;
+        uint32_t const b     = key[st];
+        bool const     valid = b != 0xFFFFu;
+        uint32_t       peers = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+        for (uint32_t i = 0; i < BITS; ++i)
+        {
+            uint32_t const bit = (b >> i) & 1u;
+            peers &= __ballot_sync(0xFFFFFFFFu, bit != 0) ^ (bit - 1u);
+        }
+        uint32_t const lt  = __popc(peers & lanemask_lt());
+        uint32_t       old = 0;
         if (valid)
         {
-            pos      = base[b] + __popc(peers & lanemask_lt());
-            out[pos] = gh_s[k];
+            old = cnt16[b];
         }
         __syncwarp();
-        if (valid && (peers & lanemask_lt()) == 0)
+        if (valid && lt == 0)
         {
-            base[b] += __popc(peers);
+            cnt16[b] = static_cast<uint16_t>(old + __popc(peers));
         }
         __syncwarp();
+        key[st] = b | ((old + lt) << 16);
     }
 }
 
-__device__ __forceinline__ void cp_async8(void *smem_dst, void const *gsrc)
+// grid (chunks, tiles)
+template <typename BinT, uint32_t GROUPS>
+__global__ void __launch_bounds__(GROUPS *k_xgthr, GROUPS == k_xgroups && sizeof(BinT) == 1 ? 2 : 1)
+    sort_kernel(Ctl const *ctl, Chunk const *bchunks, uint32_t const *brange,
+                uint32_t const *build, uint32_t const *__restrict__ rows,
+                uint4 const *__restrict__ mirror, uint64_t n_rows,
+                float2 const *__restrict__ gh, uint32_t const *tile_ids, int32_t const *tile_j,
+                uint32_t const *sel_nb, uint32_t const *cell_off, uint32_t max_nb, uint32_t nfb,
+                uint16_t *__restrict__ coff, uint32_t cs, float2 *__restrict__ payload,
+                uint64_t p_stride, float2 *hist, uint32_t total_cells)
+{
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr uint32_t per = k_mirror_bytes / sizeof(BinT);
+    uint32_t const     c   = blockIdx.x;
+    if (c >= ctl->n_bchunks)
+    {
+        return;
+    }
+    uint32_t const tile = tile_ids[blockIdx.y];
+    if (tile == k_no_sel_tile)
+    {
+        return;
+    }
+    uint32_t const crow   = (max_nb + 1) / 2; // counter words per warp
+    uint32_t const orow   = k_build_rows + chunk_pads(max_nb);
+    auto          *gh_s   = reinterpret_cast<float2 *>(smem_raw); // [rows], a pair of zeros
+    auto          *tile_s = reinterpret_cast<uint32_t *>(gh_s + k_build_rows + 2); // [8 words][rows]
+    auto          *cnt_0  = tile_s + (8 * k_build_rows);
+    uint32_t const group  = threadIdx.x / k_xgthr;
+    uint32_t const gt     = threadIdx.x % k_xgthr;
+    uint32_t const wg     = gt / 32;
+    uint32_t const lane   = threadIdx.x & 31;
+    auto          *cnt_s  = cnt_0 + (group * k_xgwarps * crow); // [warp][bin], 16 bits each
+    auto          *order_s =
+        reinterpret_cast<uint16_t *>(cnt_0 + (GROUPS * k_xgwarps * crow)) + (group * orow);
+    __shared__ uint32_t wsum_s[GROUPS][k_xgwarps];
+
+    Chunk const    ch  = bchunks[c];
+    uint32_t const c0  = brange[ch.node];
+    bool const     one = brange[ch.node + 1] - c0 == 1;
+    for (uint32_t k = threadIdx.x; k < ch.count; k += GROUPS * k_xgthr)
+    {
+        uint32_t const r  = rows[ch.begin + k];
+        uint4 const   *tp = mirror + (((uint64_t{tile} * n_rows) + r) * 2);
+        uint4 const    lo = __ldg(tp);
+        uint4 const    hi = __ldg(tp + 1);
+        gh_s[k]           = __ldg(gh + r);
+        // a plane per 4-byte word, so that a feature's codes of consecutive
+        // rows lie in consecutive banks
+        tile_s[k]                      = lo.x;
+        tile_s[k_build_rows + k]       = lo.y;
+        tile_s[(2 * k_build_rows) + k] = lo.z;
+        tile_s[(3 * k_build_rows) + k] = lo.w;
+        tile_s[(4 * k_build_rows) + k] = hi.x;
+        tile_s[(5 * k_build_rows) + k] = hi.y;
+        tile_s[(6 * k_build_rows) + k] = hi.z;
+        tile_s[(7 * k_build_rows) + k] = hi.w;
+    }
+    if (threadIdx.x == 0)
+    {
+        gh_s[k_build_rows] = make_float2(0.0F, 0.0F);
+    }
+    __syncthreads();
+    auto          *cnt16 = reinterpret_cast<uint16_t *>(cnt_s + (wg * crow));
+    auto const    *start = reinterpret_cast<uint16_t const *>(cnt_s); // after the scan
+    uint32_t const k0    = wg * (k_xsteps * 32);
+    for (uint32_t x = group; x < per; x += GROUPS)
+    {
+        int32_t const js = tile_j[(blockIdx.y * per) + x];
+        if (js < 0)
+        {
+            continue;
+        }
+        uint32_t const j  = static_cast<uint32_t>(js);
+        uint32_t const nb = sel_nb[j];
+        for (uint32_t b = lane; b < crow; b += 32)
+        {
+            cnt_s[(wg * crow) + b] = 0;
+        }
+        __syncwarp();
+        auto const *codes =
+            reinterpret_cast<unsigned char const *>(tile_s + ((x * sizeof(BinT) / 4) * k_build_rows)) +
+            ((x * sizeof(BinT)) % 4);
+        uint32_t key[k_xsteps];
+#pragma unroll
+        for (uint32_t st = 0; st < k_xsteps; ++st)
+        {
+            uint32_t const k = k0 + (st * 32) + lane;
+            key[st]          = k < ch.count
+                                   ? *reinterpret_cast<BinT const *>(codes + (size_t{k} * 4))
+                                   : 0xFFFFu;
+        }
+        // as many ballots as the feature's codes have bits (a uniform choice)
+        if (nb <= 16)
+        {
+            rank_rows<4>(key, cnt16);
+        }
+        else if (sizeof(BinT) == 1 || nb <= 256)
+        {
+            rank_rows<8>(key, cnt16);
+        }
+        else
+        {
+            rank_rows<12>(key, cnt16);
+        }
+        group_sync(group);
+        // the chunk's (padded) bin starts, and each warp's place in each bin
+        uint32_t carry = 0;
+        for (uint32_t p0 = 0; p0 < crow; p0 += k_xgthr)
+        {
+            uint32_t const p = p0 + gt;
+            uint32_t       v[k_xgwarps];
+            uint32_t       pair = 0; // two bins' counts, 16 bits each
+#pragma unroll
+            for (uint32_t w = 0; w < k_xgwarps; ++w)
+            {
+                v[w] = p < crow ? cnt_s[(w * crow) + p] : 0;
+                pair += v[w];
+            }
+            uint32_t const even = (pair + 0x00010001u) & 0xFFFEFFFEu;
+            uint32_t const both = (even & 0xFFFFu) + (even >> 16);
+            uint32_t       inc  = both;
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1)
+            {
+                uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o)
+                {
+                    inc += y;
+                }
+            }
+            if (lane == 31)
+            {
+                wsum_s[group][wg] = inc;
+            }
+            group_sync(group);
+            uint32_t before = carry + inc - both;
+#pragma unroll
+            for (uint32_t w = 0; w < k_xgwarps; ++w)
+            {
+                uint32_t const t = wsum_s[group][w];
+                before += w < wg ? t : 0;
+                carry += t;
+            }
+            // (both halves stay below 2^13: no carry between them)
+            uint32_t const second = before + (even & 0xFFFFu);
+            uint32_t       run    = before | (second << 16);
+            if (p < crow)
+            {
+#pragma unroll
+                for (uint32_t w = 0; w < k_xgwarps; ++w)
+                {
+                    cnt_s[(w * crow) + p] = run;
+                    run += v[w];
+                }
+                if ((pair & 1u) != 0)
+                {
+                    order_s[second - 1] = k_build_rows;
+                }
+                if ((pair & 0x10000u) != 0)
+                {
+                    order_s[before + both - 1] = k_build_rows;
+                }
+            }
+            group_sync(group);
+        }
+#pragma unroll
+        for (uint32_t st = 0; st < k_xsteps; ++st)
+        {
+            uint32_t const b = key[st] & 0xFFFFu;
+            if (b != 0xFFFFu)
+            {
+                order_s[cnt16[b] + (key[st] >> 16)] =
+                    static_cast<uint16_t>(k0 + (st * 32) + lane);
+            }
+        }
+        group_sync(group);
+        // (warp 0's counters are the bins' starts, carry the padded length)
+        if (one)
+        {
+            float2 *cells = hist + (static_cast<uint64_t>(build[ch.node]) * total_cells) + cell_off[j];
+            for (uint32_t b = gt; b < nb; b += k_xgthr)
+            {
+                uint32_t const s1 = b + 1 < nb ? start[b + 1] : carry;
+                float2         a  = make_float2(0.0F, 0.0F);
+#pragma unroll 2
+                for (uint32_t p = start[b]; p < s1; p += 2)
+                {
+                    uint32_t const two = *reinterpret_cast<uint32_t const *>(order_s + p);
+                    add_pair(a, gh_s[two & 0xFFFFu]);
+                    add_pair(a, gh_s[two >> 16]);
+                }
+                cells[b] = a;
+            }
+        }
+        else
+        {
+            float2 *out = payload + (j * p_stride) + chunk_at(ch.aux, c - c0, c, max_nb);
+#pragma unroll 4
+            for (uint32_t p = gt; p < carry; p += k_xgthr)
+            {
+                out[p] = gh_s[order_s[p]];
+            }
+            uint16_t      *off = coff + (((uint64_t{c} * nfb) + j) * cs);
+            uint32_t const end = (((nb + 31) / 32) * 32) + 1;
+            for (uint32_t b = gt; b < end; b += k_xgthr)
+            {
+                off[b] = b < nb ? start[b] : static_cast<uint16_t>(carry);
+            }
+        }
+        group_sync(group);
+    }
+}
+
+__device__ __forceinline__ void cp_async16(void *smem_dst, void const *gsrc)
 {
     uint32_t const s = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc));
 }
 __device__ __forceinline__ void cp_async_commit()
 {
@@ -516,86 +655,236 @@ template <int N> __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// One lane per cell: the serial float chain over the cell's contiguous
-// (g, h) run, streamed through a per-lane cp.async ring in shared memory so
-// that many bytes are in flight even when few cells exist (the root).
-// grid (build nodes, features, ceil(max_bins / 32)), one warp per CTA.
-__global__ void __launch_bounds__(32)
+// A piece of a chunk's range of 32 bins: at most k_piece pairs (a chunk of
+// evenly spread codes has 272 in 32 of 256 bins, so one piece a chunk; a bin
+// holding most rows takes several), in one of k_pslots ring slots.
+constexpr uint32_t k_piece    = 512;
+constexpr uint32_t k_pslots   = 6;
+constexpr uint32_t k_plag     = 4;  // copies under way before the oldest is handed over
+constexpr uint32_t k_cthreads = 64; // the adding warp and the copying one
+
+// Named barriers of the ring (0 is the CTA's): slot s is full, slot s is empty.
+__device__ __forceinline__ void ring_arrive(uint32_t id)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(k_cthreads) : "memory");
+}
+__device__ __forceinline__ void ring_sync(uint32_t id)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(k_cthreads) : "memory");
+}
+
+// grid (build nodes, features, ceil(max_bins / 32)). A level's time is that
+// of its largest node, whose chain of chunks is serial, so what counts is a
+// chunk's time in the adding warp: a second warp does all of the copying.
+__global__ void __launch_bounds__(k_cthreads)
     chain_kernel(Ctl const *ctl, uint32_t const *build, Chunk const *bchunks,
-                 uint32_t const *brange, uint32_t const *seg, float2 const *payload,
-                 uint64_t p_stride, uint32_t const *sel_nb, uint32_t const *cell_off,
-                 uint32_t nfb, uint32_t cs, float2 *hist, uint32_t total_cells)
+                 uint32_t const *brange, uint16_t const *__restrict__ coff,
+                 float2 const *__restrict__ payload, uint64_t p_stride, uint32_t const *sel_nb,
+                 uint32_t const *cell_off, uint32_t max_nb, uint32_t nfb, uint32_t cs,
+                 float2 *hist, uint32_t total_cells)
 {
     pdl_enter();
-    extern __shared__ float2 ring_s[];
-    uint32_t const i = blockIdx.x;
+    __shared__ __align__(16) float2 ring_s[k_pslots][k_piece];
+    // a slot's piece: first pair within the chunk | pairs << 12 | the chunk's
+    // last piece << 31
+    __shared__ uint32_t head_s[k_pslots];
+    uint32_t const      i = blockIdx.x;
     if (i >= ctl->n_build)
     {
         return;
     }
-    uint32_t const j    = blockIdx.y;
-    uint32_t const nb   = sel_nb[j];
-    uint32_t const lane = threadIdx.x;
-    uint32_t const b    = (blockIdx.z * 32) + lane;
-    if (blockIdx.z * 32 >= nb)
+    uint32_t const c0 = brange[i];
+    uint32_t const c1 = brange[i + 1];
+    uint32_t const j  = blockIdx.y;
+    uint32_t const nb = sel_nb[j];
+    uint32_t const z  = blockIdx.z * 32;
+    if (c1 - c0 == 1 || z >= nb)
     {
-        return;
+        return; // one chunk: the sort finished it
     }
-    uint32_t const  slot  = build[i];
-    uint32_t const  nbase = bchunks[brange[i]].aux;
-    uint32_t const *sg    = seg + ((static_cast<uint64_t>(i) * nfb + j) * cs);
-    uint32_t        s0    = 0;
-    uint32_t        s1    = 0;
-    if (b < nb)
+    uint32_t const  lane = threadIdx.x & 31;
+    size_t const    step = size_t{nfb} * cs;
+    uint16_t const *off  = coff + (((uint64_t{c0} * nfb) + j) * cs) + z;
+    constexpr uint32_t full  = 1;
+    constexpr uint32_t empty = 1 + k_pslots;
+    if (threadIdx.x >= 32)
     {
-        s0 = sg[b];
-        s1 = sg[b + 1];
-    }
-    float2 const *src  = payload + (static_cast<uint64_t>(j) * p_stride) + nbase;
-    float2       *ring = ring_s + (lane * k_chain_stg * k_chain_nst);
-    uint32_t      next = s0;
-    auto          issue = [&](uint32_t st)
-    {
-        float2 *dst = ring + (st * k_chain_stg);
-#pragma unroll 8
-        for (uint32_t e = 0; e < k_chain_stg; ++e)
+        // every chunk is at least one piece, if an empty one
+        uint32_t const base   = c1 > c0 ? bchunks[c0].aux : 0;
+        float2 const  *mine   = payload + (j * p_stride);
+        uint32_t       piece  = 0;
+        uint32_t       slot   = 0; // of the piece being issued
+        uint32_t       ready  = 0; // of the oldest copy under way
+        for (uint32_t cb = c0; cb < c1; cb += 32)
         {
-            if (next + e < s1)
+            // the ranges of 32 chunks at a time, a lane each
+            uint32_t const m  = min(32u, c1 - cb);
+            uint32_t       r0 = 0;
+            uint32_t       r1 = 0;
+            if (lane < m)
             {
-                cp_async8(dst + e, src + next + e);
+                r0 = off[lane * step];
+                r1 = off[(lane * step) + 32];
+            }
+            off += 32 * step;
+            for (uint32_t x = 0; x < m; ++x)
+            {
+                uint32_t       ip  = __shfl_sync(0xFFFFFFFFu, r0, x);
+                uint32_t const end = __shfl_sync(0xFFFFFFFFu, r1, x);
+                float2 const  *src = mine + chunk_at(base, cb + x - c0, cb + x, max_nb) + (2 * lane);
+                bool           more;
+                do
+                {
+                    uint32_t const len = min(k_piece, end - ip);
+                    more               = end - ip > k_piece;
+                    if (piece >= k_pslots)
+                    {
+                        ring_sync(empty + slot);
+                    }
+                    float2 const *from = src + ip; // runs are even: 16-byte copies
+                    float2       *dst  = &ring_s[slot][2 * lane];
+#pragma unroll
+                    for (uint32_t u = 0; u < k_piece / 64; ++u)
+                    {
+                        if (2 * ((u * 32) + lane) < len)
+                        {
+                            cp_async16(dst + (u * 64), from + (u * 64));
+                        }
+                    }
+                    cp_async_commit();
+                    if (lane == 0)
+                    {
+                        head_s[slot] = ip | (len << 12) | (more ? 0u : 1u << 31);
+                    }
+                    ip += len;
+                    slot = slot + 1 == k_pslots ? 0 : slot + 1;
+                    if (++piece > k_plag)
+                    {
+                        cp_async_wait<k_plag>();
+                        ring_arrive(full + ready);
+                        ready = ready + 1 == k_pslots ? 0 : ready + 1;
+                    }
+                } while (more);
             }
         }
-        next = min(s1, next + k_chain_stg);
-        cp_async_commit();
-    };
-#pragma unroll
-    for (uint32_t st = 0; st < k_chain_nst - 1; ++st)
-    {
-        issue(st);
-    }
-    float    g  = 0.0F;
-    float    h  = 0.0F;
-    uint32_t st = 0;
-    for (uint32_t s = s0; s < s1;)
-    {
-        issue((st + k_chain_nst - 1) % k_chain_nst);
-        cp_async_wait<k_chain_nst - 1>();
-        float2 const  *v = ring + (st * k_chain_stg);
-        uint32_t const n = min(k_chain_stg, s1 - s);
-        for (uint32_t e = 0; e < n; ++e)
+        cp_async_wait<0>();
+        for (uint32_t x = min(piece, k_plag); x > 0; --x)
         {
-            float2 const x = v[e];
-            g += x.x;
-            h += x.y;
+            ring_arrive(full + ready);
+            ready = ready + 1 == k_pslots ? 0 : ready + 1;
         }
-        s += n;
-        st = (st + 1) % k_chain_nst;
+        // the adding warp's last hand-backs
+        uint32_t at = (slot + k_pslots - (min(piece, k_pslots) % k_pslots)) % k_pslots;
+        for (uint32_t x = min(piece, k_pslots); x > 0; --x)
+        {
+            ring_sync(empty + at);
+            at = at + 1 == k_pslots ? 0 : at + 1;
+        }
+        return;
     }
-    cp_async_wait<0>();
-    if (b < nb)
+    off += lane;
+    uint32_t left = c1 - c0; // chunks whose offsets have not been asked for
+    auto     offs = [&](uint32_t &lo, uint32_t &hi)
     {
-        hist[(static_cast<uint64_t>(slot) * total_cells) + cell_off[j] + b] =
-            make_float2(g, h);
+        lo = 0;
+        hi = 0;
+        if (left > 0)
+        {
+            lo = off[0];
+            hi = off[1];
+            off += step;
+            --left;
+        }
+    };
+    // this lane's run in the current chunk and in the next three
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+    {
+        offs(lo[q], hi[q]);
+    }
+    // four reads of two pairs; their additions
+    auto take = [](float4(&x)[4], float4 const *v, int n)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            if (2 * q < n)
+            {
+                x[q] = v[q];
+            }
+        }
+    };
+    auto fold = [](float2 &a, float4 const(&x)[4], int n)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            if (2 * q < n)
+            {
+                add_pair(a, make_float2(x[q].x, x[q].y));
+                add_pair(a, make_float2(x[q].z, x[q].w));
+            }
+        }
+    };
+    float2   a    = make_float2(0.0F, 0.0F);
+    uint32_t slot = 0;
+    // four chunks at a time, so that each one's offsets keep their registers
+    // (moving a register waits for the load that fills it)
+    for (uint32_t c = c0; c < c1; c += 4)
+    {
+#pragma unroll
+        for (uint32_t p = 0; p < 4; ++p)
+        {
+            if (c + p >= c1)
+            {
+                break;
+            }
+            bool more;
+            do
+            {
+                ring_sync(full + slot);
+                uint32_t const head = head_s[slot];
+                uint32_t const ip   = head & 0xFFFu;
+                uint32_t const len  = (head >> 12) & 0xFFFu;
+                more                = (head >> 31) == 0;
+                // the run's part in this piece, eight pairs at a time: the
+                // next eight are on their way while these are added
+                uint32_t const e0 = max(lo[p], ip);
+                int            n  = static_cast<int>(min(hi[p], ip + len)) - static_cast<int>(e0);
+                float4 const  *v  = reinterpret_cast<float4 const *>(&ring_s[slot][0]) + ((e0 - ip) / 2);
+                float4         x[4], y[4];
+                take(x, v, n);
+                while (__any_sync(0xFFFFFFFFu, n > 8))
+                {
+                    take(y, v + 4, n - 8);
+                    fold(a, x, n);
+                    n -= 8;
+                    v += 4;
+                    if (!__any_sync(0xFFFFFFFFu, n > 8))
+                    {
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                        {
+                            x[q] = y[q];
+                        }
+                        break;
+                    }
+                    take(x, v + 4, n - 8);
+                    fold(a, y, n);
+                    n -= 8;
+                    v += 4;
+                }
+                fold(a, x, n);
+                ring_arrive(empty + slot);
+                slot = slot + 1 == k_pslots ? 0 : slot + 1;
+            } while (more);
+            offs(lo[p], hi[p]);
+        }
+    }
+    if (z + lane < nb)
+    {
+        hist[(static_cast<uint64_t>(build[i]) * total_cells) + cell_off[j] + z + lane] = a;
     }
 }
 
@@ -1831,7 +2120,6 @@ __global__ void __launch_bounds__(k_threads)
 // 2^62; integer sums are order-free, hence deterministic), a one-CTA kernel
 // turns them into FP64 Newton values, and
 // pass B applies them from the leaf id pass A recorded.
-constexpr uint32_t k_no_sel_tile = 0xFFFFFFFFu; // an unused tile slot of a selection
 constexpr uint32_t k_walk_nodes = 512;     // a depth-8 tree has at most 511
 
 struct WalkArgs
@@ -4230,7 +4518,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                               "bin_mapper.max_bin or use a host grower");
         }
     }
-    cell_stride_ = ((max_nb_ + 1 + 3) / 4) * 4;
+    cell_stride_ = offset_stride(max_nb_);
     // leafwise: a pool slot per live leaf plus the one being built; a pop
     // consumes a heap entry (at most 2 per split + the root), two nodes each
     max_front_   = cfg_.leaf ? cfg_.tp.max_leaves + 1 : 1u << cfg_.tp.max_depth;
@@ -4250,7 +4538,6 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     sel_base_      = dalloc<uint32_t>(static_cast<size_t>(nsets) * n_sel_, s);
     cell_off_base_ = dalloc<uint32_t>(static_cast<size_t>(nsets) * (n_sel_ + 1), s);
     sel_nb_base_   = dalloc<uint32_t>(static_cast<size_t>(nsets) * n_sel_, s);
-    if (quant_)
     {
         // the mirror tiles a selection can touch: all selected features (v
         // 0), and the first one alone (v 1: the last level builds only its
@@ -4379,9 +4666,11 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     }
     else
     {
-        ccount_  = dalloc<uint32_t>(static_cast<size_t>(max_bchunks_) * n_sel_ * cell_stride_, s);
-        seg_     = dalloc<uint32_t>(static_cast<size_t>(max_front_) * n_sel_ * cell_stride_, s);
-        payload_ = dalloc<float2>(static_cast<size_t>(n_sel_) * max_rows_, s);
+        coff_    = dalloc<uint16_t>(static_cast<size_t>(max_bchunks_) * n_sel_ * cell_stride_, s);
+        // every built row once, and each chunk's padding
+        p_stride_ = ((uint64_t{max_rows_} + 1) & ~uint64_t{1}) +
+                    (uint64_t{max_bchunks_} * (chunk_pads(max_nb_) + 2));
+        payload_  = dalloc<float2>(n_sel_ * p_stride_, s);
     }
     scale_ = dalloc<float2>(1, s);
     BB_CHECK(cudaMemsetAsync(scale_, 0, sizeof(float2), s));
@@ -4411,32 +4700,28 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                                   static_cast<int>(lsmem)));
     if (!quant_)
     {
-        size_t const cnt_smem   = k_warps_feat * cell_stride_ * sizeof(uint32_t);
-        size_t const bin_bytes  = plane_.u8 ? 1 : 2;
-        size_t const sc_smem    = (k_build_rows * (4 + 8)) + cnt_smem +
-                               (k_warps_feat * k_build_rows * bin_bytes);
-        size_t const chain_smem = 32 * k_chain_stg * k_chain_nst * sizeof(float2);
-        if (sc_smem > 227 * 1024)
+        if (max_nb_ > k_exact_bins)
         {
             throw ConfigError("grower: bins per feature exceed the shared-memory budget");
         }
-        auto ck = plane_.u8 ? reinterpret_cast<void const *>(&count_kernel<uint8_t>)
-                            : reinterpret_cast<void const *>(&count_kernel<uint16_t>);
-        auto sk = plane_.u8 ? reinterpret_cast<void const *>(&scatter_kernel<uint8_t>)
-                            : reinterpret_cast<void const *>(&scatter_kernel<uint16_t>);
-        BB_CHECK(cudaFuncSetAttribute(ck, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(cnt_smem)));
-        BB_CHECK(cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(sc_smem)));
-        BB_CHECK(cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(chain_smem)));
+        // four features in flight, or two where a group's counters take more
+        // (features of several thousand bins)
+        xgroups_ = sort_smem(max_nb_, k_xgroups) <= 226 * 1024 ? k_xgroups : 2;
+        auto allow = [&](auto kern)
+        {
+            BB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(sort_smem(max_nb_, xgroups_))));
+        };
+        plane_.u8 ? allow(sort_kernel<uint8_t, k_xgroups>)
+                  : (xgroups_ == 2 ? allow(sort_kernel<uint16_t, 2>)
+                                   : allow(sort_kernel<uint16_t, k_xgroups>));
     }
     BB_CHECK(cudaEventCreate(&pev_[0]));
     BB_CHECK(cudaEventCreate(&pev_[1]));
 }
 
 // Set k's tables for the ascending feature ids sel: the ids, each one's
-// first cell and bin count, and (quantised) the mirror tiles holding them
+// first cell and bin count, and the mirror tiles holding them
 // with each tile slot's selection index, unused slots marked. The host
 // vectors are pageable, so each copy has left them when it returns.
 void Grower::write_tables(uint32_t set, std::vector<uint32_t> const &sel)
@@ -4456,10 +4741,6 @@ void Grower::write_tables(uint32_t set, std::vector<uint32_t> const &sel)
                              off.data(), (n_sel_ + 1) * 4, cudaMemcpyHostToDevice, s));
     BB_CHECK(cudaMemcpyAsync(sel_nb_base_ + (static_cast<size_t>(set) * n_sel_), nb.data(),
                              n_sel_ * 4, cudaMemcpyHostToDevice, s));
-    if (!quant_)
-    {
-        return;
-    }
     uint32_t const per = k_mirror_bytes / (plane_.u8 ? 1 : 2);
     for (int v = 0; v < 2; ++v)
     {
@@ -4531,7 +4812,7 @@ Grower::~Grower()
     void *ptrs[] = {sel_base_, cell_off_base_, sel_nb_base_, ctl_, nodes_[0], nodes_[1],
                     hist_[0], hist_[1],  cand_,    best_,     pchunks_,    pleft_,
                     prbase_,  dst_,      build_,   bpair_,    brange_,     bchunks_,
-                    ccount_,  seg_,      payload_, rows_[0],  rows_[1],    scale_,
+                    coff_,    payload_, rows_[0],  rows_[1],    scale_,
                     absmax_,  qgh_,      pcr_,     nleft_,    mono_,       qscale_,
                     qgh8_,    partial_,  dtree_,   tile_ids_base_[0], tile_ids_base_[1],
                     tile_j_base_[0], tile_j_base_[1], bbase_, dirs_, btot_, done_, wacc_,
@@ -4665,9 +4946,13 @@ void Grower::quantise(float2 const *gh, uint32_t n, bool have_absmax)
     n_launch_ += 1;
 }
 
-void Grower::build(uint32_t const *rows, uint32_t nfb, int dst, bool zeroed)
+void Grower::build(uint32_t const *rows, uint32_t nfb, int dst, bool zeroed, uint32_t n_nodes)
 {
     cudaStream_t s = stream_;
+    // the root's chunks, or those of n_nodes smaller children (each at most
+    // half of its parent's rows)
+    uint32_t const n_chunks =
+        std::min(max_bchunks_, ceil_div(zeroed ? max_rows_ / 2 : max_rows_, crows_) + n_nodes);
     phase_begin();
     if (quant_)
     {
@@ -4735,45 +5020,26 @@ void Grower::build(uint32_t const *rows, uint32_t nfb, int dst, bool zeroed)
     }
     else
     {
-        size_t const bin_bytes = plane_.u8 ? 1 : 2;
-        size_t const cnt_smem  = k_warps_feat * cell_stride_ * sizeof(uint32_t);
-        size_t const sc_smem   = (k_build_rows * (4 + 8)) + cnt_smem +
-                               (k_warps_feat * k_build_rows * bin_bytes);
-        dim3 const   gcs(max_bchunks_, ceil_div(nfb, k_warps_feat));
+        int const       v    = nfb == n_sel_ ? 0 : 1;
         uint32_t const *crow = rows != nullptr ? rows : root_rows_;
-        if (plane_.u8)
+        auto            sort = [&](auto kern)
         {
-            launch_k(pdl_, count_kernel<uint8_t>, gcs, k_threads, cnt_smem, s, ctl_, bchunks_, crow,
-                     plane_.bins, plane_.n_pad, sel_, sel_nb_, nfb, ccount_, cell_stride_);
-        }
-        else
-        {
-            launch_k(pdl_, count_kernel<uint16_t>, gcs, k_threads, cnt_smem, s, ctl_, bchunks_,
-                     crow, plane_.bins, plane_.n_pad, sel_, sel_nb_, nfb, ccount_, cell_stride_);
-        }
-        BB_LAUNCH("count_kernel");
-        launch_k(pdl_, offsets_kernel, dim3(max_front_, nfb), k_threads, 0, s, ctl_, brange_,
-                 ccount_, seg_, sel_nb_, nfb, cell_stride_, bchunks_);
-        BB_LAUNCH("offsets_kernel");
-        if (plane_.u8)
-        {
-            launch_k(pdl_, scatter_kernel<uint8_t>, gcs, k_threads, sc_smem, s, ctl_, bchunks_,
-                     crow, plane_.bins, plane_.n_pad, gh_cur_, sel_, sel_nb_, nfb, ccount_,
-                     cell_stride_, payload_, max_rows_);
-        }
-        else
-        {
-            launch_k(pdl_, scatter_kernel<uint16_t>, gcs, k_threads, sc_smem, s, ctl_, bchunks_,
-                     crow, plane_.bins, plane_.n_pad, gh_cur_, sel_, sel_nb_, nfb, ccount_,
-                     cell_stride_, payload_, max_rows_);
-        }
-        BB_LAUNCH("scatter_kernel");
-        size_t const chain_smem = 32 * k_chain_stg * k_chain_nst * sizeof(float2);
-        launch_k(pdl_, chain_kernel, dim3(max_front_, nfb, ceil_div(max_nb_, 32)), 32, chain_smem,
-                 s, ctl_, build_, bchunks_, brange_, seg_, payload_, max_rows_, sel_nb_, cell_off_,
-                 nfb, cell_stride_, static_cast<float2 *>(hist_[dst]), total_cells_);
+            launch_k(pdl_, kern, dim3(n_chunks, n_tiles_[v]), xgroups_ * k_xgthr,
+                     sort_smem(max_nb_, xgroups_), s, ctl_, bchunks_, brange_, build_, crow,
+                     static_cast<uint4 const *>(plane_.mirror), plane_.n_rows, gh_cur_,
+                     tile_ids_[v], tile_j_[v], sel_nb_, cell_off_, max_nb_, nfb, coff_,
+                     cell_stride_, payload_, p_stride_, static_cast<float2 *>(hist_[dst]),
+                     total_cells_);
+        };
+        plane_.u8 ? sort(sort_kernel<uint8_t, k_xgroups>)
+                  : (xgroups_ == 2 ? sort(sort_kernel<uint16_t, 2>)
+                                   : sort(sort_kernel<uint16_t, k_xgroups>));
+        BB_LAUNCH("sort_kernel");
+        launch_k(pdl_, chain_kernel, dim3(n_nodes, nfb, ceil_div(max_nb_, 32)), k_cthreads, 0, s,
+                 ctl_, build_, bchunks_, brange_, coff_, payload_, p_stride_, sel_nb_, cell_off_,
+                 max_nb_, nfb, cell_stride_, static_cast<float2 *>(hist_[dst]), total_cells_);
         BB_LAUNCH("chain_kernel");
-        n_launch_ += 4;
+        n_launch_ += 2;
     }
     if (prof_ != nullptr)
     {
@@ -4985,7 +5251,7 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
         }
         return;
     }
-    build(rows_out, nfb, nxt, true);
+    build(rows_out, nfb, nxt, true, front);
     uint32_t const n_cells = off_h_[nfb]; // the built features: a selection prefix
     if (red_ != nullptr)
     {
@@ -5079,7 +5345,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
     n_launch_ += 1;
     // the root's rows: the quantised build reads an identity list implicitly
     build(quant_ && identity_root ? nullptr : root_rows,
-          cfg_.tp.max_depth == 0 ? 1 : n_sel_, 0);
+          cfg_.tp.max_depth == 0 ? 1 : n_sel_, 0, false, 1);
     if (red_ != nullptr)
     {
         red_->sum_u64(hist_[0], total_cells_ * cw_, s);
@@ -5243,7 +5509,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
              brange_, build_, t, crows_, n_root, nullptr, static_cast<uint2 *>(nullptr));
     BB_LAUNCH("root_setup_kernel");
     launches += 2;
-    build(rows_[0], n_sel_, 0);
+    build(rows_[0], n_sel_, 0, false, 1);
     if (quant_)
     {
         launch_k(pdl_, qroot_totals_kernel, 1, 32, 0, s, nodes_[0],
@@ -5335,7 +5601,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                      quant_ ? total_cells_ * cw_ : 0);
             BB_LAUNCH("pscatter_kernel");
             n_launch_ = 0;
-            build(rows_[1], n_sel_, 0, true);
+            build(rows_[1], n_sel_, 0, true, 1);
             uint32_t const nb = n_launch_;
             launch_k(pdl_, leaf_copyback_kernel, 148u * 8u, 256, 0, s, lout, rows_[1], rows_[0], pp);
             BB_LAUNCH("leaf_copyback_kernel");
@@ -5453,7 +5719,7 @@ void Grower::populate(float2 const *gh, uint32_t const *rows, uint32_t n, double
     launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s, ctl_, nodes_[0], n, bchunks_, brange_,
              build_, t, crows_, n, nullptr, heap_);
     BB_LAUNCH("root_setup_kernel");
-    build(rows, n_sel_, 0);
+    build(rows, n_sel_, 0, false, 1);
     std::vector<double2> cells(total_cells_);
     if (quant_)
     {

@@ -255,8 +255,10 @@ class Grower
     void grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut const &out,
                        uint32_t *leaf_id, float *scores, float lr);
     void find_nodes(void const *hist, uint32_t n_nodes, uint32_t const *slot_of);
-    // zeroed: the quantised slots were already cleared (by the partition)
-    void build(uint32_t const *rows, uint32_t n_feat_build, int dst, bool zeroed = false);
+    // the histograms of the root, or (zeroed: the quantised slots were already
+    // cleared, by the partition) of at most n_nodes smaller children
+    void build(uint32_t const *rows, uint32_t n_feat_build, int dst, bool zeroed,
+               uint32_t n_nodes);
 
     Plane const          &plane_;
     GrowConfig            cfg_;
@@ -270,7 +272,7 @@ class Grower
     uint32_t              max_rows_    = 0;
     uint32_t              max_pchunks_ = 0;
     uint32_t              max_bchunks_ = 0;
-    uint32_t              cell_stride_ = 0; // per-(chunk, feature) count stride
+    uint32_t              cell_stride_ = 0; // per-(chunk, feature) offset stride
     uint32_t              lgroup_      = 1; // nodes per level-finder group
     uint32_t              qctas_       = 1; // u8 quantised histogram CTAs per tile
     // words per quantised cell: 2 (an int64 gradient and a uint64 hessian
@@ -300,9 +302,10 @@ class Grower
     uint32_t *bbase_    = nullptr; // per build index: its payload base
     uint32_t *brange_   = nullptr; // per build index: chunk range [c0, c1)
     Chunk    *bchunks_  = nullptr;
-    uint32_t *ccount_   = nullptr; // [bchunk][n_sel][cell_stride] counts/offsets
-    uint32_t *seg_      = nullptr; // [build][n_sel][cell_stride] bin segment starts
-    float2   *payload_  = nullptr; // [n_sel][max_rows] bin-sorted (g, h)
+    uint16_t *coff_     = nullptr; // [bchunk][n_sel][cell_stride] bin starts in the chunk
+    float2   *payload_  = nullptr; // [n_sel][p_stride_] (g, h), bin-sorted within a chunk
+    uint64_t  p_stride_ = 0;       // built rows and their chunks' padding
+    uint32_t  xgroups_  = 4;       // features a sort CTA has in flight
     uint32_t *rows_[2]  = {nullptr, nullptr};
     uint32_t *pcr_      = nullptr; // per frontier slot: partition chunk range
     uint32_t *nleft_    = nullptr; // per frontier slot: rows routed left
