@@ -270,12 +270,13 @@ __global__ void fill_kernel(float *x, float v, uint64_t n)
     }
 }
 
-// Copies the scratch tree into slot *round and advances the round counter,
-// so a captured boosting round needs no per-round pointer.
+// Copies the scratch tree into slot *round + k and advances the counter by
+// step, so a captured boosting round needs no per-round pointer. (Class trees
+// grown side by side commit with step 0, and advance_kernel follows them.)
 __global__ void commit_tree_kernel(TreeOut scratch, TreeOut slots, uint32_t cap,
-                                   uint32_t *round)
+                                   uint32_t *round, uint32_t k, uint32_t step)
 {
-    uint32_t const r   = *round;
+    uint32_t const r   = *round + k;
     uint64_t const off = static_cast<uint64_t>(r) * cap;
     for (uint32_t i = threadIdx.x; i < cap; i += blockDim.x)
     {
@@ -293,10 +294,15 @@ __global__ void commit_tree_kernel(TreeOut scratch, TreeOut slots, uint32_t cap,
         slots.meta[(3 * static_cast<uint64_t>(r)) + threadIdx.x] = scratch.meta[threadIdx.x];
     }
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && step != 0)
     {
-        *round = r + 1;
+        *round = r + step;
     }
+}
+
+__global__ void advance_kernel(uint32_t *round, uint32_t step)
+{
+    *round += step;
 }
 
 template <typename T> T *dmalloc(size_t n)
@@ -789,6 +795,19 @@ class RowSampler
 
 using namespace bb;
 
+// What grows a tree: a grower on its stream, the tree it writes, and the
+// rows of that tree's sample.
+struct Lane
+{
+    std::unique_ptr<bb::Grower> grower;
+    bb::TreeStore               scratch;
+    uint32_t                   *srows  = nullptr; // the tree's kept rows, ascending
+    uint32_t                   *scount = nullptr; // their number
+    uint32_t                   *sbsum  = nullptr; // per mask block: counts, then offsets
+    cudaStream_t                stream{};
+    cudaEvent_t                 done{};
+};
+
 struct bb_booster
 {
     bb::Plane const            *plane = nullptr;
@@ -803,8 +822,8 @@ struct bb_booster
     uint32_t                   *rows      = nullptr;
     uint32_t                   *leaf_id   = nullptr;
     uint32_t                   *round     = nullptr;
-    std::unique_ptr<bb::Grower> grower;
-    bb::TreeStore               scratch;
+    std::vector<Lane>           lanes; // one, or one per class
+    cudaEvent_t                 fork{};
     bb::TreeStore               trees;
     uint32_t                    n_trees = 0;
     bool                        use_graph = false;
@@ -827,9 +846,6 @@ struct bb_booster
     // the row sample (subsample < 1): a round's masks, one tree's rows
     std::unique_ptr<RowSampler> sampler;
     uint32_t                   *sbits  = nullptr; // K x words, tree-major
-    uint32_t                   *srows  = nullptr; // the tree's kept rows, ascending
-    uint32_t                   *scount = nullptr; // their number
-    uint32_t                   *sbsum  = nullptr; // per mask block: counts, then offsets
     std::vector<uint32_t>       host_counts;      // this round's, per tree
     // the feature sample (feature_fraction < 1): the grower's std::mt19937
     std::mt19937                feat_rng;
@@ -846,8 +862,16 @@ struct bb_booster
         }
         for (uint32_t k = 0; feat_k > 0 && k < n_classes; ++k)
         {
-            grower->set_selection(k, sample_features(plane->n_feats, feat_frac, feat_rng));
+            // (on the booster's stream: after the last round, which lanes
+            // join, and before the next)
+            lane(k).grower->set_selection(
+                k, sample_features(plane->n_feats, feat_frac, feat_rng), stream);
         }
+    }
+
+    Lane &lane(uint32_t k)
+    {
+        return lanes[lanes.size() > 1 ? k : 0];
     }
 
     // Class k's tree reads table set k (the one set of a single-output fit).
@@ -855,24 +879,32 @@ struct bb_booster
     {
         if (feat_k > 0)
         {
-            grower->use_set(k);
+            lane(k).grower->use_set(k);
         }
     }
 
-    // Tree k's kept rows into srows / scount.
+    // Tree k's kept rows into its lane's srows / scount.
     RootSample sample_tree(uint32_t k)
     {
+        Lane           &L     = lane(k);
         uint64_t const  words = sampler->words();
         uint32_t const *bits  = sbits + (static_cast<uint64_t>(k) * words);
         uint32_t const  nb    = static_cast<uint32_t>(ceil_div(words, k_smp_block));
-        sample_count_kernel<<<nb, k_smp_threads, 0, stream>>>(bits, words, sbsum);
+        sample_count_kernel<<<nb, k_smp_threads, 0, L.stream>>>(bits, words, L.sbsum);
         BB_LAUNCH("sample_count_kernel");
-        sample_scan_kernel<<<1, k_scan_threads, 0, stream>>>(sbsum, nb, scount);
+        sample_scan_kernel<<<1, k_scan_threads, 0, L.stream>>>(L.sbsum, nb, L.scount);
         BB_LAUNCH("sample_scan_kernel");
-        sample_list_kernel<<<nb, k_smp_threads, 0, stream>>>(bits, words, sbsum, srows);
+        sample_list_kernel<<<nb, k_smp_threads, 0, L.stream>>>(bits, words, L.sbsum, L.srows);
         BB_LAUNCH("sample_list_kernel");
         round_launches += 3;
-        return RootSample{scount, bits};
+        return RootSample{L.scount, bits};
+    }
+
+    // Where tree k records its rows' leaves: class trees one after another
+    // overwrite each other's, so side by side only the last one records.
+    uint32_t *leaf_ids(uint32_t k)
+    {
+        return record_leaf_ids && (lanes.size() == 1 || k + 1 == n_classes) ? leaf_id : nullptr;
     }
 
     // One tree over tree k's sample: the depthwise and levelwise planes walk
@@ -880,27 +912,28 @@ struct bb_booster
     void grow_sampled(uint32_t k, float2 const *g, float *sc, NextRound const *next)
     {
         RootSample const rs = sample_tree(k);
+        Lane            &L  = lane(k);
         uint64_t const   n  = plane->n_rows;
-        uint32_t *const  li = record_leaf_ids ? leaf_id : nullptr;
-        if (grower->fuses_next())
+        uint32_t *const  li = leaf_ids(k);
+        if (L.grower->fuses_next())
         {
-            grower->grow(g, srows, static_cast<uint32_t>(n), scratch.t, li, sc, lr, false, next,
+            L.grower->grow(g, L.srows, static_cast<uint32_t>(n), L.scratch.t, li, sc, lr, false, next,
                          &rs);
             return;
         }
-        grower->grow(g, srows, host_counts[k], scratch.t, li, sc, lr, false, nullptr);
+        L.grower->grow(g, L.srows, host_counts[k], L.scratch.t, li, sc, lr, false, nullptr);
         uint32_t const grid = std::min<uint32_t>(blocks(n), 148u * 16u);
         if (plane->u8)
         {
-            route_unsampled_kernel<uint8_t><<<grid, 256, 0, stream>>>(
+            route_unsampled_kernel<uint8_t><<<grid, 256, 0, L.stream>>>(
                 static_cast<uint8_t const *>(plane->bins), plane->n_pad, n, plane->n_bins,
-                scratch.t, scratch.cap, rs.bits, sc, li, lr);
+                L.scratch.t, L.scratch.cap, rs.bits, sc, li, lr);
         }
         else
         {
-            route_unsampled_kernel<uint16_t><<<grid, 256, 0, stream>>>(
+            route_unsampled_kernel<uint16_t><<<grid, 256, 0, L.stream>>>(
                 static_cast<uint16_t const *>(plane->bins), plane->n_pad, n, plane->n_bins,
-                scratch.t, scratch.cap, rs.bits, sc, li, lr);
+                L.scratch.t, L.scratch.cap, rs.bits, sc, li, lr);
         }
         BB_LAUNCH("route_unsampled_kernel");
         round_launches += 1;
@@ -920,9 +953,9 @@ struct bb_booster
     }
 
     // one grow's kernels and the commit after it
-    void count_tree()
+    void count_tree(uint32_t k)
     {
-        round_launches += grower->launches_per_tree() + 1;
+        round_launches += lane(k).grower->launches_per_tree() + 1;
     }
 
     void eval_round()
@@ -977,8 +1010,18 @@ struct bb_booster
                                                                     n_classes, weights);
             BB_LAUNCH("softmax_gradient_kernel");
             round_launches += 1;
+            bool const side = lanes.size() > 1;
+            if (side)
+            {
+                BB_CHECK(cudaEventRecord(fork, stream));
+            }
             for (uint32_t k = 0; k < n_classes; ++k)
             {
+                Lane &L = lane(k);
+                if (L.stream != stream)
+                {
+                    BB_CHECK(cudaStreamWaitEvent(L.stream, fork, 0));
+                }
                 use_features(k);
                 if (sampler)
                 {
@@ -986,18 +1029,33 @@ struct bb_booster
                 }
                 else
                 {
-                    grower->grow(gh + (k * n), rows, static_cast<uint32_t>(n), scratch.t,
-                                 record_leaf_ids ? leaf_id : nullptr, scores + (k * n), lr,
-                                 true, nullptr);
+                    L.grower->grow(gh + (k * n), rows, static_cast<uint32_t>(n), L.scratch.t,
+                                   leaf_ids(k), scores + (k * n), lr, true, nullptr);
                 }
-                commit_tree_kernel<<<1, 256, 0, stream>>>(scratch.t, trees.t, trees.cap, round);
+                commit_tree_kernel<<<1, 256, 0, L.stream>>>(L.scratch.t, trees.t, trees.cap,
+                                                            round, side ? k : 0u, side ? 0u : 1u);
                 BB_LAUNCH("commit_tree_kernel");
-                count_tree();
+                count_tree(k);
+            }
+            for (Lane &L : lanes)
+            {
+                if (L.stream != stream)
+                {
+                    BB_CHECK(cudaEventRecord(L.done, L.stream));
+                    BB_CHECK(cudaStreamWaitEvent(stream, L.done, 0));
+                }
+            }
+            if (side)
+            {
+                advance_kernel<<<1, 1, 0, stream>>>(round, n_classes);
+                BB_LAUNCH("advance_kernel");
+                round_launches += 1;
             }
             return;
         }
         use_features(0);
-        if (!grower->fuses_next())
+        Lane &L = lanes[0];
+        if (!L.grower->fuses_next())
         {
             // the leafwise plane stamps from its leaves' segments: gradients
             // of the current scores come from their own pass
@@ -1010,12 +1068,13 @@ struct bb_booster
             }
             else
             {
-                grower->grow(gh, rows, static_cast<uint32_t>(n), scratch.t,
-                             record_leaf_ids ? leaf_id : nullptr, scores, lr, true, nullptr);
+                L.grower->grow(gh, rows, static_cast<uint32_t>(n), L.scratch.t,
+                             leaf_ids(0), scores, lr, true, nullptr);
             }
-            commit_tree_kernel<<<1, 256, 0, stream>>>(scratch.t, trees.t, trees.cap, round);
+            commit_tree_kernel<<<1, 256, 0, stream>>>(L.scratch.t, trees.t, trees.cap, round,
+                                                     0, 1);
             BB_LAUNCH("commit_tree_kernel");
-            count_tree();
+            count_tree(0);
             round_launches += 1; // the gradient pass
             return;
         }
@@ -1026,12 +1085,13 @@ struct bb_booster
         }
         else
         {
-            grower->grow(gh, rows, static_cast<uint32_t>(n), scratch.t,
-                         record_leaf_ids ? leaf_id : nullptr, scores, lr, true, &next);
+            L.grower->grow(gh, rows, static_cast<uint32_t>(n), L.scratch.t,
+                         leaf_ids(0), scores, lr, true, &next);
         }
-        commit_tree_kernel<<<1, 256, 0, stream>>>(scratch.t, trees.t, trees.cap, round);
+        commit_tree_kernel<<<1, 256, 0, stream>>>(L.scratch.t, trees.t, trees.cap, round,
+                                                     0, 1);
         BB_LAUNCH("commit_tree_kernel");
-        count_tree();
+        count_tree(0);
     }
 };
 
@@ -1162,14 +1222,50 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
         b->feat_frac  = cfg->feature_fraction;
         b->feat_rng.seed(cfg->feature_seed);
     }
-    b->grower = std::make_unique<Grower>(p, gc, selection(*cfg, p.n_feats),
-                                         static_cast<uint32_t>(n), b->stream);
-    b->grower->set_monotone(monotone(*cfg));
-    b->grower->set_interaction(interaction(*cfg, p.n_feats));
-    b->grower->set_seed(cfg->seed);
+    // One lane per class: a class tree's launches are a chain of short
+    // kernels that leaves most of the GPU idle, and the classes' trees do not
+    // depend on one another. Seven classes x 54 columns, levelwise depth 8, ms
+    // a round one after another / side by side: int8 3.56 / 1.05 at 581,012
+    // rows, 7.09 / 4.48 at 4,000,000; exact 167 / 41 at 2,000,000 (whose
+    // one-hot columns are long serial chains). One lane for all of them where
+    // their growers would not fit a quarter of the free memory, and for the
+    // leafwise plane, whose host waits for every tree.
+    b->lanes.resize(1);
+    b->lanes[0].stream = b->stream;
+    if (K > 1 && !gc.leaf)
+    {
+        size_t free = 0;
+        size_t all  = 0;
+        BB_CHECK(cudaMemGetInfo(&free, &all));
+        if (Grower::device_bytes(p, gc, selection(*cfg, p.n_feats), static_cast<uint32_t>(n)) *
+                (K - 1) <=
+            free / 4)
+        {
+            gc.lanes = K;
+            b->lanes.resize(K);
+            BB_CHECK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        }
+    }
+    for (uint32_t k = 0; k < b->lanes.size(); ++k)
+    {
+        Lane &L = b->lanes[k];
+        if (k > 0)
+        {
+            BB_CHECK(cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking));
+            BB_CHECK(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming));
+        }
+        L.grower = std::make_unique<Grower>(p, gc, selection(*cfg, p.n_feats),
+                                            static_cast<uint32_t>(n), L.stream);
+        L.grower->set_monotone(monotone(*cfg));
+        L.grower->set_interaction(interaction(*cfg, p.n_feats));
+        L.grower->set_seed(cfg->seed);
+        // tree numbers (the rounding stream): round-major, as one grower's are
+        L.grower->set_tree_numbers(k, static_cast<uint32_t>(b->lanes.size()));
+        L.scratch.alloc(L.grower->max_nodes(), 1);
+    }
     if (red != nullptr)
     {
-        b->grower->set_shard(red, row_offset, total_rows);
+        b->lanes[0].grower->set_shard(red, row_offset, total_rows);
         b->sharded = true;
     }
     if (sampled)
@@ -1179,22 +1275,24 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
         b->sampler = std::make_unique<RowSampler>(cfg->subsample, cfg->random_seed, n, K, dev,
                                                   external);
         uint64_t const words = b->sampler->words();
-        b->sbits  = dmalloc<uint32_t>(words * K);
-        b->srows  = dmalloc<uint32_t>(n);
-        b->scount = dmalloc<uint32_t>(1);
-        b->sbsum  = dmalloc<uint32_t>(ceil_div(words, k_smp_block));
+        b->sbits = dmalloc<uint32_t>(words * K);
+        for (Lane &L : b->lanes)
+        {
+            L.srows  = dmalloc<uint32_t>(n);
+            L.scount = dmalloc<uint32_t>(1);
+            L.sbsum  = dmalloc<uint32_t>(ceil_div(words, k_smp_block));
+        }
     }
-    b->scratch.alloc(b->grower->max_nodes(), 1);
-    b->trees.alloc(b->grower->max_nodes(), max_trees * K); // round-major: r * K + k
+    b->trees.alloc(b->lanes[0].grower->max_nodes(), max_trees * K); // round-major: r * K + k
     // a leafwise round reads every pop back to the host: it runs eagerly
-    b->use_graph       = cfg->use_graph != 0 && b->grower->fuses_next();
+    b->use_graph       = cfg->use_graph != 0 && b->lanes[0].grower->fuses_next();
     b->record_leaf_ids = cfg->record_leaf_ids != 0;
     if (K == 1)
     {
         gradient_kernel<<<blocks(n), 256, 0, b->stream>>>(b->objective, b->scores, b->labels,
                                                           b->gh, n, nullptr);
         BB_LAUNCH("gradient_kernel");
-        b->grower->seed_absmax(b->gh);
+        b->lanes[0].grower->seed_absmax(b->gh);
     }
     BB_CHECK(cudaEventCreate(&b->ev0));
     BB_CHECK(cudaEventCreate(&b->ev1));
@@ -1792,7 +1890,7 @@ extern "C"
                     gradient_kernel<<<blocks(n), 256, 0, b->stream>>>(
                         b->objective, b->scores, b->labels, b->gh, n, b->weights);
                     BB_LAUNCH("gradient_kernel");
-                    b->grower->seed_absmax(b->gh);
+                    b->lanes[0].grower->seed_absmax(b->gh);
                 }
                 BB_CHECK(cudaStreamSynchronize(b->stream));
             });
@@ -1930,7 +2028,14 @@ extern "C"
                      "bb_booster_profile_round: tree capacity");
                 BB_CHECK(cudaStreamSynchronize(b->stream));
                 Profile p;
-                b->grower->set_profile(&p);
+                auto const profile = [&](Profile *q)
+                {
+                    for (Lane &L : b->lanes)
+                    {
+                        L.grower->set_profile(q);
+                    }
+                };
+                profile(&p);
                 b->upload_sample();
                 BB_CHECK(cudaEventRecord(b->ev0, b->stream));
                 try
@@ -1939,10 +2044,10 @@ extern "C"
                 }
                 catch (...)
                 {
-                    b->grower->set_profile(nullptr);
+                    profile(nullptr);
                     throw;
                 }
-                b->grower->set_profile(nullptr);
+                profile(nullptr);
                 BB_CHECK(cudaEventRecord(b->ev1, b->stream));
                 BB_CHECK(cudaEventSynchronize(b->ev1));
                 float ms = 0.0F;
@@ -2093,11 +2198,30 @@ extern "C"
         }
         b->release_eval();
         b->sampler.reset();
-        b->grower.reset();
-        b->scratch.release();
+        for (Lane &L : b->lanes)
+        {
+            if (L.stream != b->stream)
+            {
+                cudaStreamSynchronize(L.stream);
+            }
+            L.grower.reset();
+            L.scratch.release();
+            cudaFree(L.srows);
+            cudaFree(L.scount);
+            cudaFree(L.sbsum);
+            if (L.stream != b->stream)
+            {
+                cudaStreamDestroy(L.stream);
+                cudaEventDestroy(L.done);
+            }
+        }
+        if (b->fork != nullptr)
+        {
+            cudaEventDestroy(b->fork);
+        }
         b->trees.release();
         void *ps[] = {b->labels, b->scores, b->gh,     b->rows,   b->leaf_id, b->round,
-                      b->sbits,  b->srows,  b->scount, b->sbsum, b->weights};
+                      b->sbits,  b->weights};
         for (void *p : ps)
         {
             cudaFree(p);

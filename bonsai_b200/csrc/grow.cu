@@ -4410,10 +4410,10 @@ __global__ void leaf_set_tree_kernel(TreeOut *dst, TreeOut t, LeafLoop *st, uint
     st->root_may  = root_may;
 }
 
-__global__ void tree_counter_kernel(uint32_t *tree_no)
+__global__ void tree_counter_kernel(uint32_t *tree_no, uint32_t step)
 {
     pdl_enter();
-    *tree_no += 1;
+    *tree_no += step;
 }
 
 template <typename T> T *dalloc(size_t n, cudaStream_t s)
@@ -4429,7 +4429,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                uint32_t max_root_rows, cudaStream_t stream)
     : plane_(plane), cfg_(cfg), sel_h_(std::move(selected)), stream_(stream)
 {
-    pdl_ = plane_.n_rows >= (uint64_t{1} << 19);
+    pdl_ = plane_.n_rows >= (uint64_t{1} << 19) && cfg_.lanes == 1;
     if (cfg_.sample_k > 0)
     {
         // per-tree samples: the first sample_k features until set_selection
@@ -4526,10 +4526,13 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     max_rows_    = std::max<uint32_t>(max_root_rows, 1);
     crows_       = quant_ ? k_qbuild_rows : k_build_rows;
     // the histogram grid: one CTA per SM for a large fit, about one per four
-    // 2,048-row chunks of the root for a small one
+    // 2,048-row chunks of the root for a small one; growers side by side share
+    // the SMs (seven classes: 1.05 ms a round at 581,012 rows against 1.17 with
+    // a CTA per SM each, 1.40 against 1.68 at 1,000,000)
     qctas_       = cfg_.hist_ctas > 0
                        ? std::min(cfg_.hist_ctas, 64u * k_qctas)
-                       : std::max(1u, std::min(k_qctas, ceil_div(max_rows_, 4 * k_qbuild_rows)));
+                       : std::max(1u, std::min(k_qctas / std::min(cfg_.lanes, k_qctas),
+                                               ceil_div(max_rows_, 4 * k_qbuild_rows)));
     max_pchunks_ = ceil_div(max_rows_, k_part_rows) + max_front_;
     max_bchunks_ = ceil_div(max_rows_, crows_) + max_front_;
 
@@ -4567,7 +4570,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     sets_h_.assign(nsets, sel_h_);
     for (uint32_t k = 0; k < nsets; ++k)
     {
-        write_tables(k, sel_h_);
+        write_tables(k, sel_h_, s);
     }
     use_set(0);
     ctl_      = dalloc<Ctl>(1, s);
@@ -4724,9 +4727,8 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
 // first cell and bin count, and the mirror tiles holding them
 // with each tile slot's selection index, unused slots marked. The host
 // vectors are pageable, so each copy has left them when it returns.
-void Grower::write_tables(uint32_t set, std::vector<uint32_t> const &sel)
+void Grower::write_tables(uint32_t set, std::vector<uint32_t> const &sel, cudaStream_t s)
 {
-    cudaStream_t          s = stream_;
     std::vector<uint32_t> off(n_sel_ + 1, 0);
     std::vector<uint32_t> nb(n_sel_, 0);
     for (uint32_t j = 0; j < n_sel_; ++j)
@@ -4769,7 +4771,7 @@ void Grower::write_tables(uint32_t set, std::vector<uint32_t> const &sel)
     }
 }
 
-void Grower::set_selection(uint32_t set, std::vector<uint32_t> const &sel)
+void Grower::set_selection(uint32_t set, std::vector<uint32_t> const &sel, cudaStream_t s)
 {
     if (cfg_.sample_k == 0 || set >= sets_h_.size() || sel.size() != n_sel_)
     {
@@ -4782,7 +4784,7 @@ void Grower::set_selection(uint32_t set, std::vector<uint32_t> const &sel)
             throw std::logic_error("grower: a feature sample must be ascending plane features");
         }
     }
-    write_tables(set, sel);
+    write_tables(set, sel, s);
     sets_h_[set] = sel;
 }
 
@@ -4897,6 +4899,36 @@ void Grower::set_shard(Reducer *r, uint64_t row_offset, uint64_t total_rows)
         gleft_ = dalloc<uint64_t>(max_front_, stream_);
         BB_CHECK(cudaStreamSynchronize(stream_));
     }
+}
+
+void Grower::set_tree_numbers(uint32_t first, uint32_t step)
+{
+    tree_step_ = step;
+    BB_CHECK(cudaMemcpyAsync(dtree_, &first, 4, cudaMemcpyHostToDevice, stream_));
+    BB_CHECK(cudaStreamSynchronize(stream_));
+}
+
+size_t Grower::device_bytes(Plane const &plane, GrowConfig const &cfg,
+                            std::vector<uint32_t> const &selected, uint32_t max_root_rows)
+{
+    size_t   cells  = 0;
+    uint32_t max_nb = 0;
+    for (uint32_t const f : selected)
+    {
+        uint32_t const nb = plane.h_cut_off[f + 1] - plane.h_cut_off[f];
+        cells += nb;
+        max_nb = std::max(max_nb, nb);
+    }
+    size_t const n     = max_root_rows;
+    size_t const front = cfg.leaf ? cfg.tp.max_leaves + 1 : size_t{1} << cfg.tp.max_depth;
+    size_t       bytes = (16 * n) + (front * ((2 * cells * 16) + (selected.size() * 32)));
+    if (cfg.mode == HistMode::exact)
+    {
+        size_t const chunks = (n / k_build_rows) + front + 1;
+        bytes += selected.size() * ((8 * (n + (chunks * (chunk_pads(max_nb) + 2)))) +
+                                    (chunks * 2 * offset_stride(max_nb)));
+    }
+    return bytes;
 }
 
 void Grower::seed_absmax(float2 const *gh)
@@ -5464,7 +5496,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         BB_LAUNCH("stamp_kernel");
         n_launch_ += 1;
     }
-    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_);
+    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_, tree_step_);
     BB_LAUNCH("tree_counter_kernel");
     n_launch_ += 2;
     if (prof_ != nullptr)
@@ -5672,7 +5704,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
     launch_k(pdl_, stamp_kernel, max_pchunks_, k_threads, 0, s, ctl_, pchunks_, nodes_[0], rows_[0],
              t, leaf_id, scores, lr);
     BB_LAUNCH("stamp_kernel");
-    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_);
+    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_, tree_step_);
     BB_LAUNCH("tree_counter_kernel");
     launches += 2;
     // the loop's verdict: a full node table or pool is the reference's

@@ -166,6 +166,9 @@ struct GrowConfig
     // for any such sample, so its launches do not depend on which
     uint32_t   sample_k = 0;
     uint32_t   sel_sets = 1;
+    // growers working side by side on streams of one fit (the class trees of a
+    // round): their kernels share the GPU
+    uint32_t   lanes    = 1;
     // rows of the whole fit (every shard's, for a row-sharded fit; 0: the
     // grower's own rows): sizes the quantised cells and fixed-point sums
     uint64_t   fit_rows = 0;
@@ -229,9 +232,9 @@ class Grower
 
     // Per-tree feature samples (GrowConfig::sample_k): writes the tables of
     // table set `set` for the ascending feature ids sel (sample_k of them),
-    // enqueued on the grower's stream; use_set picks the set the next
-    // grow() reads (a captured grow keeps the set it was captured with).
-    void set_selection(uint32_t set, std::vector<uint32_t> const &sel);
+    // enqueued on stream s; use_set picks the set the next grow() reads (a
+    // captured grow keeps the set it was captured with).
+    void set_selection(uint32_t set, std::vector<uint32_t> const &sel, cudaStream_t s);
     void use_set(uint32_t set);
 
     uint32_t max_nodes() const
@@ -360,7 +363,7 @@ class Grower
     uint32_t *sel_nb_base_   = nullptr;
     uint32_t *tile_ids_base_[2] = {nullptr, nullptr};
     int32_t  *tile_j_base_[2]   = {nullptr, nullptr};
-    void      write_tables(uint32_t set, std::vector<uint32_t> const &sel);
+    void      write_tables(uint32_t set, std::vector<uint32_t> const &sel, cudaStream_t s);
     Node const     *nodes_cur_ = nullptr;
     uint32_t const *rows_cur_  = nullptr;
     uint32_t const *root_rows_ = nullptr;
@@ -373,12 +376,19 @@ class Grower
     void      leaf_values(TreeOut const &t, bool final_level);
     uint64_t  seed_     = 0;
     uint32_t  tree_no_  = 0;
+    uint32_t  tree_step_ = 1;
 
   public:
     void set_seed(uint64_t s)
     {
         seed_ = s;
     }
+    // The number of the first tree grown (the rounding stream's), and the step
+    // to each next one: 0 and 1 unless growers take turns.
+    void set_tree_numbers(uint32_t first, uint32_t step);
+    // About the device memory a grower of this configuration takes.
+    static size_t device_bytes(Plane const &plane, GrowConfig const &cfg,
+                               std::vector<uint32_t> const &selected, uint32_t max_root_rows);
     // per-feature monotone directions (+1 / -1 / 0), copied to the device
     void set_monotone(std::vector<int8_t> const &m);
     // Interaction constraints: per feature, the groups containing it as a
