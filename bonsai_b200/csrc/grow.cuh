@@ -345,6 +345,7 @@ class Grower
     Node            *leaves_    = nullptr;
     uint32_t        *free_      = nullptr;
     void            *tree_dev_  = nullptr;
+    uint32_t        *leaf_tick_ = nullptr; // last-CTA tickets: the partition's, the pair's
     cudaGraph_t      loop_g_    = nullptr;
     cudaGraphExec_t  loop_x_    = nullptr;
     uint32_t         body_launches_ = 0;
