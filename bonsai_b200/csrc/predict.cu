@@ -21,19 +21,19 @@
 // becomes the choice of which of two staged variants of the code the node
 // reads (the heap node comment below).
 //
-// Kernel: a CTA stages 1,024 rows' codes (both variants) from the plane's
-// row-major mirror into shared memory, word-interleaved by lane so that
-// every lane's code load hits its own bank whatever feature it reads, then
-// streams the heaps through shared memory in 16 KB chunks; each of 512
-// threads walks 2 rows per tree, addressing the heap by shared-window byte
-// address (from p = base + 4n the child is 2p - base (+4)). A grid of one
-// resident wave splits the rows evenly, so no SM idles in a tail. Small
-// batches, which cannot fill the GPU with rows, split the trees across CTAs
-// too: each (row, tree) leaf value goes to a workspace and a second kernel
-// sums every row's values in tree order, so the scores stay bit-identical.
-// Ensembles deeper than 10 or planes wider than 8 mirror tiles (256 u8 / 128
-// u16 features) use the node form: the reference's layout and walk, nodes in
-// global memory.
+// Up to depth 8 a lane is a tree and a warp a row (lane_predict_kernel): 32
+// trees' heaps lie interleaved, slot by slot, so that a lane's node is in its
+// own bank whatever slot it reached, and the row's codes are a few words that
+// the lanes share -- one shared-memory wavefront for every load of the walk,
+// where a lane per row has conflicts on the lower levels' nodes. A CTA holds a
+// tile of rows and streams the trees through shared memory, 32 at a time; the
+// 32 values of each row go by shared memory to the row's thread,
+// which adds them in tree order. Batches of up to a few hundred rows take a CTA
+// per row, a thread per tree and the nodes straight from L2
+// (row_predict_kernel), up to 64 rows several CTAs per row. Depths 9 and 10 take a lane
+// per row (heap_predict_kernel). Deeper ensembles, or planes wider than 8
+// mirror tiles (256 u8 / 128 u16 features), use the node form: the reference's
+// layout and walk, nodes in global memory.
 #include "bonsai_b200.h"
 #include "ingest.cuh"
 
@@ -58,8 +58,6 @@ namespace
 constexpr uint32_t k_max_heap_depth = 10;
 constexpr uint32_t k_max_heap_tiles = 8;
 constexpr uint32_t k_chunk_bytes    = 16384;
-constexpr uint32_t k_sms            = 148;
-constexpr size_t   k_max_vals_bytes = size_t{256} << 20;
 
 void need(bool ok, char const *what)
 {
@@ -138,19 +136,320 @@ template <typename CodeT> __device__ __forceinline__ uint32_t lds_code(uint32_t 
     return v;
 }
 
-// Scores of rows [blockIdx.x * rows_per_cta, + rows_per_cta) over trees
-// [blockIdx.y * trees_per_split, + trees_per_split), taken T x R rows at a
-// time. vals == nullptr: out[r] = init + lr * sum (blockIdx.y is 0 and the
-// split holds every tree); else every (tree, row) leaf value into
-// vals[t * n_rows + r].
+// ---- a lane per tree ----
+
+constexpr uint32_t k_lane_depth   = 8;    // the deepest ensemble taken a lane per tree
+constexpr uint32_t k_lane_threads = 512;
+constexpr uint32_t k_lane_smem    = 113 * 1024; // two CTAs an SM
+constexpr uint32_t k_val_stride   = 33;   // a row's 32 values, rows in different banks
+constexpr uint32_t k_row_threads  = 1024;
+constexpr uint32_t k_row_vals     = 4096; // values a row's CTA holds at once
+// Batches up to this many rows take a CTA per row: 1,000 trees of depth 8 over
+// 1,000 rows take 37.0 us so and 41.1 a lane per tree (whose floor is one SM
+// streaming every tree), over 2,000 rows 63.0 and 41.3.
+constexpr uint32_t k_row_batch    = 1024;
+constexpr uint32_t k_few_rows     = 64; // up to these, several CTAs per row
+constexpr uint32_t k_few_threads  = 128;
+
+__device__ __forceinline__ void cp_async16(void *smem_dst, void const *gsrc)
+{
+    uint32_t const d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc));
+}
+
+// Word wd of a row's staged codes: v1 words, then v0 words.
+__device__ __forceinline__ uint32_t staged_word(uint32_t const *mirror, uint64_t n_rows,
+                                                uint64_t row, uint32_t wd, uint32_t words,
+                                                uint32_t const *last_words, bool u8)
+{
+    uint32_t const w1 = wd < words ? wd : wd - words;
+    uint32_t const c =
+        __ldg(mirror + ((((static_cast<uint64_t>(w1 / 8) * n_rows) + row) * 8) + (w1 % 8)));
+    return wd < words ? c : missing_low(c, last_words[w1], u8);
+}
+
+// R rows of a warp's tile through its lanes' trees.
+template <typename CodeT, uint32_t D, uint32_t R>
+__device__ __forceinline__ void lane_walk(unsigned char const *heap, unsigned char const *codes,
+                                          uint32_t row_bytes, uint32_t r0, float *vals)
+{
+    uint32_t const lane4 = (threadIdx.x & 31u) * 4u;
+    // byte offsets into the interleaved heaps: slot n of this lane's tree at
+    // 128 n + 4 lane, its children at 2p - 4 lane (+ 128)
+    uint32_t const cl = 0u - lane4;
+    uint32_t const cr = 128u - lane4;
+    uint32_t       p[R];
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k)
+    {
+        p[k] = 128u + lane4;
+    }
+#pragma unroll
+    for (uint32_t d = 0; d < D; ++d)
+    {
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k)
+        {
+            uint32_t const e = *reinterpret_cast<uint32_t const *>(heap + p[k]);
+            uint32_t const c = *reinterpret_cast<CodeT const *>(
+                codes + ((r0 + (k_lane_threads / 32 * k)) * row_bytes) + (e >> 16));
+            p[k] = (2u * p[k]) + (c >= (e & 0xFFFFu) ? cr : cl);
+        }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k)
+    {
+        vals[((r0 + (k_lane_threads / 32 * k)) * k_val_stride) + (lane4 / 4u)] =
+            *reinterpret_cast<float const *>(heap + p[k]);
+    }
+}
+
+// Scores of rows [blockIdx.x * rows, + rows): warp w takes rows w, w + 16, ...
+// through each 32 trees, thread r sums row r. What bounds it is shared-memory
+// wavefronts (19 a row and 32 trees at depth 8) and instruction issue, close
+// together; two CTAs an SM fill each other's barriers and group loads (one CTA
+// of 1,024 threads with two buffers: 3.16 ms for 1,000 trees over 1M rows, two
+// so: 2.72; a lane per row, whose lower levels' nodes conflict: 3.21, and 0.78
+// against 0.30 at 100,000 rows, where its passes were half empty).
+template <typename CodeT, uint32_t D>
+__global__ void __launch_bounds__(k_lane_threads, 2)
+    lane_predict_kernel(uint32_t const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
+                        uint32_t const *__restrict__ last_words,
+                        uint32_t const *__restrict__ heaps, uint32_t n_trees, uint32_t rows,
+                        float lr, float init, float *__restrict__ out)
+{
+    constexpr uint32_t group = 32u * (2u << D) * 4u; // bytes of 32 trees
+    constexpr uint32_t warps = k_lane_threads / 32;
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *const heap_s  = smem;
+    float *const         vals_s  = reinterpret_cast<float *>(smem + group);
+    uint32_t const       words   = n_tiles * 8;
+    unsigned char *const codes_s =
+        smem + group + (size_t{rows} * k_val_stride * sizeof(float));
+    uint32_t const row_bytes = words * 8;
+    uint64_t const row0      = static_cast<uint64_t>(blockIdx.x) * rows;
+    uint32_t const live      = static_cast<uint32_t>(min(static_cast<uint64_t>(rows), n_rows - row0));
+    uint32_t const warp      = threadIdx.x >> 5;
+    uint32_t const groups    = (n_trees + 31) / 32;
+    auto const     load      = [&](uint32_t c)
+    {
+        auto const *src = reinterpret_cast<unsigned char const *>(heaps) +
+                          (static_cast<size_t>(c) * group);
+        for (uint32_t i = threadIdx.x * 16u; i < group; i += k_lane_threads * 16u)
+        {
+            cp_async16(heap_s + i, src + i);
+        }
+    };
+    load(0);
+    for (uint32_t i = threadIdx.x; i < live * 2 * words; i += k_lane_threads)
+    {
+        uint32_t const r = i / (2 * words);
+        reinterpret_cast<uint32_t *>(codes_s)[i] = staged_word(
+            mirror, n_rows, row0 + r, i - (r * 2 * words), words, last_words, sizeof(CodeT) == 1);
+    }
+    float acc = 0.0F;
+    for (uint32_t c = 0; c < groups; ++c)
+    {
+        asm volatile("cp.async.wait_all;\n" ::);
+        __syncthreads(); // the group is here (and the codes; the last values are added)
+        for (uint32_t r0 = warp; r0 < live; r0 += 4 * warps)
+        {
+            // (the same for the whole warp)
+            uint32_t const left = (live - r0 + warps - 1) / warps;
+            if (left >= 4)
+            {
+                lane_walk<CodeT, D, 4>(heap_s, codes_s, row_bytes, r0, vals_s);
+            }
+            else if (left == 3)
+            {
+                lane_walk<CodeT, D, 3>(heap_s, codes_s, row_bytes, r0, vals_s);
+            }
+            else if (left == 2)
+            {
+                lane_walk<CodeT, D, 2>(heap_s, codes_s, row_bytes, r0, vals_s);
+            }
+            else
+            {
+                lane_walk<CodeT, D, 1>(heap_s, codes_s, row_bytes, r0, vals_s);
+            }
+        }
+        __syncthreads(); // the values are here, the group is done with
+        if (c + 1 < groups)
+        {
+            load(c + 1);
+        }
+        if (threadIdx.x < live)
+        {
+            float const   *v = vals_s + (threadIdx.x * k_val_stride);
+            uint32_t const m = min(32u, n_trees - (c * 32));
+            if (m == 32)
+            {
+#pragma unroll
+                for (uint32_t t = 0; t < 32; ++t)
+                {
+                    acc = acc + v[t];
+                }
+            }
+            else
+            {
+                for (uint32_t t = 0; t < m; ++t)
+                {
+                    acc = acc + v[t];
+                }
+            }
+        }
+    }
+    if (threadIdx.x < live)
+    {
+        out[row0 + threadIdx.x] = __fadd_rn(init, __fmul_rn(acc, lr));
+    }
+}
+
+// A thread's tree for a row whose staged codes are in shared memory, nodes
+// from global memory (a warp's 32 trees side by side): the leaf's value.
+template <typename CodeT>
+__device__ __forceinline__ float tree_value(uint32_t const *__restrict__ heaps, uint32_t t,
+                                            uint32_t D, uint32_t const *codes_s)
+{
+    uint32_t const *h = heaps + ((t / 32) * (size_t{32} * (2u << D))) + (t % 32);
+    uint32_t        n = 1;
+    for (uint32_t d = 0; d < D; ++d)
+    {
+        uint32_t const e = __ldg(h + (n * 32));
+        uint32_t const c = *reinterpret_cast<CodeT const *>(
+            reinterpret_cast<unsigned char const *>(codes_s) + (e >> 16));
+        n = (2 * n) + (c >= (e & 0xFFFFu) ? 1 : 0);
+    }
+    return __uint_as_float(__ldg(h + (n * 32)));
+}
+
+// m values of shared memory (16-byte aligned) onto acc, in order.
+__device__ __forceinline__ float add_values(float acc, float const *vals_s, uint32_t m)
+{
+    uint32_t i = 0;
+#pragma unroll 4
+    for (; i + 4 <= m; i += 4)
+    {
+        float4 const v = *reinterpret_cast<float4 const *>(vals_s + i);
+        acc            = acc + v.x;
+        acc            = acc + v.y;
+        acc            = acc + v.z;
+        acc            = acc + v.w;
+    }
+    for (; i < m; ++i)
+    {
+        acc = acc + vals_s[i];
+    }
+    return acc;
+}
+
+template <typename CodeT>
+__device__ __forceinline__ void stage_row(uint32_t *codes_s, uint32_t const *mirror,
+                                          uint64_t n_rows, uint64_t row, uint32_t n_tiles,
+                                          uint32_t const *last_words)
+{
+    uint32_t const words = n_tiles * 8;
+    for (uint32_t i = threadIdx.x; i < 2 * words; i += blockDim.x)
+    {
+        codes_s[i] =
+            staged_word(mirror, n_rows, row, i, words, last_words, sizeof(CodeT) == 1);
+    }
+    __syncthreads();
+}
+
+// A CTA per row, a thread per tree; then one thread adds the values in tree
+// order.
+template <typename CodeT>
+__global__ void __launch_bounds__(k_row_threads)
+    row_predict_kernel(uint32_t const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
+                       uint32_t const *__restrict__ last_words,
+                       uint32_t const *__restrict__ heaps, uint32_t D, uint32_t n_trees, float lr,
+                       float init, float *__restrict__ out)
+{
+    __shared__ __align__(16) float    vals_s[k_row_vals];
+    __shared__ __align__(16) uint32_t codes_s[k_max_heap_tiles * 16];
+    stage_row<CodeT>(codes_s, mirror, n_rows, blockIdx.x, n_tiles, last_words);
+    float acc = 0.0F;
+    for (uint32_t t0 = 0; t0 < n_trees; t0 += k_row_vals)
+    {
+        uint32_t const m = min(k_row_vals, n_trees - t0);
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
+        {
+            vals_s[i] = tree_value<CodeT>(heaps, t0 + i, D, codes_s);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            acc = add_values(acc, vals_s, m);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+    {
+        out[blockIdx.x] = __fadd_rn(init, __fmul_rn(acc, lr));
+    }
+}
+
+// The fewest rows: the trees of a row over several CTAs (one SM's load path
+// bounds a row's 1,000 walks), every value kept, then a CTA per row sums them
+// in tree order.
+template <typename CodeT>
+__global__ void __launch_bounds__(k_few_threads)
+    few_values_kernel(uint32_t const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
+                      uint32_t const *__restrict__ last_words,
+                      uint32_t const *__restrict__ heaps, uint32_t D, uint32_t n_trees,
+                      float *__restrict__ vals)
+{
+    __shared__ __align__(16) uint32_t codes_s[k_max_heap_tiles * 16];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the sum may be set up
+    stage_row<CodeT>(codes_s, mirror, n_rows, blockIdx.x, n_tiles, last_words);
+    uint32_t const t = (blockIdx.y * k_few_threads) + threadIdx.x;
+    if (t < n_trees)
+    {
+        vals[(static_cast<uint64_t>(blockIdx.x) * n_trees) + t] =
+            tree_value<CodeT>(heaps, t, D, codes_s);
+    }
+}
+
+__global__ void __launch_bounds__(k_few_threads)
+    few_sum_kernel(float const *vals, uint32_t n_trees, float lr, float init,
+                   float *__restrict__ out)
+{
+    __shared__ __align__(16) float vals_s[k_row_vals];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float const *row = vals + (static_cast<uint64_t>(blockIdx.x) * n_trees);
+    float        acc = 0.0F;
+    for (uint32_t t0 = 0; t0 < n_trees; t0 += k_row_vals)
+    {
+        uint32_t const m = min(k_row_vals, n_trees - t0);
+        for (uint32_t i = threadIdx.x; i < m; i += k_few_threads)
+        {
+            vals_s[i] = __ldcg(row + t0 + i);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            acc = add_values(acc, vals_s, m);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+    {
+        out[blockIdx.x] = __fadd_rn(init, __fmul_rn(acc, lr));
+    }
+}
+
+// ---- a lane per row (depths 9 and 10) ----
+
+// Scores of rows [blockIdx.x * rows_per_cta, + rows_per_cta), taken T x R
+// rows at a time: out[r] = init + lr * sum.
 template <typename CodeT, uint32_t D, uint32_t T, uint32_t R>
 __global__ void __launch_bounds__(T)
     heap_predict_kernel(uint4 const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
                         uint32_t const *__restrict__ last_words,
                         uint32_t const *__restrict__ heaps, uint32_t n_trees,
-                        uint32_t trees_per_split, uint32_t chunk_trees, uint32_t rows_per_cta,
-                        float lr, float init, float *__restrict__ out,
-                        float *__restrict__ vals)
+                        uint32_t chunk_trees, uint32_t rows_per_cta, float lr, float init,
+                        float *__restrict__ out)
 {
     constexpr uint32_t slots = 2u << D; // per tree: root at 1, leaves at [2^D, 2^(D+1))
     constexpr uint32_t warps = T / 32;
@@ -167,8 +466,6 @@ __global__ void __launch_bounds__(T)
     uint32_t const heap_a = static_cast<uint32_t>(__cvta_generic_to_shared(heap_s));
     uint64_t const begin = static_cast<uint64_t>(blockIdx.x) * rows_per_cta;
     uint64_t const end   = min(n_rows, begin + rows_per_cta);
-    uint32_t const t0    = blockIdx.y * trees_per_split;
-    uint32_t const t1    = min(n_trees, t0 + trees_per_split);
 
     for (uint64_t row0 = begin; row0 < end; row0 += T * R)
     {
@@ -211,9 +508,9 @@ __global__ void __launch_bounds__(T)
         {
             acc[k] = 0.0F;
         }
-        for (uint32_t c0 = t0; c0 < t1; c0 += chunk_trees)
+        for (uint32_t c0 = 0; c0 < n_trees; c0 += chunk_trees)
         {
-            uint32_t const nc = min(chunk_trees, t1 - c0);
+            uint32_t const nc = min(chunk_trees, n_trees - c0);
             __syncthreads(); // codes staged; the previous chunk's walks done
             {
                 auto const *src =
@@ -254,75 +551,18 @@ __global__ void __launch_bounds__(T)
 #pragma unroll
                 for (uint32_t k = 0; k < R; ++k)
                 {
-                    float const v = __uint_as_float(lds_u32(p[k]));
-                    if (vals == nullptr)
-                    {
-                        acc[k] = acc[k] + v;
-                    }
-                    else if (row[k] < end)
-                    {
-                        vals[(static_cast<uint64_t>(c0 + j) * n_rows) + row[k]] = v;
-                    }
+                    acc[k] = acc[k] + __uint_as_float(lds_u32(p[k]));
                 }
             }
         }
-        if (vals == nullptr)
-        {
 #pragma unroll
-            for (uint32_t k = 0; k < R; ++k)
+        for (uint32_t k = 0; k < R; ++k)
+        {
+            if (row[k] < end)
             {
-                if (row[k] < end)
-                {
-                    out[row[k]] = __fadd_rn(init, __fmul_rn(acc[k], lr));
-                }
+                out[row[k]] = __fadd_rn(init, __fmul_rn(acc[k], lr));
             }
         }
-    }
-}
-
-// Every row's leaf values summed in tree order: one thread per row.
-__global__ void sum_rows_kernel(float const *__restrict__ vals, uint64_t n_rows, uint32_t n_trees,
-                                float lr, float init, float *__restrict__ out)
-{
-    uint64_t const r = (static_cast<uint64_t>(blockIdx.x) * blockDim.x) + threadIdx.x;
-    if (r >= n_rows)
-    {
-        return;
-    }
-    float acc = 0.0F;
-#pragma unroll 8
-    for (uint32_t t = 0; t < n_trees; ++t)
-    {
-        acc = acc + vals[(static_cast<uint64_t>(t) * n_rows) + r];
-    }
-    out[r] = __fadd_rn(init, __fmul_rn(acc, lr));
-}
-
-// The same sum with one warp per row, for batches too small to fill the GPU
-// with rows: lanes load 32 trees' values at once, every lane adds them in
-// order from the shuffles.
-__global__ void sum_warp_kernel(float const *__restrict__ vals, uint64_t n_rows, uint32_t n_trees,
-                                float lr, float init, float *__restrict__ out)
-{
-    uint64_t const r    = ((static_cast<uint64_t>(blockIdx.x) * blockDim.x) + threadIdx.x) >> 5;
-    uint32_t const lane = threadIdx.x & 31u;
-    if (r >= n_rows)
-    {
-        return;
-    }
-    float acc = 0.0F;
-    for (uint32_t t0 = 0; t0 < n_trees; t0 += 32)
-    {
-        uint32_t const m = min(32u, n_trees - t0);
-        float const    v = lane < m ? vals[(static_cast<uint64_t>(t0 + lane) * n_rows) + r] : 0.0F;
-        for (uint32_t j = 0; j < m; ++j)
-        {
-            acc = acc + __shfl_sync(0xFFFFFFFFu, v, static_cast<int>(j));
-        }
-    }
-    if (lane == 0)
-    {
-        out[r] = __fadd_rn(init, __fmul_rn(acc, lr));
     }
 }
 
@@ -382,9 +622,13 @@ struct DeviceBuf
             cudaFree(p);
         }
     }
-    void upload(void const *src, size_t bytes)
+    void alloc(size_t bytes)
     {
         check(cudaMalloc(&p, std::max<size_t>(bytes, 16)), "cudaMalloc");
+    }
+    void upload(void const *src, size_t bytes)
+    {
+        alloc(bytes);
         check(cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
     }
     template <typename T> T *as() const
@@ -407,22 +651,19 @@ struct bb_predict_plan
     // heap form (depth > 0) or node form (depth == 0)
     uint32_t    depth   = 0;
     uint32_t    n_tiles = 0;
+    uint32_t    sms     = 1;
+    uint32_t    lane_rows = 0; // a lane CTA's most rows
     bb::DeviceBuf heaps;
+    bb::DeviceBuf vals;       // a few rows' leaf values
     bb::DeviceBuf last_words; // per staged code word, its features' last bins
     bb::DeviceBuf last, roots, feature, split, left, right, dl, value;
-    // per-run workspace, grown on demand; runs through one plan serialise
+    // the host runs' output, grown on demand; runs through one plan serialise
     std::mutex   mu;
-    float       *vals     = nullptr;
-    size_t       vals_cap = 0;
     float       *out      = nullptr;
     size_t       out_cap  = 0;
     cudaStream_t stream   = nullptr;
     ~bb_predict_plan()
     {
-        if (vals != nullptr)
-        {
-            cudaFree(vals);
-        }
         if (out != nullptr)
         {
             cudaFree(out);
@@ -488,6 +729,8 @@ struct HeapPacker
     uint32_t        D;
     bool            u8;
     uint32_t        words;
+    bool            lanes;  // a lane per tree: the row's words one after another
+    uint32_t        stride; // words from a heap slot to the next
     uint32_t const *cut_off;
     uint32_t const *feature;
     uint32_t const *split;
@@ -505,7 +748,7 @@ struct HeapPacker
     {
         uint32_t const wd = u8 ? f >> 2 : f >> 1;
         uint32_t const b  = u8 ? f & 3u : (f & 1u) * 2u;
-        return (((v0 ? words : 0u) + wd) * 128u) + b;
+        return (((v0 ? words : 0u) + wd) * (lanes ? 4u : 128u)) + b;
     }
     // routes_left(code, last, split, dl) == !(variant code >= thr).
     uint32_t route(uint32_t f, uint32_t split_bin, bool default_left, uint32_t last) const
@@ -527,24 +770,25 @@ struct HeapPacker
         std::memcpy(&u, &v, 4);
         return u;
     }
-    // Node i (global id; b its tree's first) into heap slot h at depth d.
+    // Node i (global id; b its tree's first) into heap slot h at depth d (slot h lies
+    // at heap[h * stride])
     void fill(uint32_t *heap, uint32_t b, uint32_t i, uint32_t h, uint32_t d) const
     {
         if (d == D)
         {
-            heap[h] = leaf_slot(value[i]);
+            heap[size_t{h} * stride] = leaf_slot(value[i]);
             return;
         }
         if (feature[i] == k_leaf_flag)
         {
             // a leaf above depth D: route everything left, repeat it below
-            heap[h] = never();
+            heap[size_t{h} * stride] = never();
             fill(heap, b, i, 2 * h, d + 1);
             fill(heap, b, i, (2 * h) + 1, d + 1);
             return;
         }
         uint32_t const f = feature[i];
-        heap[h] = route(f, split[i], dl[i] != 0, cut_off[f + 1] - cut_off[f] - 1);
+        heap[size_t{h} * stride] = route(f, split[i], dl[i] != 0, cut_off[f + 1] - cut_off[f] - 1);
         fill(heap, b, b + left[i], 2 * h, d + 1);
         fill(heap, b, b + right[i], (2 * h) + 1, d + 1);
     }
@@ -566,35 +810,46 @@ template <typename F> void set_smem(F *kern, size_t smem)
 }
 
 using HeapFn = void (*)(uint4 const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
-                        uint32_t, uint32_t, uint32_t, uint32_t, float, float, float *, float *);
+                        uint32_t, uint32_t, uint32_t, float, float, float *);
 
-// The kernel shapes: 256 threads x 1 row per pass (small batches, trees
-// split across CTAs) and 512 threads x 2 rows (1,024 rows per pass).
-template <typename CodeT, uint32_t D> HeapFn heap_fn_r(uint32_t T, uint32_t R)
+HeapFn heap_fn(bool u8, uint32_t D)
 {
-    if (T == 512 && R == 2)
+    if (D == 9)
     {
-        return heap_predict_kernel<CodeT, D, 512, 2>;
+        return u8 ? heap_predict_kernel<uint8_t, 9, 512, 2> : heap_predict_kernel<uint16_t, 9, 512, 2>;
     }
-    return heap_predict_kernel<CodeT, D, 256, 1>;
+    return u8 ? heap_predict_kernel<uint8_t, 10, 512, 2> : heap_predict_kernel<uint16_t, 10, 512, 2>;
 }
 
-template <typename CodeT> HeapFn heap_fn_d(uint32_t D, uint32_t T, uint32_t R)
+using LaneFn = void (*)(uint32_t const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
+                        uint32_t, uint32_t, float, float, float *);
+
+template <typename CodeT> LaneFn lane_fn_d(uint32_t D)
 {
     switch (D)
     {
-    case 1: return heap_fn_r<CodeT, 1>(T, R);
-    case 2: return heap_fn_r<CodeT, 2>(T, R);
-    case 3: return heap_fn_r<CodeT, 3>(T, R);
-    case 4: return heap_fn_r<CodeT, 4>(T, R);
-    case 5: return heap_fn_r<CodeT, 5>(T, R);
-    case 6: return heap_fn_r<CodeT, 6>(T, R);
-    case 7: return heap_fn_r<CodeT, 7>(T, R);
-    case 8: return heap_fn_r<CodeT, 8>(T, R);
-    case 9: return heap_fn_r<CodeT, 9>(T, R);
-    case 10: return heap_fn_r<CodeT, 10>(T, R);
-    default: throw std::logic_error("bb_predict_plan: heap depth out of range");
+    case 1: return lane_predict_kernel<CodeT, 1>;
+    case 2: return lane_predict_kernel<CodeT, 2>;
+    case 3: return lane_predict_kernel<CodeT, 3>;
+    case 4: return lane_predict_kernel<CodeT, 4>;
+    case 5: return lane_predict_kernel<CodeT, 5>;
+    case 6: return lane_predict_kernel<CodeT, 6>;
+    case 7: return lane_predict_kernel<CodeT, 7>;
+    case 8: return lane_predict_kernel<CodeT, 8>;
+    default: throw std::logic_error("bb_predict_plan: lane depth out of range");
     }
+}
+
+LaneFn lane_fn(bool u8, uint32_t D)
+{
+    return u8 ? lane_fn_d<uint8_t>(D) : lane_fn_d<uint16_t>(D);
+}
+
+// Shared memory of a lane CTA over `rows` rows.
+size_t lane_smem(uint32_t D, uint32_t n_tiles, uint32_t rows)
+{
+    return (size_t{32} * (2u << D) * 4) +
+           (size_t{rows} * ((k_val_stride * sizeof(float)) + (n_tiles * 64)));
 }
 
 uint32_t sm_count()
@@ -637,86 +892,62 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
         BB_LAUNCH("node_predict_kernel");
         return 1;
     }
-    uint32_t const tree_bytes = (2u << pl.depth) * 4u;
-    uint32_t const chunk      = std::max(1u, k_chunk_bytes / tree_bytes);
-    uint32_t const sms        = sm_count();
-    size_t const   vals_bytes = n * static_cast<size_t>(n_trees) * 4;
-    // both code variants of a row: 64 bytes per mirror tile
-    size_t const   row_bytes  = static_cast<size_t>(pl.n_tiles) * 64;
-    bool const     split_mode = ceil_div(n, 256) < sms && vals_bytes <= k_max_vals_bytes;
-    uint32_t       T          = 256;
-    uint32_t       R          = 1;
-    if (!split_mode)
+    if (pl.depth <= k_lane_depth)
     {
-        T = 512;
-        R = 2;
-    }
-    size_t const smem = (static_cast<size_t>(T) * R * row_bytes) +
-                        (static_cast<size_t>(chunk) * tree_bytes);
-    HeapFn const fn   = pl.u8 ? heap_fn_d<uint8_t>(pl.depth, T, R)
-                              : heap_fn_d<uint16_t>(pl.depth, T, R);
-    set_smem(fn, smem);
-    uint32_t rows_per_cta = T * R;
-    uint32_t splits       = 1;
-    uint32_t tps          = n_trees;
-    dim3     grid;
-    if (split_mode)
-    {
-        // few rows: the trees split across CTAs too, every leaf value kept
-        uint32_t const row_blks = ceil_div(n, rows_per_cta);
-        uint32_t const n_chunks = ceil_div(n_trees, chunk);
-        splits = std::min(ceil_div(2 * sms, row_blks), n_chunks);
-        tps    = ceil_div(ceil_div(n_trees, splits), chunk) * chunk;
-        splits = ceil_div(n_trees, tps);
-        grid   = dim3(row_blks, splits);
-    }
-    else
-    {
-        // one wave of resident CTAs, each over an equal run of rows
-        int occ = 0;
-        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, static_cast<int>(T), smem),
-              "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-        uint64_t const ctas = static_cast<uint64_t>(std::max(occ, 1)) * sms;
-        uint64_t const per  = std::max<uint64_t>(32, ((((n + ctas - 1) / ctas) + 31) / 32) * 32);
-        rows_per_cta        = static_cast<uint32_t>(per);
-        grid                = dim3(ceil_div(n, per), 1);
-    }
-    float *vals = nullptr;
-    if (splits > 1)
-    {
-        if (pl.vals_cap < vals_bytes)
+        auto const *mirror = static_cast<uint32_t const *>(p.mirror);
+        if (n <= k_few_rows)
         {
-            if (pl.vals != nullptr)
-            {
-                check(cudaFree(pl.vals), "cudaFree");
-                pl.vals     = nullptr;
-                pl.vals_cap = 0;
-            }
-            check(cudaMalloc(&pl.vals, vals_bytes), "cudaMalloc");
-            pl.vals_cap = vals_bytes;
+            auto const fn = pl.u8 ? few_values_kernel<uint8_t> : few_values_kernel<uint16_t>;
+            fn<<<dim3(static_cast<uint32_t>(n), ceil_div(n_trees, k_few_threads)), k_few_threads, 0,
+                 s>>>(mirror, n, pl.n_tiles, pl.last_words.as<uint32_t>(),
+                      pl.heaps.as<uint32_t>(), pl.depth, n_trees, pl.vals.as<float>());
+            BB_LAUNCH("few_values_kernel");
+            launch_k(true, few_sum_kernel, static_cast<uint32_t>(n), k_few_threads, 0, s,
+                     pl.vals.as<float>(), n_trees, pl.lr, pl.init, out);
+            BB_LAUNCH("few_sum_kernel");
+            return 2;
         }
-        vals = pl.vals;
-    }
-    fn<<<grid, T, smem, s>>>(static_cast<uint4 const *>(p.mirror), n, pl.n_tiles,
-                                          pl.last_words.as<uint32_t>(), pl.heaps.as<uint32_t>(),
-                                          n_trees, tps, chunk, rows_per_cta, pl.lr, pl.init, out,
-                                          vals);
-    BB_LAUNCH("heap_predict_kernel");
-    if (splits == 1)
-    {
+        if (n <= k_row_batch)
+        {
+            uint32_t const T = std::min(k_row_threads, ((n_trees + 31) / 32) * 32);
+            auto const     fn = pl.u8 ? row_predict_kernel<uint8_t> : row_predict_kernel<uint16_t>;
+            fn<<<static_cast<uint32_t>(n), T, 0, s>>>(mirror, n, pl.n_tiles,
+                                                      pl.last_words.as<uint32_t>(),
+                                                      pl.heaps.as<uint32_t>(), pl.depth, n_trees,
+                                                      pl.lr, pl.init, out);
+            BB_LAUNCH("row_predict_kernel");
+            return 1;
+        }
+        // equal tiles, in as few waves of two CTAs an SM as the largest allows
+        uint64_t const wave  = uint64_t{2} * pl.sms;
+        uint64_t const waves = (n + (wave * pl.lane_rows) - 1) / (wave * pl.lane_rows);
+        uint32_t const rows  = ceil_div(n, wave * waves);
+        lane_fn(pl.u8, pl.depth)<<<ceil_div(n, rows), k_lane_threads,
+                                   lane_smem(pl.depth, pl.n_tiles, rows), s>>>(
+            mirror, n, pl.n_tiles, pl.last_words.as<uint32_t>(), pl.heaps.as<uint32_t>(), n_trees,
+            rows, pl.lr, pl.init, out);
+        BB_LAUNCH("lane_predict_kernel");
         return 1;
     }
-    if (n < 4096)
-    {
-        sum_warp_kernel<<<ceil_div(n * 32, 256), 256, 0, s>>>(vals, n, n_trees, pl.lr, pl.init,
-                                                              out);
-    }
-    else
-    {
-        sum_rows_kernel<<<ceil_div(n, 256), 256, 0, s>>>(vals, n, n_trees, pl.lr, pl.init, out);
-    }
-    BB_LAUNCH("predict sum kernel");
-    return 2;
+    uint32_t const tree_bytes = (2u << pl.depth) * 4u;
+    uint32_t const chunk      = std::max(1u, k_chunk_bytes / tree_bytes);
+    // both code variants of a row: 64 bytes per mirror tile; two rows a thread
+    // of 512
+    size_t const smem = (size_t{1024} * pl.n_tiles * 64) + (size_t{chunk} * tree_bytes);
+    HeapFn const fn   = heap_fn(pl.u8, pl.depth);
+    set_smem(fn, smem);
+    // one wave of resident CTAs, each over an equal run of rows
+    int occ = 0;
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 512, smem),
+          "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+    uint64_t const ctas = static_cast<uint64_t>(std::max(occ, 1)) * pl.sms;
+    uint64_t const per  = std::max<uint64_t>(32, ((((n + ctas - 1) / ctas) + 31) / 32) * 32);
+    fn<<<ceil_div(n, per), 512, smem, s>>>(static_cast<uint4 const *>(p.mirror), n, pl.n_tiles,
+                                           pl.last_words.as<uint32_t>(), pl.heaps.as<uint32_t>(),
+                                           n_trees, chunk, static_cast<uint32_t>(per), pl.lr,
+                                           pl.init, out);
+    BB_LAUNCH("heap_predict_kernel");
+    return 1;
 }
 
 std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
@@ -752,14 +983,35 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
         pl->n_tiles        = n_tiles;
         size_t const   slots = static_cast<size_t>(2u << D);
         uint32_t const words = n_tiles * 8;
-        std::vector<uint32_t> h(slots * n_trees, 0u);
-        HeapPacker const      pk{D,     p.u8,      words, pl->cut_off.data(), feature, split_bin,
-                            left,  right,     default_left, value};
-        for (uint32_t t = 0; t < n_trees; ++t)
+        bool const       by_tree = D <= k_lane_depth;
+        HeapPacker const pk{D,       p.u8,      words, by_tree, by_tree ? 32u : 1u, pl->cut_off.data(),
+                            feature, split_bin, left,  right,   default_left,       value};
+        pl->sms = sm_count();
+        if (by_tree)
         {
-            pk.fill(h.data() + (t * slots), roots[t], roots[t], 1, 0);
+            // 32 trees interleaved; the last group's missing ones (never added)
+            // route every row to their left spine
+            std::vector<uint32_t> h(slots * 32 * ((n_trees + 31) / 32), pk.never());
+            for (uint32_t t = 0; t < n_trees; ++t)
+            {
+                pk.fill(h.data() + ((t / 32) * slots * 32) + (t % 32), roots[t], roots[t], 1, 0);
+            }
+            pl->heaps.upload(h.data(), h.size() * 4);
+            size_t const per_row = lane_smem(D, n_tiles, 1) - lane_smem(D, n_tiles, 0);
+            pl->lane_rows        = static_cast<uint32_t>(std::min<size_t>(
+                k_lane_threads, (k_lane_smem - lane_smem(D, n_tiles, 0)) / per_row));
+            set_smem(lane_fn(p.u8, D), k_lane_smem);
+            pl->vals.alloc(size_t{k_few_rows} * n_trees * sizeof(float));
         }
-        pl->heaps.upload(h.data(), h.size() * 4);
+        else
+        {
+            std::vector<uint32_t> h(slots * n_trees, 0u);
+            for (uint32_t t = 0; t < n_trees; ++t)
+            {
+                pk.fill(h.data() + (t * slots), roots[t], roots[t], 1, 0);
+            }
+            pl->heaps.upload(h.data(), h.size() * 4);
+        }
         // the last bin of every code lane of every staged word (padding
         // lanes: a value no code has)
         std::vector<uint32_t> lw(words, 0u);
