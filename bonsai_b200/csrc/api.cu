@@ -1397,8 +1397,8 @@ extern "C"
                 BB_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
                 try
                 {
+                    alloc_mirror(p);
                     ingest(p, X, x_on_device != 0, s);
-                    build_mirror(p, s);
                     BB_CHECK(cudaStreamSynchronize(s));
                 }
                 catch (...)
@@ -1591,7 +1591,6 @@ extern "C"
                 p.n_rows = n_rows;
                 p.n_pad  = ((n_rows + 63) / 64) * 64;
                 ingest(p, X, x_on_device != 0, p.stream, p.stage, p.stage_rows);
-                fill_mirror(p, p.stream);
                 BB_CHECK(cudaStreamSynchronize(p.stream));
             });
     }

@@ -50,6 +50,9 @@ struct Plane
 void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream,
             float *owned_stage = nullptr, uint64_t owned_rows = 0);
 
+// Allocates p.mirror; ingest() then fills it beside the feature-major codes.
+void alloc_mirror(Plane &p);
+
 // Fills p.mirror from the feature-major codes (allocating it).
 void build_mirror(Plane &p, cudaStream_t stream);
 
@@ -57,10 +60,6 @@ void build_mirror(Plane &p, cudaStream_t stream);
 // at most 64 MB, and a whole number of bin-application tiles whenever a batch
 // can take more than one chunk.
 uint64_t stage_rows_for(uint32_t n_feats, uint64_t max_rows);
-
-// Rewrites p.mirror (already allocated for at least p.n_rows rows) from the
-// feature-major codes.
-void fill_mirror(Plane &p, cudaStream_t stream);
 
 constexpr uint32_t k_mirror_bytes = 32;
 
