@@ -5,11 +5,11 @@
 // Per column of the sample: the NaN-free values as order-preserving 32-bit
 // keys (the reference's radix key: flip every bit of a negative, the sign bit
 // of a non-negative, so -0.0 sorts before +0.0 as in its sort_floats,
-// :115-157); an LSD radix sort by one CTA (four 8-bit passes, each a digit
-// histogram, a scan and a stable scatter ranked per warp with match_any);
-// then the runs of equal values (run-length encoding under operator<, so the
-// two zeros are one run whose representative is the first, -0.0 when
-// present), and the lightest exact rule: every distinct value when they fit
+// :115-157); an LSD radix sort (four 8-bit passes, each the tiles' digit
+// counts, a scan and a stable scatter ranked per warp with ballots); then the
+// runs of equal values (run-length encoding under operator<, so the two zeros
+// are one run whose representative is the first, -0.0 when present), and the
+// lightest exact rule: every distinct value when they fit
 // the cut budget, else the count-weighted greedy walk when some value is at
 // least a mean bin (greedy_weighted_cuts, :38-96; one thread walks the
 // runs), else the quantile stride over the sorted values; then the FLT_MAX
@@ -134,91 +134,179 @@ __global__ void __launch_bounds__(k_tile_rows_c)
     }
 }
 
-// Column blockIdx.x's keys sorted ascending: four stable 8-bit LSD passes
-// between a and b (the result back in a).
-__global__ void __launch_bounds__(k_cut_threads)
-    sort_keys_kernel(uint32_t *__restrict__ a, uint32_t *__restrict__ b, uint64_t n,
-                     uint32_t const *counts)
+// The columns' keys sorted ascending: four stable 8-bit LSD passes, each over
+// tiles of k_sort_tile keys -- the tiles' digit counts, their scan, and a
+// scatter in which a warp ranks a contiguous run of its tile's keys, the lanes
+// of one digit found from a ballot per bit. (One CTA per column with the match
+// instruction, which takes about 59 cycles of an SM a warp, and 1,024 keys
+// between barriers: a 200,000 x 28 fit 5.8 ms, 1.4 so.)
+constexpr uint32_t k_sort_threads = 512;
+constexpr uint32_t k_sort_warps   = k_sort_threads / 32;
+constexpr uint32_t k_sort_steps   = 16; // keys per lane
+constexpr uint32_t k_sort_tile    = k_sort_threads * k_sort_steps;
+
+// grid (tiles, columns): digit d's keys of tile t into tc[(col * tiles + t) * 256 + d].
+__global__ void __launch_bounds__(k_sort_threads)
+    sort_count_kernel(uint32_t const *__restrict__ src, uint64_t n,
+                      uint32_t const *__restrict__ counts, uint32_t shift,
+                      uint32_t *__restrict__ tc)
 {
     __shared__ uint32_t hist[256];
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t tot[256];
-    __shared__ uint16_t wc[k_cut_threads / 32][256];
-    uint32_t const      col  = blockIdx.x;
-    uint32_t const      m    = counts[col];
-    uint32_t const      t    = threadIdx.x;
-    uint32_t const      lane = t & 31u;
-    uint32_t const      w    = t >> 5;
-    uint32_t           *src  = a + (static_cast<uint64_t>(col) * n);
-    uint32_t           *dst  = b + (static_cast<uint64_t>(col) * n);
-    for (uint32_t shift = 0; shift < 32; shift += 8)
+    uint32_t const      m  = counts[blockIdx.y];
+    uint64_t const      i0 = static_cast<uint64_t>(blockIdx.x) * k_sort_tile;
+    if (i0 >= m)
     {
-        if (t < 256)
+        return;
+    }
+    uint32_t const *k = src + (static_cast<uint64_t>(blockIdx.y) * n);
+    if (threadIdx.x < 256)
+    {
+        hist[threadIdx.x] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t st = 0; st < k_sort_steps; ++st)
+    {
+        uint64_t const i = i0 + (st * k_sort_threads) + threadIdx.x;
+        if (i < m)
         {
-            hist[t] = 0;
+            atomicAdd(&hist[(k[i] >> shift) & 0xFFu], 1u);
         }
-        __syncthreads();
-        for (uint32_t i = t; i < m; i += k_cut_threads)
+    }
+    __syncthreads();
+    if (threadIdx.x < 256)
+    {
+        tc[(((static_cast<uint64_t>(blockIdx.y) * gridDim.x) + blockIdx.x) * 256) + threadIdx.x] =
+            hist[threadIdx.x];
+    }
+}
+
+// grid (columns): each tile's counts become its first places in the column,
+// digits in order, tiles in order within a digit.
+__global__ void __launch_bounds__(256)
+    sort_scan_kernel(uint32_t const *__restrict__ counts, uint32_t *__restrict__ tc,
+                     uint32_t tiles)
+{
+    __shared__ uint32_t wsum[8];
+    uint32_t const      used = (counts[blockIdx.x] + k_sort_tile - 1) / k_sort_tile;
+    uint32_t           *c    = tc + ((static_cast<uint64_t>(blockIdx.x) * tiles) * 256) + threadIdx.x;
+    uint32_t            sum  = 0;
+#pragma unroll 8
+    for (uint32_t t = 0; t < used; ++t)
+    {
+        sum += c[static_cast<uint64_t>(t) * 256];
+    }
+    uint32_t const lane = threadIdx.x & 31u;
+    uint32_t       inc  = sum;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1)
+    {
+        uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o)
         {
-            atomicAdd(&hist[(src[i] >> shift) & 0xFFu], 1u);
+            inc += y;
         }
-        __syncthreads();
-        if (t == 0)
+    }
+    if (lane == 31)
+    {
+        wsum[threadIdx.x >> 5] = inc;
+    }
+    __syncthreads();
+    uint32_t run = inc - sum;
+    for (uint32_t w = 0; w < threadIdx.x >> 5; ++w)
+    {
+        run += wsum[w];
+    }
+#pragma unroll 8
+    for (uint32_t t = 0; t < used; ++t)
+    {
+        uint32_t const v                    = c[static_cast<uint64_t>(t) * 256];
+        c[static_cast<uint64_t>(t) * 256] = run;
+        run += v;
+    }
+}
+
+// grid (tiles, columns): the tile's keys to their places.
+__global__ void __launch_bounds__(k_sort_threads)
+    sort_scatter_kernel(uint32_t const *__restrict__ src, uint32_t *__restrict__ dst, uint64_t n,
+                        uint32_t const *__restrict__ counts, uint32_t shift,
+                        uint32_t const *__restrict__ tc)
+{
+    __shared__ uint16_t wc[k_sort_warps][256];
+    __shared__ uint32_t base[256];
+    uint32_t const      m  = counts[blockIdx.y];
+    uint64_t const      i0 = static_cast<uint64_t>(blockIdx.x) * k_sort_tile;
+    if (i0 >= m)
+    {
+        return;
+    }
+    uint32_t const  lane = threadIdx.x & 31u;
+    uint32_t const  w    = threadIdx.x >> 5;
+    uint32_t const *k    = src + (static_cast<uint64_t>(blockIdx.y) * n);
+    uint64_t const  w0   = i0 + (w * (k_sort_steps * 32));
+    for (uint32_t d = lane; d < 256; d += 32)
+    {
+        wc[w][d] = 0;
+    }
+    uint32_t key[k_sort_steps];
+    uint32_t rank[k_sort_steps];
+#pragma unroll
+    for (uint32_t st = 0; st < k_sort_steps; ++st)
+    {
+        uint64_t const i = w0 + (st * 32) + lane;
+        key[st]          = i < m ? k[i] : 0u;
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t st = 0; st < k_sort_steps; ++st)
+    {
+        bool const     ok    = w0 + (st * 32) + lane < m;
+        uint32_t const d     = (key[st] >> shift) & 0xFFu;
+        uint32_t       peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+        for (uint32_t b = 0; b < 8; ++b)
         {
-            uint32_t run = 0;
-            for (uint32_t d = 0; d < 256; ++d)
-            {
-                base[d] = run;
-                run += hist[d];
-            }
+            uint32_t const bit = (d >> b) & 1u;
+            peers &= __ballot_sync(0xFFFFFFFFu, bit != 0) ^ (bit - 1u);
         }
-        __syncthreads();
-        for (uint32_t t0 = 0; t0 < m; t0 += k_cut_threads)
+        uint32_t const lt = __popc(peers & ((1u << lane) - 1u));
+        uint32_t       at = 0;
+        if (ok)
         {
-            for (uint32_t x = t; x < (k_cut_threads / 32) * 256; x += k_cut_threads)
-            {
-                wc[x / 256][x % 256] = 0;
-            }
-            __syncthreads();
-            uint32_t const i     = t0 + t;
-            bool const     ok    = i < m;
-            uint32_t const key   = ok ? src[i] : 0u;
-            uint32_t const d     = (key >> shift) & 0xFFu;
-            // lanes with the same digit, in lane order (an idle lane only
-            // matches itself)
-            uint32_t const peers = __match_any_sync(0xFFFFFFFFu, ok ? d : 256u + lane);
-            uint32_t const r     = __popc(peers & ((1u << lane) - 1u));
-            if (ok && r == 0)
-            {
-                wc[w][d] = static_cast<uint16_t>(__popc(peers));
-            }
-            __syncthreads();
-            if (t < 256)
-            {
-                uint32_t run = 0;
-                for (uint32_t x = 0; x < k_cut_threads / 32; ++x)
-                {
-                    uint32_t const c = wc[x][t];
-                    wc[x][t]         = static_cast<uint16_t>(run);
-                    run += c;
-                }
-                tot[t] = run;
-            }
-            __syncthreads();
-            if (ok)
-            {
-                dst[base[d] + wc[w][d] + r] = key;
-            }
-            __syncthreads();
-            if (t < 256)
-            {
-                base[t] += tot[t];
-            }
-            __syncthreads();
+            at = wc[w][d];
         }
-        uint32_t *x = src;
-        src         = dst;
-        dst         = x;
+        __syncwarp();
+        if (ok && lt == 0)
+        {
+            wc[w][d] = static_cast<uint16_t>(at + __popc(peers));
+        }
+        __syncwarp();
+        rank[st] = at + lt;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256)
+    {
+        uint32_t run = 0;
+#pragma unroll
+        for (uint32_t x = 0; x < k_sort_warps; ++x)
+        {
+            uint32_t const c   = wc[x][threadIdx.x];
+            wc[x][threadIdx.x] = static_cast<uint16_t>(run);
+            run += c;
+        }
+        base[threadIdx.x] =
+            tc[(((static_cast<uint64_t>(blockIdx.y) * gridDim.x) + blockIdx.x) * 256) + threadIdx.x];
+    }
+    __syncthreads();
+    uint32_t *out = dst + (static_cast<uint64_t>(blockIdx.y) * n);
+#pragma unroll
+    for (uint32_t st = 0; st < k_sort_steps; ++st)
+    {
+        if (w0 + (st * 32) + lane < m)
+        {
+            uint32_t const d                 = (key[st] >> shift) & 0xFFu;
+            out[base[d] + wc[w][d] + rank[st]] = key[st];
+        }
     }
 }
 
@@ -241,27 +329,50 @@ __global__ void __launch_bounds__(k_cut_threads)
     float              *out    = cuts + (static_cast<uint64_t>(col) * max_bin);
     uint32_t const      budget = max_bin - 2;
     // the runs of equal values: starts in order (value(i - 1) < value(i))
-    uint32_t done = 0;
-    for (uint32_t t0 = 0; t0 < m; t0 += k_cut_threads)
+    // (a thread takes eight consecutive values at a time)
+    constexpr uint32_t each = 8;
+    uint32_t           done = 0;
+    for (uint64_t t0 = 0; t0 < m; t0 += k_cut_threads * each)
     {
-        uint32_t const i    = t0 + t;
-        bool const     head = i < m && (i == 0 || value_of(k[i - 1]) < value_of(k[i]));
-        uint32_t const mask = __ballot_sync(0xFFFFFFFFu, head);
-        if (lane == 0)
+        uint64_t const i0   = t0 + (t * each);
+        uint32_t       mask = 0;
+        float          prev = i0 > 0 && i0 < m ? value_of(k[i0 - 1]) : 0.0F;
+#pragma unroll
+        for (uint32_t q = 0; q < each; ++q)
         {
-            wsum[w] = __popc(mask);
+            if (i0 + q < m)
+            {
+                float const v = value_of(k[i0 + q]);
+                mask |= i0 + q == 0 || prev < v ? 1u << q : 0u;
+                prev = v;
+            }
+        }
+        uint32_t const heads = __popc(mask);
+        uint32_t       inc   = heads;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1)
+        {
+            uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o)
+            {
+                inc += y;
+            }
+        }
+        if (lane == 31)
+        {
+            wsum[w] = inc;
         }
         __syncthreads();
-        uint32_t before = 0;
+        uint32_t before = inc - heads;
         uint32_t total  = 0;
         for (uint32_t x = 0; x < k_cut_threads / 32; ++x)
         {
             before += x < w ? wsum[x] : 0u;
             total += wsum[x];
         }
-        if (head)
+        for (; mask != 0; mask &= mask - 1)
         {
-            st[done + before + __popc(mask & ((1u << lane) - 1u))] = i;
+            st[done + before++] = static_cast<uint32_t>(i0) + __ffs(mask) - 1;
         }
         done += total;
         __syncthreads();
@@ -309,13 +420,13 @@ __global__ void __launch_bounds__(k_cut_threads)
         }
         return;
     }
-    if (t != 0)
-    {
-        return;
-    }
     uint32_t c = 0;
     if (static_cast<double>(s_maxrun) >= mean_bin)
     {
+        if (t != 0)
+        {
+            return;
+        }
         // greedy_weighted_cuts over the runs
         uint64_t n_big   = 0;
         uint64_t big_sum = 0;
@@ -367,16 +478,39 @@ __global__ void __launch_bounds__(k_cut_threads)
     }
     else
     {
-        // the quantile stride over the sorted values
-        uint64_t const q    = (static_cast<uint64_t>(m) + budget) / (budget + 1);
-        uint64_t const step = q > 0 ? q : 1;
-        for (uint64_t x = step; x < m; x += step)
+        // the quantile stride over the sorted values: fetched by every thread,
+        // then one drops the repeated ones
+        __shared__ float v_s[k_cut_threads];
+        uint64_t const   q    = (static_cast<uint64_t>(m) + budget) / (budget + 1);
+        uint64_t const   step = q > 0 ? q : 1;
+        float            last = 0.0F;
+        for (uint64_t x0 = step; x0 < m; x0 += step * k_cut_threads)
         {
-            float const v = value_of(k[x]);
-            if (c == 0 || out[c - 1] < v)
+            uint64_t const x = x0 + (step * t);
+            if (x < m)
             {
-                out[c++] = v;
+                v_s[t] = value_of(k[x]);
             }
+            __syncthreads();
+            if (t == 0)
+            {
+                uint32_t const here = static_cast<uint32_t>(
+                    min(static_cast<uint64_t>(k_cut_threads), (m - x0 + step - 1) / step));
+                for (uint32_t i = 0; i < here; ++i)
+                {
+                    float const v = v_s[i];
+                    if (c == 0 || last < v)
+                    {
+                        out[c++] = v;
+                        last     = v;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (t != 0)
+        {
+            return;
         }
     }
     if (c == 0 || out[c - 1] < FLT_MAX)
@@ -389,7 +523,7 @@ __global__ void __launch_bounds__(k_cut_threads)
 
 struct Scratch
 {
-    void *p[7] = {};
+    void *p[2] = {};
     ~Scratch()
     {
         for (void *q : p)
@@ -427,7 +561,7 @@ extern "C" int bb_fit_cuts(float const *S, uint64_t n_rows, uint32_t n_feats, in
         uint64_t const n = std::max<uint64_t>(n_rows, 1);
         // columns per group: keys twice and the run starts, 12 bytes per value
         uint32_t const group = static_cast<uint32_t>(std::max<uint64_t>(
-            1, std::min<uint64_t>(n_feats, k_cut_mem / (12 * n))));
+            1, std::min<uint64_t>({n_feats, k_cut_mem / (12 * n), 65535}))); // (a grid's rows)
         Scratch        sc;
         size_t const   s_bytes = static_cast<size_t>(n_rows) * n_feats * sizeof(float);
         float const   *Sd      = S;
@@ -437,18 +571,22 @@ extern "C" int bb_fit_cuts(float const *S, uint64_t n_rows, uint32_t n_feats, in
             check(cudaMemcpy(sc.p[0], S, s_bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
             Sd = static_cast<float const *>(sc.p[0]);
         }
-        check(cudaMalloc(&sc.p[1], static_cast<size_t>(group) * n * 4), "cudaMalloc");
-        check(cudaMalloc(&sc.p[2], static_cast<size_t>(group) * n * 4), "cudaMalloc");
-        check(cudaMalloc(&sc.p[3], static_cast<size_t>(group) * n * 4), "cudaMalloc");
-        check(cudaMalloc(&sc.p[4], static_cast<size_t>(group) * max_bin * 4), "cudaMalloc");
-        check(cudaMalloc(&sc.p[5], static_cast<size_t>(group) * 4), "cudaMalloc");
-        check(cudaMalloc(&sc.p[6], static_cast<size_t>(group) * 4), "cudaMalloc");
-        auto *ka    = static_cast<uint32_t *>(sc.p[1]);
-        auto *kb    = static_cast<uint32_t *>(sc.p[2]);
-        auto *st    = static_cast<uint32_t *>(sc.p[3]);
-        auto *cd    = static_cast<float *>(sc.p[4]);
-        auto *cn    = static_cast<uint32_t *>(sc.p[5]); // values per column
-        auto *nc    = static_cast<uint32_t *>(sc.p[6]); // cuts per column
+        // one allocation: keys twice, run starts, tile counts, cuts, and the
+        // columns' values and cuts
+        uint32_t const tiles = ceil_div(n, k_sort_tile);
+        size_t const   per   = ((static_cast<size_t>(group) * n * 4) + 255) & ~size_t{255};
+        size_t const   t_bytes = static_cast<size_t>(group) * tiles * 256 * 4;
+        size_t const   c_bytes = ((static_cast<size_t>(group) * max_bin * 4) + 255) & ~size_t{255};
+        size_t const   g_bytes = ((static_cast<size_t>(group) * 4) + 255) & ~size_t{255};
+        check(cudaMalloc(&sc.p[1], (3 * per) + t_bytes + c_bytes + (2 * g_bytes)), "cudaMalloc");
+        auto *mem   = static_cast<unsigned char *>(sc.p[1]);
+        auto *ka    = reinterpret_cast<uint32_t *>(mem);
+        auto *kb    = reinterpret_cast<uint32_t *>(mem + per);
+        auto *st    = reinterpret_cast<uint32_t *>(mem + (2 * per));
+        auto *tc    = reinterpret_cast<uint32_t *>(mem + (3 * per));
+        auto *cd    = reinterpret_cast<float *>(mem + (3 * per) + t_bytes);
+        auto *cn    = reinterpret_cast<uint32_t *>(mem + (3 * per) + t_bytes + c_bytes);
+        auto *nc    = reinterpret_cast<uint32_t *>(mem + (3 * per) + t_bytes + c_bytes + g_bytes);
         std::vector<float>    hc(static_cast<size_t>(group) * max_bin);
         std::vector<uint32_t> hn(group);
         uint32_t              at = 0;
@@ -462,8 +600,16 @@ extern "C" int bb_fit_cuts(float const *S, uint64_t n_rows, uint32_t n_feats, in
                 dim3 const grid(ceil_div(n_rows, k_tile_rows_c), ceil_div(nf, k_tile_feats_c));
                 gather_keys_kernel<<<grid, k_tile_rows_c>>>(Sd, n_rows, n_feats, f0, nf, ka, cn);
                 check(cudaGetLastError(), "gather_keys_kernel");
-                sort_keys_kernel<<<nf, k_cut_threads>>>(ka, kb, n, cn);
-                check(cudaGetLastError(), "sort_keys_kernel");
+                dim3 const tg(tiles, nf);
+                for (uint32_t shift = 0; shift < 32; shift += 8)
+                {
+                    uint32_t const *from = (shift & 8) == 0 ? ka : kb;
+                    uint32_t       *to   = (shift & 8) == 0 ? kb : ka;
+                    sort_count_kernel<<<tg, k_sort_threads>>>(from, n, cn, shift, tc);
+                    sort_scan_kernel<<<nf, 256>>>(cn, tc, tiles);
+                    sort_scatter_kernel<<<tg, k_sort_threads>>>(from, to, n, cn, shift, tc);
+                }
+                check(cudaGetLastError(), "sort kernels");
             }
             column_cuts_kernel<<<nf, k_cut_threads>>>(ka, n, cn, st, max_bin, cd, nc);
             check(cudaGetLastError(), "column_cuts_kernel");
