@@ -44,6 +44,18 @@ void set_last_error(char const *msg);
 #define BB_CHECK(call) ::bb::check((call), #call)
 #define BB_LAUNCH(what) ::bb::check(cudaGetLastError(), what)
 
+// Lets a kernel take all the dynamic shared memory its static arrays leave.
+// The limit is the kernel's, shared by every object that launches it: it is
+// always set to this one value, so that an object with smaller features does
+// not lower it under the launches of another.
+template <typename F> void allow_smem(F *kern)
+{
+    cudaFuncAttributes a{};
+    BB_CHECK(cudaFuncGetAttributes(&a, kern));
+    BB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>((227 * 1024) - a.sharedSizeBytes)));
+}
+
 // Programmatic dependent launch. A kernel launched with the programmatic
 // stream-serialization attribute may be scheduled while the kernel before it
 // in the stream still runs; its first statement waits for that kernel's

@@ -5179,35 +5179,16 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
             throw ConfigError("grower: quantised histograms of this many bins exceed "
                               "shared memory; lower bin_mapper.max_bin");
         }
-        BB_CHECK(cudaFuncSetAttribute(qhist_kernel<uint16_t>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(qsmem)));
-        BB_CHECK(cudaFuncSetAttribute(qhist_kernel<uint16_t, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(qsmem)));
-        BB_CHECK(cudaFuncSetAttribute(qhist_kernel<uint16_t, false, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(qsmem)));
-        BB_CHECK(cudaFuncSetAttribute(qhist_kernel<uint8_t, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(static_cast<size_t>(32) * max_nb_ * 8)));
-        size_t const tsmem = k_tsmem;
-        BB_CHECK(cudaFuncSetAttribute(qhist_t_kernel<false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(tsmem)));
-        BB_CHECK(cudaFuncSetAttribute(qhist_t_kernel<true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(tsmem)));
-        // the summing walk's accumulator copies at depth 8
-        int const wsmem = static_cast<int>((size_t{2} << 8) * k_wsum_copies * 8);
-        BB_CHECK(cudaFuncSetAttribute(walk_sum_kernel<true, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
-        BB_CHECK(cudaFuncSetAttribute(walk_sum_kernel<true, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
-        BB_CHECK(cudaFuncSetAttribute(walk_sum_kernel<false, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
-        BB_CHECK(cudaFuncSetAttribute(walk_sum_kernel<false, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
+        allow_smem(qhist_kernel<uint16_t>);
+        allow_smem(qhist_kernel<uint16_t, true>);
+        allow_smem(qhist_kernel<uint16_t, false, true>);
+        allow_smem(qhist_kernel<uint8_t, true>);
+        allow_smem(qhist_t_kernel<false>);
+        allow_smem(qhist_t_kernel<true>);
+        allow_smem(walk_sum_kernel<true, false>);
+        allow_smem(walk_sum_kernel<true, true>);
+        allow_smem(walk_sum_kernel<false, false>);
+        allow_smem(walk_sum_kernel<false, true>);
     }
     else
     {
@@ -5227,22 +5208,13 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     {
         throw ConfigError("grower: bins per feature exceed the shared-memory budget");
     }
-    BB_CHECK(cudaFuncSetAttribute(find_kernel<false>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(find_smem)));
-    BB_CHECK(cudaFuncSetAttribute(find_kernel<true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(find_smem)));
+    allow_smem(find_kernel<false>);
+    allow_smem(find_kernel<true>);
     // the level finder prefixes up to 16 nodes at a time in shared memory
     lgroup_ = static_cast<uint32_t>(std::min<size_t>(
         k_lfind_thr / 32, std::max<size_t>(1, (192 * 1024) / (max_nb_ * sizeof(double2)))));
-    size_t const lsmem = static_cast<size_t>(lgroup_) * max_nb_ * sizeof(double2);
-    BB_CHECK(cudaFuncSetAttribute(level_find_kernel<false>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(lsmem)));
-    BB_CHECK(cudaFuncSetAttribute(level_find_kernel<true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(lsmem)));
+    allow_smem(level_find_kernel<false>);
+    allow_smem(level_find_kernel<true>);
     if (!quant_)
     {
         if (max_nb_ > k_exact_bins)
@@ -5252,14 +5224,9 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
         // four features in flight, or two where a group's counters take more
         // (features of several thousand bins)
         xgroups_ = sort_smem(max_nb_, k_xgroups) <= 226 * 1024 ? k_xgroups : 2;
-        auto allow = [&](auto kern)
-        {
-            BB_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(sort_smem(max_nb_, xgroups_))));
-        };
-        plane_.u8 ? allow(sort_kernel<uint8_t, k_xgroups>)
-                  : (xgroups_ == 2 ? allow(sort_kernel<uint16_t, 2>)
-                                   : allow(sort_kernel<uint16_t, k_xgroups>));
+        allow_smem(sort_kernel<uint8_t, k_xgroups>);
+        allow_smem(sort_kernel<uint16_t, k_xgroups>);
+        allow_smem(sort_kernel<uint16_t, 2>);
     }
     BB_CHECK(cudaEventCreate(&pev_[0]));
     BB_CHECK(cudaEventCreate(&pev_[1]));

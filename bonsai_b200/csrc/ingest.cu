@@ -436,10 +436,7 @@ void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream, flo
     auto const kern16 = pad ? bin_apply_kernel<uint16_t, true> : bin_apply_kernel<uint16_t, false>;
     if (!by_value)
     {
-        BB_CHECK(cudaFuncSetAttribute(p.u8 ? reinterpret_cast<void const *>(kern8)
-                                           : reinterpret_cast<void const *>(kern16),
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
+        p.u8 ? allow_smem(kern8) : allow_smem(kern16);
     }
     bool const vec4 = (F % 4) == 0 &&
                       (!x_on_device || (reinterpret_cast<uintptr_t>(X) % 16) == 0);

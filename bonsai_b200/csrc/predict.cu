@@ -802,13 +802,6 @@ void plan_check_plane(bb_predict_plan const &pl, Plane const &p)
          "bb_predict_plan: the plane's bin counts differ from the plan's");
 }
 
-template <typename F> void set_smem(F *kern, size_t smem)
-{
-    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem)),
-          "cudaFuncSetAttribute");
-}
-
 using HeapFn = void (*)(uint4 const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
                         uint32_t, uint32_t, uint32_t, float, float, float *);
 
@@ -935,7 +928,7 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
     // of 512
     size_t const smem = (size_t{1024} * pl.n_tiles * 64) + (size_t{chunk} * tree_bytes);
     HeapFn const fn   = heap_fn(pl.u8, pl.depth);
-    set_smem(fn, smem);
+    allow_smem(fn);
     // one wave of resident CTAs, each over an equal run of rows
     int occ = 0;
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 512, smem),
@@ -1000,7 +993,7 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
             size_t const per_row = lane_smem(D, n_tiles, 1) - lane_smem(D, n_tiles, 0);
             pl->lane_rows        = static_cast<uint32_t>(std::min<size_t>(
                 k_lane_threads, (k_lane_smem - lane_smem(D, n_tiles, 0)) / per_row));
-            set_smem(lane_fn(p.u8, D), k_lane_smem);
+            allow_smem(lane_fn(p.u8, D));
             pl->vals.alloc(size_t{k_few_rows} * n_trees * sizeof(float));
         }
         else

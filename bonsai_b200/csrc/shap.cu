@@ -1141,9 +1141,7 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
     pl->n_trees     = static_cast<uint32_t>(views.size());
     pl->room        = tb.room;
     size_t const sm = tree_smem(F, tb.room, pl->warps);
-    check(cudaFuncSetAttribute(tree_fn(D), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(k_tree_smem)),
-          "cudaFuncSetAttribute");
+    allow_smem(tree_fn(D));
     for (uint32_t c = 0; c < 4; ++c)
     {
         cudaLaunchAttribute at{};
@@ -1394,9 +1392,7 @@ uint32_t shap_launch(bb_shap_plan &pl, Plane const &p, double *out, cudaStream_t
     };
     // one wave of resident CTAs is the target
     int occ = 0;
-    check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem_of(1))),
-          "cudaFuncSetAttribute");
+    allow_smem(fn);
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, static_cast<int>(T), smem_of(1)),
           "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     uint32_t const target = static_cast<uint32_t>(std::max(occ, 1)) * k_sms;
@@ -1430,9 +1426,6 @@ uint32_t shap_launch(bb_shap_plan &pl, Plane const &p, double *out, cudaStream_t
         pl.ws.grow(static_cast<size_t>(splits) * n * (F + 1) * sizeof(double), pl.ws_cap);
         ws = pl.ws.as<double>();
     }
-    check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem)),
-          "cudaFuncSetAttribute");
     dim3 const grid(row_blks, splits);
     fn<<<grid, T, smem, s>>>(p.u8 ? static_cast<uint8_t const *>(p.bins) : nullptr,
                              p.u8 ? nullptr : static_cast<uint16_t const *>(p.bins), p.n_pad,
