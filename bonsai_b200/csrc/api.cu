@@ -308,7 +308,8 @@ __global__ void advance_kernel(uint32_t *round, uint32_t step)
 template <typename T> T *dmalloc(size_t n)
 {
     void *p = nullptr;
-    BB_CHECK(cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(T)));
+    MemPool::with_trim([&] { return cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(T)); },
+                       "cudaMalloc");
     return static_cast<T *>(p);
 }
 
@@ -317,33 +318,20 @@ struct TreeStore
     uint32_t cap  = 0;
     uint32_t n    = 0;
     TreeOut  t{};
-    void     alloc(uint32_t capacity, uint32_t slots)
+    void     want(Arena &mem, uint32_t capacity, uint32_t slots)
     {
         cap                = capacity;
         n                  = slots;
         size_t const total = static_cast<size_t>(capacity) * slots;
-        t.feature          = dmalloc<uint32_t>(total);
-        t.value            = dmalloc<float>(total);
-        t.left             = dmalloc<uint32_t>(total);
-        t.right            = dmalloc<uint32_t>(total);
-        t.default_left     = dmalloc<uint8_t>(total);
-        t.gain             = dmalloc<float>(total);
-        t.cover            = dmalloc<float>(total);
-        t.split_bin        = dmalloc<uint32_t>(total);
-        t.meta             = dmalloc<uint32_t>(3 * static_cast<size_t>(slots));
-    }
-    void release()
-    {
-        void *ps[] = {t.feature, t.value,     t.left, t.right, t.default_left,
-                      t.gain,    t.cover,     t.split_bin, t.meta};
-        for (void *p : ps)
-        {
-            if (p != nullptr)
-            {
-                cudaFree(p);
-            }
-        }
-        t = {};
+        mem.want<uint32_t>(t.feature, total);
+        mem.want<float>(t.value, total);
+        mem.want<uint32_t>(t.left, total);
+        mem.want<uint32_t>(t.right, total);
+        mem.want<uint8_t>(t.default_left, total);
+        mem.want<float>(t.gain, total);
+        mem.want<float>(t.cover, total);
+        mem.want<uint32_t>(t.split_bin, total);
+        mem.want<uint32_t>(t.meta, 3 * static_cast<size_t>(slots));
     }
     // slots [slot, slot + count), each array's entries back to back
     void download(uint32_t slot, uint32_t *feature, float *value, uint32_t *left,
@@ -812,6 +800,7 @@ struct bb_booster
 {
     bb::Plane const            *plane = nullptr;
     cudaStream_t                stream{};
+    bb::Arena                   mem; // every array but weights and the eval's
     int                         objective = 0;
     float                       lr        = 0.1F;
     float                       init      = 0.0F;
@@ -1187,30 +1176,6 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
         float const nn = static_cast<float>(n);
         b->init = cfg->objective == 0 ? sum / nn : std::log((sum / nn) / (1.0F - (sum / nn)));
     }
-    b->labels  = dmalloc<float>(n);
-    b->scores  = dmalloc<float>(n * K);
-    b->gh      = dmalloc<float2>(n * K);
-    b->rows    = dmalloc<uint32_t>(n);
-    b->leaf_id = dmalloc<uint32_t>(n);
-    b->round   = dmalloc<uint32_t>(1);
-    BB_CHECK(cudaMemcpyAsync(b->labels, labels, n * 4, cudaMemcpyHostToDevice, b->stream));
-    if (init_scores != nullptr)
-    {
-        BB_CHECK(cudaMemcpyAsync(b->scores, init_scores, n * 4, cudaMemcpyHostToDevice,
-                                 b->stream));
-    }
-    else
-    {
-        for (uint32_t k = 0; k < K; ++k)
-        {
-            fill_kernel<<<blocks(n), 256, 0, b->stream>>>(b->scores + (k * n),
-                                                          K > 1 ? b->init_k[k] : b->init, n);
-            BB_LAUNCH("fill_kernel");
-        }
-    }
-    iota_kernel<<<blocks(n), 256, 0, b->stream>>>(b->rows, n);
-    BB_LAUNCH("iota_kernel");
-    BB_CHECK(cudaMemsetAsync(b->round, 0, 4, b->stream));
     GrowConfig gc = grow_config(*cfg);
     gc.fit_rows   = red != nullptr ? total_rows : n; // a shard's cells hold the fit's sums
     if (feat_k > 0 && feat_k < p.n_feats)
@@ -1261,7 +1226,7 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
         L.grower->set_seed(cfg->seed);
         // tree numbers (the rounding stream): round-major, as one grower's are
         L.grower->set_tree_numbers(k, static_cast<uint32_t>(b->lanes.size()));
-        L.scratch.alloc(L.grower->max_nodes(), 1);
+        L.scratch.want(b->mem, L.grower->max_nodes(), 1);
     }
     if (red != nullptr)
     {
@@ -1275,15 +1240,40 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
         b->sampler = std::make_unique<RowSampler>(cfg->subsample, cfg->random_seed, n, K, dev,
                                                   external);
         uint64_t const words = b->sampler->words();
-        b->sbits = dmalloc<uint32_t>(words * K);
+        b->mem.want<uint32_t>(b->sbits, words * K);
         for (Lane &L : b->lanes)
         {
-            L.srows  = dmalloc<uint32_t>(n);
-            L.scount = dmalloc<uint32_t>(1);
-            L.sbsum  = dmalloc<uint32_t>(ceil_div(words, k_smp_block));
+            b->mem.want<uint32_t>(L.srows, n);
+            b->mem.want<uint32_t>(L.scount, 1);
+            b->mem.want<uint32_t>(L.sbsum, ceil_div(words, k_smp_block));
         }
     }
-    b->trees.alloc(b->lanes[0].grower->max_nodes(), max_trees * K); // round-major: r * K + k
+    b->mem.want<float>(b->labels, n);
+    b->mem.want<float>(b->scores, n * K);
+    b->mem.want<float2>(b->gh, n * K);
+    b->mem.want<uint32_t>(b->rows, n);
+    b->mem.want<uint32_t>(b->leaf_id, n);
+    b->mem.want<uint32_t>(b->round, 1);
+    b->trees.want(b->mem, b->lanes[0].grower->max_nodes(), max_trees * K); // round-major: r * K + k
+    b->mem.alloc(p.pool(), b->stream);
+    BB_CHECK(cudaMemcpyAsync(b->labels, labels, n * 4, cudaMemcpyHostToDevice, b->stream));
+    if (init_scores != nullptr)
+    {
+        BB_CHECK(cudaMemcpyAsync(b->scores, init_scores, n * 4, cudaMemcpyHostToDevice,
+                                 b->stream));
+    }
+    else
+    {
+        for (uint32_t k = 0; k < K; ++k)
+        {
+            fill_kernel<<<blocks(n), 256, 0, b->stream>>>(b->scores + (k * n),
+                                                          K > 1 ? b->init_k[k] : b->init, n);
+            BB_LAUNCH("fill_kernel");
+        }
+    }
+    iota_kernel<<<blocks(n), 256, 0, b->stream>>>(b->rows, n);
+    BB_LAUNCH("iota_kernel");
+    BB_CHECK(cudaMemsetAsync(b->round, 0, 4, b->stream));
     // a leafwise round reads every pop back to the host: it runs eagerly
     b->use_graph       = cfg->use_graph != 0 && b->lanes[0].grower->fuses_next();
     b->record_leaf_ids = cfg->record_leaf_ids != 0;
@@ -1391,7 +1381,7 @@ extern "C"
                                     cudaMemcpyHostToDevice));
                 BB_CHECK(cudaMemcpy(p.n_bins, nb.data(), n_feats * 4, cudaMemcpyHostToDevice));
                 size_t const bytes = static_cast<size_t>(n_feats) * p.n_pad * (p.u8 ? 1 : 2);
-                BB_CHECK(cudaMalloc(&p.bins, bytes));
+                p.bins = dmalloc<char>(bytes);
                 BB_CHECK(cudaMemset(p.bins, 0, bytes));
                 cudaStream_t s;
                 BB_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1468,7 +1458,7 @@ extern "C"
                 BB_CHECK(cudaMemcpy(p.n_bins, nb.data(), n_feats * 4, cudaMemcpyHostToDevice));
                 size_t const el    = p.u8 ? 1 : 2;
                 size_t const bytes = static_cast<size_t>(n_feats) * p.n_pad * el;
-                BB_CHECK(cudaMalloc(&p.bins, bytes));
+                p.bins = dmalloc<char>(bytes);
                 BB_CHECK(cudaMemset(p.bins, 0, bytes));
                 BB_CHECK(cudaMemcpy2D(p.bins, p.n_pad * el, bins, n_rows * el, n_rows * el,
                                       n_feats, cudaMemcpyHostToDevice));
@@ -1558,16 +1548,16 @@ extern "C"
                 BB_CHECK(cudaMemcpy(p.n_bins, q.n_bins, F * 4, cudaMemcpyDeviceToDevice));
                 uint64_t const cap_pad = ((max_rows + 63) / 64) * 64;
                 size_t const   el      = p.u8 ? 1 : 2;
-                BB_CHECK(cudaMalloc(&p.bins, static_cast<size_t>(F) * cap_pad * el));
+                p.bins = dmalloc<char>(static_cast<size_t>(F) * cap_pad * el);
                 BB_CHECK(cudaMemset(p.bins, 0, static_cast<size_t>(F) * cap_pad * el));
                 uint32_t const per = k_mirror_bytes / (p.u8 ? 1 : 2);
                 p.n_tiles          = (F + per - 1) / per;
-                BB_CHECK(cudaMalloc(&p.mirror,
-                                    static_cast<size_t>(p.n_tiles) * max_rows * k_mirror_bytes));
+                p.mirror = dmalloc<char>(static_cast<size_t>(p.n_tiles) * max_rows *
+                                         k_mirror_bytes);
                 // host rows go up through a staging buffer of at most 64 MB
                 uint64_t const row_bytes = static_cast<uint64_t>(F) * sizeof(float);
                 p.stage_rows             = stage_rows_for(F, max_rows);
-                BB_CHECK(cudaMalloc(&p.stage, p.stage_rows * row_bytes));
+                p.stage = reinterpret_cast<float *>(dmalloc<char>(p.stage_rows * row_bytes));
                 BB_CHECK(cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking));
                 *out = pl.release();
             });
@@ -2204,10 +2194,6 @@ extern "C"
                 cudaStreamSynchronize(L.stream);
             }
             L.grower.reset();
-            L.scratch.release();
-            cudaFree(L.srows);
-            cudaFree(L.scount);
-            cudaFree(L.sbsum);
             if (L.stream != b->stream)
             {
                 cudaStreamDestroy(L.stream);
@@ -2218,13 +2204,8 @@ extern "C"
         {
             cudaEventDestroy(b->fork);
         }
-        b->trees.release();
-        void *ps[] = {b->labels, b->scores, b->gh,     b->rows,   b->leaf_id, b->round,
-                      b->sbits,  b->weights};
-        for (void *p : ps)
-        {
-            cudaFree(p);
-        }
+        cudaFree(b->weights);
+        b->mem.release();
         cudaEventDestroy(b->ev0);
         cudaEventDestroy(b->ev1);
         cudaStreamDestroy(b->stream);
@@ -2258,13 +2239,22 @@ extern "C"
                 {
                     gh[i] = make_float2(grad[i], hess[i]);
                 }
-                float2   *d_gh  = dmalloc<float2>(n);
-                uint32_t *d_rows = dmalloc<uint32_t>(std::max<uint64_t>(m, 1));
-                uint32_t *d_leaf = dmalloc<uint32_t>(n);
-                float    *d_val  = dmalloc<float>(n);
+                float2   *d_gh   = nullptr;
+                uint32_t *d_rows = nullptr;
+                uint32_t *d_leaf = nullptr;
+                float    *d_val  = nullptr;
                 TreeStore ts;
+                Arena     mem;
                 try
                 {
+                    Grower g(p, grow_config(*cfg), selection(*cfg, p.n_feats),
+                             static_cast<uint32_t>(std::max<uint64_t>(m, 1)), s);
+                    mem.want<float2>(d_gh, n);
+                    mem.want<uint32_t>(d_rows, m);
+                    mem.want<uint32_t>(d_leaf, n);
+                    mem.want<float>(d_val, n);
+                    ts.want(mem, g.max_nodes(), 1);
+                    mem.alloc(p.pool(), s);
                     BB_CHECK(cudaMemcpyAsync(d_gh, gh.data(), n * 8, cudaMemcpyHostToDevice, s));
                     if (rows == nullptr)
                     {
@@ -2277,12 +2267,9 @@ extern "C"
                     }
                     // values via the fused score update on a zeroed buffer, lr = 1
                     BB_CHECK(cudaMemsetAsync(d_val, 0, n * 4, s));
-                    Grower g(p, grow_config(*cfg), selection(*cfg, p.n_feats),
-                             static_cast<uint32_t>(std::max<uint64_t>(m, 1)), s);
                     g.set_monotone(monotone(*cfg));
                     g.set_interaction(interaction(*cfg, p.n_feats));
                     g.set_seed(cfg->seed);
-                    ts.alloc(g.max_nodes(), 1);
                     g.grow(d_gh, d_rows, static_cast<uint32_t>(m), ts.t, d_leaf, d_val, 1.0F);
                     BB_CHECK(cudaStreamSynchronize(s));
                     ts.download(0, feature, value, left, right, default_left, gain, cover,
@@ -2300,19 +2287,11 @@ extern "C"
                 }
                 catch (...)
                 {
-                    ts.release();
-                    cudaFree(d_gh);
-                    cudaFree(d_rows);
-                    cudaFree(d_leaf);
-                    cudaFree(d_val);
+                    mem.release();
                     cudaStreamDestroy(s);
                     throw;
                 }
-                ts.release();
-                cudaFree(d_gh);
-                cudaFree(d_rows);
-                cudaFree(d_leaf);
-                cudaFree(d_val);
+                mem.release();
                 BB_CHECK(cudaStreamDestroy(s));
             });
     }

@@ -5077,9 +5077,9 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
 
     cudaStream_t   s     = stream_;
     uint32_t const nsets = std::max(1u, cfg_.sel_sets);
-    sel_base_      = dalloc<uint32_t>(static_cast<size_t>(nsets) * n_sel_, s);
-    cell_off_base_ = dalloc<uint32_t>(static_cast<size_t>(nsets) * (n_sel_ + 1), s);
-    sel_nb_base_   = dalloc<uint32_t>(static_cast<size_t>(nsets) * n_sel_, s);
+    arena_.want<uint32_t>(sel_base_, static_cast<size_t>(nsets) * n_sel_);
+    arena_.want<uint32_t>(cell_off_base_, static_cast<size_t>(nsets) * (n_sel_ + 1));
+    arena_.want<uint32_t>(sel_nb_base_, static_cast<size_t>(nsets) * n_sel_);
     {
         // the mirror tiles a selection can touch: all selected features (v
         // 0), and the first one alone (v 1: the last level builds only its
@@ -5102,76 +5102,69 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                 }
             }
             n_tiles_[v]       = cap;
-            tile_ids_base_[v] = dalloc<uint32_t>(static_cast<size_t>(nsets) * cap, s);
-            tile_j_base_[v]   = dalloc<int32_t>(static_cast<size_t>(nsets) * cap * per, s);
+            arena_.want<uint32_t>(tile_ids_base_[v], static_cast<size_t>(nsets) * cap);
+            arena_.want<int32_t>(tile_j_base_[v], static_cast<size_t>(nsets) * cap * per);
         }
     }
-    sets_h_.assign(nsets, sel_h_);
-    for (uint32_t k = 0; k < nsets; ++k)
-    {
-        write_tables(k, sel_h_, s);
-    }
-    use_set(0);
-    ctl_      = dalloc<Ctl>(1, s);
-    nodes_[0] = dalloc<Node>(max_front_, s);
-    nodes_[1] = dalloc<Node>(max_front_, s);
-    hist_[0]  = dalloc<float2>(static_cast<size_t>(max_front_) * total_cells_ * cw_, s);
+    arena_.want<Ctl>(ctl_, 1);
+    arena_.want<Node>(nodes_[0], max_front_);
+    arena_.want<Node>(nodes_[1], max_front_);
+    arena_.want<float2>(hist_[0], static_cast<size_t>(max_front_) * total_cells_ * cw_);
     // (leafwise uses the first buffer as its slot pool)
-    hist_[1]  = dalloc<float2>(static_cast<size_t>(cfg_.leaf ? 1 : max_front_) * total_cells_ * cw_,
-                               s);
-    cand_     = dalloc<Best>(static_cast<size_t>(max_front_) * n_sel_, s);
-    best_     = dalloc<Best>(max_front_, s);
-    pchunks_  = dalloc<Chunk>(max_pchunks_, s);
-    pleft_    = dalloc<uint32_t>(max_pchunks_, s);
-    dirs_     = dalloc<uint32_t>(static_cast<size_t>(max_pchunks_) * (k_part_rows / 32), s);
-    prbase_   = dalloc<uint32_t>(max_pchunks_, s);
-    dst_      = dalloc<uint32_t>(max_front_ + 1, s);
-    build_    = dalloc<uint32_t>(max_front_ * 2 + 2, s);
-    bpair_    = dalloc<uint32_t>(3 * max_front_, s);
-    bbase_    = dalloc<uint32_t>(max_front_ + 1, s);
-    brange_   = dalloc<uint32_t>(max_front_ + 2, s);
-    bchunks_  = dalloc<Chunk>(max_bchunks_, s);
+    arena_.want<float2>(hist_[1],
+                        static_cast<size_t>(cfg_.leaf ? 1 : max_front_) * total_cells_ * cw_);
+    arena_.want<Best>(cand_, static_cast<size_t>(max_front_) * n_sel_);
+    arena_.want<Best>(best_, max_front_);
+    arena_.want<Chunk>(pchunks_, max_pchunks_);
+    arena_.want<uint32_t>(pleft_, max_pchunks_);
+    arena_.want<uint32_t>(dirs_, static_cast<size_t>(max_pchunks_) * (k_part_rows / 32));
+    arena_.want<uint32_t>(prbase_, max_pchunks_);
+    arena_.want<uint32_t>(dst_, max_front_ + 1);
+    arena_.want<uint32_t>(build_, max_front_ * 2 + 2);
+    arena_.want<uint32_t>(bpair_, 3 * max_front_);
+    arena_.want<uint32_t>(bbase_, max_front_ + 1);
+    arena_.want<uint32_t>(brange_, max_front_ + 2);
+    arena_.want<Chunk>(bchunks_, max_bchunks_);
     // (leafwise: two halves of one buffer, a node's segment in either)
-    rows_[0]  = dalloc<uint32_t>(static_cast<size_t>(max_rows_) * (cfg_.leaf ? 2 : 1), s);
-    rows_[1]  = cfg_.leaf ? nullptr : dalloc<uint32_t>(max_rows_, s);
-    pcr_      = dalloc<uint32_t>(max_front_ + 2, s);
-    nbound_   = dalloc<double2>(std::max<uint32_t>(max_nodes_, k_walk_nodes), s);
-    heap_     = dalloc<uint2>(k_heap_slots, s);
-    leafmap_  = dalloc<uint16_t>(k_heap_slots + 1, s);
+    arena_.want<uint32_t>(rows_[0], static_cast<size_t>(max_rows_) * (cfg_.leaf ? 2 : 1));
+    if (!cfg_.leaf)
+    {
+        arena_.want<uint32_t>(rows_[1], max_rows_);
+    }
+    arena_.want<uint32_t>(pcr_, max_front_ + 2);
+    arena_.want<double2>(nbound_, std::max<uint32_t>(max_nodes_, k_walk_nodes));
+    arena_.want<uint2>(heap_, k_heap_slots);
+    arena_.want<uint16_t>(leafmap_, k_heap_slots + 1);
     if (cfg_.leaf)
     {
-        lout_      = dalloc<LeafOut>(1, s);
-        slot_of_   = dalloc<uint32_t>(2, s);
-        loop_      = dalloc<LeafLoop>(1, s);
-        cand_heap_ = dalloc<LeafCand>(max_front_ + 2, s);
-        leaves_    = dalloc<Node>(max_front_ + 2, s);
-        free_      = dalloc<uint32_t>(max_front_ + 2, s);
-        tree_dev_  = dalloc<TreeOut>(1, s);
-        leaf_tick_ = dalloc<uint32_t>(2, s);
-        BB_CHECK(cudaMemsetAsync(leaf_tick_, 0, 8, s));
+        arena_.want<LeafOut>(lout_, 1);
+        arena_.want<uint32_t>(slot_of_, 2);
+        arena_.want<LeafLoop>(loop_, 1);
+        arena_.want<LeafCand>(cand_heap_, max_front_ + 2);
+        arena_.want<Node>(leaves_, max_front_ + 2);
+        arena_.want<uint32_t>(free_, max_front_ + 2);
+        arena_.want<TreeOut>(tree_dev_, 1);
+        arena_.want<uint32_t>(leaf_tick_, 2);
         BB_CHECK(cudaMallocHost(&lout_h_, sizeof(LeafLoop)));
     }
-    nleft_    = dalloc<uint32_t>(max_front_ + 1, s);
-    nright_   = dalloc<uint32_t>(max_front_ + 1, s);
-    dtree_    = dalloc<uint32_t>(1, s);
-    BB_CHECK(cudaMemsetAsync(dtree_, 0, 4, s));
+    arena_.want<uint32_t>(nleft_, max_front_ + 1);
+    arena_.want<uint32_t>(nright_, max_front_ + 1);
+    arena_.want<uint32_t>(dtree_, 1);
     if (quant_)
     {
-        absmax_  = dalloc<uint32_t>(2, s);
-        qscale_  = dalloc<double2>(1, s);
+        arena_.want<uint32_t>(absmax_, 2);
+        arena_.want<double2>(qscale_, 1);
         // +2: the histogram copies whole 4-byte words of codes
-        qgh8_    = dalloc<uint16_t>((max_rows_ > plane_.n_rows ? max_rows_ : plane_.n_rows) + 2, s);
+        arena_.want<uint16_t>(qgh8_, (max_rows_ > plane_.n_rows ? max_rows_ : plane_.n_rows) + 2);
         if (wide_codes_)
         {
-            qgh16_ = dalloc<uint32_t>((max_rows_ > plane_.n_rows ? max_rows_ : plane_.n_rows) + 1,
-                                      s);
+            arena_.want<uint32_t>(qgh16_, (max_rows_ > plane_.n_rows ? max_rows_ : plane_.n_rows) + 1);
         }
-        partial_ = dalloc<double2>(max_pchunks_, s);
-        btot_    = dalloc<int64_t>(2 * static_cast<size_t>(max_front_), s);
-        done_    = dalloc<uint32_t>(1, s);
-        wacc_    = dalloc<unsigned long long>(2 * k_walk_nodes, s);
-        leaf16_  = dalloc<uint16_t>(plane_.n_rows, s);
-        BB_CHECK(cudaMemsetAsync(done_, 0, 4, s));
+        arena_.want<double2>(partial_, max_pchunks_);
+        arena_.want<int64_t>(btot_, 2 * static_cast<size_t>(max_front_));
+        arena_.want<uint32_t>(done_, 1);
+        arena_.want<unsigned long long>(wacc_, 2 * k_walk_nodes);
+        arena_.want<uint16_t>(leaf16_, plane_.n_rows);
         uint32_t const per = k_mirror_bytes / (plane_.u8 ? 1 : 2);
         size_t const qsmem = static_cast<size_t>(per) * max_nb_ * 8;
         if (qsmem > 200 * 1024)
@@ -5192,14 +5185,30 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     }
     else
     {
-        coff_    = dalloc<uint16_t>(static_cast<size_t>(max_bchunks_) * n_sel_ * cell_stride_, s);
+        arena_.want<uint16_t>(coff_, static_cast<size_t>(max_bchunks_) * n_sel_ * cell_stride_);
         // every built row once, and each chunk's padding
         p_stride_ = ((uint64_t{max_rows_} + 1) & ~uint64_t{1}) +
                     (uint64_t{max_bchunks_} * (chunk_pads(max_nb_) + 2));
-        payload_  = dalloc<float2>(n_sel_ * p_stride_, s);
+        arena_.want<float2>(payload_, n_sel_ * p_stride_);
     }
-    scale_ = dalloc<float2>(1, s);
+    arena_.want<float2>(scale_, 1);
+    arena_.alloc(plane_.pool(), s);
+    sets_h_.assign(nsets, sel_h_);
+    for (uint32_t k = 0; k < nsets; ++k)
+    {
+        write_tables(k, sel_h_, s);
+    }
+    use_set(0);
     BB_CHECK(cudaMemsetAsync(scale_, 0, sizeof(float2), s));
+    BB_CHECK(cudaMemsetAsync(dtree_, 0, 4, s));
+    if (cfg_.leaf)
+    {
+        BB_CHECK(cudaMemsetAsync(leaf_tick_, 0, 8, s));
+    }
+    if (quant_)
+    {
+        BB_CHECK(cudaMemsetAsync(done_, 0, 4, s));
+    }
     BB_CHECK(cudaStreamSynchronize(s));
 
     // dynamic shared memory ceilings
@@ -5320,32 +5329,15 @@ void Grower::use_set(uint32_t set)
 
 Grower::~Grower()
 {
-    void *ptrs[] = {sel_base_, cell_off_base_, sel_nb_base_, ctl_, nodes_[0], nodes_[1],
-                    hist_[0], hist_[1],  cand_,    best_,     pchunks_,    pleft_,
-                    prbase_,  dst_,      build_,   bpair_,    brange_,     bchunks_,
-                    coff_,    payload_, rows_[0],  rows_[1],    scale_,
-                    absmax_,  qgh_,      pcr_,     nleft_,    mono_,       qscale_,
-                    qgh8_,    partial_,  dtree_,   tile_ids_base_[0], tile_ids_base_[1],
-                    tile_j_base_[0], tile_j_base_[1], bbase_, dirs_, btot_, done_, wacc_,
-                    leaf16_,  nbound_,  gleft_,   qgh16_,   fgroups_, heap_, leafmap_, nright_};
-    for (void *p : ptrs)
+    for (void *p : {static_cast<void *>(mono_), static_cast<void *>(fgroups_),
+                    static_cast<void *>(gleft_)})
     {
         if (p != nullptr)
         {
             cudaFreeAsync(p, stream_);
         }
     }
-    if (lout_ != nullptr)
-    {
-        cudaFreeAsync(lout_, stream_);
-        cudaFreeAsync(slot_of_, stream_);
-        cudaFreeAsync(loop_, stream_);
-        cudaFreeAsync(cand_heap_, stream_);
-        cudaFreeAsync(leaves_, stream_);
-        cudaFreeAsync(free_, stream_);
-        cudaFreeAsync(tree_dev_, stream_);
-        cudaFreeAsync(leaf_tick_, stream_);
-    }
+    arena_.release();
     if (loop_x_ != nullptr)
     {
         cudaGraphExecDestroy(loop_x_);

@@ -6,6 +6,7 @@
 // static shapes (capturable as a CUDA graph) and no host round trip.
 #pragma once
 
+#include "arena.cuh"
 #include "common.cuh"
 #include "ingest.cuh"
 
@@ -286,7 +287,9 @@ class Grower
     double                fix_unit_    = 274877906944.0; // fixed-point leaf-sum unit (2^38 at
                                                          // up to 2^24 rows, halved per doubling)
 
-    // device
+    // device (arena_ holds every array but the lazily made mono_, fgroups_ and
+    // gleft_)
+    Arena     arena_;
     uint32_t *sel_      = nullptr; // selected feature ids
     uint32_t *cell_off_ = nullptr; // per selected feature, its first cell
     uint32_t *sel_nb_   = nullptr; // per selected feature, its bin count
@@ -318,7 +321,6 @@ class Grower
     float2 const *gh_cur_ = nullptr;
     std::vector<uint32_t> off_h_;
     // quantised form
-    int32_t  *qgh_      = nullptr; // per row, packed (g, h) integers
     float2   *scale_    = nullptr;
     uint32_t *absmax_   = nullptr; // max |g| and max h, as float bits
     double2  *qscale_   = nullptr; // (scale_g, scale_h) in FP64

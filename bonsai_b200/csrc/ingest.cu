@@ -365,7 +365,7 @@ void alloc_mirror(Plane &p)
     uint32_t const per = k_mirror_bytes / (p.u8 ? 1 : 2);
     p.n_tiles          = (p.n_feats + per - 1) / per;
     size_t const bytes = static_cast<size_t>(p.n_tiles) * p.n_rows * k_mirror_bytes;
-    BB_CHECK(cudaMalloc(&p.mirror, bytes));
+    MemPool::with_trim([&] { return cudaMalloc(&p.mirror, bytes); }, "cudaMalloc");
 }
 
 void build_mirror(Plane &p, cudaStream_t stream)

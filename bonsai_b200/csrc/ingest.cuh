@@ -9,6 +9,7 @@
 // consecutive rows as one 16-byte store.
 #pragma once
 
+#include "arena.cuh"
 #include "common.cuh"
 
 namespace bb
@@ -42,6 +43,16 @@ struct Plane
     float       *stage      = nullptr;
     uint64_t     stage_rows = 0;
     cudaStream_t stream     = nullptr;
+    // the device's pool, held from the plane's first fit on
+    std::shared_ptr<MemPool> pool() const
+    {
+        std::call_once(pool_once_, [&] { pool_ = MemPool::of(device); });
+        return pool_;
+    }
+
+  private:
+    mutable std::once_flag           pool_once_;
+    mutable std::shared_ptr<MemPool> pool_;
 };
 
 // owned_stage (optional): a device staging buffer of owned_rows rows the
