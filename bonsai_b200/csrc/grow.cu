@@ -4964,7 +4964,6 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                uint32_t max_root_rows, cudaStream_t stream)
     : plane_(plane), cfg_(cfg), sel_h_(std::move(selected)), stream_(stream)
 {
-    pdl_ = plane_.n_rows >= (uint64_t{1} << 19) && cfg_.lanes == 1;
     if (cfg_.sample_k > 0)
     {
         // per-tree samples: the first sample_k features until set_selection
@@ -4977,6 +4976,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     }
     n_sel_ = static_cast<uint32_t>(sel_h_.size());
     quant_ = cfg_.mode != HistMode::exact;
+    pdl_   = quant_ && cfg_.lanes == 1;
     if (n_sel_ == 0)
     {
         throw ConfigError("grower: the feature selection is empty");
@@ -5064,14 +5064,17 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     max_nodes_   = cfg_.leaf ? 4 * cfg_.tp.max_leaves : (2u << cfg_.tp.max_depth) - 1;
     max_rows_    = std::max<uint32_t>(max_root_rows, 1);
     crows_       = quant_ ? k_qbuild_rows : k_build_rows;
-    // the histogram grid: one CTA per SM for a large fit, about one per four
-    // 2,048-row chunks of the root for a small one; growers side by side share
-    // the SMs (seven classes: 1.05 ms a round at 581,012 rows against 1.17 with
-    // a CTA per SM each, 1.40 against 1.68 at 1,000,000)
+    // the histogram grid: one CTA per SM for a large fit, one per 2,048-row
+    // chunk of the root for a small one (us a round at 14,000 / 40,000 /
+    // 200,000 rows x 28, depth 6: 240 / 243 / 256, against 272 / 268 / 274 with
+    // one per four chunks; 64 fits of 1,000-200,000 rows in flight 236 ms
+    // against 257 for 100 rounds); growers side by side share the SMs (seven
+    // classes: 1.05 ms a round at 581,012 rows against 1.17 with a CTA per SM
+    // each, 1.40 against 1.68 at 1,000,000)
     qctas_       = cfg_.hist_ctas > 0
                        ? std::min(cfg_.hist_ctas, 64u * k_qctas)
                        : std::max(1u, std::min(k_qctas / std::min(cfg_.lanes, k_qctas),
-                                               ceil_div(max_rows_, 4 * k_qbuild_rows)));
+                                               ceil_div(max_rows_, k_qbuild_rows)));
     max_pchunks_ = ceil_div(max_rows_, k_part_rows) + max_front_;
     max_bchunks_ = ceil_div(max_rows_, crows_) + max_front_;
 

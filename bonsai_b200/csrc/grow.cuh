@@ -420,10 +420,13 @@ class Grower
     uint32_t    n_launch_ = 0;
     // every kernel opens with pdl_enter(): launched with programmatic
     // stream serialization, a kernel's CTAs are scheduled while its
-    // predecessor drains. Set for planes of 2^19 rows or more, whose kernels
-    // each fill the GPU; small planes are the ones several boosters fit at
-    // once, where CTAs waiting for their predecessor would hold SM resources
-    // the other boosters' kernels could use.
+    // predecessor drains. Set for the quantised form, whose kernels are short:
+    // 4-6% of a round at every size and grower (us at 20,000 rows x 28:
+    // depthwise 246 -> 233, leafwise 1,096 -> 1,048; 2,000,000: 414 -> 400), and 3%
+    // of 64 fits in flight. Not for the exact form: its chain CTAs would wait
+    // in the sort's place (us at 20,000 / 400,000 / 10,000,000 rows: 631 -> 620,
+    // 973 -> 1,116, 9,808 -> 9,890; 64 fits in flight 343 -> 697 ms for 50 rounds).
+    // Not for class lanes, whose kernels already fill the gaps.
     bool        pdl_      = false;
     cudaEvent_t pev_[2]   = {nullptr, nullptr};
     void        phase_begin();
