@@ -205,6 +205,26 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *total)
     return before + x - v;
 }
 
+// True in the block that passes here last of n: its threads then see what the
+// others wrote before. (ticket: zero between launches.)
+__device__ __forceinline__ bool last_block(uint32_t *ticket, uint32_t n)
+{
+    __shared__ bool last_s;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        last_s = atomicAdd(ticket, 1u) == n - 1;
+        if (last_s)
+        {
+            *ticket = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last_s;
+}
+
 __device__ __forceinline__ void write_leaf_node(TreeOut const &t, uint32_t id, float v)
 {
     t.feature[id]      = k_leaf_flag;
@@ -226,12 +246,39 @@ __device__ __forceinline__ float leaf_value(Node const &nd, TreeParams const &tp
 // n_root_dev (nullable): the root's row count lives on the device (a row
 // sample drawn for this tree); an unsharded root's global count is then the
 // same number.
-__global__ void root_setup_kernel(Ctl *ctl, Node *nodes, uint32_t n_root, Chunk *bchunks,
-                                  uint32_t *brange, uint32_t *build, TreeOut t,
-                                  uint32_t crows, uint32_t g_root, uint32_t const *n_root_dev,
-                                  uint2 *heap)
+} // namespace
+
+struct RootArgs
 {
-    pdl_enter();
+    Ctl            *ctl;
+    Node           *nodes;
+    uint32_t        n_root;
+    Chunk          *bchunks;
+    uint32_t       *brange;
+    uint32_t       *build;
+    TreeOut         t;
+    uint32_t        crows;
+    uint32_t        g_root;
+    uint32_t const *n_root_dev;
+    uint2          *heap;
+};
+
+namespace
+{
+
+__device__ __forceinline__ void root_setup(RootArgs const &A)
+{
+    Ctl *const            ctl        = A.ctl;
+    Node *const           nodes      = A.nodes;
+    uint32_t              n_root     = A.n_root;
+    Chunk *const          bchunks    = A.bchunks;
+    uint32_t *const       brange     = A.brange;
+    uint32_t *const       build      = A.build;
+    TreeOut const        &t          = A.t;
+    uint32_t const        crows      = A.crows;
+    uint32_t              g_root     = A.g_root;
+    uint32_t const *const n_root_dev = A.n_root_dev;
+    uint2 *const          heap       = A.heap;
     for (uint32_t i = threadIdx.x; heap != nullptr && i < k_heap_slots; i += blockDim.x)
     {
         heap[i] = make_uint2(k_no_tile << 8, k_heap_pass);
@@ -271,6 +318,12 @@ __global__ void root_setup_kernel(Ctl *ctl, Node *nodes, uint32_t n_root, Chunk 
         uint32_t const b = c * crows;
         bchunks[c]       = {0, b, min(crows, n_root - b), 0};
     }
+}
+
+__global__ void root_setup_kernel(RootArgs A)
+{
+    pdl_enter();
+    root_setup(A);
 }
 
 // Node totals from the first selected feature's cells: double sums over
@@ -1523,79 +1576,417 @@ __device__ __forceinline__ void qscore_group(QCell<CW2> const (&v)[k_qfind_group
     }
 }
 
-template <bool CW2>
-__global__ void __launch_bounds__(k_qfind_warps * 32)
+// Cuts n row segments (n <= NT) into chunks of `rows` rows with the
+// whole block: segment i owns chunks [range[i], range[i + 1]), and
+// seg(i, start, count, aux) describes it. One thread per segment stages its
+// chunk origin and description in shared memory first (range and what seg
+// reads are in global memory, written before a barrier), so a chunk's binary
+// search and lookup read no global memory.
+template <uint32_t NT, typename Seg>
+__device__ __forceinline__ void fill_chunk_table(uint32_t n, uint32_t const *range,
+                                                 uint32_t total, uint32_t rows, Seg seg,
+                                                 Chunk *out)
+{
+    __shared__ uint32_t range_s[NT];
+    __shared__ uint32_t start_s[NT];
+    __shared__ uint32_t count_s[NT];
+    __shared__ uint32_t aux_s[NT];
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+    {
+        uint32_t st  = 0;
+        uint32_t cnt = 0;
+        uint32_t aux = 0;
+        seg(i, st, cnt, aux);
+        range_s[i] = range[i];
+        start_s[i] = st;
+        count_s[i] = cnt;
+        aux_s[i]   = aux;
+    }
+    __syncthreads();
+    for (uint32_t c = threadIdx.x; c < total; c += blockDim.x)
+    {
+        uint32_t lo = 0;
+        uint32_t hi = n;
+        while (hi - lo > 1)
+        {
+            uint32_t const mid = (lo + hi) >> 1;
+            if (range_s[mid] <= c)
+            {
+                lo = mid;
+            }
+            else
+            {
+                hi = mid;
+            }
+        }
+        uint32_t const b = (c - range_s[lo]) * rows;
+        out[c]           = {lo, start_s[lo] + b, min(rows, count_s[lo] - b), aux_s[lo]};
+    }
+}
+
+struct PlanArgs
+{
+    uint32_t const *sel;
+    float const    *cuts;
+    uint32_t const *cut_off;
+    TreeParams      tp;
+    TreeOut         t;
+    Chunk          *pchunks;
+    uint32_t       *pcr;
+    double2        *nbound;
+    HeapOut         ho;
+    uint32_t       *nleft;
+    uint32_t       *nright;
+};
+
+// The frontier's splits and leaves written into the tree, and the partition's
+// chunk table, from every node's best split (one block of NT threads, a thread
+// per node).
+template <uint32_t NT>
+__device__ __forceinline__ void plan_level(Ctl *ctl, Node *nodes, Best const *best, uint32_t n_cur,
+                                           PlanArgs const &A)
+{
+    TreeParams const      tp      = A.tp;
+    TreeOut const        &t       = A.t;
+    HeapOut const        &ho      = A.ho;
+    uint32_t const *const cut_off = A.cut_off;
+    uint32_t *const       pcr     = A.pcr;
+    uint32_t const i     = threadIdx.x;
+    bool const     live  = i < n_cur;
+    Best const     bs    = live ? best[i] : Best{};
+    bool const     split = live && bs.valid != 0;
+    uint32_t       n_split_total = 0;
+    uint32_t const rank  = block_excl_scan<NT>(split ? 1 : 0, &n_split_total);
+    uint32_t const n_nodes0 = ctl->n_nodes;
+    Node           nd       = live ? nodes[i] : Node{};
+    if (live)
+    {
+        A.nleft[i]      = 0; // the one-pass partition's per-node counters
+        A.nright[i]     = 0;
+        A.nbound[nd.id] = make_double2(nd.lo, nd.hi); // for a later leaf renewal
+        if (split)
+        {
+            uint32_t const f     = A.sel[bs.feature];
+            uint32_t const left  = n_nodes0 + (2 * rank);
+            uint32_t const right = left + 1;
+            t.feature[nd.id]      = f;
+            t.value[nd.id]        = A.cuts[cut_off[f] + bs.bin];
+            t.left[nd.id]         = left;
+            t.right[nd.id]        = right;
+            t.default_left[nd.id] = static_cast<uint8_t>(bs.dl);
+            t.gain[nd.id]         = static_cast<float>(bs.gain);
+            t.split_bin[nd.id]    = bs.bin;
+            write_leaf_node(t, left, 0.0F);
+            write_leaf_node(t, right, 0.0F);
+            t.gain[left]   = 0.0F;
+            t.gain[right]  = 0.0F;
+            t.cover[left]  = 0.0F;
+            t.cover[right] = 0.0F;
+            nd.flags       = 1;
+            if (ho.heap != nullptr && nd.heap < k_heap_slots)
+            {
+                ho.heap[nd.heap] = heap_entry(f, ho.per, bs.bin,
+                                              cut_off[f + 1] - cut_off[f] - 1, bs.dl != 0);
+            }
+        }
+        else
+        {
+            heap_leaf(ho, nd.heap, nd.id);
+            write_leaf_node(t, nd.id, leaf_value(nd, tp));
+            nd.flags = 0;
+        }
+        nodes[i] = nd;
+    }
+    // partition chunk table over every frontier node
+    uint32_t const nch    = live ? (nd.count + k_part_rows - 1) / k_part_rows : 0;
+    uint32_t       total  = 0;
+    uint32_t const c0     = block_excl_scan<NT>(nch, &total);
+    if (live)
+    {
+        pcr[i] = c0;
+    }
+    if (i == 0)
+    {
+        pcr[n_cur]      = total;
+        ctl->n_pchunks  = total;
+        ctl->n_psplit   = n_split_total;
+        ctl->n_nodes    = n_nodes0 + (2 * n_split_total);
+        ctl->n_leaves  += n_cur - n_split_total;
+    }
+    __syncthreads();
+    fill_chunk_table<NT>(
+        n_cur, pcr, total, k_part_rows,
+        [&](uint32_t x, uint32_t &st, uint32_t &cnt, uint32_t &aux)
+        {
+            Node const nx = nodes[x];
+            st            = nx.start;
+            cnt           = nx.count;
+            aux           = 0;
+        },
+        A.pchunks);
+}
+
+// The quantised form's node totals: exact integer sums of the first selected
+// feature's cells with one warp (order-free), every lane holding them.
+__device__ __forceinline__ void warp_qtotals(unsigned long long const *cells, uint32_t nb,
+                                             uint32_t cw, int64_t &g, int64_t &h)
+{
+    int64_t sg = 0;
+    int64_t sh = 0;
+    for (uint32_t b = threadIdx.x & 31; b < nb; b += 32)
+    {
+        int64_t cg, ch;
+        qcell(cells, b, cw, cg, ch);
+        sg += cg;
+        sh += ch;
+    }
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1)
+    {
+        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, o);
+        sh += __shfl_xor_sync(0xFFFFFFFFu, sh, o);
+    }
+    g = sg;
+    h = sh;
+}
+
+// The level chain: for a walked tree with packed cells and a split per node,
+// the find also subtracts the larger children (parent - smaller, exact
+// integers) while it reads them, a node's last block picks its split and takes
+// its left totals off the split's cells, and the find's last block plans the
+// partition, so that a level is the build, this, the partition and the next
+// frontier's plan: four launches for six, and one pass less over the cells.
+// With the tree opened beside its quantisation and the leaves renewed by the
+// walk's last block, a round of depth 6 x 28 features is 33 launches for 45: us
+// at 1,000 / 20,000 / 200,000 rows 233 / 249 / 250 before, 228 / 241 / 244 now,
+// 64 fits in flight 235 ms for 100 rounds before, 221 now. What was measured and
+// left: the partition's last block planning the next frontier (registers: the
+// partition 24 to 32 us at 10,000,000 rows); two-word cells (500,000 rows 328 to
+// 334) and the levelwise find (its few blocks subtract slowly: 525 to 535).
+struct FindChain
+{
+    Ctl                      *ctl;
+    Node                     *nodes;
+    Best                     *best;
+    int64_t                  *ltot;    // per node: (G, H) left of its split
+    uint32_t                 *ticket;  // [0] the launch's, [1 + i] node i's
+    unsigned long long       *hist;    // this level's cells
+    unsigned long long const *parents; // the level above's; null at the root
+    uint32_t const           *bpair;
+    PlanArgs                  plan;
+};
+
+// (G, H) of the rows that a split sends left, off the node's cells of the
+// split feature (a warp; lane 0 writes them).
+__device__ __forceinline__ void left_totals(unsigned long long const *cells, uint32_t nb,
+                                            uint32_t cw, Best const &bs, int64_t *out)
+{
+    int64_t sg = 0;
+    int64_t sh = 0;
+    for (uint32_t b = threadIdx.x & 31; b < nb; b += 32)
+    {
+        if (b <= bs.bin || (b == nb - 1 && bs.dl != 0))
+        {
+            int64_t cg, ch;
+            qcell(cells, b, cw, cg, ch);
+            sg += cg;
+            sh += ch;
+        }
+    }
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1)
+    {
+        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, o);
+        sh += __shfl_xor_sync(0xFFFFFFFFu, sh, o);
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+        out[0] = sg;
+        out[1] = sh;
+    }
+}
+
+// The first feature (ascending) with the largest gain among a node's
+// candidates (a warp; every lane returns it).
+__device__ __forceinline__ Best best_candidate(Best const *cand, uint32_t n_sel)
+{
+    double   g = 0.0;
+    uint32_t o = 0xFFFFFFFFu;
+    for (uint32_t j = threadIdx.x & 31; j < n_sel; j += 32)
+    {
+        Best const c = cand[j];
+        if (c.valid != 0 && (c.gain > g || (c.gain == g && j < o)))
+        {
+            g = c.gain;
+            o = j;
+        }
+    }
+    warp_best(g, o);
+    o = __shfl_sync(0xFFFFFFFFu, o, 0);
+    return o == 0xFFFFFFFFu ? Best{0.0, 0, 0, 1, 0} : cand[o];
+}
+
+template <bool CW2, bool CHAIN>
+__global__ void __launch_bounds__(k_qfind_warps * 32, CW2 ? 1 : 3)
     qfind_warp_kernel(Ctl const *ctl, Node const *nodes, void const *hist_v,
                       uint32_t total_cells, uint32_t const *cell_off, uint32_t const *sel_nb,
                       uint32_t const *sel, uint32_t n_sel, int8_t const *mono, uint32_t n_mono,
-                      TreeParams tp, Best *cand, double2 const *qscale, uint64_t const *fgroups)
+                      TreeParams tp, Best *cand, double2 const *qscale, uint64_t const *fgroups,
+                      FindChain C)
 {
     pdl_enter();
-    uint32_t const i = blockIdx.x;
-    if (i >= ctl->n_cur)
+    constexpr uint32_t cw    = CW2 ? 2 : 1;
+    uint32_t const     i     = blockIdx.x;
+    uint32_t const     n_cur = ctl->n_cur;
+    if (i >= n_cur && (!CHAIN || n_cur != 0 || i + blockIdx.y != 0))
     {
-        return;
+        return; // (an empty frontier is planned by the first block)
     }
     uint32_t const lane = threadIdx.x & 31;
     uint32_t const j    = (blockIdx.y * k_qfind_warps) + (threadIdx.x >> 5);
-    if (j >= n_sel)
+    if (i < n_cur && j < n_sel)
     {
-        return;
-    }
-    Node const     nd  = nodes[i];
-    uint32_t const nb  = sel_nb[j];
-    uint32_t const f   = sel[j];
-    Best           out = {0.0, j, 0, 1, 0};
-    if (nd.gcount < 2 * tp.min_data_in_leaf || nb < 2 || !interaction_allows(nd, fgroups, f))
-    {
+        Node           nd   = nodes[i];
+        uint32_t const nb   = sel_nb[j];
+        uint32_t const f    = sel[j];
+        uint32_t const off  = cell_off[j];
+        auto const    *base = static_cast<unsigned long long const *>(hist_v);
+        auto const *src = base + (((static_cast<uint64_t>(i) * total_cells) + off) * cw);
+        // the larger child's cells: its parent's less its sibling's
+        bool                      large = false;
+        unsigned long long const *par   = nullptr;
+        unsigned long long const *sib   = nullptr;
+        if constexpr (CHAIN)
+        {
+            if (C.parents != nullptr)
+            {
+                uint32_t const *pair = C.bpair + (3 * (i >> 1));
+                large                = pair[2] == i;
+                par = C.parents + (((static_cast<uint64_t>(pair[0]) * total_cells) + off) * cw);
+                sib = base + (((static_cast<uint64_t>(pair[1]) * total_cells) + off) * cw);
+            }
+            else
+            {
+                warp_qtotals(src, nb, cw, nd.qg, nd.qh); // the root: every row is in one cell
+            }
+        }
+        auto const cell = [&](uint32_t b, bool keep)
+        {
+            QCell<CW2> c;
+            if (CHAIN && large)
+            {
+                QCell<CW2> o;
+                c.load(par, b);
+                o.load(sib, b);
+                c.sub(o);
+                if (keep)
+                {
+                    c.store(C.hist + (((static_cast<uint64_t>(i) * total_cells) + off) * cw), b);
+                }
+            }
+            else
+            {
+                c.load(src, b);
+            }
+            return c;
+        };
+        Best       out     = {0.0, j, 0, 1, 0};
+        bool const open    = nd.gcount >= 2 * tp.min_data_in_leaf && nb >= 2;
+        bool const allowed = open && interaction_allows(nd, fgroups, f);
+        if (allowed)
+        {
+            uint32_t const   n_cut = nb - 2;
+            double2 const    sc    = *qscale;
+            QCell<CW2> const miss  = cell(nb - 1, lane == 0);
+            if (CHAIN && large && lane == 0)
+            {
+                cell(nb - 2, true);
+            }
+            QNode n;
+            n.start(nd.qg, nd.qh, miss.g(), miss.h(), nd,
+                    (mono != nullptr && f < n_mono) ? mono[f] : 0, sc, tp);
+            __shared__ QHand<CW2> hand_s[k_qfind_warps];
+            QHand<CW2>           &hand  = hand_s[threadIdx.x >> 5];
+            double                best  = 0.0;
+            uint32_t              order = 0xFFFFFFFFu;
+            QCell<CW2>            carry, before;
+            carry.clear();
+            for (uint32_t c0 = 0; c0 < n_cut; c0 += 32 * k_qfind_group)
+            {
+                QCell<CW2> v[k_qfind_group];
+#pragma unroll
+                for (uint32_t q = 0; q < k_qfind_group; ++q)
+                {
+                    uint32_t const b = c0 + (q * 32) + lane;
+                    v[q].clear();
+                    if (b < n_cut)
+                    {
+                        v[q] = cell(b, true);
+                    }
+                }
+                qscan_group<CW2>(v, hand, carry, before);
+                qscore_group<CW2>(v, before, c0, n_cut, n, sc, tp, best, order);
+            }
+            warp_best(best, order);
+            if (order != 0xFFFFFFFFu)
+            {
+                out.gain  = best;
+                out.bin   = order >> 1;
+                out.dl    = (order & 1) == 0 ? 1 : 0;
+                out.valid = 1;
+            }
+        }
+        else if (CHAIN && large && open)
+        {
+            // (a constrained feature's cells: the children may ask for them)
+            for (uint32_t b = lane; b < nb; b += 32)
+            {
+                cell(b, true);
+            }
+        }
         if (lane == 0)
         {
             cand[(i * n_sel) + j] = out;
         }
-        return;
     }
-    uint32_t const n_cut = nb - 2;
-    auto const    *src   = static_cast<unsigned long long const *>(hist_v) +
-                      (((static_cast<uint64_t>(i) * total_cells) + cell_off[j]) * (CW2 ? 2 : 1));
-    double2 const sc = *qscale;
-    QCell<CW2>    miss;
-    miss.load(src, nb - 1);
-    QNode n;
-    n.start(nd.qg, nd.qh, miss.g(), miss.h(), nd, (mono != nullptr && f < n_mono) ? mono[f] : 0, sc,
-            tp);
-    __shared__ QHand<CW2> hand_s[k_qfind_warps];
-    QHand<CW2>           &hand  = hand_s[threadIdx.x >> 5];
-    double                best  = 0.0;
-    uint32_t              order = 0xFFFFFFFFu;
-    QCell<CW2>            carry, before;
-    carry.clear();
-    for (uint32_t c0 = 0; c0 < n_cut; c0 += 32 * k_qfind_group)
+    if constexpr (CHAIN)
     {
-        QCell<CW2> v[k_qfind_group];
-#pragma unroll
-        for (uint32_t q = 0; q < k_qfind_group; ++q)
+        if (i < n_cur)
         {
-            uint32_t const b = c0 + (q * 32) + lane;
-            v[q].clear();
-            if (b < n_cut)
+            if (!last_block(C.ticket + 1 + i, gridDim.y))
             {
-                v[q].load(src, b);
+                return;
+            }
+            if (threadIdx.x < 32)
+            {
+                auto const *cells = C.hist + (static_cast<uint64_t>(i) * total_cells * cw);
+                Best const  bs    = best_candidate(cand + (static_cast<uint64_t>(i) * n_sel), n_sel);
+                if (lane == 0)
+                {
+                    C.best[i] = bs;
+                }
+                if (bs.valid != 0)
+                {
+                    left_totals(cells + (static_cast<uint64_t>(cell_off[bs.feature]) * cw),
+                                sel_nb[bs.feature], cw, bs, C.ltot + (2 * i));
+                }
+                if (C.parents == nullptr)
+                {
+                    int64_t g, h;
+                    warp_qtotals(cells, sel_nb[0], cw, g, h);
+                    if (lane == 0)
+                    {
+                        C.nodes[0].qg = g;
+                        C.nodes[0].qh = h;
+                    }
+                }
+            }
+            if (!last_block(C.ticket, n_cur))
+            {
+                return;
             }
         }
-        qscan_group<CW2>(v, hand, carry, before);
-        qscore_group<CW2>(v, before, c0, n_cut, n, sc, tp, best, order);
-    }
-    warp_best(best, order);
-    if (lane == 0)
-    {
-        if (order != 0xFFFFFFFFu)
-        {
-            out.gain  = best;
-            out.bin   = order >> 1;
-            out.dl    = (order & 1) == 0 ? 1 : 0;
-            out.valid = 1;
-        }
-        cand[(i * n_sel) + j] = out;
+        plan_level<k_qfind_warps * 32>(C.ctl, C.nodes, C.best, n_cur, C.plan);
     }
 }
 
@@ -1874,61 +2265,11 @@ __global__ void __launch_bounds__(k_lfind_thr)
     }
 }
 
-// Cuts n row segments (n <= k_plan_thr) into chunks of `rows` rows with the
-// whole block: segment i owns chunks [range[i], range[i + 1]), and
-// seg(i, start, count, aux) describes it. One thread per segment stages its
-// chunk origin and description in shared memory first (range and what seg
-// reads are in global memory, written before a barrier), so a chunk's binary
-// search and lookup read no global memory.
-template <typename Seg>
-__device__ __forceinline__ void fill_chunk_table(uint32_t n, uint32_t const *range,
-                                                 uint32_t total, uint32_t rows, Seg seg,
-                                                 Chunk *out)
-{
-    __shared__ uint32_t range_s[k_plan_thr];
-    __shared__ uint32_t start_s[k_plan_thr];
-    __shared__ uint32_t count_s[k_plan_thr];
-    __shared__ uint32_t aux_s[k_plan_thr];
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-    {
-        uint32_t st  = 0;
-        uint32_t cnt = 0;
-        uint32_t aux = 0;
-        seg(i, st, cnt, aux);
-        range_s[i] = range[i];
-        start_s[i] = st;
-        count_s[i] = cnt;
-        aux_s[i]   = aux;
-    }
-    __syncthreads();
-    for (uint32_t c = threadIdx.x; c < total; c += blockDim.x)
-    {
-        uint32_t lo = 0;
-        uint32_t hi = n;
-        while (hi - lo > 1)
-        {
-            uint32_t const mid = (lo + hi) >> 1;
-            if (range_s[mid] <= c)
-            {
-                lo = mid;
-            }
-            else
-            {
-                hi = mid;
-            }
-        }
-        uint32_t const b = (c - range_s[lo]) * rows;
-        out[c]           = {lo, start_s[lo] + b, min(rows, count_s[lo] - b), aux_s[lo]};
-    }
-}
-
 // ------------------------------------------------------------- planning ----
 
 __global__ void __launch_bounds__(k_plan_thr)
     plan_kernel(Ctl *ctl, Node *nodes, Best const *cand, Best *best, uint32_t n_sel,
-                uint32_t const *sel, float const *cuts, uint32_t const *cut_off,
-                TreeParams tp, TreeOut t, Chunk *pchunks, uint32_t *pcr, double2 *nbound,
-                bool level, HeapOut ho, uint32_t *nleft, uint32_t *nright)
+                bool level, PlanArgs A)
 {
     pdl_enter();
     __shared__ Best    level_s;
@@ -1985,79 +2326,7 @@ __global__ void __launch_bounds__(k_plan_thr)
         }
     }
     __syncthreads();
-    uint32_t const i     = threadIdx.x;
-    bool const     live  = i < n_cur;
-    Best const     bs    = live ? best[i] : Best{};
-    bool const     split = live && bs.valid != 0;
-    uint32_t       n_split_total = 0;
-    uint32_t const rank  = block_excl_scan<k_plan_thr>(split ? 1 : 0, &n_split_total);
-    uint32_t const n_nodes0 = ctl->n_nodes;
-    Node           nd       = live ? nodes[i] : Node{};
-    if (live)
-    {
-        nleft[i]      = 0; // the one-pass partition's per-node counters
-        nright[i]     = 0;
-        nbound[nd.id] = make_double2(nd.lo, nd.hi); // for a later leaf renewal
-        if (split)
-        {
-            uint32_t const f     = sel[bs.feature];
-            uint32_t const left  = n_nodes0 + (2 * rank);
-            uint32_t const right = left + 1;
-            t.feature[nd.id]      = f;
-            t.value[nd.id]        = cuts[cut_off[f] + bs.bin];
-            t.left[nd.id]         = left;
-            t.right[nd.id]        = right;
-            t.default_left[nd.id] = static_cast<uint8_t>(bs.dl);
-            t.gain[nd.id]         = static_cast<float>(bs.gain);
-            t.split_bin[nd.id]    = bs.bin;
-            write_leaf_node(t, left, 0.0F);
-            write_leaf_node(t, right, 0.0F);
-            t.gain[left]   = 0.0F;
-            t.gain[right]  = 0.0F;
-            t.cover[left]  = 0.0F;
-            t.cover[right] = 0.0F;
-            nd.flags       = 1;
-            if (ho.heap != nullptr && nd.heap < k_heap_slots)
-            {
-                ho.heap[nd.heap] = heap_entry(f, ho.per, bs.bin,
-                                              cut_off[f + 1] - cut_off[f] - 1, bs.dl != 0);
-            }
-        }
-        else
-        {
-            heap_leaf(ho, nd.heap, nd.id);
-            write_leaf_node(t, nd.id, leaf_value(nd, tp));
-            nd.flags = 0;
-        }
-        nodes[i] = nd;
-    }
-    // partition chunk table over every frontier node
-    uint32_t const nch    = live ? (nd.count + k_part_rows - 1) / k_part_rows : 0;
-    uint32_t       total  = 0;
-    uint32_t const c0     = block_excl_scan<k_plan_thr>(nch, &total);
-    if (live)
-    {
-        pcr[i] = c0;
-    }
-    if (i == 0)
-    {
-        pcr[n_cur]      = total;
-        ctl->n_pchunks  = total;
-        ctl->n_psplit   = n_split_total;
-        ctl->n_nodes    = n_nodes0 + (2 * n_split_total);
-        ctl->n_leaves  += n_cur - n_split_total;
-    }
-    __syncthreads();
-    fill_chunk_table(
-        n_cur, pcr, total, k_part_rows,
-        [&](uint32_t x, uint32_t &st, uint32_t &cnt, uint32_t &aux)
-        {
-            Node const nx = nodes[x];
-            st            = nx.start;
-            cnt           = nx.count;
-            aux           = 0;
-        },
-        pchunks);
+    plan_level<k_plan_thr>(ctl, nodes, best, n_cur, A);
 }
 
 // ----------------------------------------------------------------- leafwise ----
@@ -2314,25 +2583,93 @@ __global__ void __launch_bounds__(k_plan_thr)
     }
 }
 
-__global__ void __launch_bounds__(k_plan_thr)
-    plan2_kernel(Ctl *ctl, Node *nodes, Node *next, Best const *best,
-                 Chunk const *pchunks, uint32_t const *pcr, uint32_t *pleft,
-                 uint32_t *prbase, uint32_t *nleft, uint32_t *dst, uint32_t *bpair,
-                 uint32_t *build, uint32_t *brange, Chunk *bchunks, TreeParams tp,
-                 TreeOut t, uint32_t crows, uint32_t *bbase, bool level,
-                 uint64_t const *gleft, uint64_t const *fgroups, HeapOut ho, bool fused)
+struct Plan2Args
 {
-    pdl_enter();
+    Ctl            *ctl;
+    Node           *nodes;
+    Node           *next;
+    Best const     *best;
+    Chunk const    *pchunks;
+    uint32_t const *pcr;
+    uint32_t       *pleft, *prbase, *nleft, *dst, *bpair, *build, *brange;
+    Chunk          *bchunks;
+    TreeParams      tp;
+    TreeOut         t;
+    uint32_t        crows;
+    uint32_t       *bbase;
+    bool            level;
+    uint64_t const *gleft;
+    uint64_t const *fgroups;
+    HeapOut         ho;
+    // one-pass partition: per node, the exact sums of its left child, from
+    // which both children take their totals and monotone bounds
+    int64_t const  *ltot;
+    uint32_t const *sel;
+    int8_t const   *mono;
+    uint32_t        n_mono;
+    double2 const  *qscale;
+};
+
+// The children's bounds after a split on a constrained feature, from their
+// integer totals.
+__device__ __forceinline__ void split_bounds(Node &L, Node &R, Node const &par, int mc,
+                                             double2 const &sc, TreeParams const &tp)
+{
+    double const l1  = tp.lambda_l1;
+    double const l2  = tp.lambda_l2;
+    double const wl  = bounded_leaf_weight(static_cast<double>(L.qg) * sc.x,
+                                           static_cast<double>(L.qh) * sc.y, l1, l2, par.lo,
+                                           par.hi);
+    double const wr  = bounded_leaf_weight(static_cast<double>(R.qg) * sc.x,
+                                           static_cast<double>(R.qh) * sc.y, l1, l2, par.lo,
+                                           par.hi);
+    double const mid = 0.5 * (wl + wr);
+    if (mc > 0)
+    {
+        L.hi = fmin(L.hi, mid);
+        R.lo = fmax(R.lo, mid);
+    }
+    else
+    {
+        L.lo = fmax(L.lo, mid);
+        R.hi = fmin(R.hi, mid);
+    }
+}
+
+// After a level's partition: the next frontier, its smaller children's build
+// chunks, and the demotion of splits that left a side empty (one block of NT
+// threads, a thread per node). FUSED: the one-pass partition, which has
+// counted and placed the rows already; the frontier advances here.
+template <uint32_t NT, bool FUSED> __device__ __forceinline__ void plan_children(Plan2Args const &A)
+{
+    Ctl *const            ctl     = A.ctl;
+    Node *const           nodes   = A.nodes;
+    Node *const           next    = A.next;
+    Chunk const *const    pchunks = A.pchunks;
+    uint32_t const *const pcr     = A.pcr;
+    uint32_t *const       pleft   = A.pleft;
+    uint32_t *const       prbase  = A.prbase;
+    uint32_t *const       nleft   = A.nleft;
+    uint32_t *const       bpair   = A.bpair;
+    uint32_t *const       build   = A.build;
+    uint32_t *const       brange  = A.brange;
+    uint32_t *const       bbase   = A.bbase;
+    TreeParams const      tp      = A.tp;
+    TreeOut const        &t       = A.t;
+    uint32_t const        crows   = A.crows;
+    bool const            level   = A.level;
+    uint64_t const *const gleft   = A.gleft;
+    HeapOut const        &ho      = A.ho;
     __shared__ uint32_t grand_s;
-    __shared__ uint32_t flags_s[k_plan_thr]; // per node: flags, start, prefix origin
-    __shared__ uint32_t start_s[k_plan_thr];
-    __shared__ uint32_t p0_s[k_plan_thr];
+    __shared__ uint32_t flags_s[NT]; // per node: flags, start, prefix origin
+    __shared__ uint32_t start_s[NT];
+    __shared__ uint32_t p0_s[NT];
     uint32_t const      n_cur = ctl->n_cur;
     uint32_t const      n_ch  = ctl->n_pchunks;
     // A. exclusive prefix of the chunks' left counts over the whole level
     //    (leaf chunks count zero), each thread a contiguous run of chunks
     //    (the one-pass partition placed its rows already: no chunk runs)
-    uint32_t const per = fused ? 0 : (n_ch + k_plan_thr - 1) / k_plan_thr;
+    uint32_t const per = FUSED ? 0 : (n_ch + NT - 1) / NT;
     uint32_t const c_a = min(n_ch, threadIdx.x * per);
     uint32_t const c_b = min(n_ch, c_a + per);
     uint32_t       sum = 0;
@@ -2341,7 +2678,7 @@ __global__ void __launch_bounds__(k_plan_thr)
         sum += pleft[c];
     }
     uint32_t       grand = 0;
-    uint32_t const base  = block_excl_scan<k_plan_thr>(sum, &grand);
+    uint32_t const base  = block_excl_scan<NT>(sum, &grand);
     for (uint32_t c = c_a, run = base; c < c_b; ++c)
     {
         uint32_t const v = pleft[c];
@@ -2363,7 +2700,7 @@ __global__ void __launch_bounds__(k_plan_thr)
     uint32_t       p0   = 0;
     if (live && (nd.flags & 1) != 0)
     {
-        if (fused)
+        if (FUSED)
         {
             nl = nleft[i]; // the one-pass partition's left counter
         }
@@ -2401,7 +2738,7 @@ __global__ void __launch_bounds__(k_plan_thr)
     }
     __syncthreads();
     // C. per chunk of a split node: its left and right write bases
-    for (uint32_t c = threadIdx.x; !fused && c < n_ch; c += k_plan_thr)
+    for (uint32_t c = threadIdx.x; !FUSED && c < n_ch; c += NT)
     {
         Chunk const    ch = pchunks[c];
         uint32_t const fl = flags_s[ch.node];
@@ -2416,16 +2753,16 @@ __global__ void __launch_bounds__(k_plan_thr)
     // D. survivors: their children in the next frontier, and the chunk table
     //    of the smaller children whose histograms are built
     uint32_t       n_surv     = 0;
-    uint32_t const k          = block_excl_scan<k_plan_thr>(surv ? 1 : 0, &n_surv);
+    uint32_t const k          = block_excl_scan<NT>(surv ? 1 : 0, &n_surv);
     uint32_t       rows_total = 0;
-    uint32_t const start = block_excl_scan<k_plan_thr>(surv ? nd.count : 0, &rows_total);
+    uint32_t const start = block_excl_scan<NT>(surv ? nd.count : 0, &rows_total);
     uint32_t small_count = 0;
     if (surv)
     {
         // the children's rows: compacted by pscatter, or where the one-pass
         // partition left them (the parent's segment, lefts first)
-        uint32_t const s0   = fused ? nd.start : start;
-        dst[i]              = s0;
+        uint32_t const s0   = FUSED ? nd.start : start;
+        A.dst[i]            = s0;
         uint32_t const nr   = nd.count - nl;
         uint32_t const gnr  = nd.gcount - gnl;
         uint32_t const lid  = t.left[nd.id];
@@ -2434,7 +2771,20 @@ __global__ void __launch_bounds__(k_plan_thr)
         Node           R{s0 + nl, nr, rid, 0, 0.0F, 0.0F, nd.lo, nd.hi, 0, 0, gnr, 0, 0};
         L.heap              = (2 * nd.heap) + 1;
         R.heap              = (2 * nd.heap) + 2;
-        interaction_children(nd, fgroups, t.feature[nd.id], L, R);
+        interaction_children(nd, A.fgroups, t.feature[nd.id], L, R);
+        if (FUSED && A.ltot != nullptr)
+        {
+            L.qg              = A.ltot[2 * i];
+            L.qh              = A.ltot[(2 * i) + 1];
+            R.qg              = nd.qg - L.qg;
+            R.qh              = nd.qh - L.qh;
+            uint32_t const f  = A.sel[A.best[i].feature];
+            int const      mc = (A.mono != nullptr && f < A.n_mono) ? A.mono[f] : 0;
+            if (mc != 0)
+            {
+                split_bounds(L, R, nd, mc, *A.qscale, tp);
+            }
+        }
         next[2 * k]         = L;
         next[(2 * k) + 1]   = R;
         t.cover[lid]        = static_cast<float>(gnl);
@@ -2449,21 +2799,25 @@ __global__ void __launch_bounds__(k_plan_thr)
     }
     uint32_t const nch   = surv ? (small_count + crows - 1) / crows : 0;
     uint32_t       nch_t = 0;
-    uint32_t const c0    = block_excl_scan<k_plan_thr>(nch, &nch_t);
+    uint32_t const c0    = block_excl_scan<NT>(nch, &nch_t);
     uint32_t       built = 0;
-    uint32_t const pbase = block_excl_scan<k_plan_thr>(small_count, &built);
+    uint32_t const pbase = block_excl_scan<NT>(small_count, &built);
     if (surv)
     {
         brange[k] = c0;
         bbase[k]  = pbase; // the built node's payload base
     }
     uint32_t n_dem = 0;
-    block_excl_scan<k_plan_thr>((live && (nd.flags & 2) != 0) ? 1 : 0, &n_dem);
+    block_excl_scan<NT>((live && (nd.flags & 2) != 0) ? 1 : 0, &n_dem);
     if (i == 0)
     {
         brange[n_surv]  = nch_t;
         ctl->n_leaves  += n_dem;
         ctl->n_next     = 2 * n_surv;
+        if (FUSED && A.ltot != nullptr)
+        {
+            ctl->n_cur = 2 * n_surv;
+        }
         ctl->n_splits   = n_surv;
         ctl->n_build    = n_surv;
         ctl->n_bchunks  = nch_t;
@@ -2474,7 +2828,7 @@ __global__ void __launch_bounds__(k_plan_thr)
         }
     }
     __syncthreads();
-    fill_chunk_table(
+    fill_chunk_table<NT>(
         n_surv, brange, nch_t, crows,
         [&](uint32_t x, uint32_t &st, uint32_t &cnt, uint32_t &aux)
         {
@@ -2483,7 +2837,13 @@ __global__ void __launch_bounds__(k_plan_thr)
             cnt           = sm.count;
             aux           = bbase[x];
         },
-        bchunks);
+        A.bchunks);
+}
+
+template <bool FUSED> __global__ void __launch_bounds__(k_plan_thr) plan2_kernel(Plan2Args A)
+{
+    pdl_enter();
+    plan_children<k_plan_thr, FUSED>(A);
 }
 
 // Rows of this level's leaves (never split, or demoted): their leaf id and
@@ -2767,13 +3127,53 @@ __device__ __forceinline__ bool in_sample(uint32_t const *bits, uint64_t r)
 constexpr uint32_t k_wsum_thr    = 512;
 constexpr uint32_t k_wsum_copies = 16;
 
+// The quantised form's leaf values from pass A's sums: FP64 Newton values
+// under each leaf's monotone bounds (one block). Run by pass A's last block,
+// which then clears the gradients' maxima for the next round's where asked;
+// a shard's sums are the fit's only after a reduction, so that it takes a
+// launch of its own.
+struct FixArgs
+{
+    Ctl const                *ctl;
+    TreeOut                   t;
+    unsigned long long const *acc;
+    double2 const            *nbound;
+    uint32_t const           *absmax;
+    TreeParams                tp;
+    double                    fix_unit;
+    uint32_t                 *ticket; // null: not in pass A
+    uint32_t                 *clear;  // the maxima to zero, or null
+};
+
+__device__ __forceinline__ void leaf_fix(FixArgs const &F)
+{
+    TreeOut const &t   = F.t;
+    float const  mgx = __uint_as_float(F.absmax[0]);
+    float const  mhx = __uint_as_float(F.absmax[1]);
+    double const fg  = mgx > 0.0F ? F.fix_unit / static_cast<double>(mgx) : 1.0;
+    double const fh  = mhx > 0.0F ? F.fix_unit / static_cast<double>(mhx) : 1.0;
+    uint32_t const n_nodes = min(F.ctl->n_nodes, k_walk_nodes);
+    for (uint32_t i = threadIdx.x; i < n_nodes; i += blockDim.x)
+    {
+        if (t.feature[i] != k_leaf_flag)
+        {
+            continue;
+        }
+        double const g = static_cast<double>(static_cast<int64_t>(F.acc[2 * i])) / fg;
+        double const h = static_cast<double>(static_cast<int64_t>(F.acc[(2 * i) + 1])) / fh;
+        double2 const b = F.nbound[i];
+        t.value[i] = static_cast<float>(
+            bounded_leaf_weight(g, h, F.tp.lambda_l1, F.tp.lambda_l2, b.x, b.y));
+    }
+}
+
 template <bool U8, bool MULTI>
 __global__ void __launch_bounds__(k_wsum_thr)
     walk_sum_kernel(Ctl const *ctl, uint4 const *__restrict__ mirror, uint64_t n_rows,
                     uint2 const *heap, uint16_t const *leafmap, uint32_t depth,
                     float2 const *__restrict__ gh, uint32_t const *absmax,
                     uint16_t *__restrict__ leaf16, unsigned long long *acc,
-                    uint32_t const *__restrict__ bits, double fix_unit)
+                    uint32_t const *__restrict__ bits, double fix_unit, FixArgs F)
 {
     pdl_enter();
     extern __shared__ unsigned long long acc_s[];
@@ -2844,33 +3244,21 @@ __global__ void __launch_bounds__(k_wsum_thr)
             atomicAdd(&acc[(2 * leaf_s[x >> 1]) + (x & 1)], v);
         }
     }
+    if (F.ticket != nullptr && last_block(F.ticket, gridDim.x))
+    {
+        leaf_fix(F);
+        __syncthreads();
+        if (F.clear != nullptr && threadIdx.x < 2)
+        {
+            F.clear[threadIdx.x] = 0;
+        }
+    }
 }
 
-// The quantised form's leaf values from pass A's sums: FP64 Newton values
-// under each leaf's monotone bounds.
-__global__ void __launch_bounds__(k_threads)
-    leaf_fix_kernel(Ctl const *ctl, TreeOut t, unsigned long long const *acc,
-                    double2 const *nbound, uint32_t const *absmax, TreeParams tp,
-                    double fix_unit)
+__global__ void __launch_bounds__(k_threads) leaf_fix_kernel(FixArgs F)
 {
     pdl_enter();
-    float const  mgx = __uint_as_float(absmax[0]);
-    float const  mhx = __uint_as_float(absmax[1]);
-    double const fg  = mgx > 0.0F ? fix_unit / static_cast<double>(mgx) : 1.0;
-    double const fh  = mhx > 0.0F ? fix_unit / static_cast<double>(mhx) : 1.0;
-    uint32_t const n_nodes = min(ctl->n_nodes, k_walk_nodes);
-    for (uint32_t i = threadIdx.x; i < n_nodes; i += k_threads)
-    {
-        if (t.feature[i] != k_leaf_flag)
-        {
-            continue;
-        }
-        double const g = static_cast<double>(static_cast<int64_t>(acc[2 * i])) / fg;
-        double const h = static_cast<double>(static_cast<int64_t>(acc[(2 * i) + 1])) / fh;
-        double2 const b = nbound[i];
-        t.value[i] = static_cast<float>(
-            bounded_leaf_weight(g, h, tp.lambda_l1, tp.lambda_l2, b.x, b.y));
-    }
+    leaf_fix(F);
 }
 
 // Pass B of the quantised form: apply the renewed values by pass A's leaf ids.
@@ -3267,7 +3655,8 @@ __global__ void __launch_bounds__(k_threads)
 // (and, quantised, the leaf renewal) run chunk by chunk as on any level.
 __global__ void __launch_bounds__(k_plan_thr)
     final_kernel(Ctl *ctl, Node *nodes, TreeParams tp, TreeOut t, Chunk *pchunks,
-                 uint32_t *pcr, double2 *nbound, HeapOut ho)
+                 uint32_t *pcr, double2 *nbound, HeapOut ho, uint32_t *tree_no,
+                 uint32_t tree_step)
 {
     pdl_enter();
     uint32_t const n    = ctl->n_cur;
@@ -3297,9 +3686,10 @@ __global__ void __launch_bounds__(k_plan_thr)
         t.meta[0]       = ctl->n_nodes;
         t.meta[1]       = ctl->depth;
         t.meta[2]       = ctl->n_leaves;
+        *tree_no       += tree_step; // (the tree's roundings are done)
     }
     __syncthreads();
-    fill_chunk_table(
+    fill_chunk_table<k_plan_thr>(
         n, pcr, total, k_part_rows,
         [&](uint32_t x, uint32_t &st, uint32_t &cnt, uint32_t &aux)
         {
@@ -3385,6 +3775,21 @@ __global__ void __launch_bounds__(k_threads)
     }
 }
 
+} // namespace
+
+// What a tree starts with, done beside its quantisation (zero null: by
+// launches of their own): the root's cells and the walk's sums zeroed, the root.
+struct OpenArgs
+{
+    unsigned long long *zero;
+    uint64_t            n_zero;
+    unsigned long long *wacc;
+    RootArgs            root;
+};
+
+namespace
+{
+
 // W16: int16 codes (scales max / 32767, g in the low half of a 32-bit word,
 // h in the high half) instead of int8 (max / 127, a 16-bit word).
 template <bool W16>
@@ -3392,9 +3797,22 @@ __global__ void __launch_bounds__(k_threads)
     quantise_kernel(float2 const *__restrict__ gh, uint32_t n,
                     uint32_t const *__restrict__ absmax, uint2 key,
                     uint32_t const *__restrict__ tree_no, void *__restrict__ qout,
-                    double2 *__restrict__ scale, uint64_t row_off)
+                    double2 *__restrict__ scale, uint64_t row_off, OpenArgs O)
 {
     pdl_enter();
+    for (uint64_t x = (uint64_t{blockIdx.x} * k_threads) + threadIdx.x; x < O.n_zero;
+         x += uint64_t{gridDim.x} * k_threads)
+    {
+        O.zero[x] = 0ULL;
+    }
+    if (O.zero != nullptr && blockIdx.x == gridDim.x - 1)
+    {
+        for (uint32_t x = threadIdx.x; x < 2 * k_walk_nodes; x += k_threads)
+        {
+            O.wacc[x] = 0ULL;
+        }
+        root_setup(O.root);
+    }
     constexpr double qmax = W16 ? 32767.0 : 127.0;
     constexpr int    imax = W16 ? 32767 : 127;
     double const mg = __uint_as_float(absmax[0]);
@@ -3830,30 +4248,6 @@ __global__ void __launch_bounds__(k_tthreads, 1)
                   hist + (static_cast<uint64_t>(build[node]) * total_cells * (CW2 ? 2 : 1)));
 }
 
-// The quantised form's node totals: exact integer sums of the first selected
-// feature's cells with one warp (order-free), every lane holding them.
-__device__ __forceinline__ void warp_qtotals(unsigned long long const *cells, uint32_t nb,
-                                             uint32_t cw, int64_t &g, int64_t &h)
-{
-    int64_t sg = 0;
-    int64_t sh = 0;
-    for (uint32_t b = threadIdx.x & 31; b < nb; b += 32)
-    {
-        int64_t cg, ch;
-        qcell(cells, b, cw, cg, ch);
-        sg += cg;
-        sh += ch;
-    }
-#pragma unroll
-    for (uint32_t o = 16; o > 0; o >>= 1)
-    {
-        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, o);
-        sh += __shfl_xor_sync(0xFFFFFFFFu, sh, o);
-    }
-    g = sg;
-    h = sh;
-}
-
 __global__ void qroot_totals_kernel(Node *nodes, unsigned long long const *hist,
                                     uint32_t const *sel_nb, uint32_t cw)
 {
@@ -3954,26 +4348,7 @@ __global__ void __launch_bounds__(k_threads)
         int const      mc = (mono != nullptr && f < n_mono) ? mono[f] : 0;
         if (mc != 0)
         {
-            double2 const sc  = *qscale;
-            double const  l1  = tp.lambda_l1;
-            double const  l2  = tp.lambda_l2;
-            double const  wl  = bounded_leaf_weight(static_cast<double>(L.qg) * sc.x,
-                                                    static_cast<double>(L.qh) * sc.y, l1, l2,
-                                                    par.lo, par.hi);
-            double const  wr  = bounded_leaf_weight(static_cast<double>(R.qg) * sc.x,
-                                                    static_cast<double>(R.qh) * sc.y, l1, l2,
-                                                    par.lo, par.hi);
-            double const  mid = 0.5 * (wl + wr);
-            if (mc > 0)
-            {
-                L.hi = fmin(L.hi, mid);
-                R.lo = fmax(R.lo, mid);
-            }
-            else
-            {
-                L.lo = fmax(L.lo, mid);
-                R.hi = fmin(R.hi, mid);
-            }
+            split_bounds(L, R, par, mc, *qscale, tp);
         }
         next[2 * k]       = L;
         next[(2 * k) + 1] = R;
@@ -4945,12 +5320,6 @@ __global__ void leaf_set_tree_kernel(TreeOut *dst, TreeOut t, LeafLoop *st, uint
     st->root_may  = root_may;
 }
 
-__global__ void tree_counter_kernel(uint32_t *tree_no, uint32_t step)
-{
-    pdl_enter();
-    *tree_no += step;
-}
-
 template <typename T> T *dalloc(size_t n, cudaStream_t s)
 {
     void *p = nullptr;
@@ -5195,6 +5564,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
         arena_.want<float2>(payload_, n_sel_ * p_stride_);
     }
     arena_.want<float2>(scale_, 1);
+    arena_.want<uint32_t>(ticket_, max_front_ + 1);
     arena_.alloc(plane_.pool(), s);
     sets_h_.assign(nsets, sel_h_);
     for (uint32_t k = 0; k < nsets; ++k)
@@ -5204,6 +5574,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     use_set(0);
     BB_CHECK(cudaMemsetAsync(scale_, 0, sizeof(float2), s));
     BB_CHECK(cudaMemsetAsync(dtree_, 0, 4, s));
+    BB_CHECK(cudaMemsetAsync(ticket_, 0, (max_front_ + 1) * 4, s));
     if (cfg_.leaf)
     {
         BB_CHECK(cudaMemsetAsync(leaf_tick_, 0, 8, s));
@@ -5451,11 +5822,13 @@ void Grower::seed_absmax(float2 const *gh)
     BB_LAUNCH("absmax_kernel");
 }
 
-void Grower::quantise(float2 const *gh, uint32_t n, bool have_absmax)
+void Grower::quantise(float2 const *gh, uint32_t n, bool have_absmax, OpenArgs const &open)
 {
     cudaStream_t s = stream_;
-    uint32_t const grid = std::min<uint32_t>(ceil_div(std::max<uint32_t>(n, 1), k_threads),
-                                             148u * 8u);
+    uint32_t const grid = std::min<uint32_t>(
+        std::max<uint32_t>(ceil_div(std::max<uint32_t>(n, 1), k_threads),
+                           ceil_div(open.n_zero, 4 * k_threads)),
+        148u * 8u);
     if (!have_absmax)
     {
         BB_CHECK(cudaMemsetAsync(absmax_, 0, 8, s));
@@ -5472,12 +5845,12 @@ void Grower::quantise(float2 const *gh, uint32_t n, bool have_absmax)
     if (wide_codes_)
     {
         launch_k(pdl_, quantise_kernel<true>, grid, k_threads, 0, s, gh, n, absmax_, key, dtree_,
-                 qgh16_, qscale_, row_off_);
+                 qgh16_, qscale_, row_off_, open);
     }
     else
     {
         launch_k(pdl_, quantise_kernel<false>, grid, k_threads, 0, s, gh, n, absmax_, key, dtree_,
-                 qgh8_, qscale_, row_off_);
+                 qgh8_, qscale_, row_off_, open);
     }
     BB_LAUNCH("quantise_kernel");
     n_launch_ += 1;
@@ -5494,7 +5867,7 @@ void Grower::build(uint32_t const *rows, uint32_t nfb, int dst, bool zeroed, uin
     if (quant_)
     {
         int const v = nfb == n_sel_ ? 0 : 1;
-        if (!zeroed)
+        if (!zeroed && !chain_)
         {
             launch_k(pdl_, zero_build_kernel, max_front_, k_threads, 0, s, ctl_, build_,
                      static_cast<unsigned long long *>(hist_[dst]), total_cells_ * cw_,
@@ -5626,28 +5999,34 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     size_t const find_smem = max_nb_ * (sizeof(double2) + (sizeof(unsigned long long) * cw_));
     phase_begin();
     dim3 const fgrid(front, n_sel_);
+    HeapOut const ho{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)};
+    PlanArgs const plan{sel_, plane_.cuts, plane_.cut_off, cfg_.tp, t,      pchunks_,
+                        pcr_, nbound_,     ho,             nleft_,  nright_};
+    FindChain const chain{ctl_,
+                          nodes_[cur],
+                          best_,
+                          btot_,
+                          ticket_,
+                          static_cast<unsigned long long *>(hist_[cur]),
+                          L > 0 ? static_cast<unsigned long long const *>(hist_[nxt]) : nullptr,
+                          bpair_,
+                          plan};
     if (cfg_.level)
     {
         size_t const lsmem = static_cast<size_t>(lgroup_) * max_nb_ * sizeof(double2);
-        if (quant_)
-        {
-            launch_k(pdl_, level_find_kernel<true>, n_sel_, k_lfind_thr, lsmem, s, ctl_,
-                     nodes_[cur], hist_[cur], total_cells_, cell_off_, sel_nb_, n_sel_, cfg_.tp,
-                     cand_, max_nb_, lgroup_, qscale_, cw_);
-        }
-        else
-        {
-            launch_k(pdl_, level_find_kernel<false>, n_sel_, k_lfind_thr, lsmem, s, ctl_,
-                     nodes_[cur], hist_[cur], total_cells_, cell_off_, sel_nb_, n_sel_, cfg_.tp,
-                     cand_, max_nb_, lgroup_, qscale_, cw_);
-        }
+        auto const   kern  = quant_ ? level_find_kernel<true> : level_find_kernel<false>;
+        launch_k(pdl_, kern, n_sel_, k_lfind_thr, lsmem, s, ctl_, nodes_[cur], hist_[cur],
+                 total_cells_, cell_off_, sel_nb_, n_sel_, cfg_.tp, cand_, max_nb_, lgroup_,
+                 qscale_, cw_);
     }
     else if (quant_)
     {
-        launch_k(pdl_, cw_ == 2 ? qfind_warp_kernel<true> : qfind_warp_kernel<false>,
-                 dim3(front, ceil_div(n_sel_, k_qfind_warps)), k_qfind_warps * 32, 0, s, ctl_,
-                 nodes_[cur], hist_[cur], total_cells_, cell_off_, sel_nb_, sel_, n_sel_, mono_,
-                 n_mono_, cfg_.tp, cand_, qscale_, fgroups_);
+        auto const kern = packed_  ? qfind_warp_kernel<false, true>
+                          : cw_ == 2 ? qfind_warp_kernel<true, false>
+                                     : qfind_warp_kernel<false, false>;
+        launch_k(pdl_, kern, dim3(front, ceil_div(n_sel_, k_qfind_warps)), k_qfind_warps * 32, 0, s,
+                 ctl_, nodes_[cur], hist_[cur], total_cells_, cell_off_, sel_nb_, sel_, n_sel_,
+                 mono_, n_mono_, cfg_.tp, cand_, qscale_, fgroups_, chain);
     }
     else
     {
@@ -5656,10 +6035,12 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
                  cfg_.tp, cand_, max_nb_, qscale_, nullptr, cw_, fgroups_);
     }
     BB_LAUNCH("find_kernel");
-    launch_k(pdl_, plan_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[cur], cand_, best_, n_sel_, sel_,
-             plane_.cuts, plane_.cut_off, cfg_.tp, t, pchunks_, pcr_, nbound_, cfg_.level,
-             HeapOut{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)}, nleft_, nright_);
-    BB_LAUNCH("plan_kernel");
+    if (!packed_)
+    {
+        launch_k(pdl_, plan_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[cur], cand_, best_, n_sel_,
+                 cfg_.level, plan);
+        BB_LAUNCH("plan_kernel");
+    }
     if (prof_ != nullptr)
     {
         phase_end(prof_->find_ms);
@@ -5668,10 +6049,14 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     bool const     last     = (L + 1) == cfg_.tp.max_depth;
     uint32_t const nfb      = last ? 1 : n_sel_;
     uint32_t const n_zcells = quant_ && !last ? off_h_[nfb] * cw_ : 0;
+    Plan2Args const plan2{ctl_,   nodes_[cur], nodes_[nxt], best_,   pchunks_, pcr_,
+                          pleft_, prbase_,     nleft_,      dst_,    bpair_,   build_,
+                          brange_, bchunks_,   cfg_.tp,     t,       crows_,   bbase_,
+                          cfg_.level, red_ != nullptr ? gleft_ : nullptr, fgroups_, ho,
+                          packed_ ? btot_ : nullptr, sel_, mono_, n_mono_, qscale_};
     // a walked quantised tree (unsharded) partitions in one pass: nothing
     // downstream of its row lists depends on the rows' order inside a node
-    bool const     fused    = quant_ && walk_ && red_ == nullptr;
-    if (fused)
+    if (chain_)
     {
         auto const kern = plane_.u8 ? (last ? psplit_kernel<uint8_t, false>
                                             : psplit_kernel<uint8_t, true>)
@@ -5694,10 +6079,7 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
                  nodes_[cur], best_, rows_in, plane_.bins, plane_.n_pad, sel_, sel_nb_, pleft_,
                  dirs_, LeafPlanArgs{});
     }
-    if (!fused)
-    {
-        BB_LAUNCH("pcount_kernel");
-    }
+    BB_LAUNCH("partition kernel");
     if (red_ != nullptr)
     {
         launch_k(pdl_, node_left_kernel, 1, k_plan_thr, 0, s, ctl_, pcr_, pleft_, gleft_,
@@ -5706,10 +6088,7 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
         red_->sum_u64(gleft_, max_front_, s);
         n_launch_ += 1;
     }
-    launch_k(pdl_, plan2_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[cur], nodes_[nxt], best_,
-             pchunks_, pcr_, pleft_, prbase_, nleft_, dst_, bpair_, build_, brange_, bchunks_,
-             cfg_.tp, t, crows_, bbase_, cfg_.level, red_ != nullptr ? gleft_ : nullptr, fgroups_,
-             HeapOut{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)}, fused);
+    launch_k(pdl_, chain_ ? plan2_kernel<true> : plan2_kernel<false>, 1, k_plan_thr, 0, s, plan2);
     BB_LAUNCH("plan2_kernel");
     nodes_cur_ = nodes_[cur];
     rows_cur_  = rows_in;
@@ -5723,6 +6102,19 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
                  rows_in, t, leaf_id, scores, lr);
         BB_LAUNCH("stamp_kernel");
         n_launch_ += 1;
+    }
+    if (packed_)
+    {
+        if (prof_ != nullptr)
+        {
+            phase_end(prof_->partition_ms);
+        }
+        n_launch_ += 3;
+        if (!last)
+        {
+            build(rows_out, nfb, nxt, true, front);
+        }
+        return;
     }
     if (quant_ && last && walk_)
     {
@@ -5750,10 +6142,10 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
         }
         return;
     }
-    if (!fused)
+    if (!chain_)
     {
-        launch_k(pdl_, pscatter_kernel, pch, k_threads, 0, s, ctl_, pchunks_,
-                 nodes_[cur], best_, pleft_, prbase_, nleft_, dst_, rows_in, rows_out, dirs_,
+        launch_k(pdl_, pscatter_kernel, pch, k_threads, 0, s, ctl_, pchunks_, nodes_[cur], best_,
+                 pleft_, prbase_, nleft_, dst_, rows_in, rows_out, dirs_,
                  static_cast<unsigned long long *>(hist_[nxt]), build_, total_cells_ * cw_,
                  n_zcells);
         BB_LAUNCH("pscatter_kernel");
@@ -5762,7 +6154,7 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     {
         phase_end(prof_->partition_ms);
     }
-    n_launch_ += fused ? 4 : 5;
+    n_launch_ += chain_ ? 4 : 5;
     if (quant_ && last)
     {
         // the last level's nodes are leaves: the quantised form needs their
@@ -5844,7 +6236,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         walk_ = false;
         if (quant_)
         {
-            quantise(gh, static_cast<uint32_t>(plane_.n_rows), false);
+            quantise(gh, static_cast<uint32_t>(plane_.n_rows), false, OpenArgs{});
         }
         grow_leafwise(root_rows, n_root, t, leaf_id, scores, lr);
         return;
@@ -5865,21 +6257,33 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         throw ConfigError("grower: a sharded fit needs the quantised form and every row as "
                           "the root");
     }
+    // (a shard's cells are the fit's only after a reduction between launches)
+    chain_  = quant_ && walk_ && red_ == nullptr;
+    packed_ = chain_ && !cfg_.level && cw_ == 1 && cfg_.tp.max_depth > 0;
+    uint32_t const g_root = red_ != nullptr ? static_cast<uint32_t>(total_rows_) : n_root;
+    RootArgs const root{ctl_, nodes_[0], n_root, bchunks_, brange_, build_, t, crows_, g_root,
+                        sample != nullptr ? sample->count : nullptr, heap_};
     if (quant_)
     {
         phase_begin();
-        quantise(gh, static_cast<uint32_t>(plane_.n_rows), next != nullptr);
+        OpenArgs open{};
+        if (chain_)
+        {
+            open = OpenArgs{static_cast<unsigned long long *>(hist_[0]),
+                            uint64_t{off_h_[cfg_.tp.max_depth == 0 ? 1 : n_sel_]} * cw_, wacc_, root};
+        }
+        quantise(gh, static_cast<uint32_t>(plane_.n_rows), next != nullptr, open);
         if (prof_ != nullptr)
         {
             phase_end(prof_->other_ms);
         }
     }
-    uint32_t const g_root = red_ != nullptr ? static_cast<uint32_t>(total_rows_) : n_root;
-    launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s, ctl_, nodes_[0], n_root, bchunks_,
-             brange_, build_, t, crows_, g_root, sample != nullptr ? sample->count : nullptr,
-             heap_);
-    BB_LAUNCH("root_setup_kernel");
-    n_launch_ += 1;
+    if (!chain_)
+    {
+        launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s, root);
+        BB_LAUNCH("root_setup_kernel");
+        n_launch_ += 1;
+    }
     // the root's rows: the quantised build reads an identity list implicitly
     build(quant_ && identity_root ? nullptr : root_rows,
           cfg_.tp.max_depth == 0 ? 1 : n_sel_, 0, false, 1);
@@ -5888,19 +6292,22 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         red_->sum_u64(hist_[0], total_cells_ * cw_, s);
     }
     phase_begin();
-    if (quant_)
+    if (!packed_)
     {
-        launch_k(pdl_, qroot_totals_kernel, 1, 32, 0, s, nodes_[0],
-                 static_cast<unsigned long long const *>(hist_[0]), sel_nb_, cw_);
-        BB_LAUNCH("qroot_totals_kernel");
+        if (quant_)
+        {
+            launch_k(pdl_, qroot_totals_kernel, 1, 32, 0, s, nodes_[0],
+                     static_cast<unsigned long long const *>(hist_[0]), sel_nb_, cw_);
+            BB_LAUNCH("qroot_totals_kernel");
+        }
+        else
+        {
+            launch_k(pdl_, root_totals_kernel, 1, 32, 0, s, nodes_[0],
+                     static_cast<float2 const *>(hist_[0]), sel_nb_);
+            BB_LAUNCH("root_totals_kernel");
+        }
+        n_launch_ += 1;
     }
-    else
-    {
-        launch_k(pdl_, root_totals_kernel, 1, 32, 0, s, nodes_[0],
-                 static_cast<float2 const *>(hist_[0]), sel_nb_);
-        BB_LAUNCH("root_totals_kernel");
-    }
-    n_launch_ += 1;
     if (prof_ != nullptr)
     {
         phase_end(prof_->other_ms);
@@ -5915,7 +6322,8 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
     phase_begin();
     int const fin = static_cast<int>(cfg_.tp.max_depth & 1);
     launch_k(pdl_, final_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[fin], cfg_.tp, t, pchunks_, pcr_,
-             nbound_, HeapOut{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)});
+             nbound_, HeapOut{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)},
+             dtree_, tree_step_);
     BB_LAUNCH("final_kernel");
     nodes_cur_ = nodes_[fin];
     rows_cur_  = rows_in;
@@ -5939,7 +6347,13 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         a.absmax    = next != nullptr && quant_ ? absmax_ : nullptr;
         if (quant_)
         {
-            BB_CHECK(cudaMemsetAsync(wacc_, 0, sizeof(unsigned long long) * 2 * k_walk_nodes, s));
+            if (!chain_)
+            {
+                BB_CHECK(cudaMemsetAsync(wacc_, 0, sizeof(unsigned long long) * 2 * k_walk_nodes,
+                                         s));
+            }
+            FixArgs const fix{ctl_,    t,         wacc_, nbound_, absmax_, cfg_.tp, fix_unit_,
+                              chain_ ? ticket_ : nullptr, next != nullptr ? absmax_ : nullptr};
             auto sum = [&](auto kern)
             {
                 uint32_t const wgrid =
@@ -5947,7 +6361,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
                 launch_k(pdl_, kern, wgrid, k_wsum_thr,
                          (size_t{2} << depth) * k_wsum_copies * sizeof(unsigned long long), s,
                          ctl_, mir, plane_.n_rows, heap_, leafmap_, depth, gh_cur_, absmax_,
-                         leaf16_, wacc_, sample != nullptr ? sample->bits : nullptr, fix_unit_);
+                         leaf16_, wacc_, sample != nullptr ? sample->bits : nullptr, fix_unit_, fix);
             };
             if (plane_.u8)
             {
@@ -5962,17 +6376,20 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
             {
                 red_->sum_u64(wacc_, 2 * static_cast<size_t>(k_walk_nodes), s);
             }
-            launch_k(pdl_, leaf_fix_kernel, 1, k_threads, 0, s, ctl_, t, wacc_, nbound_, absmax_,
-                     cfg_.tp, fix_unit_);
-            BB_LAUNCH("leaf_fix_kernel");
-            if (next != nullptr)
+            if (!chain_)
             {
-                BB_CHECK(cudaMemsetAsync(absmax_, 0, 8, s));
+                launch_k(pdl_, leaf_fix_kernel, 1, k_threads, 0, s, fix);
+                BB_LAUNCH("leaf_fix_kernel");
+                n_launch_ += 1;
+                if (next != nullptr)
+                {
+                    BB_CHECK(cudaMemsetAsync(absmax_, 0, 8, s));
+                }
             }
             launch_k(pdl_, walk_apply_kernel, grid, k_threads, 0, s, ctl_, t, plane_.n_rows,
                      leaf16_, a);
             BB_LAUNCH("walk_apply_kernel");
-            n_launch_ += 3;
+            n_launch_ += 2;
         }
         else
         {
@@ -6001,9 +6418,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         BB_LAUNCH("stamp_kernel");
         n_launch_ += 1;
     }
-    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_, tree_step_);
-    BB_LAUNCH("tree_counter_kernel");
-    n_launch_ += 2;
+    n_launch_ += 1;
     if (prof_ != nullptr)
     {
         phase_end(prof_->other_ms);
@@ -6046,8 +6461,8 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                              s));
     launch_k(pdl_, leaf_set_tree_kernel, 1, 1, 0, s, tdev, t, st, tp.max_depth > 0 ? 1u : 0u);
     BB_LAUNCH("leaf_set_tree_kernel");
-    launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s, ctl_, nodes_[0], n_root, bchunks_,
-             brange_, build_, t, crows_, n_root, nullptr, static_cast<uint2 *>(nullptr));
+    launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s,
+             RootArgs{ctl_, nodes_[0], n_root, bchunks_, brange_, build_, t, crows_, n_root, nullptr, nullptr});
     BB_LAUNCH("root_setup_kernel");
     launches += 2;
     build(rows_[0], n_sel_, 0, false, 1);
@@ -6071,10 +6486,10 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
         if (quant_)
         {
             // (the root's only: the pairs are found by leaf_pair_kernel)
-            launch_k(pdl_, cw_ == 2 ? qfind_warp_kernel<true> : qfind_warp_kernel<false>,
+            launch_k(pdl_, cw_ == 2 ? qfind_warp_kernel<true, false> : qfind_warp_kernel<false, false>,
                      dim3(2, ceil_div(n_sel_, k_qfind_warps)), k_qfind_warps * 32, 0, s, ctl_,
                      nodes, pool, total_cells_, cell_off_, sel_nb_, sel_, n_sel_, mono_, n_mono_,
-                     tp, cand_, qscale_, fgroups_);
+                     tp, cand_, qscale_, fgroups_, FindChain{});
         }
         else
         {
@@ -6195,7 +6610,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
     // write_leaf for every leaf, then (quantised) the FP64 renewal, then the
     // rows' leaf ids and score updates from the leaves' segments
     launch_k(pdl_, final_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[0], tp, t, pchunks_, pcr_,
-             nbound_, HeapOut{nullptr, nullptr, 0, 1});
+             nbound_, HeapOut{nullptr, nullptr, 0, 1}, dtree_, tree_step_);
     BB_LAUNCH("final_kernel");
     launches += 1;
     nodes_cur_ = nodes_[0];
@@ -6206,9 +6621,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
     launch_k(pdl_, stamp_kernel, max_pchunks_, k_threads, 0, s, ctl_, pchunks_, nodes_[0], rows_[0],
              t, leaf_id, scores, lr);
     BB_LAUNCH("stamp_kernel");
-    launch_k(pdl_, tree_counter_kernel, 1, 1, 0, s, dtree_, tree_step_);
-    BB_LAUNCH("tree_counter_kernel");
-    launches += 2;
+    launches += 1;
     // the loop's verdict: a full node table or pool is the reference's
     // capacity refusal
     auto *lh = static_cast<LeafLoop *>(lout_h_);
@@ -6247,11 +6660,13 @@ void Grower::populate(float2 const *gh, uint32_t const *rows, uint32_t n, double
     t.default_left = reinterpret_cast<uint8_t *>(scratch + 32);
     if (quant_)
     {
-        quantise(gh, static_cast<uint32_t>(plane_.n_rows), false);
+        quantise(gh, static_cast<uint32_t>(plane_.n_rows), false, OpenArgs{});
     }
-    walk_ = false;
-    launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s, ctl_, nodes_[0], n, bchunks_, brange_,
-             build_, t, crows_, n, nullptr, heap_);
+    walk_   = false;
+    chain_  = false;
+    packed_ = false;
+    launch_k(pdl_, root_setup_kernel, 1, k_threads, 0, s,
+             RootArgs{ctl_, nodes_[0], n, bchunks_, brange_, build_, t, crows_, n, nullptr, heap_});
     BB_LAUNCH("root_setup_kernel");
     build(rows, n_sel_, 0, false, 1);
     std::vector<double2> cells(total_cells_);

@@ -84,6 +84,8 @@ struct RootSample
     uint32_t const *bits;
 };
 
+struct OpenArgs;
+
 struct TreeOut
 {
     uint32_t *feature;
@@ -370,8 +372,12 @@ class Grower
     Node const     *nodes_cur_ = nullptr;
     uint32_t const *rows_cur_  = nullptr;
     uint32_t const *root_rows_ = nullptr;
-    void      quantise(float2 const *gh, uint32_t n, bool have_absmax);
-    bool      walk_ = false; // this tree's rows are stamped by the final walk
+    void      quantise(float2 const *gh, uint32_t n, bool have_absmax, OpenArgs const &open);
+    bool      walk_  = false; // this tree's rows are stamped by the final walk
+    bool      chain_ = false; // a walked, unsharded quantised tree: opened beside its
+                              // quantisation, partitioned in one pass
+    bool      packed_ = false; // and its levels are the level chain (FindChain)
+    uint32_t *ticket_ = nullptr; // last-block counters: the launch's, each node's
     Reducer  *red_        = nullptr; // shard reducer, or none
     uint64_t  row_off_    = 0;       // the shard's first row in the fit
     uint64_t  total_rows_ = 0;       // rows of the whole fit
