@@ -31,7 +31,8 @@
 // which adds them in tree order. Batches of up to a few hundred rows take a CTA
 // per row, a thread per tree and the nodes straight from L2
 // (row_predict_kernel), up to 64 rows several CTAs per row. Depths 9 and 10 take a lane
-// per row (heap_predict_kernel). Deeper ensembles, or planes wider than 8
+// per row (heap_predict_kernel), and so do shallow trees over batches that fill
+// its passes. Deeper ensembles, or planes wider than 8
 // mirror tiles (256 u8 / 128 u16 features), use the node form: the reference's
 // layout and walk, nodes in global memory.
 #include "bonsai_b200.h"
@@ -439,11 +440,15 @@ __global__ void __launch_bounds__(k_few_threads)
     }
 }
 
-// ---- a lane per row (depths 9 and 10) ----
+// ---- a lane per row (depths 9 and 10, and full waves of shallow trees) ----
 
+// BY32: the heaps are those of the lane-per-tree form (32 trees interleaved, a
+// row's words one after another) and are turned while they are staged: each
+// tree's slots together, an odd stride from tree to tree, the code offsets
+// for a lane's column of the staged codes.
 // Scores of rows [blockIdx.x * rows_per_cta, + rows_per_cta), taken T x R
 // rows at a time: out[r] = init + lr * sum.
-template <typename CodeT, uint32_t D, uint32_t T, uint32_t R>
+template <typename CodeT, uint32_t D, uint32_t T, uint32_t R, bool BY32>
 __global__ void __launch_bounds__(T)
     heap_predict_kernel(uint4 const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
                         uint32_t const *__restrict__ last_words,
@@ -452,6 +457,7 @@ __global__ void __launch_bounds__(T)
                         float *__restrict__ out)
 {
     constexpr uint32_t slots = 2u << D; // per tree: root at 1, leaves at [2^D, 2^(D+1))
+    constexpr uint32_t pitch = slots + (BY32 ? 1u : 0u);
     constexpr uint32_t warps = T / 32;
     constexpr bool     u8    = sizeof(CodeT) == 1;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -512,6 +518,32 @@ __global__ void __launch_bounds__(T)
         {
             uint32_t const nc = min(chunk_trees, n_trees - c0);
             __syncthreads(); // codes staged; the previous chunk's walks done
+            if constexpr (BY32)
+            {
+                // four trees' words of a slot at a time; a chunk is whole
+                // groups of 32 trees, or a part of one
+                auto const *src  = reinterpret_cast<uint4 const *>(heaps);
+                auto const  turn = [](uint32_t e, bool inner)
+                { return inner ? ((e & 0xFFFC0000u) << 5) | (e & 0x3FFFFu) : e; };
+                uint32_t const wide = min(8u, chunk_trees / 4u);
+                uint32_t const q0   = c0 / 4u;
+                uint32_t const n16  = ((nc + (4u * wide) - 1) / (4u * wide)) * slots * wide;
+                for (uint32_t i = threadIdx.x; i < n16; i += T)
+                {
+                    uint32_t const sub   = i % wide;
+                    uint32_t const slot  = (i / wide) % slots;
+                    uint32_t const blk   = i / (wide * slots);
+                    uint4 const    x     = src[(((((q0 / 8u) + blk) * slots) + slot) * 8u) +
+                                        (q0 % 8u) + sub];
+                    bool const     inner = slot < (1u << D);
+                    uint32_t      *dst   = heap_s + (((blk * 32u) + (sub * 4u)) * pitch) + slot;
+                    dst[0]               = turn(x.x, inner);
+                    dst[pitch]           = turn(x.y, inner);
+                    dst[2 * pitch]       = turn(x.z, inner);
+                    dst[3 * pitch]       = turn(x.w, inner);
+                }
+            }
+            else
             {
                 auto const *src =
                     reinterpret_cast<uint4 const *>(heaps + (static_cast<size_t>(c0) * slots));
@@ -528,7 +560,7 @@ __global__ void __launch_bounds__(T)
                 // byte addresses in the shared window: slot i of this tree
                 // at tb + 4i; from p = tb + 4n the child 2n (+1) is
                 // 2p - tb (+4)
-                uint32_t const tb = heap_a + (j * slots * 4u);
+                uint32_t const tb = heap_a + (j * pitch * 4u);
                 uint32_t const cl = 0u - tb;
                 uint32_t const cr = 4u - tb;
                 uint32_t p[R];
@@ -653,6 +685,7 @@ struct bb_predict_plan
     uint32_t    n_tiles = 0;
     uint32_t    sms     = 1;
     uint32_t    lane_rows = 0; // a lane CTA's most rows
+    uint64_t    heap_ctas = 0; // resident CTAs of the lane-per-row form; 0: not taken
     bb::DeviceBuf heaps;
     bb::DeviceBuf vals;       // a few rows' leaf values
     bb::DeviceBuf last_words; // per staged code word, its features' last bins
@@ -805,13 +838,44 @@ void plan_check_plane(bb_predict_plan const &pl, Plane const &p)
 using HeapFn = void (*)(uint4 const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
                         uint32_t, uint32_t, uint32_t, float, float, float *);
 
+template <typename CodeT> HeapFn heap_fn_d(uint32_t D)
+{
+    switch (D)
+    {
+    case 1: return heap_predict_kernel<CodeT, 1, 512, 2, true>;
+    case 2: return heap_predict_kernel<CodeT, 2, 512, 2, true>;
+    case 3: return heap_predict_kernel<CodeT, 3, 512, 2, true>;
+    case 4: return heap_predict_kernel<CodeT, 4, 512, 2, true>;
+    case 5: return heap_predict_kernel<CodeT, 5, 512, 2, true>;
+    case 6: return heap_predict_kernel<CodeT, 6, 512, 2, true>;
+    case 7: return heap_predict_kernel<CodeT, 7, 512, 2, true>;
+    case 8: return heap_predict_kernel<CodeT, 8, 512, 2, true>;
+    case 9: return heap_predict_kernel<CodeT, 9, 512, 2, false>;
+    case 10: return heap_predict_kernel<CodeT, 10, 512, 2, false>;
+    default: throw std::logic_error("bb_predict_plan: heap depth out of range");
+    }
+}
+
 HeapFn heap_fn(bool u8, uint32_t D)
 {
-    if (D == 9)
-    {
-        return u8 ? heap_predict_kernel<uint8_t, 9, 512, 2> : heap_predict_kernel<uint16_t, 9, 512, 2>;
-    }
-    return u8 ? heap_predict_kernel<uint8_t, 10, 512, 2> : heap_predict_kernel<uint16_t, 10, 512, 2>;
+    return u8 ? heap_fn_d<uint8_t>(D) : heap_fn_d<uint16_t>(D);
+}
+
+// A lane per row: the trees of a chunk, and the shared memory of a CTA of 1,024
+// rows (both code variants, 64 bytes a row and mirror tile) with it.
+uint32_t heap_chunk(uint32_t D)
+{
+    uint32_t const tree_bytes = (2u << D) * 4u;
+    uint32_t const chunk      = std::max(1u, k_chunk_bytes / tree_bytes);
+    // (depth 8: half a group of 32, depth 7: one; of 16 KB, 8 and 16 trees, whose
+    // reads are not whole lines, a pass took 8% and 4% longer)
+    return D <= 6 ? chunk & ~31u : (D <= k_lane_depth ? 2 * chunk : chunk);
+}
+
+size_t heap_smem(uint32_t D, uint32_t n_tiles)
+{
+    size_t const tree_bytes = ((2u << D) + (D <= k_lane_depth ? 1u : 0u)) * 4u;
+    return (size_t{1024} * n_tiles * 64) + (heap_chunk(D) * tree_bytes);
 }
 
 using LaneFn = void (*)(uint32_t const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
@@ -852,6 +916,42 @@ uint32_t sm_count()
     check(cudaGetDevice(&dev), "cudaGetDevice");
     check(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
     return static_cast<uint32_t>(std::max(n, 1));
+}
+
+// A lane per row: one wave of resident CTAs, each over an equal run of rows.
+uint32_t heap_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, float *out,
+                     cudaStream_t s)
+{
+    uint64_t const n   = p.n_rows;
+    uint64_t const per = std::max<uint64_t>(
+        32, ((((n + pl.heap_ctas - 1) / pl.heap_ctas) + 31) / 32) * 32);
+    heap_fn(pl.u8, pl.depth)<<<ceil_div(n, per), 512, heap_smem(pl.depth, pl.n_tiles), s>>>(
+        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words.as<uint32_t>(),
+        pl.heaps.as<uint32_t>(), n_trees, heap_chunk(pl.depth), static_cast<uint32_t>(per), pl.lr,
+        pl.init, out);
+    BB_LAUNCH("heap_predict_kernel");
+    return 1;
+}
+
+// Whether a lane per row is the faster form at depths up to k_lane_depth. It has
+// no step between a walk's end and the sum, but takes whole passes of 1,024
+// rows a CTA. Measured at full passes, picoseconds a row over all SMs: about
+// 34 + 0.31 x trees x depth (0.33 at depth 8, staged in half lines), and a fifth
+// more with two mirror tiles; a lane per tree: 20 and, for every 32 trees,
+// 25 + 7 x depth. (589,039 rows, 100 trees of depth 4 / 250 of depth 5: 84 / 236 us
+// a lane per row, 132 / 279 a lane per tree; 150,000 rows, half a pass: 55 / 132
+// and 44 / 86; 300,000 rows, 1,000 trees of depth 8: 885 and 811.)
+bool by_row(bb_predict_plan const &pl, uint64_t n, uint32_t n_trees)
+{
+    uint64_t const pass   = uint64_t{1024} * pl.heap_ctas;
+    double const   passes = static_cast<double>(((n + pass - 1) / pass) * pass);
+    double const   node   = pl.depth == 8 ? 0.333 : 0.31;
+    double const   row =
+        passes * (34.0 + (node * n_trees * pl.depth)) * (pl.n_tiles > 1 ? 1.2 : 1.0);
+    double const   tree =
+        static_cast<double>(n) * (20.0 + (25.0 * (pl.n_tiles - 1)) +
+                                  (((n_trees + 31) / 32) * (25.0 + (7.0 * pl.depth))));
+    return row < tree;
 }
 
 // Enqueues the scores of the plan's first n_trees trees over plane p into
@@ -911,6 +1011,10 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
             BB_LAUNCH("row_predict_kernel");
             return 1;
         }
+        if (pl.heap_ctas != 0 && by_row(pl, n, n_trees))
+        {
+            return heap_launch(pl, p, n_trees, out, s);
+        }
         // equal tiles, in as few waves of two CTAs an SM as the largest allows
         uint64_t const wave  = uint64_t{2} * pl.sms;
         uint64_t const waves = (n + (wave * pl.lane_rows) - 1) / (wave * pl.lane_rows);
@@ -922,25 +1026,7 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
         BB_LAUNCH("lane_predict_kernel");
         return 1;
     }
-    uint32_t const tree_bytes = (2u << pl.depth) * 4u;
-    uint32_t const chunk      = std::max(1u, k_chunk_bytes / tree_bytes);
-    // both code variants of a row: 64 bytes per mirror tile; two rows a thread
-    // of 512
-    size_t const smem = (size_t{1024} * pl.n_tiles * 64) + (size_t{chunk} * tree_bytes);
-    HeapFn const fn   = heap_fn(pl.u8, pl.depth);
-    allow_smem(fn);
-    // one wave of resident CTAs, each over an equal run of rows
-    int occ = 0;
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 512, smem),
-          "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    uint64_t const ctas = static_cast<uint64_t>(std::max(occ, 1)) * pl.sms;
-    uint64_t const per  = std::max<uint64_t>(32, ((((n + ctas - 1) / ctas) + 31) / 32) * 32);
-    fn<<<ceil_div(n, per), 512, smem, s>>>(static_cast<uint4 const *>(p.mirror), n, pl.n_tiles,
-                                           pl.last_words.as<uint32_t>(), pl.heaps.as<uint32_t>(),
-                                           n_trees, chunk, static_cast<uint32_t>(per), pl.lr,
-                                           pl.init, out);
-    BB_LAUNCH("heap_predict_kernel");
-    return 1;
+    return heap_launch(pl, p, n_trees, out, s);
 }
 
 std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
@@ -1004,6 +1090,16 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
                 pk.fill(h.data() + (t * slots), roots[t], roots[t], 1, 0);
             }
             pl->heaps.upload(h.data(), h.size() * 4);
+        }
+        if (D > k_lane_depth || n_tiles <= 2)
+        {
+            HeapFn const fn = heap_fn(p.u8, D);
+            allow_smem(fn);
+            int occ = 0;
+            check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 512,
+                                                                heap_smem(D, n_tiles)),
+                  "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+            pl->heap_ctas = static_cast<uint64_t>(std::max(occ, 1)) * pl->sms;
         }
         // the last bin of every code lane of every staged word (padding
         // lanes: a value no code has)
