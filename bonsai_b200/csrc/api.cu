@@ -270,34 +270,10 @@ __global__ void fill_kernel(float *x, float v, uint64_t n)
     }
 }
 
-// Copies the scratch tree into slot *round + k and advances the counter by
-// step, so a captured boosting round needs no per-round pointer. (Class trees
-// grown side by side commit with step 0, and advance_kernel follows them.)
-__global__ void commit_tree_kernel(TreeOut scratch, TreeOut slots, uint32_t cap,
-                                   uint32_t *round, uint32_t k, uint32_t step)
+// A leafwise tree, which no walk ends, into its slot.
+__global__ void commit_tree_kernel(TreeOut scratch, TreeCommit c)
 {
-    uint32_t const r   = *round + k;
-    uint64_t const off = static_cast<uint64_t>(r) * cap;
-    for (uint32_t i = threadIdx.x; i < cap; i += blockDim.x)
-    {
-        slots.feature[off + i]      = scratch.feature[i];
-        slots.value[off + i]        = scratch.value[i];
-        slots.left[off + i]         = scratch.left[i];
-        slots.right[off + i]        = scratch.right[i];
-        slots.default_left[off + i] = scratch.default_left[i];
-        slots.gain[off + i]         = scratch.gain[i];
-        slots.cover[off + i]        = scratch.cover[i];
-        slots.split_bin[off + i]    = scratch.split_bin[i];
-    }
-    if (threadIdx.x < 3)
-    {
-        slots.meta[(3 * static_cast<uint64_t>(r)) + threadIdx.x] = scratch.meta[threadIdx.x];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && step != 0)
-    {
-        *round = r + step;
-    }
+    commit_tree(scratch, c);
 }
 
 __global__ void advance_kernel(uint32_t *round, uint32_t step)
@@ -907,7 +883,7 @@ struct bb_booster
         if (L.grower->fuses_next())
         {
             L.grower->grow(g, L.srows, static_cast<uint32_t>(n), L.scratch.t, li, sc, lr, false, next,
-                         &rs);
+                           &rs, slot(k));
             return;
         }
         L.grower->grow(g, L.srows, host_counts[k], L.scratch.t, li, sc, lr, false, nullptr);
@@ -941,10 +917,24 @@ struct bb_booster
         }
     }
 
-    // one grow's kernels and the commit after it
-    void count_tree(uint32_t k)
+    // Where tree k of the round goes.
+    bb::TreeCommit slot(uint32_t k)
     {
-        round_launches += lane(k).grower->launches_per_tree() + 1;
+        bool const side = lanes.size() > 1;
+        return {trees.t, trees.cap, round, side ? k : 0u, side ? 0u : 1u};
+    }
+
+    // After a grow: a leafwise tree into its slot, the grow's launches counted.
+    void finish_tree(uint32_t k)
+    {
+        Lane &L = lane(k);
+        if (!L.grower->fuses_next())
+        {
+            commit_tree_kernel<<<1, 256, 0, L.stream>>>(L.scratch.t, slot(k));
+            BB_LAUNCH("commit_tree_kernel");
+            round_launches += 1;
+        }
+        round_launches += L.grower->launches_per_tree();
     }
 
     void eval_round()
@@ -1019,12 +1009,10 @@ struct bb_booster
                 else
                 {
                     L.grower->grow(gh + (k * n), rows, static_cast<uint32_t>(n), L.scratch.t,
-                                   leaf_ids(k), scores + (k * n), lr, true, nullptr);
+                                   leaf_ids(k), scores + (k * n), lr, true, nullptr, nullptr,
+                                   slot(k));
                 }
-                commit_tree_kernel<<<1, 256, 0, L.stream>>>(L.scratch.t, trees.t, trees.cap,
-                                                            round, side ? k : 0u, side ? 0u : 1u);
-                BB_LAUNCH("commit_tree_kernel");
-                count_tree(k);
+                finish_tree(k);
             }
             for (Lane &L : lanes)
             {
@@ -1060,10 +1048,7 @@ struct bb_booster
                 L.grower->grow(gh, rows, static_cast<uint32_t>(n), L.scratch.t,
                              leaf_ids(0), scores, lr, true, nullptr);
             }
-            commit_tree_kernel<<<1, 256, 0, stream>>>(L.scratch.t, trees.t, trees.cap, round,
-                                                     0, 1);
-            BB_LAUNCH("commit_tree_kernel");
-            count_tree(0);
+            finish_tree(0);
             round_launches += 1; // the gradient pass
             return;
         }
@@ -1075,12 +1060,9 @@ struct bb_booster
         else
         {
             L.grower->grow(gh, rows, static_cast<uint32_t>(n), L.scratch.t,
-                         leaf_ids(0), scores, lr, true, &next);
+                           leaf_ids(0), scores, lr, true, &next, nullptr, slot(0));
         }
-        commit_tree_kernel<<<1, 256, 0, stream>>>(L.scratch.t, trees.t, trees.cap, round,
-                                                     0, 1);
-        BB_LAUNCH("commit_tree_kernel");
-        count_tree(0);
+        finish_tree(0);
     }
 };
 

@@ -2608,6 +2608,11 @@ struct Plan2Args
     int8_t const   *mono;
     uint32_t        n_mono;
     double2 const  *qscale;
+    // the last level of such a tree: the children are its last leaves
+    bool      last;
+    double2  *nbound;
+    uint32_t *tree_no;
+    uint32_t  tree_step;
 };
 
 // The children's bounds after a split on a constrained feature, from their
@@ -2785,6 +2790,13 @@ template <uint32_t NT, bool FUSED> __device__ __forceinline__ void plan_children
                 split_bounds(L, R, nd, mc, *A.qscale, tp);
             }
         }
+        if (FUSED && A.last)
+        {
+            A.nbound[lid] = make_double2(L.lo, L.hi);
+            A.nbound[rid] = make_double2(R.lo, R.hi);
+            heap_leaf(ho, L.heap, lid); // (leaves of value 0 until the walk's sums)
+            heap_leaf(ho, R.heap, rid);
+        }
         next[2 * k]         = L;
         next[(2 * k) + 1]   = R;
         t.cover[lid]        = static_cast<float>(gnl);
@@ -2826,6 +2838,17 @@ template <uint32_t NT, bool FUSED> __device__ __forceinline__ void plan_children
         {
             ctl->depth += 1;
         }
+        if (FUSED && A.last)
+        {
+            t.meta[0]   = ctl->n_nodes;
+            t.meta[1]   = ctl->depth;
+            t.meta[2]   = ctl->n_leaves + (2 * n_surv);
+            *A.tree_no += A.tree_step; // (the tree's roundings are done)
+        }
+    }
+    if (FUSED && A.last)
+    {
+        return;
     }
     __syncthreads();
     fill_chunk_table<NT>(
@@ -2909,6 +2932,7 @@ struct WalkArgs
     float2       *gh;
     uint32_t     *absmax;
     float const  *weights;
+    TreeCommit    commit; // the finished tree's slot, or none
 };
 
 __device__ __forceinline__ uint32_t pick_word(uint32_t const w[8], uint32_t i)
@@ -3109,6 +3133,10 @@ __global__ void __launch_bounds__(k_threads)
     {
         block_absmax(mg, mh, a.absmax);
     }
+    if (a.commit.round != nullptr && blockIdx.x == gridDim.x - 1)
+    {
+        commit_tree(t, a.commit);
+    }
 }
 
 __device__ __forceinline__ bool in_sample(uint32_t const *bits, uint64_t r)
@@ -3291,6 +3319,10 @@ __global__ void __launch_bounds__(k_threads)
     if (a.absmax != nullptr)
     {
         block_absmax(mg, mh, a.absmax);
+    }
+    if (a.commit.round != nullptr && blockIdx.x == gridDim.x - 1)
+    {
+        commit_tree(t, a.commit);
     }
 }
 
@@ -6053,7 +6085,8 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
                           pleft_, prbase_,     nleft_,      dst_,    bpair_,   build_,
                           brange_, bchunks_,   cfg_.tp,     t,       crows_,   bbase_,
                           cfg_.level, red_ != nullptr ? gleft_ : nullptr, fgroups_, ho,
-                          packed_ ? btot_ : nullptr, sel_, mono_, n_mono_, qscale_};
+                          packed_ ? btot_ : nullptr, sel_, mono_, n_mono_, qscale_,
+                          packed_ && last, nbound_, dtree_, tree_step_};
     // a walked quantised tree (unsharded) partitions in one pass: nothing
     // downstream of its row lists depends on the rows' order inside a node
     if (chain_)
@@ -6216,7 +6249,8 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
 
 void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
                   TreeOut const &t, uint32_t *leaf_id, float *scores, float lr,
-                  bool identity_root, NextRound const *next, RootSample const *sample)
+                  bool identity_root, NextRound const *next, RootSample const *sample,
+                  TreeCommit const &commit)
 {
     if (n_root > max_rows_)
     {
@@ -6321,10 +6355,16 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
     }
     phase_begin();
     int const fin = static_cast<int>(cfg_.tp.max_depth & 1);
-    launch_k(pdl_, final_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[fin], cfg_.tp, t, pchunks_, pcr_,
-             nbound_, HeapOut{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)},
-             dtree_, tree_step_);
-    BB_LAUNCH("final_kernel");
+    if (!packed_)
+    {
+        launch_k(pdl_, final_kernel, 1, k_plan_thr, 0, s, ctl_, nodes_[fin], cfg_.tp, t, pchunks_,
+                 pcr_, nbound_,
+                 HeapOut{heap_, leafmap_, cfg_.tp.max_depth,
+                         k_mirror_bytes / (plane_.u8 ? 1u : 2u)},
+                 dtree_, tree_step_);
+        BB_LAUNCH("final_kernel");
+        n_launch_ += 1;
+    }
     nodes_cur_ = nodes_[fin];
     rows_cur_  = rows_in;
     if (walk_)
@@ -6337,6 +6377,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         auto const    *mir   = static_cast<uint4 const *>(plane_.mirror);
         uint32_t const depth = cfg_.tp.max_depth;
         WalkArgs a{};
+        a.commit    = commit;
         a.scores    = scores;
         a.leaf_id   = leaf_id;
         a.lr        = lr;
@@ -6418,7 +6459,6 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
         BB_LAUNCH("stamp_kernel");
         n_launch_ += 1;
     }
-    n_launch_ += 1;
     if (prof_ != nullptr)
     {
         phase_end(prof_->other_ms);

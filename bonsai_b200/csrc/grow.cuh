@@ -151,6 +151,57 @@ struct NextRound
     float const *weights   = nullptr; // per row, or nullptr (unweighted)
 };
 
+// Where a finished tree goes: slot *round + k of slots, and *round advanced by
+// step, so a captured boosting round needs no per-round pointer. (Class trees
+// grown side by side commit with step 0; the booster advances after them.)
+struct TreeCommit
+{
+    TreeOut   slots{};
+    uint32_t  cap   = 0;
+    uint32_t *round = nullptr; // null: not committed here
+    uint32_t  k     = 0;
+    uint32_t  step  = 0;
+};
+
+#ifdef __CUDACC__
+// By one block. (The walk's last block does it beside the others' rows: a launch
+// of its own took 6-11 us of a round.)
+__device__ __forceinline__ void commit_tree(TreeOut const &scratch, TreeCommit const &c)
+{
+    uint32_t const r   = *c.round + c.k;
+    uint64_t const off = static_cast<uint64_t>(r) * c.cap;
+#pragma unroll 2
+    for (uint32_t i = threadIdx.x; i < c.cap; i += blockDim.x)
+    {
+        uint32_t const feature   = scratch.feature[i];
+        float const    value     = scratch.value[i];
+        uint32_t const left      = scratch.left[i];
+        uint32_t const right     = scratch.right[i];
+        uint8_t const  dl        = scratch.default_left[i];
+        float const    gain      = scratch.gain[i];
+        float const    cover     = scratch.cover[i];
+        uint32_t const split_bin = scratch.split_bin[i];
+        c.slots.feature[off + i]      = feature;
+        c.slots.value[off + i]        = value;
+        c.slots.left[off + i]         = left;
+        c.slots.right[off + i]        = right;
+        c.slots.default_left[off + i] = dl;
+        c.slots.gain[off + i]         = gain;
+        c.slots.cover[off + i]        = cover;
+        c.slots.split_bin[off + i]    = split_bin;
+    }
+    if (threadIdx.x < 3)
+    {
+        c.slots.meta[(3 * static_cast<uint64_t>(r)) + threadIdx.x] = scratch.meta[threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && c.step != 0)
+    {
+        *c.round = r + c.step;
+    }
+}
+#endif
+
 struct GrowConfig
 {
     TreeParams tp;
@@ -211,7 +262,8 @@ class Grower
     void grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
               TreeOut const &out, uint32_t *leaf_id, float *scores, float lr,
               bool identity_root = false, NextRound const *next = nullptr,
-              RootSample const *sample = nullptr);
+              RootSample const *sample = nullptr,
+              TreeCommit const &commit = {});
     // The quantised form's gradient maxima of gh (every dataset row), for a
     // first grow() whose next round is fused.
     void seed_absmax(float2 const *gh);
