@@ -105,14 +105,16 @@ __device__ __forceinline__ uint64_t l2_policy_last()
     return p;
 }
 
-// A read-only 16-byte load that skips L1 and carries an L2 policy.
-__device__ __forceinline__ uint4 ld_nc_v4(uint4 const *src, uint64_t pol)
+// A row's 32 bytes of a mirror tile (32-byte aligned) in one load: two of 16
+// bytes looked the sector up twice, and where the first's line had left L1 by
+// the second, fetched it twice.
+__device__ __forceinline__ void ld_nc_row(uint4 const *src, uint64_t pol, uint4 &a, uint4 &b)
 {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v8.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z),
+                   "=r"(b.w)
                  : "l"(src), "l"(pol));
-    return v;
 }
 
 // A 4-byte load with an L2 policy, through the coherent path.
@@ -3111,10 +3113,9 @@ __global__ void __launch_bounds__(k_threads)
         uint64_t const r1  = r0 + stride;
         bool const     two = r1 < n_rows;
         uint64_t const rb  = two ? r1 : r0;
-        uint4 const    a0  = ld_nc_v4(mt + (r0 * 2), pol);
-        uint4 const    b0  = ld_nc_v4(mt + (r0 * 2) + 1, pol);
-        uint4 const    a1  = ld_nc_v4(mt + (rb * 2), pol);
-        uint4 const    b1  = ld_nc_v4(mt + (rb * 2) + 1, pol);
+        uint4          a0, b0, a1, b1;
+        ld_nc_row(mt + (r0 * 2), pol, a0, b0);
+        ld_nc_row(mt + (rb * 2), pol, a1, b1);
         float const    s0  = a.scores != nullptr ? a.scores[r0] : 0.0F;
         float const    s1  = a.scores != nullptr ? a.scores[rb] : 0.0F;
         float const    y0  = a.gh != nullptr ? a.labels[r0] : 0.0F;
@@ -3237,10 +3238,9 @@ __global__ void __launch_bounds__(k_wsum_thr)
         uint64_t const r1  = r0 + stride;
         bool const     two = r1 < n_rows;
         uint64_t const rb  = two ? r1 : r0;
-        uint4 const    a0  = ld_nc_v4(mt + (r0 * 2), pol);
-        uint4 const    b0  = ld_nc_v4(mt + (r0 * 2) + 1, pol);
-        uint4 const    a1  = ld_nc_v4(mt + (rb * 2), pol);
-        uint4 const    b1  = ld_nc_v4(mt + (rb * 2) + 1, pol);
+        uint4          a0, b0, a1, b1;
+        ld_nc_row(mt + (r0 * 2), pol, a0, b0);
+        ld_nc_row(mt + (rb * 2), pol, a1, b1);
         // a row outside this tree's sample takes its leaf but adds nothing
         float2 const   g0  = in_sample(bits, r0) ? gh[r0] : make_float2(0.0F, 0.0F);
         float2 const   g1  = in_sample(bits, rb) ? gh[rb] : make_float2(0.0F, 0.0F);
@@ -4051,12 +4051,18 @@ __global__ void __launch_bounds__(k_qthreads, 3)
 // Persistent: a grid of up to k_qctas CTAs per tile (one per SM; fewer for a
 // small dataset, so several fits share the GPU), each walking a
 // contiguous range of the level's chunks (node-ordered), so no wave tail.
-// The gathers are software-pipelined through registers: while a chunk's rows
-// are added, the thread's loads of the next chunk's row ids, gradient codes
-// and 32-byte tiles (two 16-byte non-coherent loads per row) are in flight,
-// the loop unrolled by two so the prefetched registers are never moved (a
-// move would wait for its load); with no shared staging the load/store path
-// carries only the reductions. The shared
+// The loads are software-pipelined through registers: while a chunk's rows are
+// added, the next chunk's codes and 32-byte tiles (one load a row), the row ids
+// of the one after and the descriptor of the one after that are in flight, so
+// that no load waits for the one that addresses it; the loop is unrolled by two
+// so the prefetched registers are never moved (a move would wait for its
+// load); with no shared staging the load/store path carries only the reductions
+// (a reduction takes two cycles of it; the root's build is at 85% of that bound,
+// the lower levels' wait for scattered DRAM sectors). 10,000,000 rows x 28, us:
+// the root 132 before, 110 now, the next two levels 75 and 72, 60 and 70, the
+// others as before; the round at 1,000,000 x depth 8 436 and 383. Shared memory
+// beyond the table costs L1, which the loads in flight need (72 KB more: 96 to
+// 108 us a level). The shared
 // histogram flushes -- one packed 64-bit global add per touched cell,
 // gradient in the high word (two's complement), hessian in the low word --
 // only when the node changes. The 32-bit shared words cannot overflow in
@@ -4085,38 +4091,70 @@ __device__ __forceinline__ void red_shared_u32_hi(uint32_t addr, uint32_t v)
     asm volatile("red.shared.add.u32 [%0+128], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
+// The table into the node's cells, and zeroed. Warp w takes bins [8w, 8w + 8):
+// read lane = feature, turned in their own place so that eight lanes add one
+// feature's eight consecutive cells (a lane per feature sent every add to a
+// sector of its own: 8,192 a flush).
 template <bool CW2>
-__device__ __forceinline__ void qflush_t(uint32_t *tbl, uint32_t max_nb, int32_t const *j_s,
-                                         uint32_t const *sel_nb, uint32_t const *cell_off,
-                                         unsigned long long *dst)
+__device__ __forceinline__ void qflush_t(uint32_t *tbl, uint32_t max_nb, uint32_t const *nb_s,
+                                         uint32_t const *off_s, unsigned long long *dst)
 {
     __syncthreads();
-    for (uint32_t x = threadIdx.x; x < 256 * 32; x += k_tthreads)
+    uint32_t const lane = threadIdx.x & 31;
+    uint32_t const b0   = (threadIdx.x >> 5) * 8;
+    uint32_t      *mine = tbl + (b0 * 64);
+    auto          *turn = reinterpret_cast<unsigned long long *>(mine);
+    if (b0 < max_nb)
     {
-        uint32_t const f  = x & 31;
-        uint32_t const bb = x >> 5;
-        uint32_t const gi = (bb * 64) + f;
-        uint32_t const g  = tbl[gi];
-        uint32_t const h  = tbl[gi + 32];
-        int32_t const  j2 = j_s[f];
-        if (bb < max_nb && j2 >= 0 && bb < sel_nb[j2] && (g != 0 || h != 0))
+        unsigned long long v[8];
+#pragma unroll
+        for (uint32_t b = 0; b < 8; ++b)
         {
-            uint64_t const cell = cell_off[j2] + bb;
-            if constexpr (CW2)
+            v[b] = (static_cast<unsigned long long>(mine[(b * 64) + lane]) << 32) |
+                   mine[(b * 64) + 32 + lane];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t b = 0; b < 8; ++b)
+        {
+            turn[(lane * 8) + (b ^ (lane & 7))] = v[b];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q)
+        {
+            uint32_t const f = (q * 4) + (lane >> 3);
+            v[q]             = turn[(f * 8) + ((lane ^ f) & 7)];
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t x = 0; x < 4; ++x)
+        {
+            reinterpret_cast<uint4 *>(mine)[(x * 32) + lane] = make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q)
+        {
+            uint32_t const f = (q * 4) + (lane >> 3);
+            uint32_t const b = b0 + (lane & 7);
+            if (v[q] != 0 && b < nb_s[f]) // (0 bins: not selected)
             {
-                // two-word cells: the int64 gradient sum, the uint64 hessian sum
-                atomicAdd(&dst[2 * cell], static_cast<unsigned long long>(
-                                              static_cast<int64_t>(static_cast<int32_t>(g))));
-                atomicAdd(&dst[(2 * cell) + 1], static_cast<unsigned long long>(h));
-            }
-            else
-            {
-                atomicAdd(&dst[cell], (static_cast<unsigned long long>(g) << 32) +
-                                          static_cast<unsigned long long>(h));
+                uint64_t const cell = off_s[f] + b;
+                if constexpr (CW2)
+                {
+                    // two-word cells: the int64 gradient sum, the uint64 hessian sum
+                    atomicAdd(&dst[2 * cell],
+                              static_cast<unsigned long long>(static_cast<int64_t>(
+                                  static_cast<int32_t>(static_cast<uint32_t>(v[q] >> 32)))));
+                    atomicAdd(&dst[(2 * cell) + 1],
+                              static_cast<unsigned long long>(static_cast<uint32_t>(v[q])));
+                }
+                else
+                {
+                    atomicAdd(&dst[cell], v[q]);
+                }
             }
         }
-        tbl[gi]      = 0;
-        tbl[gi + 32] = 0;
     }
     __syncthreads();
 }
@@ -4169,7 +4207,8 @@ __global__ void __launch_bounds__(k_tthreads, 1)
 {
     pdl_enter();
     extern __shared__ uint4 t_smem[];
-    __shared__ int32_t      j_s[32];
+    __shared__ uint32_t     nb_s[32]; // per tile slot: its feature's bins (0: not selected)
+    __shared__ uint32_t     off_s[32];
     uint32_t const          total = ctl->n_bchunks;
     uint32_t const          c_a   = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x) * total) / gridDim.x);
     uint32_t const          c_b   = static_cast<uint32_t>((static_cast<uint64_t>(blockIdx.x + 1) * total) / gridDim.x);
@@ -4186,13 +4225,65 @@ __global__ void __launch_bounds__(k_tthreads, 1)
     uint32_t const lane = tid & 31;
     auto          *tbl  = reinterpret_cast<uint32_t *>(t_smem);
     uint32_t const base = static_cast<uint32_t>(__cvta_generic_to_shared(tbl));
+    uint4 const   *mt    = mirror + (static_cast<uint64_t>(tile) * n_rows * 2);
+    uint64_t const pol_t = l2_policy_first();
+    uint64_t const pol_q = l2_policy_last();
+    // a chunk's share of this thread: two rows, their codes and tiles
+    struct Stage
+    {
+        uint32_t q[k_tper]; // k_no_row: no row
+        uint4    a[k_tper];
+        uint4    b[k_tper];
+    };
+    // a chunk, its row ids and its rows are each loaded an iteration apart, so
+    // that none waits for the one it is addressed by
+    auto const chunk = [&](uint32_t c) { return c < c_b ? bchunks[c] : Chunk{0, 0, 0, 0}; };
+    auto const ids   = [&](Chunk const &ch, uint32_t id[k_tper])
+    {
+#pragma unroll
+        for (uint32_t m = 0; m < k_tper; ++m)
+        {
+            uint32_t const k = (m * k_tthreads) + tid;
+            id[m] = k < ch.count ? (rows != nullptr ? rows[ch.begin + k] : ch.begin + k)
+                                 : k_no_row;
+        }
+    };
+    auto const gather = [&](uint32_t const id[k_tper], Stage &S)
+    {
+#pragma unroll
+        for (uint32_t m = 0; m < k_tper; ++m)
+        {
+            S.q[m] = k_no_row;
+            if (id[m] != k_no_row)
+            {
+                uint4 const *src = mt + (static_cast<uint64_t>(id[m]) * 2);
+                S.q[m]           = ld_nc_u16(qgh + id[m], pol_q);
+                ld_nc_row(src, pol_t, S.a[m], S.b[m]);
+            }
+        }
+    };
+    Chunk    ch0 = chunk(c_a);     // of stage s0, then of the rows after s1's
+    Chunk    ch1 = chunk(c_a + 1);
+    uint32_t node  = ch0.node;
+    uint32_t node0 = node;         // of s0's rows, of s1's
+    uint32_t node1 = ch1.node;
+    uint32_t id[k_tper];
+    Stage    s0;
+    Stage    s1;
+    ids(ch0, id);
+    gather(id, s0);
+    ids(ch1, id);
+    ch0 = chunk(c_a + 2);
+    ch1 = chunk(c_a + 3);
     if (tid < 32)
     {
-        j_s[tid] = tile_j[(blockIdx.y * 32) + tid];
+        int32_t const j = tile_j[(blockIdx.y * 32) + tid];
+        nb_s[tid]       = j >= 0 ? sel_nb[j] : 0;
+        off_s[tid]      = j >= 0 ? cell_off[j] : 0;
     }
-    for (uint32_t x = tid; x < k_ttable_bytes / 4; x += k_tthreads)
+    for (uint32_t x = tid; x < k_ttable_bytes / 16; x += k_tthreads)
     {
-        tbl[x] = 0;
+        t_smem[x] = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
     uint32_t sel[4];
@@ -4203,81 +4294,47 @@ __global__ void __launch_bounds__(k_tthreads, 1)
     }
     uint32_t const lane4 = lane * 4;
     uint32_t const wsel  = lane >> 2;
-    uint4 const   *mt    = mirror + (static_cast<uint64_t>(tile) * n_rows * 2);
-    uint64_t const pol_t = l2_policy_first();
-    uint64_t const pol_q = l2_policy_last();
-    // one chunk's share of this thread: two rows, their codes and tiles
-    struct Stage
+    auto           flush = [&]()
     {
-        uint32_t id[k_tper];
-        uint32_t q[k_tper];
-        uint4    a[k_tper];
-        uint4    b[k_tper];
-        uint32_t node;
+        qflush_t<CW2>(tbl, max_nb, nb_s, off_s,
+                      hist + (static_cast<uint64_t>(build[node]) * total_cells * (CW2 ? 2 : 1)));
     };
-    auto load = [&](uint32_t c, Stage &S)
+    auto run = [&](Stage const &S, uint32_t of)
     {
-        Chunk const ch = c < c_b ? bchunks[c] : Chunk{0, 0, 0, 0};
-        S.node         = ch.node;
-#pragma unroll
-        for (uint32_t m = 0; m < k_tper; ++m)
+        if (of != node)
         {
-            uint32_t const k = (m * k_tthreads) + tid;
-            S.id[m] = k < ch.count ? (rows != nullptr ? rows[ch.begin + k] : ch.begin + k)
-                                   : k_no_row;
+            flush();
+            node = of;
         }
 #pragma unroll
         for (uint32_t m = 0; m < k_tper; ++m)
         {
-            if (S.id[m] != k_no_row)
-            {
-                uint4 const *src = mt + (static_cast<uint64_t>(S.id[m]) * 2);
-                S.q[m]           = ld_nc_u16(qgh + S.id[m], pol_q);
-                S.a[m]           = ld_nc_v4(src, pol_t);
-                S.b[m]           = ld_nc_v4(src + 1, pol_t);
-            }
-            else
-            {
-                S.q[m] = 0;
-                S.a[m] = make_uint4(0, 0, 0, 0);
-                S.b[m] = make_uint4(0, 0, 0, 0);
-            }
-        }
-    };
-    uint32_t node = bchunks[c_a].node;
-    auto     run  = [&](Stage const &S)
-    {
-        if (S.node != node)
-        {
-            qflush_t<CW2>(tbl, max_nb, j_s, sel_nb, cell_off,
-                          hist + (static_cast<uint64_t>(build[node]) * total_cells * (CW2 ? 2 : 1)));
-            node = S.node;
-        }
-#pragma unroll
-        for (uint32_t m = 0; m < k_tper; ++m)
-        {
-            if (S.id[m] != k_no_row)
+            if (S.q[m] != k_no_row)
             {
                 qrow_t(base, lane4, wsel, sel, S.a[m], S.b[m], S.q[m]);
             }
         }
     };
-    Stage s0;
-    Stage s1;
-    load(c_a, s0);
     for (uint32_t c = c_a; c < c_b; c += 2)
     {
-        load(c + 1, s1);
-        run(s0);
+        gather(id, s1); // chunk c + 1
+        ids(ch0, id);   // c + 2
+        uint32_t const n0 = ch0.node;
+        ch0               = chunk(c + 4);
+        run(s0, node0);
         if (c + 1 >= c_b)
         {
             break;
         }
-        load(c + 2, s0);
-        run(s1);
+        node0 = n0;
+        gather(id, s0); // c + 2
+        ids(ch1, id);   // c + 3
+        uint32_t const n1 = ch1.node;
+        ch1               = chunk(c + 5);
+        run(s1, node1);
+        node1 = n1;
     }
-    qflush_t<CW2>(tbl, max_nb, j_s, sel_nb, cell_off,
-                  hist + (static_cast<uint64_t>(build[node]) * total_cells * (CW2 ? 2 : 1)));
+    flush();
 }
 
 __global__ void qroot_totals_kernel(Node *nodes, unsigned long long const *hist,
