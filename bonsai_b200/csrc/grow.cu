@@ -1639,6 +1639,7 @@ struct PlanArgs
     HeapOut         ho;
     uint32_t       *nleft;
     uint32_t       *nright;
+    uint4          *route; // per node: its split's feature, last bin, bin, direction
 };
 
 // The frontier's splits and leaves written into the tree, and the partition's
@@ -1684,11 +1685,12 @@ __device__ __forceinline__ void plan_level(Ctl *ctl, Node *nodes, Best const *be
             t.gain[right]  = 0.0F;
             t.cover[left]  = 0.0F;
             t.cover[right] = 0.0F;
-            nd.flags       = 1;
+            nd.flags            = 1;
+            uint32_t const last = cut_off[f + 1] - cut_off[f] - 1;
+            A.route[i]          = make_uint4(f, last, bs.bin, bs.dl);
             if (ho.heap != nullptr && nd.heap < k_heap_slots)
             {
-                ho.heap[nd.heap] = heap_entry(f, ho.per, bs.bin,
-                                              cut_off[f + 1] - cut_off[f] - 1, bs.dl != 0);
+                ho.heap[nd.heap] = heap_entry(f, ho.per, bs.bin, last, bs.dl != 0);
             }
         }
         else
@@ -3428,23 +3430,31 @@ constexpr uint32_t k_psteps = k_warp_rows / 32; // 32-row steps of a partition w
 
 // One warp's 512 rows of a one-pass partition chunk: their ids (the level's
 // list and the split column's codes are read once here, evict-first: the
-// gradient codes and the next lists are what the level reads again), their
-// codes of the split feature, their directions (lane i keeps step i's bits).
-template <bool FULL, typename BinT>
-__device__ __forceinline__ void psplit_route(Chunk const &ch, uint32_t const *__restrict__ rows,
-                                             BinT const *col, uint32_t last, Best const &bs,
-                                             uint32_t w0, uint32_t lane, uint32_t (&r)[k_psteps],
-                                             uint32_t &mword, uint32_t &n)
+// gradient codes and the next lists are what the level reads again) ...
+template <bool FULL>
+__device__ __forceinline__ void psplit_ids(Chunk const &ch, uint32_t const *__restrict__ rows,
+                                           uint32_t w0, uint32_t lane, uint32_t (&r)[k_psteps])
 {
     uint64_t const pol = l2_policy_first();
 #pragma unroll
     for (uint32_t i = 0; i < k_psteps; ++i)
     {
         uint32_t const k = w0 + (32 * i) + lane;
-        r[i]             = FULL || k < ch.count ? ld_hint_b32(rows + ch.begin + k, pol)
-                                                : k_leaf_flag;
+        r[i]             = !FULL && k >= ch.count ? k_leaf_flag
+                           : rows != nullptr      ? ld_hint_b32(rows + ch.begin + k, pol)
+                                                  : ch.begin + k; // (the root's, every row)
     }
-    uint32_t b[k_psteps];
+}
+
+// ... their codes of the split feature, their directions (lane i keeps step
+// i's bits).
+template <bool FULL, typename BinT>
+__device__ __forceinline__ void psplit_route(BinT const *col, uint4 const &route, uint32_t lane,
+                                             uint32_t const (&r)[k_psteps], uint32_t &mword,
+                                             uint32_t &n)
+{
+    uint64_t const pol = l2_policy_first();
+    uint32_t       b[k_psteps];
 #pragma unroll
     for (uint32_t i = 0; i < k_psteps; ++i)
     {
@@ -3453,8 +3463,8 @@ __device__ __forceinline__ void psplit_route(Chunk const &ch, uint32_t const *__
 #pragma unroll
     for (uint32_t i = 0; i < k_psteps; ++i)
     {
-        bool const lf =
-            (FULL || r[i] != k_leaf_flag) && routes_left(b[i], last, bs.bin, bs.dl != 0);
+        bool const lf = (FULL || r[i] != k_leaf_flag) &&
+                        routes_left(b[i], route.y, route.z, route.w != 0);
         uint32_t const m = __ballot_sync(0xFFFFFFFFu, lf);
         mword            = lane == i ? m : mword;
         n += __popc(m);
@@ -3511,19 +3521,41 @@ __device__ __forceinline__ void psplit_place(Chunk const &ch, uint32_t w0, uint3
 // the next level's histogram slots [0, 2 x splits) for the build's adds.
 template <typename BinT, bool SCATTER>
 __global__ void __launch_bounds__(k_threads)
-    psplit_kernel(Ctl const *ctl, Chunk const *pchunks, Node const *nodes, Best const *best,
+    psplit_kernel(Ctl const *ctl, Chunk const *pchunks, Node const *nodes, uint4 const *routes,
                   uint32_t const *__restrict__ rows, uint32_t *__restrict__ rows_out,
-                  void const *__restrict__ bins, uint64_t n_pad, uint32_t const *sel,
-                  uint32_t const *sel_nb, uint32_t *nleft, uint32_t *nright,
+                  void const *__restrict__ bins, uint64_t n_pad, uint32_t *nleft, uint32_t *nright,
                   unsigned long long *zhist, uint32_t total_cells, uint32_t n_zcells)
 {
     pdl_enter();
     __shared__ uint32_t wsum[k_threads / 32];
     __shared__ uint32_t base_s[2];
-    uint32_t const      c = blockIdx.x;
+    uint32_t const      c    = blockIdx.x;
+    Chunk const         ch   = pchunks[c]; // (a slot of the table, used or not)
+    uint32_t const      n_ch = ctl->n_pchunks;
+    uint32_t const      n_z  = ctl->n_psplit;
+    uint32_t const      lane = threadIdx.x & 31;
+    uint32_t const      w    = threadIdx.x >> 5;
+    uint32_t const      w0   = w * k_warp_rows;
+    // a warp whose 512 rows all lie in the chunk (the common case) skips the
+    // per-row range checks
+    bool const full = w0 + k_warp_rows <= ch.count;
+    uint32_t   r[k_psteps];
+    uint4      route{};
+    uint32_t   start = 0;
+    uint32_t   count = 0;
+    bool       split = false;
+    if (c < n_ch)
+    {
+        // the row ids, the node and its split all at once; a leaf's are unused
+        full ? psplit_ids<true>(ch, rows, w0, lane, r) : psplit_ids<false>(ch, rows, w0, lane, r);
+        route = routes[ch.node];
+        start = nodes[ch.node].start;
+        count = nodes[ch.node].count;
+        split = (nodes[ch.node].flags & 1) != 0;
+    }
     if constexpr (SCATTER)
     {
-        uint64_t const nz = 2ULL * ctl->n_psplit * n_zcells;
+        uint64_t const nz = 2ULL * n_z * n_zcells;
         for (uint64_t x = (static_cast<uint64_t>(c) * k_threads) + threadIdx.x; x < nz;
              x += static_cast<uint64_t>(gridDim.x) * k_threads)
         {
@@ -3531,37 +3563,15 @@ __global__ void __launch_bounds__(k_threads)
             zhist[(i * total_cells) + (x - (i * n_zcells))] = 0ULL;
         }
     }
-    if (c >= ctl->n_pchunks)
+    if (!split)
     {
-        return;
+        return; // past the last chunk, or a leaf's, which routes nothing
     }
-    Chunk const ch = pchunks[c];
-    Node const  nd = nodes[ch.node];
-    if ((nd.flags & 1) == 0)
-    {
-        return; // a leaf's chunk routes nothing
-    }
-    Best const     bs   = best[ch.node];
-    uint32_t const f    = sel[bs.feature];
-    uint32_t const last = sel_nb[bs.feature] - 1;
-    BinT const    *col  = static_cast<BinT const *>(bins) + (static_cast<uint64_t>(f) * n_pad);
-    uint32_t const lane = threadIdx.x & 31;
-    uint32_t const w    = threadIdx.x >> 5;
-    uint32_t const w0   = w * k_warp_rows;
-    // a warp whose 512 rows all lie in the chunk (the common case) skips the
-    // per-row range checks
-    bool const     full = w0 + k_warp_rows <= ch.count;
-    uint32_t       r[k_psteps];
-    uint32_t       mword = 0; // lane i: step i's direction bits
-    uint32_t       n     = 0;
-    if (full)
-    {
-        psplit_route<true>(ch, rows, col, last, bs, w0, lane, r, mword, n);
-    }
-    else
-    {
-        psplit_route<false>(ch, rows, col, last, bs, w0, lane, r, mword, n);
-    }
+    BinT const *col   = static_cast<BinT const *>(bins) + (static_cast<uint64_t>(route.x) * n_pad);
+    uint32_t    mword = 0; // lane i: step i's direction bits
+    uint32_t    n     = 0;
+    full ? psplit_route<true>(col, route, lane, r, mword, n)
+         : psplit_route<false>(col, route, lane, r, mword, n);
     if (lane == 0)
     {
         wsum[w] = n;
@@ -3588,9 +3598,9 @@ __global__ void __launch_bounds__(k_threads)
     {
         lb += wsum[x];
     }
-    uint32_t const lo  = nd.start + base_s[0] + lb;                       // next left
+    uint32_t const lo  = start + base_s[0] + lb;                       // next left
     uint32_t const rk  = base_s[1] + (min(w0, ch.count) - lb);            // next right's rank
-    uint32_t const top = nd.start + nd.count - 1;                          // rights count down
+    uint32_t const top = start + count - 1;                          // rights count down
     if (full)
     {
         psplit_place<true>(ch, w0, lane, r, mword, lo, rk, top, rows_out);
@@ -5576,6 +5586,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
                         static_cast<size_t>(cfg_.leaf ? 1 : max_front_) * total_cells_ * cw_);
     arena_.want<Best>(cand_, static_cast<size_t>(max_front_) * n_sel_);
     arena_.want<Best>(best_, max_front_);
+    arena_.want<uint4>(route_, max_front_);
     arena_.want<Chunk>(pchunks_, max_pchunks_);
     arena_.want<uint32_t>(pleft_, max_pchunks_);
     arena_.want<uint32_t>(dirs_, static_cast<size_t>(max_pchunks_) * (k_part_rows / 32));
@@ -6090,7 +6101,7 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     dim3 const fgrid(front, n_sel_);
     HeapOut const ho{heap_, leafmap_, cfg_.tp.max_depth, k_mirror_bytes / (plane_.u8 ? 1u : 2u)};
     PlanArgs const plan{sel_, plane_.cuts, plane_.cut_off, cfg_.tp, t,      pchunks_,
-                        pcr_, nbound_,     ho,             nleft_,  nright_};
+                        pcr_, nbound_,     ho,             nleft_,  nright_, route_};
     FindChain const chain{ctl_,
                           nodes_[cur],
                           best_,
@@ -6152,8 +6163,8 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
                                             : psplit_kernel<uint8_t, true>)
                                     : (last ? psplit_kernel<uint16_t, false>
                                             : psplit_kernel<uint16_t, true>);
-        launch_k(pdl_, kern, pch, k_threads, 0, s, ctl_, pchunks_, nodes_[cur], best_,
-                 rows_in, rows_out, plane_.bins, plane_.n_pad, sel_, sel_nb_, nleft_, nright_,
+        launch_k(pdl_, kern, pch, k_threads, 0, s, ctl_, pchunks_, nodes_[cur], route_,
+                 rows_in, rows_out, plane_.bins, plane_.n_pad, nleft_, nright_,
                  static_cast<unsigned long long *>(hist_[nxt]), total_cells_ * cw_, n_zcells);
         BB_LAUNCH("psplit_kernel");
     }
@@ -6403,7 +6414,7 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
     {
         phase_end(prof_->other_ms);
     }
-    uint32_t const *rows_in = root_rows;
+    uint32_t const *rows_in = chain_ && identity_root ? nullptr : root_rows;
     for (uint32_t L = 0; L < cfg_.tp.max_depth; ++L)
     {
         uint32_t *rows_out = rows_[L & 1];

@@ -352,6 +352,7 @@ class Grower
     void     *hist_[2]  = {nullptr, nullptr}; // [front][total_cells] cells
     Best     *cand_     = nullptr;             // [front][n_sel]
     Best     *best_     = nullptr;             // [front]
+    uint4    *route_    = nullptr;             // [front] the splits as the partition reads them
     Chunk    *pchunks_  = nullptr;
     uint32_t *pleft_    = nullptr; // per partition chunk: left count, then base
     uint32_t *prbase_   = nullptr;
