@@ -2939,30 +2939,6 @@ struct WalkArgs
     TreeCommit    commit; // the finished tree's slot, or none
 };
 
-__device__ __forceinline__ uint32_t pick_word(uint32_t const w[8], uint32_t i)
-{
-    uint32_t const a = (i & 1) != 0 ? w[1] : w[0];
-    uint32_t const b = (i & 1) != 0 ? w[3] : w[2];
-    uint32_t const c = (i & 1) != 0 ? w[5] : w[4];
-    uint32_t const d = (i & 1) != 0 ? w[7] : w[6];
-    uint32_t const e = (i & 2) != 0 ? b : a;
-    uint32_t const f = (i & 2) != 0 ? d : c;
-    return (i & 4) != 0 ? f : e;
-}
-
-template <bool U8>
-__device__ __forceinline__ uint32_t tile_code(uint32_t const w[8], uint32_t pos)
-{
-    if constexpr (U8)
-    {
-        return __byte_perm(pick_word(w, pos >> 2), 0u, 0x4440u | (pos & 3u));
-    }
-    else
-    {
-        return __byte_perm(pick_word(w, pos >> 1), 0u, 0x4410u | ((pos & 1u) * 0x22u));
-    }
-}
-
 // The walk steps through the tree's decision heap (filled by the plan
 // kernels): slot h's children are 2h + 1 and 2h + 2, so a step reads one
 // 8-byte entry and no child ids. A leaf above the last level repeats down
@@ -2975,14 +2951,23 @@ __device__ __forceinline__ uint32_t heap_step(uint2 const e, uint32_t code, uint
     return (2 * h) + (left ? 1u : 2u);
 }
 
+// A staged entry's x: the code's byte offset in the walking lane's column of the
+// staged tile words (below 1,024), and the tile above it.
+constexpr uint32_t k_no_staged_tile = k_no_tile & 0x3FFFFFu;
+
 // The heap's entries and leaf map, staged in shared memory by the block.
+template <bool U8>
 __device__ __forceinline__ void load_heap(uint2 *heap_s, uint16_t *leaf_s, uint2 const *heap,
                                           uint16_t const *leafmap, uint32_t depth)
 {
     uint32_t const n_int = (1u << depth) - 1;
     for (uint32_t i = threadIdx.x; i < n_int; i += blockDim.x)
     {
-        heap_s[i] = heap[i];
+        uint2 const    e   = heap[i];
+        uint32_t const pos = e.x & 0xFFu;
+        uint32_t const off = U8 ? ((pos >> 2) * 128) + (pos & 3u)
+                                : ((pos >> 1) * 128) + ((pos & 1u) * 2);
+        heap_s[i]          = make_uint2(((e.x >> 8) << 10) | off, e.y);
     }
     for (uint32_t i = threadIdx.x; i <= n_int; i += blockDim.x)
     {
@@ -2991,47 +2976,73 @@ __device__ __forceinline__ void load_heap(uint2 *heap_s, uint16_t *leaf_s, uint2
     __syncthreads();
 }
 
-// Row r's last-level slot (leaf_s names its leaf): its tile of the root's
-// feature is passed in; with MULTI the walk fetches another tile when a
-// slot's feature lives there.
-template <bool U8, bool MULTI>
-__device__ __forceinline__ uint32_t walk_heap(uint2 const *heap_s,
-                                              uint4 const *__restrict__ mirror, uint64_t n_rows,
-                                              uint64_t r, uint32_t depth, uint4 ta, uint4 tb,
-                                              uint32_t held)
+// Two rows' tiles in shared memory, word j of lane l's row at word 32 j + l of
+// its warp's part, so a lane finds any code in its own bank.
+__device__ __forceinline__ void stage_tile(uint32_t *col, uint4 const &a, uint4 const &b)
 {
-    uint32_t w[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
-    uint32_t h    = 0;
+    uint32_t const w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j)
+    {
+        col[32 * j] = w[j];
+    }
+}
+
+// The last-level slots (leaf_s names their leaves) of a thread's two rows, step
+// by step together: their tiles of the root's feature are staged; with MULTI
+// the walk stages another tile when a slot's feature lives there. (Picked out
+// of registers a code took a tree of selects, 30 instructions a step: pass A
+// over 10,000,000 rows 135 us before, WALK_NOW now.)
+template <bool U8, bool MULTI>
+__device__ __forceinline__ void walk_heap(uint2 const *heap_s, uint32_t *col,
+                                          uint4 const *__restrict__ mirror, uint64_t n_rows,
+                                          uint64_t const (&r)[2], uint32_t depth, uint32_t held,
+                                          uint32_t (&slot)[2])
+{
+    uint32_t const of[2]   = {0, 256};
+    uint32_t       h[2]    = {0, 0};
+    uint32_t       tile[2] = {held, held};
 #pragma unroll
     for (uint32_t d = 0; d < 8; ++d)
     {
         if (d < depth)
         {
-            uint2 const e = heap_s[h];
-            if constexpr (MULTI)
+            uint2 e[2];
+#pragma unroll
+            for (uint32_t k = 0; k < 2; ++k)
             {
-                uint32_t const tile = e.x >> 8;
-                if (tile != held && tile != k_no_tile)
+                e[k] = heap_s[h[k]];
+                if constexpr (MULTI)
                 {
-                    uint4 const *src = mirror + (((static_cast<uint64_t>(tile) * n_rows) + r) * 2);
-                    uint4 const  xa  = src[0];
-                    uint4 const  xb  = src[1];
-                    w[0] = xa.x; w[1] = xa.y; w[2] = xa.z; w[3] = xa.w;
-                    w[4] = xb.x; w[5] = xb.y; w[6] = xb.z; w[7] = xb.w;
-                    held = tile;
+                    uint32_t const t = e[k].x >> 10;
+                    if (t != tile[k] && t != k_no_staged_tile)
+                    {
+                        uint4 const *src =
+                            mirror + (((static_cast<uint64_t>(t) * n_rows) + r[k]) * 2);
+                        stage_tile(col + of[k], src[0], src[1]);
+                        tile[k] = t;
+                    }
                 }
             }
-            h = heap_step(e, tile_code<U8>(w, e.x & 0xFFu), h);
+#pragma unroll
+            for (uint32_t k = 0; k < 2; ++k)
+            {
+                auto const *at = reinterpret_cast<unsigned char const *>(col + of[k]) +
+                                 (e[k].x & 1023u);
+                uint32_t const code = U8 ? *at : *reinterpret_cast<uint16_t const *>(at);
+                h[k]                = heap_step(e[k], code, h[k]);
+            }
         }
     }
-    return h - ((1u << depth) - 1); // the row's slot among the last level's 2^depth
+    slot[0] = h[0] - ((1u << depth) - 1);
+    slot[1] = h[1] - ((1u << depth) - 1);
 }
 
 // The tile that holds the root's feature (0 when the root is a leaf).
 __device__ __forceinline__ uint32_t heap_root_tile(uint2 const *heap_s, uint32_t depth)
 {
-    uint32_t const t = depth > 0 ? heap_s[0].x >> 8 : k_no_tile;
-    return t == k_no_tile ? 0u : t;
+    uint32_t const t = depth > 0 ? heap_s[0].x >> 10 : k_no_staged_tile;
+    return t == k_no_staged_tile ? 0u : t;
 }
 
 // Block maxima of |g| and h into the quantiser's two words.
@@ -3102,7 +3113,9 @@ __global__ void __launch_bounds__(k_threads)
     {
         val_s[i] = t.value[i];
     }
-    load_heap(heap_s, leaf_s, heap, leafmap, depth);
+    __shared__ uint32_t codes_s[k_threads * 16];
+    uint32_t *const     col = codes_s + ((threadIdx.x >> 5) * 512) + (threadIdx.x & 31);
+    load_heap<U8>(heap_s, leaf_s, heap, leafmap, depth);
     uint32_t const root_tile = heap_root_tile(heap_s, depth);
     uint4 const   *mt        = mirror + (static_cast<uint64_t>(root_tile) * n_rows * 2);
     float          mg        = 0.0F;
@@ -3122,10 +3135,13 @@ __global__ void __launch_bounds__(k_threads)
         float const    s1  = a.scores != nullptr ? a.scores[rb] : 0.0F;
         float const    y0  = a.gh != nullptr ? a.labels[r0] : 0.0F;
         float const    y1  = a.gh != nullptr ? a.labels[rb] : 0.0F;
-        uint32_t const n0 =
-            leaf_s[walk_heap<U8, MULTI>(heap_s, mirror, n_rows, r0, depth, a0, b0, root_tile)];
-        uint32_t const n1 =
-            leaf_s[walk_heap<U8, MULTI>(heap_s, mirror, n_rows, rb, depth, a1, b1, root_tile)];
+        uint64_t const rr[2] = {r0, rb};
+        uint32_t       o[2];
+        stage_tile(col, a0, b0);
+        stage_tile(col + 256, a1, b1);
+        walk_heap<U8, MULTI>(heap_s, col, mirror, n_rows, rr, depth, root_tile, o);
+        uint32_t const n0 = leaf_s[o[0]];
+        uint32_t const n1 = leaf_s[o[1]];
         apply_leaf(a, r0, n0, s0, y0, val_s[n0], mg, mh);
         if (two)
         {
@@ -3215,7 +3231,9 @@ __global__ void __launch_bounds__(k_wsum_thr)
     {
         acc_s[i] = 0ULL;
     }
-    load_heap(heap_s, leaf_s, heap, leafmap, depth);
+    __shared__ uint32_t codes_s[k_wsum_thr * 16];
+    uint32_t *const     col = codes_s + ((threadIdx.x >> 5) * 512) + (threadIdx.x & 31);
+    load_heap<U8>(heap_s, leaf_s, heap, leafmap, depth);
     uint32_t const root_tile = heap_root_tile(heap_s, depth);
     uint4 const   *mt        = mirror + (static_cast<uint64_t>(root_tile) * n_rows * 2);
     float const    mgx       = __uint_as_float(absmax[0]);
@@ -3246,10 +3264,13 @@ __global__ void __launch_bounds__(k_wsum_thr)
         // a row outside this tree's sample takes its leaf but adds nothing
         float2 const   g0  = in_sample(bits, r0) ? gh[r0] : make_float2(0.0F, 0.0F);
         float2 const   g1  = in_sample(bits, rb) ? gh[rb] : make_float2(0.0F, 0.0F);
-        uint32_t const o0 =
-            walk_heap<U8, MULTI>(heap_s, mirror, n_rows, r0, depth, a0, b0, root_tile);
-        uint32_t const o1 =
-            walk_heap<U8, MULTI>(heap_s, mirror, n_rows, rb, depth, a1, b1, root_tile);
+        uint64_t const rr[2] = {r0, rb};
+        uint32_t       o[2];
+        stage_tile(col, a0, b0);
+        stage_tile(col + 256, a1, b1);
+        walk_heap<U8, MULTI>(heap_s, col, mirror, n_rows, rr, depth, root_tile, o);
+        uint32_t const o0 = o[0];
+        uint32_t const o1 = o[1];
         leaf16[r0] = leaf_s[o0];
         add(o0, g0);
         if (two)
