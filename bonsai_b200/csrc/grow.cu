@@ -333,7 +333,7 @@ __global__ void root_setup_kernel(RootArgs A)
 // never -0), every lane adds them all and keeps the sum at its own. The chain is
 // one dependent add a term; the shuffles that feed it run ahead. (One thread
 // that read, added and wrote a cell at a time took 40 ns a bin; of a level of
-// 20,640 rows x 8 the find 14.7 us and the totals 14.7 before, FIND_NOW and SUB_NOW now.)
+// 20,640 rows x 8 the find 14.7 us and the totals 14.7 before, 10.6 and 9.3 now, under ncu.)
 __device__ __forceinline__ double warp_serial_sum(double term, double &sum)
 {
     uint32_t const lane = threadIdx.x & 31;
@@ -350,15 +350,15 @@ __device__ __forceinline__ double warp_serial_sum(double term, double &sum)
 // Node totals from the first selected feature's cells: double sums over
 // every cell in bin order, rounded to float once (Histogram::totals), with
 // one warp, each lane holding them.
-__device__ __forceinline__ void warp_totals(float2 const *cells, uint32_t nb, float &g,
-                                            float &h)
+template <typename Cells>
+__device__ __forceinline__ void warp_totals(Cells const &cells, uint32_t nb, float &g, float &h)
 {
     uint32_t const lane = threadIdx.x & 31;
     double         sg   = 0.0;
     double         sh   = 0.0;
     for (uint32_t b0 = 0; b0 < nb; b0 += 32)
     {
-        float2 const c = b0 + lane < nb ? cells[b0 + lane] : make_float2(0.0F, 0.0F);
+        float2 const c = b0 + lane < nb ? cells(b0 + lane) : make_float2(0.0F, 0.0F);
         warp_serial_sum(c.x, sg);
         warp_serial_sum(c.y, sh);
     }
@@ -370,7 +370,7 @@ __global__ void root_totals_kernel(Node *nodes, float2 const *hist, uint32_t con
 {
     pdl_enter();
     float g, h;
-    warp_totals(hist, sel_nb[0], g, h);
+    warp_totals([&](uint32_t b) { return hist[b]; }, sel_nb[0], g, h);
     if (threadIdx.x == 0)
     {
         nodes[0].sum_g = g;
@@ -494,7 +494,7 @@ __device__ __forceinline__ void rank_rows(uint32_t (&key)[k_xsteps], uint16_t *c
     }
 }
 
-// grid (chunks, tiles)
+// grid (chunks, tiles, parts of a tile's features)
 template <typename BinT, uint32_t GROUPS>
 __global__ void __launch_bounds__(GROUPS *k_xgthr, GROUPS == k_xgroups && sizeof(BinT) == 1 ? 2 : 1)
     sort_kernel(Ctl const *ctl, Chunk const *bchunks, uint32_t const *brange,
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(GROUPS *k_xgthr, GROUPS == k_xgroups && sizeof
     auto          *cnt16 = reinterpret_cast<uint16_t *>(cnt_s + (wg * crow));
     auto const    *start = reinterpret_cast<uint16_t const *>(cnt_s); // after the scan
     uint32_t const k0    = wg * (k_xsteps * 32);
-    for (uint32_t x = group; x < per; x += GROUPS)
+    for (uint32_t x = group + (GROUPS * blockIdx.z); x < per; x += GROUPS * gridDim.z)
     {
         int32_t const js = tile_j[(blockIdx.y * per) + x];
         if (js < 0)
@@ -3013,7 +3013,7 @@ __device__ __forceinline__ void stage_tile(uint32_t *col, uint4 const &a, uint4 
 // by step together: their tiles of the root's feature are staged; with MULTI
 // the walk stages another tile when a slot's feature lives there. (Picked out
 // of registers a code took a tree of selects, 30 instructions a step: pass A
-// over 10,000,000 rows 135 us before, WALK_NOW now.)
+// over 10,000,000 rows 135 us before, 113 now.)
 template <bool U8, bool MULTI>
 __device__ __forceinline__ void walk_heap(uint2 const *heap_s, uint32_t *col,
                                           uint4 const *__restrict__ mirror, uint64_t n_rows,
@@ -3653,8 +3653,12 @@ __global__ void __launch_bounds__(k_threads)
     }
 }
 
+constexpr uint32_t k_sub_cells = 1024; // cells per subtraction CTA
+
 // Larger child = parent - smaller child, cell by cell in float
-// (finish_split); then both children's totals and monotone bounds.
+// (finish_split), 1,024 cells a block; both children's totals, summed from the
+// same differences, and monotone bounds by each split's first block. (One block
+// a split: 20.8 us a level of 28 features x 256 bins under ncu; now 9.0.)
 __global__ void __launch_bounds__(k_threads)
     subtract_totals_kernel(Ctl *ctl, uint32_t const *bpair, float2 const *hist_cur,
                            float2 *hist_nxt, uint32_t total_cells, uint32_t n_cells,
@@ -3664,7 +3668,7 @@ __global__ void __launch_bounds__(k_threads)
 {
     pdl_enter();
     uint32_t const k = blockIdx.x;
-    if (k == 0 && threadIdx.x == 0)
+    if (k == 0 && blockIdx.y == 0 && threadIdx.x == 0)
     {
         ctl->n_cur = ctl->n_next; // the level's last kernel advances the frontier
     }
@@ -3678,21 +3682,40 @@ __global__ void __launch_bounds__(k_threads)
     float2 const  *hp = hist_cur + (static_cast<uint64_t>(p) * total_cells);
     float2 const  *hs = hist_nxt + (static_cast<uint64_t>(s) * total_cells);
     float2        *hl = hist_nxt + (static_cast<uint64_t>(l) * total_cells);
-    for (uint32_t x = threadIdx.x; x < n_cells; x += k_threads)
+    uint32_t const x0 = blockIdx.y * k_sub_cells;
+    uint32_t const x1 = min(n_cells, x0 + k_sub_cells);
+#pragma unroll 4
+    for (uint32_t x = x0 + threadIdx.x; x < x1; x += k_threads)
     {
         float2 const a = hp[x];
         float2 const b = hs[x];
         hl[x]          = make_float2(a.x - b.x, a.y - b.y);
     }
-    __syncthreads();
+    if (blockIdx.y != 0)
+    {
+        return;
+    }
     // the children's totals: warp c sums child c's first feature
     __shared__ float tot_s[4];
     uint32_t const   wc = threadIdx.x >> 5;
     if (wc < 2)
     {
         float g, h;
-        warp_totals(hist_nxt + (static_cast<uint64_t>((2 * k) + wc) * total_cells), sel_nb[0],
-                    g, h);
+        if ((2 * k) + wc == s)
+        {
+            warp_totals([&](uint32_t b) { return hs[b]; }, sel_nb[0], g, h);
+        }
+        else
+        {
+            warp_totals(
+                [&](uint32_t b)
+                {
+                    float2 const a = hp[b];
+                    float2 const c = hs[b];
+                    return make_float2(a.x - c.x, a.y - c.y);
+                },
+                sel_nb[0], g, h);
+        }
         if ((threadIdx.x & 31) == 0)
         {
             tot_s[2 * wc]       = g;
@@ -4402,8 +4425,6 @@ __global__ void qroot_totals_kernel(Node *nodes, unsigned long long const *hist,
     }
 }
 
-constexpr uint32_t k_sub_cells = 1024; // cells per subtraction CTA
-
 // Larger child = parent - smaller child in exact integers (both packed
 // words subtract without borrow: a child's hessian sum never exceeds its
 // parent's); children's totals and monotone bounds from the integer sums.
@@ -4761,7 +4782,8 @@ __global__ void leaf_totals_kernel(Ctl *ctl, LeafOut const *out, Node *next,
     if (wc < 2)
     {
         float g, h;
-        warp_totals(pool + (static_cast<uint64_t>(slot_of[wc]) * total_cells), sel_nb[0], g, h);
+        float2 const *cells = pool + (static_cast<uint64_t>(slot_of[wc]) * total_cells);
+        warp_totals([&](uint32_t b) { return cells[b]; }, sel_nb[0], g, h);
         if ((threadIdx.x & 31) == 0)
         {
             tot_s[2 * wc]       = g;
@@ -6074,9 +6096,18 @@ void Grower::build(uint32_t const *rows, uint32_t nfb, int dst, bool zeroed, uin
     {
         int const       v    = nfb == n_sel_ ? 0 : 1;
         uint32_t const *crow = rows != nullptr ? rows : root_rows_;
-        auto            sort = [&](auto kern)
+        // a small build's chunks leave SMs idle: a tile's features are then
+        // split over several CTAs, each staging the chunk's rows, up to two CTAs
+        // an SM (20,000 rows x 28: the root's sort 65.9 us in one part, 19.7 in seven; the
+        // round 618 and 332, leafwise 2,797 and 1,629, 24 fits in flight 126 and
+        // 94 ms for 50 rounds)
+        uint32_t const per   = k_mirror_bytes / (plane_.u8 ? 1 : 2);
+        uint32_t const parts = std::max(
+            1u, std::min(ceil_div(nfb == 1 ? 1u : std::min(per, plane_.n_feats), xgroups_),
+                         296u / (n_chunks * n_tiles_[v])));
+        auto           sort = [&](auto kern)
         {
-            launch_k(pdl_, kern, dim3(n_chunks, n_tiles_[v]), xgroups_ * k_xgthr,
+            launch_k(pdl_, kern, dim3(n_chunks, n_tiles_[v], parts), xgroups_ * k_xgthr,
                      sort_smem(max_nb_, xgroups_), s, ctl_, bchunks_, brange_, build_, crow,
                      static_cast<uint4 const *>(plane_.mirror), plane_.n_rows, gh_cur_,
                      tile_ids_[v], tile_j_[v], sel_nb_, cell_off_, max_nb_, nfb, coff_,
@@ -6344,7 +6375,9 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     }
     else
     {
-        launch_k(pdl_, subtract_totals_kernel, front, k_threads, 0, s, ctl_, bpair_,
+        launch_k(pdl_, subtract_totals_kernel,
+                 dim3(front, std::max(1u, ceil_div(n_cells, k_sub_cells))), k_threads, 0, s, ctl_,
+                 bpair_,
                  static_cast<float2 const *>(hist_[cur]), static_cast<float2 *>(hist_[nxt]),
                  total_cells_, n_cells, nodes_[cur], nodes_[nxt], best_, sel_, sel_nb_, mono_,
                  n_mono_, cfg_.tp);
