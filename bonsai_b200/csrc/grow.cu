@@ -8,7 +8,7 @@
 //                                262-374), demote_empty_splits
 //                                (src/grower_impl.hpp:262-298),
 //                                commit_children (:303-326)
-//   count/offsets/scatter/chain  the column fill's serial cell order
+//   sort/chain                   the column fill's serial cell order
 //                                (src/fill/columns.hpp:31-89)
 //   subtract_totals_kernel       finish_split (src/step/primitives.hpp:
 //                                156-173), Histogram::totals
@@ -1075,20 +1075,17 @@ __device__ __forceinline__ void interaction_children(Node const &par, uint64_t c
     R.ipath  = path;
 }
 
-template <bool Q>
 __global__ void __launch_bounds__(k_find_thr)
     find_kernel(Ctl const *ctl, Node const *nodes, void const *hist_v,
                 uint32_t total_cells, uint32_t const *cell_off, uint32_t const *sel_nb,
                 uint32_t const *sel, uint32_t n_sel, int8_t const *mono, uint32_t n_mono,
-                TreeParams tp, Best *cand, uint32_t max_nb, double2 const *qscale,
-                uint32_t const *slot_of, uint32_t cw, uint64_t const *fgroups)
+                TreeParams tp, Best *cand, uint32_t max_nb, uint32_t const *slot_of,
+                uint64_t const *fgroups)
 {
     pdl_enter();
     extern __shared__ unsigned char smem_raw[];
     __shared__ double   bg_s[k_find_thr / 32];
     __shared__ uint32_t bo_s[k_find_thr / 32];
-    __shared__ int64_t  wg_s[k_find_thr / 32];
-    __shared__ int64_t  wh_s[k_find_thr / 32];
     uint32_t const      i = blockIdx.x;
     if (i >= ctl->n_cur)
     {
@@ -1099,7 +1096,7 @@ __global__ void __launch_bounds__(k_find_thr)
     uint32_t const w    = tid >> 5;
     uint32_t const j    = blockIdx.y;
     auto          *pref = reinterpret_cast<double2 *>(smem_raw);                  // [max_nb]
-    auto          *raw  = reinterpret_cast<unsigned long long *>(pref + max_nb); // [max_nb]
+    auto          *cell = reinterpret_cast<float2 *>(pref + max_nb);              // [max_nb]
     Node const     nd   = nodes[i];
     uint32_t const nb   = sel_nb[j];
     Best           out  = {0.0, j, 0, 1, 0};
@@ -1113,111 +1110,40 @@ __global__ void __launch_bounds__(k_find_thr)
         return;
     }
     uint32_t const n_cut = nb - 2;
-    // the cells, 8 bytes each (packed integers or a float2); a node's slot
-    // is its frontier index unless slot_of names it (the leafwise pool)
+    // a node's slot is its frontier index unless slot_of names it (the
+    // leafwise pool)
     uint32_t const slot = slot_of != nullptr ? slot_of[i] : i;
-    auto const *src = static_cast<unsigned long long const *>(hist_v) +
-                      (((static_cast<uint64_t>(slot) * total_cells) + cell_off[j]) * cw);
-    for (uint32_t b = tid; b < nb * cw; b += k_find_thr)
+    auto const    *src  = static_cast<float2 const *>(hist_v) +
+                      ((static_cast<uint64_t>(slot) * total_cells) + cell_off[j]);
+    for (uint32_t b = tid; b < nb; b += k_find_thr)
     {
-        raw[b] = src[b];
+        cell[b] = src[b];
     }
     __syncthreads();
-    using MissT = typename std::conditional<Q, double, float>::type;
-    MissT        mg;
-    MissT        mh;
-    double       node_sc;
-    double       real_g;
-    double       real_h;
-    bool         miss_empty;
     double const l1 = tp.lambda_l1;
     double const l2 = tp.lambda_l2;
-    if constexpr (Q)
+    if (w < 2)
     {
-        double2 const  sc  = *qscale;
-        uint32_t const run = (n_cut + k_find_thr - 1) / k_find_thr;
-        uint32_t const b0  = min(n_cut, tid * run);
-        uint32_t const b1  = min(n_cut, b0 + run);
-        int64_t        tg  = 0;
-        int64_t        th  = 0;
-        for (uint32_t b = b0; b < b1; ++b)
+        // warp 0 the gradients' running sums, warp 1 the hessians'
+        double sum = 0.0;
+        for (uint32_t b0 = 0; b0 < n_cut; b0 += 32)
         {
-            int64_t cg, ch;
-            qcell(raw, b, cw, cg, ch);
-            tg += cg;
-            th += ch;
-        }
-        int64_t eg = tg;
-        int64_t eh = th;
-#pragma unroll
-        for (uint32_t o = 1; o < 32; o <<= 1)
-        {
-            int64_t const ug = __shfl_up_sync(0xFFFFFFFFu, eg, o);
-            int64_t const uh = __shfl_up_sync(0xFFFFFFFFu, eh, o);
-            if (lane >= o)
+            uint32_t const b    = b0 + lane;
+            float const    v    = b < n_cut ? (w == 0 ? cell[b].x : cell[b].y) : 0.0F;
+            double const   mine = warp_serial_sum(v, sum);
+            if (b < n_cut)
             {
-                eg += ug;
-                eh += uh;
+                (w == 0 ? pref[b].x : pref[b].y) = mine;
             }
         }
-        if (lane == 31)
-        {
-            wg_s[w] = eg;
-            wh_s[w] = eh;
-        }
-        __syncthreads();
-        int64_t pg = eg - tg;
-        int64_t ph = eh - th;
-        for (uint32_t x = 0; x < w; ++x)
-        {
-            pg += wg_s[x];
-            ph += wh_s[x];
-        }
-        for (uint32_t b = b0; b < b1; ++b)
-        {
-            int64_t cg, ch;
-            qcell(raw, b, cw, cg, ch);
-            pg += cg;
-            ph += ch;
-            pref[b] = make_double2(static_cast<double>(pg) * sc.x,
-                                   static_cast<double>(ph) * sc.y);
-        }
-        int64_t mqg, mqh;
-        qcell(raw, nb - 1, cw, mqg, mqh);
-        mg         = static_cast<double>(mqg) * sc.x;
-        mh         = static_cast<double>(mqh) * sc.y;
-        node_sc    = split_score(static_cast<double>(nd.qg) * sc.x,
-                                 static_cast<double>(nd.qh) * sc.y, l1, l2);
-        real_g     = static_cast<double>(nd.qg - mqg) * sc.x;
-        real_h     = static_cast<double>(nd.qh - mqh) * sc.y;
-        miss_empty = mqg == 0 && mqh == 0;
     }
-    else
-    {
-        auto const *cell = reinterpret_cast<float2 const *>(raw);
-        if (w < 2)
-        {
-            // warp 0 the gradients' running sums, warp 1 the hessians'
-            double sum = 0.0;
-            for (uint32_t b0 = 0; b0 < n_cut; b0 += 32)
-            {
-                uint32_t const b    = b0 + lane;
-                float const    v    = b < n_cut ? (w == 0 ? cell[b].x : cell[b].y) : 0.0F;
-                double const   mine = warp_serial_sum(v, sum);
-                if (b < n_cut)
-                {
-                    (w == 0 ? pref[b].x : pref[b].y) = mine;
-                }
-            }
-        }
-        mg      = cell[nb - 1].x;
-        mh      = cell[nb - 1].y;
-        node_sc = split_score(nd.sum_g, nd.sum_h, l1, l2);
-        // float fields subtract in float, then widen (src/split.cpp:117-118)
-        real_g     = static_cast<double>(nd.sum_g - mg);
-        real_h     = static_cast<double>(nd.sum_h - mh);
-        miss_empty = mg == 0.0F && mh == 0.0F;
-    }
+    float const  mg      = cell[nb - 1].x;
+    float const  mh      = cell[nb - 1].y;
+    double const node_sc = split_score(nd.sum_g, nd.sum_h, l1, l2);
+    // float fields subtract in float, then widen (src/split.cpp:117-118)
+    double const real_g     = static_cast<double>(nd.sum_g - mg);
+    double const real_h     = static_cast<double>(nd.sum_h - mh);
+    bool const   miss_empty = mg == 0.0F && mh == 0.0F;
     __syncthreads();
     uint32_t const f        = sel[j];
     int const      mc       = (mono != nullptr && f < n_mono) ? mono[f] : 0;
@@ -1231,7 +1157,7 @@ __global__ void __launch_bounds__(k_find_thr)
         for (uint32_t d = 0; d < n_dir; ++d)
         {
             double gain = 0.0;
-            if (candidate_gain<MissT>(p.x, p.y, mg, mh, real_g, real_h, d == 0, node_sc, tp,
+            if (candidate_gain<float>(p.x, p.y, mg, mh, real_g, real_h, d == 0, node_sc, tp,
                                       mc, nd.lo, nd.hi, gain) &&
                 gain > best && gain >= min_gain)
             {
@@ -2400,10 +2326,32 @@ struct LeafPlanArgs
     uint32_t      *slot_of;
     LeafOut       *out;
     uint32_t       crows;
-    uint32_t       half; // rows of one half of the row buffer
+    uint32_t       half; // rows of one half of the row buffer; 0: the children's rows are
+                          // copied back into their parent's places
     LeafPop const *pp;
     uint32_t      *ticket;
 };
+
+// The popped node's scattered rows back into its segment (unless the
+// partition emptied a side, which scatters nothing).
+constexpr uint32_t k_far_rows = 0x80000000u;
+
+__global__ void __launch_bounds__(k_threads)
+    leaf_copyback_kernel(LeafPop const *pp, LeafOut const *out, uint32_t const *from, uint32_t *to)
+{
+    pdl_enter();
+    if (out->split == 0)
+    {
+        return;
+    }
+    uint64_t const start = pp->node.start;
+    uint64_t const count = pp->node.count;
+    for (uint64_t i = (uint64_t{blockIdx.x} * k_threads) + threadIdx.x; i < count;
+         i += uint64_t{gridDim.x} * k_threads)
+    {
+        to[start + i] = from[start + i];
+    }
+}
 
 template <uint32_t NT> __device__ __forceinline__ void leaf_plan(LeafPlanArgs const &A)
 {
@@ -2431,7 +2379,9 @@ template <uint32_t NT> __device__ __forceinline__ void leaf_plan(LeafPlanArgs co
     bool const     split = nl != 0 && nl != count;
     bool const     sl    = nl <= nr; // the left child wins a size tie
     uint32_t const sc    = sl ? nl : nr;
-    uint32_t const to0   = p.node.start >= A.half ? p.node.start - A.half : p.node.start + A.half;
+    uint32_t const to0   = A.half == 0                ? p.node.start
+                           : p.node.start >= A.half ? p.node.start - A.half
+                                                    : p.node.start + A.half;
     uint32_t const sb    = to0 + (sl ? 0 : nl);
     uint32_t const nchb  = split ? (sc + A.crows - 1) / A.crows : 0;
     if (threadIdx.x == 0)
@@ -5524,10 +5474,6 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
             throw ConfigError("grower: leafwise needs 1 <= max_leaves <= 512 and "
                               "max_depth <= 255");
         }
-        if (max_root_rows >= 0x80000000u)
-        {
-            throw ConfigError("grower: leafwise takes fewer than 2^31 rows");
-        }
     }
     else if (cfg_.tp.max_depth > 8)
     {
@@ -5661,9 +5607,12 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     arena_.want<uint32_t>(bbase_, max_front_ + 1);
     arena_.want<uint32_t>(brange_, max_front_ + 2);
     arena_.want<Chunk>(bchunks_, max_bchunks_);
-    // (leafwise: two halves of one buffer, a node's segment in either)
-    arena_.want<uint32_t>(rows_[0], static_cast<size_t>(max_rows_) * (cfg_.leaf ? 2 : 1));
-    if (!cfg_.leaf)
+    // (leafwise: two halves of one buffer, a node's segment in either, while a
+    // 32-bit index reaches both; from 2^31 rows on a second buffer, whose rows
+    // each pop copies back)
+    bool const far = max_rows_ >= k_far_rows;
+    arena_.want<uint32_t>(rows_[0], static_cast<size_t>(max_rows_) * (cfg_.leaf && !far ? 2 : 1));
+    if (!cfg_.leaf || far)
     {
         arena_.want<uint32_t>(rows_[1], max_rows_);
     }
@@ -5755,8 +5704,7 @@ Grower::Grower(Plane const &plane, GrowConfig const &cfg, std::vector<uint32_t> 
     {
         throw ConfigError("grower: bins per feature exceed the shared-memory budget");
     }
-    allow_smem(find_kernel<false>);
-    allow_smem(find_kernel<true>);
+    allow_smem(find_kernel);
     // the level finder prefixes up to 16 nodes at a time in shared memory
     lgroup_ = static_cast<uint32_t>(std::min<size_t>(
         k_lfind_thr / 32, std::max<size_t>(1, (192 * 1024) / (max_nb_ * sizeof(double2)))));
@@ -6203,9 +6151,9 @@ void Grower::level(uint32_t L, uint32_t const *rows_in, uint32_t *rows_out,
     }
     else
     {
-        launch_k(pdl_, find_kernel<false>, fgrid, k_find_thr, find_smem, s, ctl_, nodes_[cur],
+        launch_k(pdl_, find_kernel, fgrid, k_find_thr, find_smem, s, ctl_, nodes_[cur],
                  hist_[cur], total_cells_, cell_off_, sel_nb_, sel_, n_sel_, mono_, n_mono_,
-                 cfg_.tp, cand_, max_nb_, qscale_, nullptr, cw_, fgroups_);
+                 cfg_.tp, cand_, max_nb_, nullptr, fgroups_);
     }
     BB_LAUNCH("find_kernel");
     if (!packed_)
@@ -6634,6 +6582,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
     auto             *cand      = static_cast<LeafCand *>(cand_heap_);
     auto             *tdev      = static_cast<TreeOut *>(tree_dev_);
     LeafPop const    *pp        = &st->pop;
+    bool const        far       = max_rows_ >= k_far_rows;
     void             *pool      = hist_[0];
     uint32_t          launches  = 0;
     LeafTurn const    turn{st,       cand,           leaves_,          free_,    lout,
@@ -6676,9 +6625,9 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
         }
         else
         {
-            launch_k(pdl_, find_kernel<false>, fgrid, k_find_thr, find_smem, s, ctl_, nodes, pool,
+            launch_k(pdl_, find_kernel, fgrid, k_find_thr, find_smem, s, ctl_, nodes, pool,
                      total_cells_, cell_off_, sel_nb_, sel_, n_sel_, mono_, n_mono_, tp, cand_,
-                     max_nb_, qscale_, slot_of, cw_, fgroups_);
+                     max_nb_, slot_of, fgroups_);
         }
         BB_LAUNCH("find_kernel");
         launch_k(pdl_, leaf_best_kernel, 2, k_best_thr, 0, s, ctl_, cand_, n_sel_, nodes, lout,
@@ -6719,7 +6668,8 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
         {
             LeafPlanArgs const lp{ctl_,   pchunks_, pleft_, prbase_,   nleft_,     dst_,
                                   build_, brange_,  bbase_, bchunks_,  bpair_,     nodes_[0],
-                                  nodes_[1], slot_of_, lout, crows_,   max_rows_,  pp, leaf_tick_};
+                                  nodes_[1], slot_of_, lout, crows_,   far ? 0u : max_rows_,
+                                  pp,     leaf_tick_};
             auto count = [&](auto kern)
             {
                 launch_k(pdl_, kern, max_pchunks_, k_threads, 0, s, ctl_, pchunks_, nodes_[0],
@@ -6729,10 +6679,16 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
             plane_.u8 ? count(pcount_kernel<uint8_t, true>) : count(pcount_kernel<uint16_t, true>);
             BB_LAUNCH("pcount_kernel");
             launch_k(pdl_, pscatter_kernel, max_pchunks_, k_threads, 0, s, ctl_, pchunks_,
-                     nodes_[0], best_, pleft_, prbase_, nleft_, dst_, rows_[0], rows_[0], dirs_,
-                     static_cast<unsigned long long *>(pool), build_, total_cells_ * cw_,
+                     nodes_[0], best_, pleft_, prbase_, nleft_, dst_, rows_[0], rows_[far ? 1 : 0],
+                     dirs_, static_cast<unsigned long long *>(pool), build_, total_cells_ * cw_,
                      quant_ ? total_cells_ * cw_ : 0);
             BB_LAUNCH("pscatter_kernel");
+            if (far)
+            {
+                launch_k(pdl_, leaf_copyback_kernel, 148 * 4, k_threads, 0, s, pp, lout, rows_[1],
+                         rows_[0]);
+                BB_LAUNCH("leaf_copyback_kernel");
+            }
             n_launch_ = 0;
             build(rows_[0], n_sel_, 0, true, 1);
             uint32_t const nb = n_launch_;
@@ -6761,7 +6717,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                 launch_k(pdl_, leaf_turn_kernel, 1, k_pop_thr, 0, s, turn, handle);
                 BB_LAUNCH("leaf_turn_kernel");
                 // count, scatter, the build, subtraction, totals, find, best, turn
-                body_launches_ = 2 + nb + 5;
+                body_launches_ = 2 + nb + 5 + (far ? 1 : 0);
             }
         }
         catch (...)
