@@ -5811,6 +5811,19 @@ void Grower::use_set(uint32_t set)
         }
     }
     sel_h_ = sets_h_[set];
+    set_   = set;
+}
+
+Grower::LoopGraph::~LoopGraph()
+{
+    if (x != nullptr)
+    {
+        cudaGraphExecDestroy(x);
+    }
+    if (g != nullptr)
+    {
+        cudaGraphDestroy(g);
+    }
 }
 
 Grower::~Grower()
@@ -5824,14 +5837,7 @@ Grower::~Grower()
         }
     }
     arena_.release();
-    if (loop_x_ != nullptr)
-    {
-        cudaGraphExecDestroy(loop_x_);
-    }
-    if (loop_g_ != nullptr)
-    {
-        cudaGraphDestroy(loop_g_);
-    }
+    loops_.clear();
     cudaStreamSynchronize(stream_);
     if (lout_h_ != nullptr)
     {
@@ -6644,14 +6650,27 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
 
     // one pop as a fixed sequence of launches, repeated by the loop graph's
     // WHILE node until leaf_commit_kernel says the heap is done; captured
-    // once (the loop's buffers and the tree's device record do not move)
-    if (loop_x_ == nullptr)
+    // once for these gradients and this table set (the loop's other buffers and
+    // the tree's device record do not move)
+    float2 const *const lgh  = quant_ ? nullptr : gh_cur_; // (the codes have one place)
+    LoopGraph const    *loop = nullptr;
+    for (auto const &l : loops_)
+    {
+        if (l->gh == lgh && l->set == set_)
+        {
+            loop = l.get();
+        }
+    }
+    if (loop == nullptr)
     {
         Profile *const saved = prof_;
         prof_                = nullptr; // no per-phase events inside the loop graph
-        BB_CHECK(cudaGraphCreate(&loop_g_, 0));
+        auto made            = std::make_unique<LoopGraph>();
+        made->gh             = lgh;
+        made->set            = set_;
+        BB_CHECK(cudaGraphCreate(&made->g, 0));
         cudaGraphConditionalHandle handle{};
-        BB_CHECK(cudaGraphConditionalHandleCreate(&handle, loop_g_, 1,
+        BB_CHECK(cudaGraphConditionalHandleCreate(&handle, made->g, 1,
                                                   cudaGraphCondAssignDefault));
         cudaGraphNodeParams cp{};
         cp.type               = cudaGraphNodeTypeConditional;
@@ -6659,7 +6678,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
         cp.conditional.type   = cudaGraphCondTypeWhile;
         cp.conditional.size   = 1;
         cudaGraphNode_t cnode{};
-        BB_CHECK(cudaGraphAddNode(&cnode, loop_g_, nullptr, 0, &cp));
+        BB_CHECK(cudaGraphAddNode(&cnode, made->g, nullptr, 0, &cp));
         cudaGraph_t const body = cp.conditional.phGraph_out[0];
         BB_CHECK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
@@ -6730,15 +6749,21 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
         }
         cudaGraph_t captured{};
         BB_CHECK(cudaStreamEndCapture(s, &captured));
-        BB_CHECK(cudaGraphInstantiate(&loop_x_, loop_g_, 0));
+        BB_CHECK(cudaGraphInstantiate(&made->x, made->g, 0));
         prof_     = saved;
         n_launch_ = n0;
+        if (loops_.size() == k_loops)
+        {
+            loops_.erase(loops_.begin()); // (every tree before this one was waited for)
+        }
+        loops_.push_back(std::move(made));
+        loop = loops_.back().get();
     }
     if (prof_ != nullptr)
     {
         phase_begin();
     }
-    BB_CHECK(cudaGraphLaunch(loop_x_, s));
+    BB_CHECK(cudaGraphLaunch(loop->x, s));
     if (prof_ != nullptr)
     {
         phase_end(prof_->other_ms);

@@ -396,15 +396,25 @@ class Grower
     uint32_t *slot_of_  = nullptr; // the children's pool slots
     // the device-side pop loop: its state (the candidate heap, free pool
     // slots, the leaves, the node count), the tree being grown, and the
-    // loop's graph (a conditional WHILE node over one pop's launches)
+    // loop's graphs (a conditional WHILE node over one pop's launches). A graph
+    // holds the gradients' address (exact form) and its table set's: a softmax
+    // round, whose class trees take turns, has one per class
     void            *loop_      = nullptr;
     void            *cand_heap_ = nullptr;
     Node            *leaves_    = nullptr;
     uint32_t        *free_      = nullptr;
     void            *tree_dev_  = nullptr;
     uint32_t        *leaf_tick_ = nullptr; // last-CTA tickets: the partition's, the pair's
-    cudaGraph_t      loop_g_    = nullptr;
-    cudaGraphExec_t  loop_x_    = nullptr;
+    struct LoopGraph
+    {
+        float2 const   *gh  = nullptr;
+        uint32_t        set = 0;
+        cudaGraph_t     g   = nullptr;
+        cudaGraphExec_t x   = nullptr;
+        ~LoopGraph();
+    };
+    std::vector<std::unique_ptr<LoopGraph>> loops_; // at most k_loops, the oldest first
+    static constexpr size_t                 k_loops = 16; // (the most classes)
     uint32_t         body_launches_ = 0;
     uint32_t  crows_    = 0;       // rows per histogram-build chunk
     bool      quant_    = false;
@@ -416,6 +426,7 @@ class Grower
     // tile tables point into set k's part); unused tile slots hold
     // k_no_sel_tile, so their CTAs exit
     std::vector<std::vector<uint32_t>> sets_h_;
+    uint32_t  set_           = 0; // the set in use
     uint32_t *sel_base_      = nullptr;
     uint32_t *cell_off_base_ = nullptr;
     uint32_t *sel_nb_base_   = nullptr;
