@@ -1206,14 +1206,25 @@ __global__ void __launch_bounds__(k_find_thr)
 //
 // What bounds it is instructions: a candidate's rule in FP64, two divisions
 // among it, is about 100 of them. So the children's scores are first
-// approximated in float from the exact integer sums (relative error below
-// 2^-20: four conversions, a reciprocal and a few products), and only
-// candidates whose approximation comes within 2^-14 of the warp's largest take
-// the rule: the true maximum and all its ties are among them, and their gains
-// are the serial scan's, bit for bit. A bin without rows is skipped: its
-// candidates are the bin before's over again, later in the scan's order. (Over
-// 2,000 features: the root's find 15.3 to 10.5 us under ncu, 1,834 to 1,209
-// instructions a warp; both children of a pop 27 to 15.6 us.)
+// approximated in float from the exact integer sums (four conversions, a
+// reciprocal and a few products), and only candidates whose approximation comes
+// within 2^-14 of the warp's largest take the rule: where the approximation is
+// off by less than 2^-15, the true maximum and all its ties are among them, and
+// their gains are the serial scan's, bit for bit. Its steps are off by 2^-20
+// together, but for t = |g| - l1, which may cancel. So l1 is taken 2^-20 of itself
+// too small, which makes t at least its true value less 2^-22 of it and at most
+// e = 2^-19 l1 more, and a score s, the sum of t^2 / h over both children, at
+// most 2 e sqrt(2 / (the least h)) sqrt(s) too large: what the largest score may
+// have too much is taken off before it is compared (QNode::slack). The rule's own
+// sums are right to E = 2^-49 M, M = l1 + (largest code x rows) a bound of them
+// all, which changes s by 2 x + x^2 of itself, x = E sqrt(2 / (the least h) / s):
+// x is at most 2^-17 where s is at least 2^-63 M^2 / (the least h), and the screen
+// decides only where the warp's largest score is (QNode::floor, with a factor of
+// 4 to spare). A bin without rows is skipped: its candidates are the bin before's
+// over again, later in the scan's order. (Over 2,000 features: the root's find
+// 15.3 to 10.5 us under ncu, 1,834 to 1,209 instructions a warp; both children of
+// a pop 27 to 15.6 us. |g| - l1 in FP64 instead: 2-3% of a round; the rule for
+// every candidate where l1 is not 0: 7-20% of such a round.)
 
 constexpr uint32_t k_qfind_warps = 8;
 constexpr uint32_t k_qfind_group = 8; // cells held per lane
@@ -1321,12 +1332,14 @@ struct QNode
     double   mg, mh, node_sc, real_g, real_h, lo, hi;
     int64_t  img, irg, irh; // the missing bin's g; g and h without it
     float    fmh, l1, l2, sure, maybe;
+    float    slack, floor; // of the largest score's root, and the least one that decides
     uint32_t n_dir;
     int      mc;
 
+    // qmax: the largest code
     __device__ __forceinline__ void start(int64_t qg, int64_t qh, int64_t mqg, int64_t mqh,
                                           Node const &nd, int mono, double2 const &sc,
-                                          TreeParams const &tp)
+                                          TreeParams const &tp, float qmax)
     {
         mg      = static_cast<double>(mqg) * sc.x;
         mh      = static_cast<double>(mqh) * sc.y;
@@ -1345,11 +1358,18 @@ struct QNode
         // (an inf or NaN here makes every candidate take the rule)
         float const sx = 1.0F / static_cast<float>(sc.x);
         float const sy = 1.0F / static_cast<float>(sc.y);
-        l1             = tp.lambda_l1 * sx;
+        l1             = tp.lambda_l1 * sx * (1.0F - 0x1p-20F);
         l2             = tp.lambda_l2 * sy;
         // min_child_hess, which the rule compares in FP64, from both sides
         sure  = tp.min_child_hess * sy * (1.0F + 0x1p-18F);
         maybe = tp.min_child_hess * sy * (1.0F - 0x1p-18F);
+        // (where nothing else keeps h off 0 it is a whole number, or the score is
+        // not finite)
+        float const least = fmaxf(maybe, 0.0F) + l2;
+        float const q     = sqrtf(2.0F / (least > 0.0F ? least : 1.0F));
+        float const m     = 0x1p-31F * q * (l1 + (qmax * static_cast<float>(nd.gcount)));
+        floor             = fmaxf(1e-30F, m * m);
+        slack             = 0x1p-18F * q * l1;
     }
 };
 
@@ -1474,10 +1494,11 @@ __device__ __forceinline__ void qscore_group(QCell<CW2> const (&v)[k_qfind_group
     {
         top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
     }
+    top = top - (n.slack * sqrtf(fmaxf(top, 0.0F)));
     // monotone candidates are chosen among by their leaf weights too, and
     // scores past the normal float range say nothing about the order: the
     // rule for them all
-    float const bar = n.mc != 0 || !(top < 1e37F && top > 1e-30F && n.l2 < 1e30F && n.l1 < 1e30F)
+    float const bar = n.mc != 0 || !(top < 1e37F && top > n.floor && n.l2 < 1e30F && n.l1 < 1e30F)
                           ? -0.5F
                           : top * (1.0F - 0x1p-14F);
     uint32_t todo = 0;
@@ -1851,7 +1872,8 @@ __global__ void __launch_bounds__(k_qfind_warps * 32, CW2 ? 1 : 3)
             }
             QNode n;
             n.start(nd.qg, nd.qh, miss.g(), miss.h(), nd,
-                    (mono != nullptr && f < n_mono) ? mono[f] : 0, sc, tp);
+                    (mono != nullptr && f < n_mono) ? mono[f] : 0, sc, tp,
+                    CW2 ? 32767.0F : 127.0F);
             __shared__ QHand<CW2> hand_s[k_qfind_warps];
             QHand<CW2>           &hand  = hand_s[threadIdx.x >> 5];
             double                best  = 0.0;
@@ -5293,7 +5315,7 @@ __global__ void __launch_bounds__(k_pop_thr)
                              interaction_allows(nd, fgroups, f);
             QNode n;
             n.start(qg, qh, miss.g(), miss.h(), nd, (mono != nullptr && f < n_mono) ? mono[f] : 0,
-                    sc, tp);
+                    sc, tp, CW2 ? 32767.0F : 127.0F);
             if (held)
             {
                 if (may)
