@@ -31,10 +31,10 @@
 // which adds them in tree order. Batches of up to a few hundred rows take a CTA
 // per row, a thread per tree and the nodes straight from L2
 // (row_predict_kernel), up to 64 rows several CTAs per row. Depths 9 and 10 take a lane
-// per row (heap_predict_kernel), and so do shallow trees over batches that fill
-// its passes. Deeper ensembles, or planes wider than 8
-// mirror tiles (256 u8 / 128 u16 features), use the node form: the reference's
-// layout and walk, nodes in global memory.
+// per row (heap_predict_kernel), the trees split over CTAs where the rows do not fill
+// the GPU, and so do shallow trees over batches that fill its passes. Deeper
+// ensembles, or planes wider than 8 mirror tiles (256 u8 / 128 u16 features), use
+// the node form: the reference's layout and walk, nodes in global memory.
 #include "bonsai_b200.h"
 #include "ingest.cuh"
 
@@ -151,6 +151,8 @@ constexpr uint32_t k_row_vals     = 4096; // values a row's CTA holds at once
 constexpr uint32_t k_row_batch    = 1024;
 constexpr uint32_t k_few_rows     = 64; // up to these, several CTAs per row
 constexpr uint32_t k_few_threads  = 128;
+constexpr size_t   k_max_smem     = 227 * 1024;
+constexpr size_t   k_max_vals     = size_t{256} << 20; // bytes of a split batch's leaf values
 
 __device__ __forceinline__ void cp_async16(void *smem_dst, void const *gsrc)
 {
@@ -447,14 +449,17 @@ __global__ void __launch_bounds__(k_few_threads)
 // tree's slots together, an odd stride from tree to tree, the code offsets
 // for a lane's column of the staged codes.
 // Scores of rows [blockIdx.x * rows_per_cta, + rows_per_cta), taken T x R
-// rows at a time: out[r] = init + lr * sum.
-template <typename CodeT, uint32_t D, uint32_t T, uint32_t R, bool BY32>
+// rows at a time: out[r] = init + lr * sum. SPLIT, with vals not null: the trees
+// [blockIdx.y * trees_per_split, + trees_per_split) only, every (tree, row) leaf
+// value into vals[t * n_rows + r].
+template <typename CodeT, uint32_t D, uint32_t T, uint32_t R, bool BY32, bool SPLIT>
 __global__ void __launch_bounds__(T)
     heap_predict_kernel(uint4 const *__restrict__ mirror, uint64_t n_rows, uint32_t n_tiles,
                         uint32_t const *__restrict__ last_words,
                         uint32_t const *__restrict__ heaps, uint32_t n_trees,
                         uint32_t chunk_trees, uint32_t rows_per_cta, float lr, float init,
-                        float *__restrict__ out)
+                        float *__restrict__ out, uint32_t trees_per_split,
+                        float *__restrict__ vals)
 {
     constexpr uint32_t slots = 2u << D; // per tree: root at 1, leaves at [2^D, 2^(D+1))
     constexpr uint32_t pitch = slots + (BY32 ? 1u : 0u);
@@ -472,6 +477,8 @@ __global__ void __launch_bounds__(T)
     uint32_t const heap_a = static_cast<uint32_t>(__cvta_generic_to_shared(heap_s));
     uint64_t const begin = static_cast<uint64_t>(blockIdx.x) * rows_per_cta;
     uint64_t const end   = min(n_rows, begin + rows_per_cta);
+    uint32_t const t0    = SPLIT ? blockIdx.y * trees_per_split : 0;
+    uint32_t const t1    = SPLIT ? min(n_trees, t0 + trees_per_split) : n_trees;
 
     for (uint64_t row0 = begin; row0 < end; row0 += T * R)
     {
@@ -514,9 +521,9 @@ __global__ void __launch_bounds__(T)
         {
             acc[k] = 0.0F;
         }
-        for (uint32_t c0 = 0; c0 < n_trees; c0 += chunk_trees)
+        for (uint32_t c0 = t0; c0 < t1; c0 += chunk_trees)
         {
-            uint32_t const nc = min(chunk_trees, n_trees - c0);
+            uint32_t const nc = min(chunk_trees, t1 - c0);
             __syncthreads(); // codes staged; the previous chunk's walks done
             if constexpr (BY32)
             {
@@ -583,18 +590,72 @@ __global__ void __launch_bounds__(T)
 #pragma unroll
                 for (uint32_t k = 0; k < R; ++k)
                 {
-                    acc[k] = acc[k] + __uint_as_float(lds_u32(p[k]));
+                    float const v = __uint_as_float(lds_u32(p[k]));
+                    if (!SPLIT || vals == nullptr)
+                    {
+                        acc[k] = acc[k] + v;
+                    }
+                    else if (row[k] < end)
+                    {
+                        vals[(static_cast<uint64_t>(c0 + j) * n_rows) + row[k]] = v;
+                    }
                 }
             }
         }
 #pragma unroll
         for (uint32_t k = 0; k < R; ++k)
         {
-            if (row[k] < end)
+            if (row[k] < end && (!SPLIT || vals == nullptr))
             {
                 out[row[k]] = __fadd_rn(init, __fmul_rn(acc[k], lr));
             }
         }
+    }
+}
+
+// Every row's leaf values summed in tree order: one thread per row.
+__global__ void sum_rows_kernel(float const *__restrict__ vals, uint64_t n_rows, uint32_t n_trees,
+                                float lr, float init, float *__restrict__ out)
+{
+    uint64_t const r = (static_cast<uint64_t>(blockIdx.x) * blockDim.x) + threadIdx.x;
+    if (r >= n_rows)
+    {
+        return;
+    }
+    float acc = 0.0F;
+#pragma unroll 8
+    for (uint32_t t = 0; t < n_trees; ++t)
+    {
+        acc = acc + vals[(static_cast<uint64_t>(t) * n_rows) + r];
+    }
+    out[r] = __fadd_rn(init, __fmul_rn(acc, lr));
+}
+
+// The same sum with one warp per row, for batches too small to fill the GPU
+// with rows: lanes load 32 trees' values at once, every lane adds them in
+// order from the shuffles.
+__global__ void sum_warp_kernel(float const *__restrict__ vals, uint64_t n_rows, uint32_t n_trees,
+                                float lr, float init, float *__restrict__ out)
+{
+    uint64_t const r    = ((static_cast<uint64_t>(blockIdx.x) * blockDim.x) + threadIdx.x) >> 5;
+    uint32_t const lane = threadIdx.x & 31u;
+    if (r >= n_rows)
+    {
+        return;
+    }
+    float acc = 0.0F;
+    for (uint32_t t0 = 0; t0 < n_trees; t0 += 32)
+    {
+        uint32_t const m = min(32u, n_trees - t0);
+        float const    v = lane < m ? vals[(static_cast<uint64_t>(t0 + lane) * n_rows) + r] : 0.0F;
+        for (uint32_t j = 0; j < m; ++j)
+        {
+            acc = acc + __shfl_sync(0xFFFFFFFFu, v, static_cast<int>(j));
+        }
+    }
+    if (lane == 0)
+    {
+        out[r] = __fadd_rn(init, __fmul_rn(acc, lr));
     }
 }
 
@@ -643,7 +704,8 @@ __global__ void node_predict_kernel(BinT const *__restrict__ bins, uint64_t n_pa
 // A device buffer released with its owner.
 struct DeviceBuf
 {
-    void *p = nullptr;
+    void  *p   = nullptr;
+    size_t cap = 0;
     DeviceBuf() = default;
     DeviceBuf(DeviceBuf const &) = delete;
     DeviceBuf &operator=(DeviceBuf const &) = delete;
@@ -657,6 +719,21 @@ struct DeviceBuf
     void alloc(size_t bytes)
     {
         check(cudaMalloc(&p, std::max<size_t>(bytes, 16)), "cudaMalloc");
+        cap = std::max<size_t>(bytes, 16);
+    }
+    // At least this many bytes, whatever they hold.
+    void grow(size_t bytes)
+    {
+        if (cap < bytes)
+        {
+            if (p != nullptr)
+            {
+                check(cudaFree(p), "cudaFree");
+                p   = nullptr;
+                cap = 0;
+            }
+            alloc(bytes);
+        }
     }
     void upload(void const *src, size_t bytes)
     {
@@ -687,7 +764,7 @@ struct bb_predict_plan
     uint32_t    lane_rows = 0; // a lane CTA's most rows
     uint64_t    heap_ctas = 0; // resident CTAs of the lane-per-row form; 0: not taken
     bb::DeviceBuf heaps;
-    bb::DeviceBuf vals;       // a few rows' leaf values
+    bb::DeviceBuf vals;       // a few rows' leaf values; a split batch's (depths 9, 10)
     bb::DeviceBuf last_words; // per staged code word, its features' last bins
     bb::DeviceBuf last, roots, feature, split, left, right, dl, value;
     // the host runs' output, grown on demand; runs through one plan serialise
@@ -836,33 +913,40 @@ void plan_check_plane(bb_predict_plan const &pl, Plane const &p)
 }
 
 using HeapFn = void (*)(uint4 const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
-                        uint32_t, uint32_t, uint32_t, float, float, float *);
+                        uint32_t, uint32_t, uint32_t, float, float, float *, uint32_t, float *);
 
-template <typename CodeT> HeapFn heap_fn_d(uint32_t D)
+// The shapes of a lane per row: 512 threads of two rows, and for depths 9 and 10
+// 256 of one, whose codes leave room on planes of four to eight mirror tiles.
+template <typename CodeT> HeapFn heap_fn_d(uint32_t D, uint32_t T)
 {
+    if (T == 256)
+    {
+        return D == 9 ? heap_predict_kernel<CodeT, 9, 256, 1, false, true>
+                      : heap_predict_kernel<CodeT, 10, 256, 1, false, true>;
+    }
     switch (D)
     {
-    case 1: return heap_predict_kernel<CodeT, 1, 512, 2, true>;
-    case 2: return heap_predict_kernel<CodeT, 2, 512, 2, true>;
-    case 3: return heap_predict_kernel<CodeT, 3, 512, 2, true>;
-    case 4: return heap_predict_kernel<CodeT, 4, 512, 2, true>;
-    case 5: return heap_predict_kernel<CodeT, 5, 512, 2, true>;
-    case 6: return heap_predict_kernel<CodeT, 6, 512, 2, true>;
-    case 7: return heap_predict_kernel<CodeT, 7, 512, 2, true>;
-    case 8: return heap_predict_kernel<CodeT, 8, 512, 2, true>;
-    case 9: return heap_predict_kernel<CodeT, 9, 512, 2, false>;
-    case 10: return heap_predict_kernel<CodeT, 10, 512, 2, false>;
+    case 1: return heap_predict_kernel<CodeT, 1, 512, 2, true, false>;
+    case 2: return heap_predict_kernel<CodeT, 2, 512, 2, true, false>;
+    case 3: return heap_predict_kernel<CodeT, 3, 512, 2, true, false>;
+    case 4: return heap_predict_kernel<CodeT, 4, 512, 2, true, false>;
+    case 5: return heap_predict_kernel<CodeT, 5, 512, 2, true, false>;
+    case 6: return heap_predict_kernel<CodeT, 6, 512, 2, true, false>;
+    case 7: return heap_predict_kernel<CodeT, 7, 512, 2, true, false>;
+    case 8: return heap_predict_kernel<CodeT, 8, 512, 2, true, false>;
+    case 9: return heap_predict_kernel<CodeT, 9, 512, 2, false, false>;
+    case 10: return heap_predict_kernel<CodeT, 10, 512, 2, false, false>;
     default: throw std::logic_error("bb_predict_plan: heap depth out of range");
     }
 }
 
-HeapFn heap_fn(bool u8, uint32_t D)
+HeapFn heap_fn(bool u8, uint32_t D, uint32_t T)
 {
-    return u8 ? heap_fn_d<uint8_t>(D) : heap_fn_d<uint16_t>(D);
+    return u8 ? heap_fn_d<uint8_t>(D, T) : heap_fn_d<uint16_t>(D, T);
 }
 
-// A lane per row: the trees of a chunk, and the shared memory of a CTA of 1,024
-// rows (both code variants, 64 bytes a row and mirror tile) with it.
+// A lane per row: the trees of a chunk, and the shared memory of a CTA of T
+// threads (both code variants, 64 bytes a row and mirror tile) with it.
 uint32_t heap_chunk(uint32_t D)
 {
     uint32_t const tree_bytes = (2u << D) * 4u;
@@ -872,10 +956,16 @@ uint32_t heap_chunk(uint32_t D)
     return D <= 6 ? chunk & ~31u : (D <= k_lane_depth ? 2 * chunk : chunk);
 }
 
-size_t heap_smem(uint32_t D, uint32_t n_tiles)
+size_t heap_smem(uint32_t D, uint32_t n_tiles, uint32_t T)
 {
     size_t const tree_bytes = ((2u << D) + (D <= k_lane_depth ? 1u : 0u)) * 4u;
-    return (size_t{1024} * n_tiles * 64) + (heap_chunk(D) * tree_bytes);
+    return (size_t{T == 512 ? 1024u : T} * n_tiles * 64) + (heap_chunk(D) * tree_bytes);
+}
+
+// The larger shape whose rows' codes fit.
+uint32_t heap_threads(uint32_t D, uint32_t n_tiles)
+{
+    return heap_smem(D, n_tiles, 512) <= k_max_smem ? 512 : 256;
 }
 
 using LaneFn = void (*)(uint32_t const *, uint64_t, uint32_t, uint32_t const *, uint32_t const *,
@@ -923,14 +1013,57 @@ uint32_t heap_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
                      cudaStream_t s)
 {
     uint64_t const n   = p.n_rows;
+    uint32_t const T   = heap_threads(pl.depth, pl.n_tiles);
     uint64_t const per = std::max<uint64_t>(
         32, ((((n + pl.heap_ctas - 1) / pl.heap_ctas) + 31) / 32) * 32);
-    heap_fn(pl.u8, pl.depth)<<<ceil_div(n, per), 512, heap_smem(pl.depth, pl.n_tiles), s>>>(
+    heap_fn(pl.u8, pl.depth, T)<<<ceil_div(n, per), T, heap_smem(pl.depth, pl.n_tiles, T), s>>>(
         static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words.as<uint32_t>(),
         pl.heaps.as<uint32_t>(), n_trees, heap_chunk(pl.depth), static_cast<uint32_t>(per), pl.lr,
-        pl.init, out);
+        pl.init, out, n_trees, nullptr);
     BB_LAUNCH("heap_predict_kernel");
     return 1;
+}
+
+// Depths 9 and 10 where the rows alone leave SMs idle: the trees split over CTAs
+// of 256 rows, every leaf value kept, then summed in tree order. (500 trees of
+// depth 10 over 28 features, 64 / 4,000 / 30,000 rows: 31 / 60 / 192 us; a wave
+// of CTAs that each take every tree 379 / 383 / 585.)
+uint32_t split_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, float *out,
+                      cudaStream_t s)
+{
+    uint64_t const n        = p.n_rows;
+    uint32_t const chunk    = heap_chunk(pl.depth);
+    uint32_t const row_blks = ceil_div(n, 256);
+    uint32_t const n_chunks = ceil_div(n_trees, chunk);
+    uint32_t       splits   = std::min(ceil_div(2 * pl.sms, row_blks), n_chunks);
+    uint32_t const tps      = ceil_div(ceil_div(n_trees, splits), chunk) * chunk;
+    splits                  = ceil_div(n_trees, tps);
+    float *vals             = nullptr;
+    if (splits > 1)
+    {
+        pl.vals.grow(n * static_cast<size_t>(n_trees) * sizeof(float));
+        vals = pl.vals.as<float>();
+    }
+    heap_fn(pl.u8, pl.depth, 256)<<<dim3(row_blks, splits), 256,
+                                    heap_smem(pl.depth, pl.n_tiles, 256), s>>>(
+        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words.as<uint32_t>(),
+        pl.heaps.as<uint32_t>(), n_trees, chunk, 256, pl.lr, pl.init, out, tps, vals);
+    BB_LAUNCH("heap_predict_kernel");
+    if (splits == 1)
+    {
+        return 1;
+    }
+    if (n < 4096)
+    {
+        sum_warp_kernel<<<ceil_div(n * 32, 256), 256, 0, s>>>(vals, n, n_trees, pl.lr, pl.init,
+                                                              out);
+    }
+    else
+    {
+        sum_rows_kernel<<<ceil_div(n, 256), 256, 0, s>>>(vals, n, n_trees, pl.lr, pl.init, out);
+    }
+    BB_LAUNCH("predict sum kernel");
+    return 2;
 }
 
 // Whether a lane per row is the faster form at depths up to k_lane_depth. It has
@@ -1026,6 +1159,10 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
         BB_LAUNCH("lane_predict_kernel");
         return 1;
     }
+    if (ceil_div(n, 256) < pl.sms && n * static_cast<size_t>(n_trees) * sizeof(float) <= k_max_vals)
+    {
+        return split_launch(pl, p, n_trees, out, s);
+    }
     return heap_launch(pl, p, n_trees, out, s);
 }
 
@@ -1093,11 +1230,16 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
         }
         if (D > k_lane_depth || n_tiles <= 2)
         {
-            HeapFn const fn = heap_fn(p.u8, D);
+            uint32_t const T  = heap_threads(D, n_tiles);
+            HeapFn const   fn = heap_fn(p.u8, D, T);
             allow_smem(fn);
+            if (D > k_lane_depth)
+            {
+                allow_smem(heap_fn(p.u8, D, 256));
+            }
             int occ = 0;
-            check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 512,
-                                                                heap_smem(D, n_tiles)),
+            check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, static_cast<int>(T),
+                                                                heap_smem(D, n_tiles, T)),
                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
             pl->heap_ctas = static_cast<uint64_t>(std::max(occ, 1)) * pl->sms;
         }
