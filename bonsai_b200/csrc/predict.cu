@@ -28,7 +28,7 @@
 // where a lane per row has conflicts on the lower levels' nodes. A CTA holds a
 // tile of rows and streams the trees through shared memory, 32 at a time; the
 // 32 values of each row go by shared memory to the row's thread,
-// which adds them in tree order. Batches of up to a few hundred rows take a CTA
+// which adds them in tree order. Batches of up to some 1,000 rows take a CTA
 // per row, a thread per tree and the nodes straight from L2
 // (row_predict_kernel), up to 64 rows several CTAs per row. Depths 9 and 10 take a lane
 // per row (heap_predict_kernel), the trees split over CTAs where the rows do not fill
@@ -145,10 +145,6 @@ constexpr uint32_t k_lane_smem    = 113 * 1024; // two CTAs an SM
 constexpr uint32_t k_val_stride   = 33;   // a row's 32 values, rows in different banks
 constexpr uint32_t k_row_threads  = 1024;
 constexpr uint32_t k_row_vals     = 4096; // values a row's CTA holds at once
-// Batches up to this many rows take a CTA per row: 1,000 trees of depth 8 over
-// 1,000 rows take 37.0 us so and 41.1 a lane per tree (whose floor is one SM
-// streaming every tree), over 2,000 rows 63.0 and 41.3.
-constexpr uint32_t k_row_batch    = 1024;
 constexpr uint32_t k_few_rows     = 64; // up to these, several CTAs per row
 constexpr uint32_t k_few_threads  = 128;
 constexpr size_t   k_max_smem     = 227 * 1024;
@@ -1008,6 +1004,31 @@ uint32_t sm_count()
     return static_cast<uint32_t>(std::max(n, 1));
 }
 
+// Whether a batch takes a CTA per row: while the rows' CTAs of 256 threads all
+// run at once, eight an SM, and over two such waves where there are many trees,
+// which every CTA of the lane-per-tree form streams whole. (28 features, device
+// us a CTA per row / a lane per tree: 1,000 trees of depth 8, 1,100 rows 22.8 / 41.3,
+// 1,700 rows 39.4 / 42.0, 2,500 rows 55.2 / 43.3; 300 trees of depth 8, 1,100 rows
+// 11.7 / 16.7, 1,700 rows 18.8 / 16.8.)
+bool row_form(uint64_t n, uint32_t n_trees, uint32_t sms)
+{
+    uint64_t const wave = uint64_t{8} * sms;
+    return n <= wave || (n <= 2 * wave && n_trees > 500);
+}
+
+// Threads of a row's CTA: the most, up to 1,024, that let every row's CTA run at
+// once. (1,000 trees of depth 8 over 1,000 rows: 38.8 us with 1,024, 28.9 with 512,
+// 20.9 with 256; over 150 rows 12.5, 12.6, 14.6.)
+uint32_t row_threads(uint64_t n, uint32_t sms)
+{
+    uint32_t T = k_row_threads;
+    while (T > 256 && n * T > uint64_t{2048} * sms)
+    {
+        T /= 2;
+    }
+    return T;
+}
+
 // A lane per row: one wave of resident CTAs, each over an equal run of rows.
 uint32_t heap_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, float *out,
                      cudaStream_t s)
@@ -1133,9 +1154,9 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
             BB_LAUNCH("few_sum_kernel");
             return 2;
         }
-        if (n <= k_row_batch)
+        if (row_form(n, n_trees, pl.sms))
         {
-            uint32_t const T = std::min(k_row_threads, ((n_trees + 31) / 32) * 32);
+            uint32_t const T = std::min(row_threads(n, pl.sms), ((n_trees + 31) / 32) * 32);
             auto const     fn = pl.u8 ? row_predict_kernel<uint8_t> : row_predict_kernel<uint16_t>;
             fn<<<static_cast<uint32_t>(n), T, 0, s>>>(mirror, n, pl.n_tiles,
                                                       pl.last_words.as<uint32_t>(),
