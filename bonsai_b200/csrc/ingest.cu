@@ -11,10 +11,16 @@ namespace
 constexpr uint32_t k_tile_rows  = 256; // rows per CTA tile
 constexpr uint32_t k_tile_feats = 32;  // features per CTA tile
 constexpr uint32_t k_threads    = 256;
-constexpr uint32_t k_bin_ctas   = 148 * 2; // two CTAs' tiles and cuts fit an SM
-// batches that take a thread per value (a refill of 10,007 x 28 from device
-// memory: 23.6 us so, 33.7 by row tiles; 30,000 rows take the tiles, 28.6 us)
-constexpr uint64_t k_small_rows = 16384;
+constexpr uint32_t k_bin_ctas   = 148 * 2; // two CTAs' padded tables and tiles fit an SM
+constexpr size_t   k_max_smem   = 227 * 1024;
+// Batches of up to this many values (whole tiles of features counted) take a
+// thread per value. It writes single bytes to columns far apart and reads its cuts
+// from L2, so what it costs goes with the values, where a wave of row tiles takes
+// about 20 us whatever is in it. Refills from device memory, wall us by value / by
+// row tiles, 255 cuts: 8,000 x 28 26.4 / 33.4, 16,000 x 28 31.5 / 33.8; 1,000 x
+// 333 32.7 / 34.8, 2,000 x 333 40.4 / 36.6; 250 x 1,000 30.0 / 35.7, 500 x 1,000
+// 36.7 / 34.0, 8,000 x 1,000 260 / 99.
+constexpr uint64_t k_small_values = 3 << 17;
 constexpr uint32_t k_pad_cuts   = 256;
 
 // lower_bound for K values over K tables of cuts at once (cut(k, i) is table
@@ -116,7 +122,7 @@ __device__ __forceinline__ void bin_features(float const *c_s, uint32_t const *c
 // tile(s), which leave its registers whole; the columns leave through shared
 // memory as 16-byte runs of rows. A CTA keeps its features' cuts over all its
 // row tiles and has the next tile's values on their way (cp.async) while it
-// searches. PAD: every table of at most k_pad_cuts cuts, each filled up to
+// searches, where its shared memory holds two (TWO). PAD: every table of at most k_pad_cuts cuts, each filled up to
 // that many with +inf, so that the search is eight steps of a load at a
 // constant offset, a compare and a conditional add (3 instructions a step;
 // tables of any length take about 20). (A thread per 16 rows of a feature,
@@ -126,7 +132,7 @@ __device__ __forceinline__ void bin_features(float const *c_s, uint32_t const *c
 constexpr uint32_t k_x_stride = k_tile_feats + 4; // floats: rows' 16-byte quarters in
                                                   // different banks
 
-template <typename BinT, bool PAD>
+template <typename BinT, bool PAD, bool TWO>
 __global__ void __launch_bounds__(k_threads, 2)
     bin_apply_kernel(float const *__restrict__ X, uint64_t n_rows, uint32_t F,
                      uint64_t row0, float const *__restrict__ cuts,
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(k_threads, 2)
 {
     extern __shared__ __align__(16) float smem[];
     constexpr uint32_t x_floats = k_tile_rows * k_x_stride;
-    float             *c_s      = smem + (2 * x_floats);
+    float             *c_s      = smem + ((TWO ? 2 : 1) * x_floats);
     uint32_t          *coff_s   = reinterpret_cast<uint32_t *>(c_s + max_tile_cuts);
     constexpr uint32_t per      = 16 / sizeof(BinT);
     constexpr uint32_t words    = k_tile_feats * sizeof(BinT) / 4; // of a row's codes
@@ -209,12 +215,19 @@ __global__ void __launch_bounds__(k_threads, 2)
             c_s[i] = cuts[c_begin + i];
         }
     }
-    for (uint32_t b = 0; r0 < n_rows; r0 += stride, b ^= 1)
+    for (uint32_t b = 0; r0 < n_rows; r0 += stride, b ^= TWO ? 1 : 0)
     {
         uint32_t const nr =
             static_cast<uint32_t>(n_rows - r0 < k_tile_rows ? n_rows - r0 : k_tile_rows);
-        load(r0 + stride, b ^ 1);
-        asm volatile("cp.async.wait_group 1;\n" ::);
+        if constexpr (TWO)
+        {
+            load(r0 + stride, b ^ 1);
+            asm volatile("cp.async.wait_group 1;\n" ::);
+        }
+        else
+        {
+            asm volatile("cp.async.wait_all;\n" ::);
+        }
         __syncthreads(); // the tile is here (and the cuts)
         float         *tile = smem + (b * x_floats);
         uint32_t const rr   = threadIdx.x;
@@ -291,6 +304,10 @@ __global__ void __launch_bounds__(k_threads, 2)
             }
         }
         __syncthreads(); // the columns have left: the buffer may be filled again
+        if constexpr (!TWO)
+        {
+            load(r0 + stride, 0);
+        }
     }
     asm volatile("cp.async.wait_all;\n" ::);
 }
@@ -421,19 +438,21 @@ void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream, flo
     {
         max_tile_cuts = k_tile_feats * k_pad_cuts;
     }
-    size_t const smem = (2 * k_tile_rows * k_x_stride * sizeof(float)) +
-                        (max_tile_cuts * sizeof(float)) +
-                        ((k_tile_feats + 1) * sizeof(uint32_t));
-    // (one tile of values beside the cuts is what the capacity stands for)
-    if ((k_tile_rows * (k_tile_feats + 1) * sizeof(float)) + (max_tile_cuts * sizeof(float)) +
-            ((k_tile_feats + 1) * sizeof(uint32_t)) >
-        227 * 1024)
+    size_t const one   = k_tile_rows * k_x_stride * sizeof(float); // a tile of values
+    size_t const table = (max_tile_cuts * sizeof(float)) + ((k_tile_feats + 1) * sizeof(uint32_t));
+    // (a tile of values, rows 33 apart, beside the cuts is what the capacity stands for)
+    if ((k_tile_rows * (k_tile_feats + 1) * sizeof(float)) + table > k_max_smem)
     {
         throw ConfigError("ingest: a 32-feature tile's cuts exceed shared memory");
     }
-    bool const by_value = smem > 227 * 1024; // two tiles do not fit beside them
-    auto const kern8  = pad ? bin_apply_kernel<uint8_t, true> : bin_apply_kernel<uint8_t, false>;
-    auto const kern16 = pad ? bin_apply_kernel<uint16_t, true> : bin_apply_kernel<uint16_t, false>;
+    bool const   two_tiles = (2 * one) + table <= k_max_smem;
+    bool const   by_value  = one + table > k_max_smem;
+    size_t const smem      = ((two_tiles ? 2 : 1) * one) + table;
+    // (u8 codes have at most 256 cuts a feature: padded tables, two tiles)
+    auto const kern8  = bin_apply_kernel<uint8_t, true, true>;
+    auto const kern16 = pad         ? bin_apply_kernel<uint16_t, true, true>
+                        : two_tiles ? bin_apply_kernel<uint16_t, false, true>
+                                    : bin_apply_kernel<uint16_t, false, false>;
     if (!by_value)
     {
         p.u8 ? allow_smem(kern8) : allow_smem(kern16);
@@ -443,10 +462,10 @@ void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream, flo
 
     auto launch = [&](float const *Xd, uint64_t rows, uint64_t row0)
     {
-        if (rows <= k_small_rows || by_value)
+        uint32_t const per   = k_mirror_bytes / (p.u8 ? 1 : 2);
+        uint32_t const slots = p.n_tiles * per;
+        if (rows * slots <= k_small_values || by_value)
         {
-            uint32_t const per   = k_mirror_bytes / (p.u8 ? 1 : 2);
-            uint32_t const slots = p.n_tiles * per;
             uint32_t const grid  = ceil_div(rows * slots, k_threads);
             if (p.u8)
             {
@@ -463,11 +482,11 @@ void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream, flo
             BB_LAUNCH("bin_rows_kernel");
             return;
         }
-        // a CTA keeps its features' cuts over its row tiles: no more CTAs than
-        // about fit the GPU at once
+        // a CTA keeps its features' cuts over its row tiles: no more CTAs than about
+        // fit the GPU at once (one more than fit takes as long again: 333 features
+        // as 27 x 11 CTAs, of which 296 fit, 54.0 us for 8,000 rows, as 26 x 11 50.1)
         uint32_t const ftiles = ceil_div(F, k_tile_feats);
-        dim3 const     grid(std::min(ceil_div(rows, k_tile_rows),
-                                     std::max(1u, ceil_div(k_bin_ctas, ftiles))),
+        dim3 const     grid(std::min(ceil_div(rows, k_tile_rows), std::max(1u, k_bin_ctas / ftiles)),
                             ftiles);
         if (p.u8)
         {
