@@ -281,6 +281,19 @@ __global__ void advance_kernel(uint32_t *round, uint32_t step)
     *round += step;
 }
 
+// The largest of n codes. (A loop of its own, with nothing in it but the maximum:
+// with the refusal in the loop it took 21 or 36 ms over 56 million codes, as the
+// compiler happened to inline it.)
+template <typename T> T largest(T const *codes, uint64_t n)
+{
+    T most = 0;
+    for (uint64_t i = 0; i < n; ++i)
+    {
+        most = std::max(most, codes[i]);
+    }
+    return most;
+}
+
 template <typename T> T *dmalloc(size_t n)
 {
     void *p = nullptr;
@@ -1403,17 +1416,16 @@ extern "C"
                 need(is_u8 == 0 || max_nb <= 256, "bb_plane_from_bins: u8 codes need <= 256 bins");
                 need(max_nb <= 65535, "bb_plane_from_bins: more than 65535 bins");
                 // every code indexes a histogram cell: check them all
-                for (uint32_t f = 0; f < n_feats; ++f)
+                auto const check_codes = [&](auto const *codes)
                 {
-                    uint32_t const nb = cut_off[f + 1] - cut_off[f];
-                    for (uint64_t r = 0; r < n_rows; ++r)
+                    for (uint32_t f = 0; f < n_feats; ++f)
                     {
-                        uint32_t const b =
-                            is_u8 != 0 ? static_cast<uint8_t const *>(bins)[(f * n_rows) + r]
-                                       : static_cast<uint16_t const *>(bins)[(f * n_rows) + r];
-                        need(b < nb, "bb_plane_from_bins: a code is not below its bin count");
+                        need(largest(codes + (f * n_rows), n_rows) < cut_off[f + 1] - cut_off[f],
+                             "bb_plane_from_bins: a code is not below its bin count");
                     }
-                }
+                };
+                is_u8 != 0 ? check_codes(static_cast<uint8_t const *>(bins))
+                           : check_codes(static_cast<uint16_t const *>(bins));
                 auto   pl = std::make_unique<bb_plane>();
                 Plane &p  = pl->p;
                 p.n_rows  = n_rows;
