@@ -1376,13 +1376,12 @@ extern "C"
                                     cudaMemcpyHostToDevice));
                 BB_CHECK(cudaMemcpy(p.n_bins, nb.data(), n_feats * 4, cudaMemcpyHostToDevice));
                 size_t const bytes = static_cast<size_t>(n_feats) * p.n_pad * (p.u8 ? 1 : 2);
-                p.bins = dmalloc<char>(bytes);
+                alloc_codes(p, n_rows);
                 BB_CHECK(cudaMemset(p.bins, 0, bytes));
                 cudaStream_t s;
                 BB_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
                 try
                 {
-                    alloc_mirror(p);
                     ingest(p, X, x_on_device != 0, s);
                     BB_CHECK(cudaStreamSynchronize(s));
                 }
@@ -1452,7 +1451,7 @@ extern "C"
                 BB_CHECK(cudaMemcpy(p.n_bins, nb.data(), n_feats * 4, cudaMemcpyHostToDevice));
                 size_t const el    = p.u8 ? 1 : 2;
                 size_t const bytes = static_cast<size_t>(n_feats) * p.n_pad * el;
-                p.bins = dmalloc<char>(bytes);
+                alloc_codes(p, n_rows);
                 BB_CHECK(cudaMemset(p.bins, 0, bytes));
                 BB_CHECK(cudaMemcpy2D(p.bins, p.n_pad * el, bins, n_rows * el, n_rows * el,
                                       n_feats, cudaMemcpyHostToDevice));
@@ -1542,12 +1541,8 @@ extern "C"
                 BB_CHECK(cudaMemcpy(p.n_bins, q.n_bins, F * 4, cudaMemcpyDeviceToDevice));
                 uint64_t const cap_pad = ((max_rows + 63) / 64) * 64;
                 size_t const   el      = p.u8 ? 1 : 2;
-                p.bins = dmalloc<char>(static_cast<size_t>(F) * cap_pad * el);
+                alloc_codes(p, max_rows);
                 BB_CHECK(cudaMemset(p.bins, 0, static_cast<size_t>(F) * cap_pad * el));
-                uint32_t const per = k_mirror_bytes / (p.u8 ? 1 : 2);
-                p.n_tiles          = (F + per - 1) / per;
-                p.mirror = dmalloc<char>(static_cast<size_t>(p.n_tiles) * max_rows *
-                                         k_mirror_bytes);
                 // host rows go up through a staging buffer of at most 64 MB
                 uint64_t const row_bytes = static_cast<uint64_t>(F) * sizeof(float);
                 p.stage_rows             = stage_rows_for(F, max_rows);
@@ -1593,7 +1588,6 @@ extern "C"
         }
         cudaFree(p.stage);
         cudaFree(p.bins);
-        cudaFree(p.mirror);
         cudaFree(p.cuts);
         cudaFree(p.cut_off);
         cudaFree(p.n_bins);

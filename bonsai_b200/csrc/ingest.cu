@@ -377,17 +377,20 @@ __global__ void __launch_bounds__(k_threads)
 
 } // namespace
 
-void alloc_mirror(Plane &p)
+void alloc_codes(Plane &p, uint64_t rows)
 {
-    uint32_t const per = k_mirror_bytes / (p.u8 ? 1 : 2);
-    p.n_tiles          = (p.n_feats + per - 1) / per;
-    size_t const bytes = static_cast<size_t>(p.n_tiles) * p.n_rows * k_mirror_bytes;
-    MemPool::with_trim([&] { return cudaMalloc(&p.mirror, bytes); }, "cudaMalloc");
+    uint32_t const per   = k_mirror_bytes / (p.u8 ? 1 : 2);
+    p.n_tiles            = (p.n_feats + per - 1) / per;
+    uint64_t const pad   = ((rows + 63) / 64) * 64;
+    size_t const   codes = ((static_cast<size_t>(p.n_feats) * pad * (p.u8 ? 1 : 2)) + 255) &
+                         ~size_t{255};
+    size_t const bytes   = codes + (static_cast<size_t>(p.n_tiles) * rows * k_mirror_bytes);
+    MemPool::with_trim([&] { return cudaMalloc(&p.bins, bytes); }, "cudaMalloc");
+    p.mirror = static_cast<char *>(p.bins) + codes;
 }
 
 void build_mirror(Plane &p, cudaStream_t stream)
 {
-    alloc_mirror(p);
     dim3 const grid(ceil_div(p.n_rows, k_threads), p.n_tiles);
     if (p.u8)
     {

@@ -24,7 +24,7 @@ struct Plane
     uint64_t  n_pad    = 0;
     uint32_t  n_feats  = 0;
     bool      u8       = true;
-    void     *bins     = nullptr; // uint8_t or uint16_t
+    void     *bins     = nullptr; // uint8_t or uint16_t; its block holds the mirror too
     // Row-major mirror for gathered reads: features in tiles of 32 bytes
     // (32 u8 or 16 u16 codes), tile t of row r at mirror[(t * n_rows + r) * 32],
     // so one gathered row costs one 32-byte DRAM sector per tile.
@@ -61,10 +61,13 @@ struct Plane
 void ingest(Plane &p, float const *X, bool x_on_device, cudaStream_t stream,
             float *owned_stage = nullptr, uint64_t owned_rows = 0);
 
-// Allocates p.mirror; ingest() then fills it beside the feature-major codes.
-void alloc_mirror(Plane &p);
+// Allocates p.bins and p.mirror (and sets p.n_tiles) for up to `rows` rows: one
+// block, freed through p.bins. (Each mapping of memory takes 0.3 ms and more, and
+// ingest() needs both before it starts: of 2,000,000 x 28 device rows a plane took
+// 2.43 ms to make with two, 1.79 with one.)
+void alloc_codes(Plane &p, uint64_t rows);
 
-// Fills p.mirror from the feature-major codes (allocating it).
+// Fills p.mirror from the feature-major codes.
 void build_mirror(Plane &p, cudaStream_t stream);
 
 // Rows of a request plane's staging buffer for batches of up to max_rows:
