@@ -557,6 +557,102 @@ __device__ __forceinline__ void tree_node(TreeWalk<M> &w, double const (&G)[M], 
     }
 }
 
+// Small batches of deep trees give a warp a subtree: a tree is one warp's chain of
+// dependent operations (depth 8: 80 us), and a few rows leave most warps idle. A
+// node's sum is linear in A_L and A_R, so a subtree's warp adds its own part of
+// every node above it: with A_s what the subtree hands up times the edges' factors
+// from a node's child down to it, plus or minus sum_k G_k (...) A_s,k there. The
+// units are the subtrees at level J (3, or 2 up to depth 6), and leaves above it. (28 features,
+// depth 8, one row: 100 trees 96 us a warp per tree, 33 so; 1,000 trees 94 and
+// 80; a path at a time, as deeper ensembles take it, 50 and 70.)
+struct TreeUnit
+{
+    uint32_t rec[3];     // the records above it, offsets in the blob
+    uint32_t begin, end; // its own; none: a leaf
+    float    leaf;
+    uint32_t len;        // records above it
+    uint32_t dirs;       // bit l: left at the path's level l
+};
+constexpr uint32_t k_unit_levels = 3;
+constexpr uint32_t k_unit_rec    = sizeof(NodeRec) + sizeof(MergedRec);
+constexpr uint32_t k_unit_path   = k_unit_levels * k_unit_rec; // bytes before a subtree's records
+
+// Levels above the units of a plan of at most D levels.
+__host__ __device__ constexpr uint32_t unit_levels(uint32_t D)
+{
+    return D == 8 ? 3 : (D == 6 ? 2 : 0);
+}
+
+// The unit u below its path's level-L node (at level L = u.len: the unit itself),
+// its records at shared address `first`.
+template <uint32_t D, uint32_t M, uint32_t J, uint32_t L>
+__device__ __forceinline__ void unit_node(TreeWalk<M> &w, TreeUnit const &u, uint32_t first,
+                                          double const (&G)[M], double (&A)[M])
+{
+    if constexpr (L == J)
+    {
+        if (u.begin != u.end)
+        {
+            w.at = first + k_unit_path;
+            tree_node<D, M, L>(w, G, A);
+            return;
+        }
+    }
+    if (u.len == L)
+    {
+        double const vd = u.leaf;
+#pragma unroll
+        for (uint32_t k = 0; k < M; ++k)
+        {
+            A[k] = vd;
+        }
+        return;
+    }
+    if constexpr (L < J)
+    {
+        uint32_t const rec    = first + (L * k_unit_rec);
+        uint4 const    h      = lds_u4(rec);
+        double2 const  z      = lds_d2(rec + 16);
+        uint32_t const f      = (h.x & 0xFFFFu) * k_tree_rows;
+        bool const     merged = L > 0 && (h.x & k_nr_merged) != 0;
+        uint32_t const code   = w.codes[f];
+        bool const     left = code == (h.y >> 16) ? (h.x & k_nr_dl) != 0 : code <= (h.y & 0xFFFFu);
+        bool const     onp  = !merged || ((w.on >> ((h.x >> k_nr_level) & 15u)) & 1u) != 0;
+        double const   d    = (left && onp ? 1.0 : 0.0) - z.x;
+        double const   dp   = merged ? lds_d2(rec + 32).x : 0.0;
+        bool const     down = ((u.dirs >> L) & 1u) != 0; // to the left
+        w.on |= (down == left) && onp ? 1u << L : 0u;
+        // (the earlier edge's 1 / f_p: 1 where there is none)
+        auto const r = [&](uint32_t k)
+        {
+            if (!merged)
+            {
+                return 1.0;
+            }
+            double2 const r2 = lds_d2(rec + 48 + ((k & ~1u) * 8));
+            return (k & 1u) == 0 ? r2.x : r2.y;
+        };
+        auto const rho = [&](uint32_t k) { return onp ? __fma_rn(d, w.t[k], z.x) * r(k) : z.y; };
+        double     GX[M];
+#pragma unroll
+        for (uint32_t k = 0; k < M; ++k)
+        {
+            double const x = rho(k) * G[k];
+            GX[k]          = down ? x : G[k] - x;
+        }
+        unit_node<D, M, J, L + 1>(w, u, first, GX, A);
+        double sg = 0.0;
+#pragma unroll
+        for (uint32_t k = 0; k < M; ++k)
+        {
+            double const x = rho(k);
+            sg             = __fma_rn(G[k] * A[k], __fma_rn(-dp, x, d) * r(k), sg);
+            A[k] *= down ? x : 1.0 - x;
+        }
+        w.phi[f] += onp ? (down ? sg : -sg) : 0.0;
+    }
+}
+
 __device__ __forceinline__ uint32_t cluster_rank()
 {
     uint32_t r;
@@ -585,14 +681,14 @@ __device__ __forceinline__ double ld_cluster(uint32_t a, uint32_t rank)
 
 // grid (cluster CTAs x row tiles, splits), blockDim.x / 32 warps: warp v of
 // the cluster and split takes trees v, v + V, v + 2 V ... of all V warps that
-// share its rows. A split writes its raw sums into ws, the only split composes
-// the row.
-template <uint32_t D>
+// share its rows (J > 0: units). A split writes its raw sums into ws, the only
+// split composes the row.
+template <uint32_t D, uint32_t J>
 __global__ void __launch_bounds__(tree_warps(D) * 32, 1)
     shap_tree_kernel(uint8_t const *__restrict__ bins8, uint16_t const *__restrict__ bins16,
                      uint64_t n_pad, uint64_t n_rows, uint32_t F,
                      unsigned char const *__restrict__ blob, uint32_t const *__restrict__ blob_off,
-                     uint32_t n_trees, uint32_t room, Gauss g, double lr, double bias, double init,
+                     TreeUnit const *__restrict__ units, uint32_t n_trees, uint32_t room, Gauss g, double lr, double bias, double init,
                      double *__restrict__ out, double *__restrict__ ws)
 {
     constexpr uint32_t M = D / 2;
@@ -642,6 +738,32 @@ __global__ void __launch_bounds__(tree_warps(D) * 32, 1)
     uint32_t const       V     = gridDim.y * C * W;
     for (uint32_t t = (((blockIdx.y * C) + rank) * W) + wid; t < n_trees; t += V)
     {
+        if constexpr (J > 0)
+        {
+            TreeUnit const u = units[t];
+            __syncwarp(); // the previous unit is done
+#pragma unroll
+            for (uint32_t l = 0; l < J; ++l)
+            {
+                // (a record alone may be shorter: what follows it is not read)
+                if (l < u.len && lane < k_unit_rec / 16)
+                {
+                    *reinterpret_cast<uint4 *>(mine + (l * k_unit_rec) + (lane * 16)) =
+                        __ldg(reinterpret_cast<uint4 const *>(blob + u.rec[l]) + lane);
+                }
+            }
+            for (uint32_t x = lane * 16; x < u.end - u.begin; x += 512)
+            {
+                *reinterpret_cast<uint4 *>(mine + k_unit_path + x) =
+                    __ldg(reinterpret_cast<uint4 const *>(blob + u.begin + x));
+            }
+            __syncwarp();
+            double A[M];
+            w.on   = 0;
+            w.went = 0;
+            unit_node<D, M, J, 0>(w, u, first, G, A);
+            continue;
+        }
         uint32_t const b0 = blob_off[t];
         uint32_t const nb = blob_off[t + 1] - b0;
         __syncwarp(); // the previous tree is done
@@ -894,6 +1016,11 @@ struct TreeBlob
     std::vector<unsigned char> bytes;
     std::vector<uint32_t>      off; // n_trees + 1
     uint32_t                   room = 0;
+    // the units at level J (0: none): a path's records so far, and theirs
+    uint32_t              J         = 0;
+    uint32_t              unit_room = 0;
+    uint32_t              rec[k_unit_levels] = {};
+    std::vector<TreeUnit> units;
 };
 
 // Levels of split nodes; 0 where the tree form cannot take the tree (over 8
@@ -931,9 +1058,22 @@ struct PathEdge
     double   z; // merged cover fraction
 };
 
+// Node id's subtree; dirs: the path's left turns, bit by level.
 void pack_node(TreeView const &t, uint32_t const *last, uint32_t id, std::vector<PathEdge> &path,
-               std::vector<double> const &gx, std::vector<unsigned char> &out)
+               std::vector<double> const &gx, TreeBlob &tb, uint32_t dirs)
 {
+    std::vector<unsigned char> &out   = tb.bytes;
+    uint32_t const              level = static_cast<uint32_t>(path.size());
+    uint32_t const              begin = static_cast<uint32_t>(out.size());
+    auto const                  unit  = [&](uint32_t b, uint32_t e, float leaf, uint32_t len, uint32_t d)
+    {
+        tb.units.push_back({{tb.rec[0], tb.rec[1], tb.rec[2]}, b, e, leaf, len, d});
+        tb.unit_room = std::max(tb.unit_room, k_unit_path + (e - b));
+    };
+    if (level < tb.J)
+    {
+        tb.rec[level] = begin;
+    }
     uint32_t const f     = t.feature[id];
     uint32_t const l     = t.left[id];
     uint32_t const r     = t.right[id];
@@ -972,12 +1112,21 @@ void pack_node(TreeView const &t, uint32_t const *last, uint32_t id, std::vector
     for (int side = 0; side < 2; ++side)
     {
         uint32_t const child = side == 0 ? l : r;
+        uint32_t const d     = dirs | (side == 0 ? 1u << level : 0u);
         if (t.feature[child] != k_leaf_flag)
         {
             path.push_back({f, zp * (side == 0 ? fl : fr)});
-            pack_node(t, last, child, path, gx, out);
+            pack_node(t, last, child, path, gx, tb, d);
             path.pop_back();
         }
+        else if (level < tb.J)
+        {
+            unit(0, 0, t.value[child], level + 1, d);
+        }
+    }
+    if (level == tb.J && tb.J > 0)
+    {
+        unit(begin, static_cast<uint32_t>(out.size()), 0.0F, level, dirs);
     }
 }
 
@@ -997,9 +1146,13 @@ struct ShapBuf
             cudaFree(p);
         }
     }
-    void upload(void const *src, size_t bytes)
+    void alloc(size_t bytes)
     {
         check(cudaMalloc(&p, std::max<size_t>(bytes, 16)), "cudaMalloc");
+    }
+    void upload(void const *src, size_t bytes)
+    {
+        alloc(bytes);
         if (bytes > 0)
         {
             check(cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
@@ -1047,7 +1200,14 @@ struct bb_shap_plan
     uint32_t              room       = 0;
     uint32_t              warps      = 0;
     uint32_t              resident[4] = {};
-    bb::ShapBuf           blob, blob_off;
+    uint32_t              unit_level = 0; // small batches' units: their level (0: none)
+    uint32_t              n_units    = 0;
+    uint32_t              unit_room  = 0;
+    uint32_t              unit_warps = 0;
+    bb::ShapBuf           tables; // of the tree form: the three below
+    uint32_t             *blob_off = nullptr;
+    bb::TreeUnit         *units    = nullptr;
+    unsigned char        *blob     = nullptr;
     std::mutex            mu;
     bb::ShapBuf           ws, out;
     size_t                ws_cap = 0, out_cap = 0;
@@ -1067,12 +1227,21 @@ namespace
 {
 
 using TreeFn = void (*)(uint8_t const *, uint16_t const *, uint64_t, uint64_t, uint32_t,
-                        unsigned char const *, uint32_t const *, uint32_t, uint32_t, Gauss, double,
-                        double, double, double *, double *);
+                        unsigned char const *, uint32_t const *, TreeUnit const *, uint32_t,
+                        uint32_t, Gauss, double, double, double, double *, double *);
 
-TreeFn tree_fn(uint32_t D)
+// J: the units' level, 0 for whole trees.
+TreeFn tree_fn(uint32_t D, uint32_t J)
 {
-    return D == 4 ? shap_tree_kernel<4> : (D == 6 ? shap_tree_kernel<6> : shap_tree_kernel<8>);
+    switch ((10 * D) + J)
+    {
+    case 40: return shap_tree_kernel<4, 0>;
+    case 60: return shap_tree_kernel<6, 0>;
+    case 62: return shap_tree_kernel<6, 2>;
+    case 80: return shap_tree_kernel<8, 0>;
+    case 83: return shap_tree_kernel<8, 3>;
+    default: throw std::logic_error("bb_shap_plan: no such tree form");
+    }
 }
 
 size_t tree_smem(uint32_t F, uint32_t room, uint32_t warps)
@@ -1116,12 +1285,14 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
     }
     TreeBlob              tb;
     std::vector<PathEdge> path;
+    // (trees for several rounds of all the GPU's warps even them out by themselves)
+    tb.J = views.size() < size_t{4} * k_sms * tree_warps(D) ? unit_levels(D) : 0;
     for (TreeView const &tv : views)
     {
         tb.off.push_back(static_cast<uint32_t>(tb.bytes.size()));
         if (tv.feature[0] != k_leaf_flag)
         {
-            pack_node(tv, last.data(), 0, path, gx, tb.bytes);
+            pack_node(tv, last.data(), 0, path, gx, tb, 0);
         }
         if (tb.bytes.size() > 0x7FFFFFFFu)
         {
@@ -1130,9 +1301,14 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
         tb.room = std::max(tb.room, static_cast<uint32_t>(tb.bytes.size()) - tb.off.back());
     }
     tb.off.push_back(static_cast<uint32_t>(tb.bytes.size()));
-    size_t const one = tree_smem(F, tb.room, 1) - tree_smem(F, tb.room, 0);
-    pl->warps        = static_cast<uint32_t>(
-        std::min<size_t>(tree_warps(D), (k_tree_smem - tree_smem(F, tb.room, 0)) / one));
+    // the warps whose slices and trees (or units) of `room` bytes fit a CTA
+    auto const warps = [&](uint32_t room)
+    {
+        size_t const one = tree_smem(F, room, 1) - tree_smem(F, room, 0);
+        return static_cast<uint32_t>(
+            std::min<size_t>(tree_warps(D), (k_tree_smem - tree_smem(F, room, 0)) / one));
+    };
+    pl->warps = warps(tb.room);
     if (pl->warps < 2)
     {
         return nullptr;
@@ -1141,18 +1317,38 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
     pl->n_trees     = static_cast<uint32_t>(views.size());
     pl->room        = tb.room;
     size_t const sm = tree_smem(F, tb.room, pl->warps);
-    allow_smem(tree_fn(D));
+    allow_smem(tree_fn(D, 0));
     for (uint32_t c = 0; c < 4; ++c)
     {
         cudaLaunchAttribute at{};
         cudaLaunchConfig_t  cfg = tree_config(&at, 1u << c, dim3(1u << c), pl->warps, sm, nullptr);
         int                 n   = 0;
-        check(cudaOccupancyMaxActiveClusters(&n, tree_fn(D), &cfg),
+        check(cudaOccupancyMaxActiveClusters(&n, tree_fn(D, 0), &cfg),
               "cudaOccupancyMaxActiveClusters");
         pl->resident[c] = static_cast<uint32_t>(n) << c;
     }
-    pl->blob.upload(tb.bytes.data(), tb.bytes.size());
-    pl->blob_off.upload(tb.off.data(), tb.off.size() * 4);
+    if (tb.J > 0)
+    {
+        allow_smem(tree_fn(D, tb.J));
+        pl->unit_level = tb.J;
+        pl->n_units    = static_cast<uint32_t>(tb.units.size());
+        pl->unit_room  = tb.unit_room;
+        pl->unit_warps = std::max(1u, warps(pl->unit_room));
+    }
+    // the offsets, the units and the blob, in one allocation (a unit's path reads whole
+    // records: some bytes past the blob, whatever they hold)
+    size_t const n_off = ((tb.off.size() * 4) + 15) & ~size_t{15};
+    size_t const n_un  = tb.units.size() * sizeof(TreeUnit);
+    pl->tables.alloc(n_off + n_un + tb.bytes.size() + k_unit_rec);
+    auto *const at = pl->tables.as<unsigned char>();
+    pl->blob_off   = reinterpret_cast<uint32_t *>(at);
+    pl->units      = reinterpret_cast<TreeUnit *>(at + n_off);
+    pl->blob       = at + n_off + n_un;
+    auto const up  = [](void *to, void const *from, size_t n)
+    { check(cudaMemcpy(to, from, n, cudaMemcpyHostToDevice), "cudaMemcpy"); };
+    up(pl->blob_off, tb.off.data(), tb.off.size() * 4);
+    up(pl->units, tb.units.data(), n_un);
+    up(pl->blob, tb.bytes.data(), tb.bytes.size());
     return pl;
 }
 
@@ -1305,15 +1501,39 @@ uint32_t tree_launch(bb_shap_plan &pl, Plane const &p, double *out, cudaStream_t
     uint64_t const n      = p.n_rows;
     uint32_t const F      = pl.n_feats;
     uint32_t const tiles  = ceil_div(n, k_tree_rows);
-    uint32_t       W      = std::min(pl.warps, pl.n_trees);
+    uint32_t       J      = 0;
+    uint32_t       count  = pl.n_trees;
+    uint32_t       room   = pl.room;
+    uint32_t       most   = pl.warps;
+    uint32_t       W      = std::min(most, count);
     uint32_t       C      = 1;
     uint32_t       splits = 1;
     if (n < k_tree_split)
     {
-        // about one CTA per SM, a tree at a time in each of its warps
-        splits = std::min(std::max(1u, k_sms / tiles), pl.n_trees);
-        W      = std::min(pl.warps, ceil_div(pl.n_trees, splits));
-        splits = std::min(splits, ceil_div(pl.n_trees, W));
+        // about one CTA per SM, a tree (a unit) at a time in each of its warps: the
+        // form whose rounds over them take less, a unit 1 / 40 of a tree beside its
+        // share of it
+        uint32_t const ctas  = std::max(1u, k_sms / tiles);
+        uint32_t const trees = ceil_div(count, ctas * most) * 40;
+        uint32_t const share = (40 >> pl.unit_level) + 1;
+        if (pl.unit_level > 0 && ceil_div(pl.n_units, ctas * pl.unit_warps) * share < trees)
+        {
+            J     = pl.unit_level;
+            count = pl.n_units;
+            room  = pl.unit_room;
+            most  = pl.unit_warps;
+        }
+        splits = std::min(ctas, count);
+        W      = std::min(most, ceil_div(count, splits));
+        splits = std::min(splits, ceil_div(count, W));
+        if (pl.tree_depth == 4 && count <= 8 * most && pl.resident[3] != 0)
+        {
+            // short trees: a cluster's warps take one each, without the second
+            // launch that sums the splits
+            C      = 8;
+            W      = ceil_div(count, 8);
+            splits = 1;
+        }
     }
     else
     {
@@ -1345,13 +1565,14 @@ uint32_t tree_launch(bb_shap_plan &pl, Plane const &p, double *out, cudaStream_t
     }
     cudaLaunchAttribute at{};
     cudaLaunchConfig_t  cfg = tree_config(&at, C, dim3(tiles * C, splits), W,
-                                          tree_smem(F, pl.room, W), s);
+                                          tree_smem(F, room, W), s);
     check(cudaLaunchKernelEx(
-              &cfg, tree_fn(pl.tree_depth),
+              &cfg, tree_fn(pl.tree_depth, J),
               p.u8 ? static_cast<uint8_t const *>(p.bins) : static_cast<uint8_t const *>(nullptr),
               p.u8 ? static_cast<uint16_t const *>(nullptr) : static_cast<uint16_t const *>(p.bins),
-              p.n_pad, n, F, static_cast<unsigned char const *>(pl.blob.p),
-              static_cast<uint32_t const *>(pl.blob_off.p), pl.n_trees, pl.room, pl.gauss, pl.lr,
+              p.n_pad, n, F, static_cast<unsigned char const *>(pl.blob),
+              static_cast<uint32_t const *>(pl.blob_off), static_cast<TreeUnit const *>(pl.units),
+              count, room, pl.gauss, pl.lr,
               pl.bias, pl.init, out, ws),
           "shap_tree_kernel");
     if (splits == 1)
