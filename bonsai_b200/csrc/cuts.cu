@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(256)
                      uint32_t tiles)
 {
     __shared__ uint32_t wsum[8];
-    uint32_t const      used = (counts[blockIdx.x] + k_sort_tile - 1) / k_sort_tile;
+    uint32_t const      used =
+        static_cast<uint32_t>((uint64_t{counts[blockIdx.x]} + k_sort_tile - 1) / k_sort_tile);
     uint32_t           *c    = tc + ((static_cast<uint64_t>(blockIdx.x) * tiles) * 256) + threadIdx.x;
     uint32_t            sum  = 0;
 #pragma unroll 8
