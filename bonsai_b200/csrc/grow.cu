@@ -6726,15 +6726,15 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                      dirs_, static_cast<unsigned long long *>(pool), build_, total_cells_ * cw_,
                      quant_ ? total_cells_ * cw_ : 0);
             BB_LAUNCH("pscatter_kernel");
+            n_launch_ = 2; // the body's so far: count, scatter
             if (far)
             {
                 launch_k(pdl_, leaf_copyback_kernel, 148 * 4, k_threads, 0, s, pp, lout, rows_[1],
                          rows_[0]);
                 BB_LAUNCH("leaf_copyback_kernel");
+                n_launch_ += 1;
             }
-            n_launch_ = 0;
             build(rows_[0], n_sel_, 0, true, 1);
-            uint32_t const nb = n_launch_;
             if (quant_)
             {
                 launch_k(pdl_, cw_ == 2 ? leaf_pair_kernel<true> : leaf_pair_kernel<false>,
@@ -6743,7 +6743,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                          n_sel_, mono_, n_mono_, tp, qscale_, fgroups_, cand_, leaf_tick_ + 1,
                          handle);
                 BB_LAUNCH("leaf_pair_kernel");
-                body_launches_ = 2 + nb + 1; // count, scatter, the build, the pair
+                n_launch_ += 1;
             }
             else
             {
@@ -6759,9 +6759,9 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
                 find(nodes_[1], slot_of_, &st->may_split);
                 launch_k(pdl_, leaf_turn_kernel, 1, k_pop_thr, 0, s, turn, handle);
                 BB_LAUNCH("leaf_turn_kernel");
-                // count, scatter, the build, subtraction, totals, find, best, turn
-                body_launches_ = 2 + nb + 5 + (far ? 1 : 0);
+                n_launch_ += 5; // subtraction, totals, find, best, turn
             }
+            body_launches_ = n_launch_;
         }
         catch (...)
         {
