@@ -1269,7 +1269,7 @@ bb_booster *create_booster(bb_plane const *plane, float const *labels, float con
     iota_kernel<<<blocks(n), 256, 0, b->stream>>>(b->rows, n);
     BB_LAUNCH("iota_kernel");
     BB_CHECK(cudaMemsetAsync(b->round, 0, 4, b->stream));
-    // a leafwise round reads every pop back to the host: it runs eagerly
+    // a leafwise round waits on the host for each tree: it runs eagerly
     b->use_graph       = cfg->use_graph != 0 && b->lanes[0].grower->fuses_next();
     b->record_leaf_ids = cfg->record_leaf_ids != 0;
     if (K == 1)

@@ -1031,10 +1031,6 @@ __device__ __forceinline__ void warp_best(double &gain, uint32_t &order)
     }
 }
 
-// grid (frontier, n_sel): one CTA of k_find_thr threads per (node,
-// feature), each thread a few candidates. The exact form's prefix is one
-// serial FP64 chain (the reference's summation order); the quantised form's
-// is an exact integer block scan.
 // Interaction constraints (allowed_features / propagate_interaction_state,
 // src/grower_impl.hpp:114-160). fgroups[f]: the groups containing feature f
 // as a bit mask (at most 64 groups). A node may split on f when its path is
@@ -1075,6 +1071,9 @@ __device__ __forceinline__ void interaction_children(Node const &par, uint64_t c
     R.ipath  = path;
 }
 
+// The exact form's find. grid (frontier, n_sel): one CTA of k_find_thr threads per
+// (node, feature), the prefix one serial FP64 chain (the reference's summation
+// order), then each thread a few candidates.
 __global__ void __launch_bounds__(k_find_thr)
     find_kernel(Ctl const *ctl, Node const *nodes, void const *hist_v,
                 uint32_t total_cells, uint32_t const *cell_off, uint32_t const *sel_nb,
@@ -6588,19 +6587,11 @@ void Grower::grow(float2 const *gh, uint32_t const *root_rows, uint32_t n_root,
     ++tree_no_;
 }
 
-namespace
-{
-
-// A leaf awaiting expansion (Candidate, src/step/primitives.hpp:440-450): its
-// node, its best split, its depth and the pool slot holding its histograms.
-
-} // namespace
-
-// LeafwiseGrower::grow with the host as the control plane: the same gain
-// heap (max gain, the lower node id on a tie), child ids allocated at the
-// pop, demotion when the partition empties a side (its two children stay as
-// zero leaf placeholders), no children's split at the depth cap, the leaf
-// budget; every pop's data plane on the device, one read-back per pop.
+// LeafwiseGrower::grow on the device: the same gain heap (max gain, the lower
+// node id on a tie), child ids allocated at the pop, demotion when the
+// partition empties a side (its two children stay as zero leaf placeholders),
+// no children's split at the depth cap, the leaf budget; the host launches the
+// loop once and reads its verdict after the tree.
 void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut const &t,
                            uint32_t *leaf_id, float *scores, float lr)
 {
@@ -6673,7 +6664,7 @@ void Grower::grow_leafwise(uint32_t const *root_rows, uint32_t n_root, TreeOut c
     launches += 4;
 
     // one pop as a fixed sequence of launches, repeated by the loop graph's
-    // WHILE node until leaf_commit_kernel says the heap is done; captured
+    // WHILE node until a turn (leaf_turn) finds nothing to pop; captured
     // once for these gradients and this table set (the loop's other buffers and
     // the tree's device record do not move)
     float2 const *const lgh  = quant_ ? nullptr : gh_cur_; // (the codes have one place)

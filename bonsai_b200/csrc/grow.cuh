@@ -473,7 +473,7 @@ class Grower
         prof_ = p;
     }
     // whether grow() can take a fused next round (and be graph-captured):
-    // not on the leafwise plane, whose host reads each pop back
+    // not on the leafwise plane, whose host waits for every tree's verdict
     bool fuses_next() const
     {
         return !cfg_.leaf;

@@ -23,8 +23,8 @@
 // Ensembles of depth at most 8 take another form of the sum, tree by tree (the
 // tree form, below). For the others, the ensemble's paths are packed once
 // (bb_shap_plan_create; the reference's cuda_shap_plan,
-// include/bonsai/cuda/shap.hpp:31-35) into fixed-stride records of K elements (K = 8, 16 or 32 by the longest path) and streamed
-// through shared memory in chunks. A CTA covers a tile of rows crossed with
+// include/bonsai/cuda/shap.hpp:31-35) into fixed-stride records of K elements
+// (K = 8, 16 or 32 by the longest path) and streamed through shared memory in chunks. A CTA covers a tile of rows crossed with
 // PL path lanes: thread (row, lane) takes every PL-th path of the chunk
 // against its row's codes (staged in shared memory) and accumulates into its
 // own FP64 slice; with PL = 1 every thread of a warp reads the same path

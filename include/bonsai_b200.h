@@ -194,7 +194,15 @@ typedef struct
  * (src/objective.cpp:76-83, :124-131, :293-308) is then used.
  * Replaces Booster<Obj, DepthwiseGrower<CudaHistogramEngine>, AllRows> with
  * the resident round armed (include/bonsai/booster.hpp:630-676) and the
- * engine's resident_begin (histogram_engine.hpp:251-253). */
+ * engine's resident_begin (histogram_engine.hpp:251-253).
+ *
+ * Device memory: a fit's arrays come from a pool per device that keeps up to
+ * 1 GiB mapped between fits, from a plane's first fit until the last fitted
+ * plane is destroyed (this process's other allocations take it back when they
+ * need it; other processes cannot have it). A softmax booster that is not
+ * leafwise grows its class trees side by side, each with a grower's arrays of
+ * its own, where the further ones fit a quarter of the free memory, and one
+ * after another otherwise. */
 int bb_booster_create(bb_plane const *plane, float const *labels,
                       float const *init_scores, bb_train_cfg const *cfg,
                       uint32_t max_trees, bb_booster **out);
@@ -445,10 +453,12 @@ int bb_predict_plan_run(bb_predict_plan *plan, bb_plane const *plane, uint32_t n
 
 /* bb_predict_plan_run enqueued on a caller's stream (a cudaStream_t; NULL is
  * the legacy default stream) into device out_device, without waiting.
- * *launches (if not NULL) receives the kernels enqueued. Small batches use a
- * workspace the plan owns: one launch per plan in flight at a time, and the
- * first launch of a new largest small batch allocates it (not inside a
- * stream capture). */
+ * *launches (if not NULL) receives the kernels enqueued. Some batches use a
+ * workspace the plan owns, so that one such launch per plan may be in flight at
+ * a time: of plans of depth 1 to 8, batches of up to 64 rows (the workspace is
+ * there from the plan's creation); of plans of depth 9 and 10, batches of under
+ * 256 rows per SM, the first launch of a new largest one allocating it (not
+ * inside a stream capture). Other launches use none and never allocate. */
 int bb_predict_plan_launch(bb_predict_plan *plan, bb_plane const *plane, uint32_t n_trees,
                            float *out_device, void *stream, uint32_t *launches);
 
