@@ -759,9 +759,11 @@ struct bb_predict_plan
     uint32_t    sms     = 1;
     uint32_t    lane_rows = 0; // a lane CTA's most rows
     uint64_t    heap_ctas = 0; // resident CTAs of the lane-per-row form; 0: not taken
-    bb::DeviceBuf heaps;
-    bb::DeviceBuf vals;       // a few rows' leaf values; a split batch's (depths 9, 10)
-    bb::DeviceBuf last_words; // per staged code word, its features' last bins
+    bb::DeviceBuf tables; // of the heap form, in one allocation:
+    uint32_t     *heaps      = nullptr;
+    uint32_t     *last_words = nullptr; // per staged code word, its features' last bins
+    float        *few_vals   = nullptr; // a few rows' leaf values (depths to 8)
+    bb::DeviceBuf vals;                 // a split batch's leaf values (depths 9, 10)
     bb::DeviceBuf last, roots, feature, split, left, right, dl, value;
     // the host runs' output, grown on demand; runs through one plan serialise
     std::mutex   mu;
@@ -1038,8 +1040,8 @@ uint32_t heap_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
     uint64_t const per = std::max<uint64_t>(
         32, ((((n + pl.heap_ctas - 1) / pl.heap_ctas) + 31) / 32) * 32);
     heap_fn(pl.u8, pl.depth, T)<<<ceil_div(n, per), T, heap_smem(pl.depth, pl.n_tiles, T), s>>>(
-        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words.as<uint32_t>(),
-        pl.heaps.as<uint32_t>(), n_trees, heap_chunk(pl.depth), static_cast<uint32_t>(per), pl.lr,
+        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words,
+        pl.heaps, n_trees, heap_chunk(pl.depth), static_cast<uint32_t>(per), pl.lr,
         pl.init, out, n_trees, nullptr);
     BB_LAUNCH("heap_predict_kernel");
     return 1;
@@ -1067,8 +1069,8 @@ uint32_t split_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, flo
     }
     heap_fn(pl.u8, pl.depth, 256)<<<dim3(row_blks, splits), 256,
                                     heap_smem(pl.depth, pl.n_tiles, 256), s>>>(
-        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words.as<uint32_t>(),
-        pl.heaps.as<uint32_t>(), n_trees, chunk, 256, pl.lr, pl.init, out, tps, vals);
+        static_cast<uint4 const *>(p.mirror), n, pl.n_tiles, pl.last_words,
+        pl.heaps, n_trees, chunk, 256, pl.lr, pl.init, out, tps, vals);
     BB_LAUNCH("heap_predict_kernel");
     if (splits == 1)
     {
@@ -1146,11 +1148,11 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
         {
             auto const fn = pl.u8 ? few_values_kernel<uint8_t> : few_values_kernel<uint16_t>;
             fn<<<dim3(static_cast<uint32_t>(n), ceil_div(n_trees, k_few_threads)), k_few_threads, 0,
-                 s>>>(mirror, n, pl.n_tiles, pl.last_words.as<uint32_t>(),
-                      pl.heaps.as<uint32_t>(), pl.depth, n_trees, pl.vals.as<float>());
+                 s>>>(mirror, n, pl.n_tiles, pl.last_words,
+                      pl.heaps, pl.depth, n_trees, pl.few_vals);
             BB_LAUNCH("few_values_kernel");
             launch_k(true, few_sum_kernel, static_cast<uint32_t>(n), k_few_threads, 0, s,
-                     pl.vals.as<float>(), n_trees, pl.lr, pl.init, out);
+                     pl.few_vals, n_trees, pl.lr, pl.init, out);
             BB_LAUNCH("few_sum_kernel");
             return 2;
         }
@@ -1159,8 +1161,8 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
             uint32_t const T = std::min(row_threads(n, pl.sms), ((n_trees + 31) / 32) * 32);
             auto const     fn = pl.u8 ? row_predict_kernel<uint8_t> : row_predict_kernel<uint16_t>;
             fn<<<static_cast<uint32_t>(n), T, 0, s>>>(mirror, n, pl.n_tiles,
-                                                      pl.last_words.as<uint32_t>(),
-                                                      pl.heaps.as<uint32_t>(), pl.depth, n_trees,
+                                                      pl.last_words,
+                                                      pl.heaps, pl.depth, n_trees,
                                                       pl.lr, pl.init, out);
             BB_LAUNCH("row_predict_kernel");
             return 1;
@@ -1175,7 +1177,7 @@ uint32_t plan_launch(bb_predict_plan &pl, Plane const &p, uint32_t n_trees, floa
         uint32_t const rows  = ceil_div(n, wave * waves);
         lane_fn(pl.u8, pl.depth)<<<ceil_div(n, rows), k_lane_threads,
                                    lane_smem(pl.depth, pl.n_tiles, rows), s>>>(
-            mirror, n, pl.n_tiles, pl.last_words.as<uint32_t>(), pl.heaps.as<uint32_t>(), n_trees,
+            mirror, n, pl.n_tiles, pl.last_words, pl.heaps, n_trees,
             rows, pl.lr, pl.init, out);
         BB_LAUNCH("lane_predict_kernel");
         return 1;
@@ -1224,30 +1226,22 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
         HeapPacker const pk{D,       p.u8,      words, by_tree, by_tree ? 32u : 1u, pl->cut_off.data(),
                             feature, split_bin, left,  right,   default_left,       value};
         pl->sms = sm_count();
+        // the heaps, then the last words
+        size_t const          n_heap = slots * (by_tree ? 32 * ((n_trees + 31) / 32) : n_trees);
+        std::vector<uint32_t> h(n_heap + words, by_tree ? pk.never() : 0u);
+        for (uint32_t t = 0; t < n_trees; ++t)
+        {
+            // 32 trees interleaved (the last group's missing ones, never added, route
+            // every row to their left spine), or one after another
+            size_t const at = by_tree ? ((t / 32) * slots * 32) + (t % 32) : t * slots;
+            pk.fill(h.data() + at, roots[t], roots[t], 1, 0);
+        }
         if (by_tree)
         {
-            // 32 trees interleaved; the last group's missing ones (never added)
-            // route every row to their left spine
-            std::vector<uint32_t> h(slots * 32 * ((n_trees + 31) / 32), pk.never());
-            for (uint32_t t = 0; t < n_trees; ++t)
-            {
-                pk.fill(h.data() + ((t / 32) * slots * 32) + (t % 32), roots[t], roots[t], 1, 0);
-            }
-            pl->heaps.upload(h.data(), h.size() * 4);
             size_t const per_row = lane_smem(D, n_tiles, 1) - lane_smem(D, n_tiles, 0);
             pl->lane_rows        = static_cast<uint32_t>(std::min<size_t>(
                 k_lane_threads, (k_lane_smem - lane_smem(D, n_tiles, 0)) / per_row));
             allow_smem(lane_fn(p.u8, D));
-            pl->vals.alloc(size_t{k_few_rows} * n_trees * sizeof(float));
-        }
-        else
-        {
-            std::vector<uint32_t> h(slots * n_trees, 0u);
-            for (uint32_t t = 0; t < n_trees; ++t)
-            {
-                pk.fill(h.data() + (t * slots), roots[t], roots[t], 1, 0);
-            }
-            pl->heaps.upload(h.data(), h.size() * 4);
         }
         if (D > k_lane_depth || n_tiles <= 2)
         {
@@ -1266,8 +1260,7 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
         }
         // the last bin of every code lane of every staged word (padding
         // lanes: a value no code has)
-        std::vector<uint32_t> lw(words, 0u);
-        uint32_t const        lanes = p.u8 ? 4u : 2u;
+        uint32_t const lanes = p.u8 ? 4u : 2u;
         for (uint32_t wd = 0; wd < words; ++wd)
         {
             uint32_t v = 0;
@@ -1278,9 +1271,14 @@ std::unique_ptr<bb_predict_plan> make_plan(Plane const &p, uint32_t n_trees,
                                                     : (p.u8 ? 0xFFu : 0xFFFFu);
                 v |= last << (k * (32u / lanes));
             }
-            lw[wd] = v;
+            h[n_heap + wd] = v;
         }
-        pl->last_words.upload(lw.data(), lw.size() * 4);
+        size_t const n_few = by_tree ? size_t{k_few_rows} * n_trees : 0;
+        pl->tables.alloc((h.size() + n_few) * 4);
+        pl->heaps      = pl->tables.as<uint32_t>();
+        pl->last_words = pl->heaps + n_heap;
+        pl->few_vals   = reinterpret_cast<float *>(pl->last_words + words);
+        check(cudaMemcpy(pl->heaps, h.data(), h.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy");
     }
     else
     {
