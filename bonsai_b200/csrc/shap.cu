@@ -1019,6 +1019,7 @@ struct TreeBlob
     // the units at level J (0: none): a path's records so far, and theirs
     uint32_t              J         = 0;
     uint32_t              unit_room = 0;
+    uint64_t              nodes     = 0;
     uint32_t              rec[k_unit_levels] = {};
     std::vector<TreeUnit> units;
 };
@@ -1070,6 +1071,7 @@ void pack_node(TreeView const &t, uint32_t const *last, uint32_t id, std::vector
         tb.units.push_back({{tb.rec[0], tb.rec[1], tb.rec[2]}, b, e, leaf, len, d});
         tb.unit_room = std::max(tb.unit_room, k_unit_path + (e - b));
     };
+    ++tb.nodes;
     if (level < tb.J)
     {
         tb.rec[level] = begin;
@@ -1204,6 +1206,8 @@ struct bb_shap_plan
     uint32_t              n_units    = 0;
     uint32_t              unit_room  = 0;
     uint32_t              unit_warps = 0;
+    double                tree_cost = 0.0; // nodes of a tree, and of a unit with its path
+    double                unit_cost = 0.0;
     bb::ShapBuf           tables; // of the tree form: the three below
     uint32_t             *blob_off = nullptr;
     bb::TreeUnit         *units    = nullptr;
@@ -1334,11 +1338,14 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
         pl->n_units    = static_cast<uint32_t>(tb.units.size());
         pl->unit_room  = tb.unit_room;
         pl->unit_warps = std::max(1u, warps(pl->unit_room));
+        pl->tree_cost  = static_cast<double>(tb.nodes) / static_cast<double>(views.size());
+        pl->unit_cost  = (static_cast<double>(tb.nodes) / pl->n_units) + 8.0;
     }
     // the offsets, the units and the blob, in one allocation (a unit's path reads whole
     // records: some bytes past the blob, whatever they hold)
-    size_t const n_off = ((tb.off.size() * 4) + 15) & ~size_t{15};
-    size_t const n_un  = tb.units.size() * sizeof(TreeUnit);
+    auto const   lines = [](size_t n) { return (n + 127) & ~size_t{127}; };
+    size_t const n_off = lines(tb.off.size() * 4);
+    size_t const n_un  = lines(tb.units.size() * sizeof(TreeUnit));
     pl->tables.alloc(n_off + n_un + tb.bytes.size() + k_unit_rec);
     auto *const at = pl->tables.as<unsigned char>();
     pl->blob_off   = reinterpret_cast<uint32_t *>(at);
@@ -1347,7 +1354,7 @@ std::unique_ptr<bb_shap_plan> make_tree_plan(std::vector<TreeView> const &views,
     auto const up  = [](void *to, void const *from, size_t n)
     { check(cudaMemcpy(to, from, n, cudaMemcpyHostToDevice), "cudaMemcpy"); };
     up(pl->blob_off, tb.off.data(), tb.off.size() * 4);
-    up(pl->units, tb.units.data(), n_un);
+    up(pl->units, tb.units.data(), tb.units.size() * sizeof(TreeUnit));
     up(pl->blob, tb.bytes.data(), tb.bytes.size());
     return pl;
 }
@@ -1511,12 +1518,12 @@ uint32_t tree_launch(bb_shap_plan &pl, Plane const &p, double *out, cudaStream_t
     if (n < k_tree_split)
     {
         // about one CTA per SM, a tree (a unit) at a time in each of its warps: the
-        // form whose rounds over them take less, a unit 1 / 40 of a tree beside its
-        // share of it
+        // form whose rounds over them visit fewer nodes one after another (a unit's
+        // path and its start are worth about eight)
         uint32_t const ctas  = std::max(1u, k_sms / tiles);
-        uint32_t const trees = ceil_div(count, ctas * most) * 40;
-        uint32_t const share = (40 >> pl.unit_level) + 1;
-        if (pl.unit_level > 0 && ceil_div(pl.n_units, ctas * pl.unit_warps) * share < trees)
+        double const   trees = pl.tree_cost * ceil_div(count, ctas * most);
+        if (pl.unit_level > 0 &&
+            pl.unit_cost * ceil_div(pl.n_units, ctas * pl.unit_warps) < trees)
         {
             J     = pl.unit_level;
             count = pl.n_units;
