@@ -1648,6 +1648,10 @@ __device__ __forceinline__ void plan_level(Ctl *ctl, Node *nodes, Best const *be
             t.gain[right]  = 0.0F;
             t.cover[left]  = 0.0F;
             t.cover[right] = 0.0F;
+            // a demoted split's children keep these: nothing comes after to
+            // write their bounds, and leaf_fix reads every leaf's
+            A.nbound[left]  = make_double2(-INFINITY, INFINITY);
+            A.nbound[right] = make_double2(-INFINITY, INFINITY);
             nd.flags            = 1;
             uint32_t const last = cut_off[f + 1] - cut_off[f] - 1;
             A.route[i]          = make_uint4(f, last, bs.bin, bs.dl);
