@@ -4941,8 +4941,9 @@ struct LeafTurn
 // commit_split_node (src/grower_impl.hpp:189-206) into the node table, a pool
 // slot for the smaller child, and the popped node's partition chunks (the
 // setup of one pop). With nothing to pop it sets the no-op flag and leaves no
-// chunks, so that an iteration after it does nothing. Returns whether it
-// popped.
+// chunks and no split, so that an iteration after it does nothing (a tree that
+// is its root alone still runs the loop's body once, and without chunks no
+// CTA of it plans children). Returns whether it popped.
 constexpr uint32_t k_pop_thr = 256;
 
 __device__ __forceinline__ bool leaf_pop(LeafTurn const &T)
@@ -4966,6 +4967,7 @@ __device__ __forceinline__ bool leaf_pop(LeafTurn const &T)
             T.ctl->n_bchunks = 0;
             T.pcr[0]         = 0;
             T.pcr[1]         = 0;
+            T.out->split     = 0;
             T.st->pop.node.count = 0;
         }
     }
@@ -5035,6 +5037,7 @@ __device__ __forceinline__ bool leaf_pop(LeafTurn const &T)
             T.ctl->n_bchunks     = 0;
             T.pcr[0]             = 0;
             T.pcr[1]             = 0;
+            T.out->split         = 0;
             T.st->pop.node.count = 0;
             go_s               = 0;
         }
